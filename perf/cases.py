@@ -20,6 +20,7 @@ import torch
 import torch.distributed as dist
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.utils.checkpoint import checkpoint
 
 from yafsdp_b200 import MixedPrecisionPolicy, fully_shard
 from yafsdp_b200.models.llama import CONFIGS, LlamaConfig, LlamaDecoderLayer, LlamaForCausalLM
@@ -281,3 +282,124 @@ def tolerance(case: dict[str, Any]) -> dict[str, float]:
     operations is 4-7 % further off.  Two correct implementations are up to 1.4 times these figures apart.  ``modules``: library kernels
     throughout, one bf16 rounding of the gradients on the way."""
     return {"rel": {"train": 0.03, "layer": 0.025, "eval": 0.02, "modules": 0.01}[case["kind"]]}
+
+
+# ----------------------------------------------------------------------------------------- the same in 64 bits
+def exact(case: dict[str, Any], seed: int) -> dict[str, Any]:
+    """What the first ``run`` after ``prepare(case, seed)`` returns, in plain torch operations in 64 bits: the weights as the
+    compute type holds them, nothing rounded on the way."""
+    return _EXACT[case["kind"]](case, prepare(case, seed))
+
+
+def _exact_norm(x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
+    return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps) * w
+
+
+def _exact_head(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
+    """Causal attention of one sequence and head."""
+    hidden = torch.ones(q.shape[0], q.shape[0], dtype=torch.bool, device=q.device).triu_(1)
+    return (q @ k.T / math.sqrt(q.shape[1])).masked_fill_(hidden, -math.inf).softmax(-1) @ v
+
+
+def _exact_layer(x: torch.Tensor, w: dict[str, torch.Tensor], cfg: LlamaConfig, batch: int, seq: int) -> torch.Tensor:
+    hq, hkv, hd, half = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim, cfg.head_dim // 2
+    pos = torch.arange(seq, dtype=torch.float64, device=x.device)
+    ang = pos[:, None] * cfg.rope_theta ** (torch.arange(half, dtype=torch.float64, device=x.device) * (-2.0 / hd))
+    cos, sin = ang.cos()[None, :, None, :], ang.sin()[None, :, None, :]
+
+    def heads(name: str, n: int, rotate: bool) -> torch.Tensor:
+        t = (n1 @ w[f"self_attn.{name}_proj.weight"].T).view(batch, seq, n, hd)
+        if rotate:
+            a, b = t[..., :half], t[..., half:]
+            t = torch.cat([a * cos - b * sin, b * cos + a * sin], dim=-1)
+        return t.transpose(1, 2)
+
+    n1 = _exact_norm(x, w["input_layernorm.weight"], cfg.rms_norm_eps)
+    q, k, v = heads("q", hq, True), heads("k", hkv, True), heads("v", hkv, False)
+    att = torch.stack([checkpoint(_exact_head, q[b, h], k[b, h * hkv // hq], v[b, h * hkv // hq], use_reentrant=False)
+                       for b in range(batch) for h in range(hq)])
+    att = att.view(batch, hq, seq, hd).transpose(1, 2).reshape(batch * seq, hq * hd)
+    x = x + att @ w["self_attn.o_proj.weight"].T
+    n2 = _exact_norm(x, w["post_attention_layernorm.weight"], cfg.rms_norm_eps)
+    return x + (F.silu(n2 @ w["mlp.gate_proj.weight"].T) * (n2 @ w["mlp.up_proj.weight"].T)) @ w["mlp.down_proj.weight"].T
+
+
+def _exact_logits(ids: torch.Tensor, w: dict[str, torch.Tensor], cfg: LlamaConfig) -> torch.Tensor:
+    x = w["model.embed_tokens.weight"][ids.reshape(-1)]
+    for i in range(cfg.num_hidden_layers):
+        pre = f"model.layers.{i}."
+        x = _exact_layer(x, {n[len(pre) :]: t for n, t in w.items() if n.startswith(pre)}, cfg, *ids.shape)
+    return _exact_norm(x, w["model.norm.weight"], cfg.rms_norm_eps) @ w["lm_head.weight"].T
+
+
+def _exact_weights(model: nn.Module, groups: list[Any]) -> tuple[dict[str, torch.Tensor], list[list[str]]]:
+    """The parameters of a sharded model (one rank) as its compute type holds them, and their names by group in flat order."""
+    names = {p: n for n, p in model.named_parameters()}
+    order = [[names[sp.sharded_param] for sp in g.params] for g in groups]
+    w = {}
+    for g, members in zip(groups, order):
+        for name, sp in zip(members, g.params):
+            at = sp.placement.shard_offset
+            w[name] = g.master_flat[at : at + sp.numel].view(sp.orig_shape).bfloat16().double().requires_grad_(True)
+    return w, order
+
+
+def _exact_step(w: dict[str, torch.Tensor], order: list[list[str]], groups: list[Any], clip: float, clipped_grads: bool) -> dict[str, Any]:
+    """The first AdamW step from the masters of ``groups`` with the gradients in ``w``."""
+    norm = torch.stack([t.grad.norm() for t in w.values()]).norm()
+    coef = float(torch.clamp(clip / (norm + 1e-6), max=1.0)) if clip else 1.0
+    out: dict[str, Any] = {"weights": [], "grads": [], "exp_avg": [], "exp_avg_sq": []}
+    for g, members in zip(groups, order):
+        grad = torch.zeros(g.master_flat.numel(), dtype=torch.float64, device=g.master_flat.device)
+        for name, sp in zip(members, g.params):
+            at = sp.placement.shard_offset
+            grad[at : at + sp.numel] = w[name].grad.reshape(-1)
+            w[name].grad = None
+        m, v = grad * (0.1 * coef), grad.pow(2).mul_(0.05 * coef * coef)
+        p = g.master_flat.double().mul_(1 - 1e-5 * 0.1).addcdiv_(m, (v / 0.05).sqrt_().add_(1e-8), value=-1e-5 / 0.1)
+        for key, value in (("weights", p), ("grads", grad.mul_(coef) if clipped_grads else grad), ("exp_avg", m), ("exp_avg_sq", v)):
+            out[key].append(value)
+    return out
+
+
+def _exact_train(case: dict[str, Any], s: dict[str, Any]) -> dict[str, Any]:
+    w, order = _exact_weights(s["model"], s["groups"])
+    total = torch.zeros((), dtype=torch.float64, device=s["device"])
+    for ids, labels in s["batches"][: case["micro"]]:
+        target = torch.cat([labels[:, 1:], torch.full_like(labels[:, :1], -100)], dim=1).to(s["device"]).reshape(-1)
+        loss = F.cross_entropy(_exact_logits(ids.to(s["device"]), w, _config(case)), target, ignore_index=-100, reduction="sum")
+        loss = loss / (target >= 0).sum().clamp(min=1) / case["micro"]
+        loss.backward()
+        total += loss.detach()
+    return {"loss": total, **_exact_step(w, order, s["groups"], case["clip"], clipped_grads=False)}
+
+
+def _exact_eval(case: dict[str, Any], s: dict[str, Any]) -> dict[str, Any]:
+    with torch.no_grad():
+        w = {n: p.double() for n, p in s["model"].named_parameters()}
+        return {"logits": _exact_logits(s["ids"], w, _config(case)).view(case["batch"], case["seq"], -1)}
+
+
+def _exact_layer_pass(case: dict[str, Any], s: dict[str, Any]) -> dict[str, Any]:
+    w = {n: p.detach().double().requires_grad_(True) for n, p in s["params"].items()}
+    x = s["x"].detach().double().requires_grad_(True)
+    out = _exact_layer(x, w, _config(case), case["batch"], case["seq"])
+    out.backward(s["dout"].double())
+    return {"out": out.detach(), "dx": x.grad, "grads": {n: t.grad for n, t in w.items()}}
+
+
+def _exact_modules(case: dict[str, Any], s: dict[str, Any]) -> dict[str, Any]:
+    w, order = _exact_weights(s["model"], s["groups"])
+    x0 = s["x"].detach().double().requires_grad_(True)
+    x = x0
+    for i in range(case["layers"]):
+        n = F.layer_norm(x, x.shape[-1:], w[f"{i}.norm.weight"], w[f"{i}.norm.bias"])
+        h = F.gelu(F.linear(n, w[f"{i}.up.weight"], w[f"{i}.up.bias"]))
+        x = x + F.linear(h, w[f"{i}.down.weight"], w[f"{i}.down.bias"])
+    loss = F.mse_loss(x, s["y"].double())
+    loss.backward()
+    step = _exact_step(w, order, s["groups"], case["clip"], clipped_grads=True)
+    return {"loss": loss.detach(), "dx": x0.grad, "weights": step["weights"], "grads": step["grads"]}
+
+
+_EXACT = {"train": _exact_train, "eval": _exact_eval, "layer": _exact_layer_pass, "modules": _exact_modules}
