@@ -1,7 +1,7 @@
 // bf16 GEMM family for sm_100a: C[M,N] = alpha * A[M,K] * B[N,K]^T (+ C), fp32 accumulation in TMEM.
 //
 // Persistent, warp-specialised kernel, one CTA per SM:
-//   warp 0     TMA producer  (cp.async.bulk.tensor, 128-byte swizzle, no multicast)
+//   warp 0     TMA producer  (cp.async.bulk.tensor, 128-byte swizzle, no multicast); plain mode: warps 0 and 6 in turn
 //   warp 1     MMA issuer    (tcgen05.mma cta_group::1, M=128, N=BLOCK_N, K=16 per instruction)
 //   warps 2-5  epilogue      (tcgen05.ld 32x32b, convert, store; overlaps the next tile's main loop
 //                             through two TMEM accumulators)
@@ -11,6 +11,8 @@
 // buffer (the cast and the micro-batch accumulation of a sharded-data-parallel step).
 #include <stdlib.h>
 #include <string.h>
+
+#include <atomic>
 
 #include "common.cuh"
 #include "yafsdp_b200.h"
@@ -23,11 +25,13 @@ constexpr int BLOCK_M = 128;
 constexpr int BLOCK_K = 64;   // 64 bf16 = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
 constexpr int GEMM_THREADS = 192;
-constexpr int GATHER_THREADS = 224;  // gather mode: one more warp, for the communication role
+constexpr int WIDE_THREADS = 224;  // one more warp: plain mode's second TMA producer, gather mode's communication role
 
-// MODE_PLAIN: C is stored locally through TMA.  MODE_SCATTER: GEMM -> reduce-scatter, the fp32 rows of C are pushed to the
+// MODE_PLAIN: C is stored locally through TMA; MODE_SPLIT: so too, and the last wave's tiles are split along K (an
+// instantiation of its own: the exchange's code alone costs the plain kernel 0.3 us per tile).  MODE_SCATTER: GEMM -> reduce-scatter, the fp32 rows of C are pushed to the
 // ranks that own them.  MODE_GATHER: all-gather -> GEMM, the kernel also gathers the layer that B is part of (see FusedArgs).
-constexpr int MODE_PLAIN = 0, MODE_SCATTER = 1, MODE_GATHER = 2;
+constexpr int MODE_PLAIN = 0, MODE_SCATTER = 1, MODE_GATHER = 2, MODE_SPLIT = 3;
+__host__ __device__ constexpr bool is_plain(int mode) { return mode == MODE_PLAIN || mode == MODE_SPLIT; }
 constexpr int SCATTER_COLS = 64;                         // columns per pushed row piece: 256 bytes of fp32
 constexpr int SCATTER_PITCH = SCATTER_COLS * 4 + 16;     // row pitch of the staging block (16 B of padding: no bank conflicts)
 
@@ -40,12 +44,14 @@ struct GemmCfg {
   static constexpr int RING_BYTES = (MODE == MODE_GATHER) ? 6 * 16384 : 0;  // the communication role's ring (COMM_SLOTS pieces)
   static constexpr int STAGES = (MODE == MODE_SCATTER) ? (STAGE_BYTES == 49152 ? 3 : 4)
                                 : (MODE == MODE_GATHER) ? (STAGE_BYTES == 49152 ? 2 : 3)
-                                                        : ((STAGE_BYTES == 49152) ? 4 : 6);
-  static constexpr int TMEM_COLS = 2 * BLOCK_N;  // two accumulators (power of two: 256 or 512)
-  // plain: two [128 rows x 128 B] swizzled blocks for TMA stores; scatter: two [128 rows x 256 B (+ padding)] linear blocks
+                                                        : 196608 / STAGE_BYTES;  // 192 KB of operands in flight
+  static constexpr int TMEM_COLS = 2 * BLOCK_N;  // two accumulators (a power of two)
+  // plain: two [32 rows x 128 B] swizzled blocks per warp for TMA stores; scatter: two [128 rows x 256 B (+ padding)] linear blocks
   static constexpr int STAGING_BYTES = (MODE == MODE_SCATTER) ? 2 * BLOCK_M * SCATTER_PITCH : 2 * 16384 + RING_BYTES;
   static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + STAGING_BYTES + 256;
 };
+
+constexpr int MAX_SPLITS = 4;  // K ranges of one tile (split mode)
 
 constexpr int MAX_RANKS = 16;
 constexpr int MAX_GROUP = 4;  // problems of one grouped launch (the weight-gradient GEMMs of a decoder layer)
@@ -60,6 +66,18 @@ struct GemmArgs {
   // mode): a block's "x + proj(...)" costs no pass of its own over the activations
   const void* R;
   long long ldr;
+  // Split tiles (split mode).  The number of tiles modulo the number of units is what a last wave would leave most units
+  // idle for: so many tiles, [0, split_tiles), are computed in `splits` K ranges each, the others whole.  Work items are
+  // dealt round-robin: range 0 of every split tile, range 1 of every split tile, and so on - the units that run at the same
+  // time read the same part of K (L2) - and then the whole tiles, whose main loops hide the exchange of the sums.  A
+  // range's fp32 sums go to its slot of `slots` ([128 rows x BLOCK_N] per CTA); the CTA that arrives last at the tile's
+  // counter adds the ranges in their order (the result does not depend on which one that is) and writes the output.
+  // Nobody waits.  A counter is (nonce << 8 | arrivals): the nonce is new in every launch, so what the workspace held
+  // before does not matter and nothing has to be cleared; the last one leaves a zero (replays of a captured launch).
+  int split_tiles, splits;
+  unsigned long long nonce;
+  unsigned long long* counters;
+  float* slots;
   // Grouped launch (scatter mode): n_prob problems that share K and the operand majors, in the order of their positions in
   // the flat layer gradient.  Tiles are numbered problem by problem, rows first (= in flat order); tile_prefix[p] = number
   // of tiles in front of problem p; own_start[o] = first tile whose rows begin in the shard of rank o.  The launch deals the
@@ -73,6 +91,26 @@ struct GemmArgs {
   int own_start[MAX_RANKS + 1];
   int steps;   // world * (largest number of tiles of one owner)
 };
+
+// one piece of work of a unit: K blocks [kb0, kb1) of a tile; part < 0: all of them
+struct WorkItem {
+  int tile, kb0, kb1, part;
+};
+template <int MODE>
+YF_DEVINL WorkItem work_item(const GemmArgs& args, int i, int num_k) {
+  WorkItem w = {i, 0, num_k, -1};
+  if constexpr (MODE == MODE_SPLIT) {
+    if (i < args.split_tiles * args.splits) {
+      w.part = i / args.split_tiles;
+      w.tile = i - w.part * args.split_tiles;
+      w.kb0 = (int)((long long)num_k * w.part / args.splits);
+      w.kb1 = (int)((long long)num_k * (w.part + 1) / args.splits);
+    } else {
+      w.tile = i - args.split_tiles * (args.splits - 1);
+    }
+  }
+  return w;
+}
 
 // operand tensor maps of up to MAX_GROUP problems (entry 0 alone for an ordinary launch)
 struct GroupMaps {
@@ -118,6 +156,21 @@ YF_DEVINL unsigned long long ld_relaxed_gpu_u64(const unsigned long long* p) {
 }
 YF_DEVINL void red_add_relaxed_gpu_u64(unsigned long long* p, unsigned long long v) {
   asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+// counters of split tiles: has every other range arrived / arrive (true: as the last one)
+YF_DEVINL bool split_others_arrived(unsigned long long* ctr, unsigned long long nonce, int splits) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(ctr) : "memory");
+  return v == ((nonce << 8) | (unsigned long long)(splits - 1));
+}
+YF_DEVINL bool split_arrive(unsigned long long* ctr, unsigned long long nonce, int splits) {
+  unsigned long long old = ld_relaxed_gpu_u64(ctr);
+  for (;;) {  // ends: a failed exchange means that another range of the tile has arrived
+    const unsigned long long n = ((old >> 8) == nonce ? (old & 255ull) : 0ull) + 1ull;
+    const unsigned long long seen = atomicCAS(ctr, old, (nonce << 8) | n);
+    if (seen == old) return n == (unsigned long long)splits;
+    old = seen;
+  }
 }
 YF_DEVINL void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
@@ -213,7 +266,7 @@ __device__ void gather_comm_role(const FusedArgs& fa, long long b_bytes, long lo
 }
 
 template <int BLOCK_N, int CG, int MODE>
-__global__ void __launch_bounds__(MODE == MODE_GATHER ? GATHER_THREADS : GEMM_THREADS, 1)
+__global__ void __maxnreg__(128)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ CUtensorMap tma_c, GemmArgs args, FusedArgs fa) {
   using Cfg = GemmCfg<BLOCK_N, CG, MODE>;
   // CG == 2: the grid is a sequence of CTA pairs (clusters of two); a pair works on one 256 x BLOCK_N tile, CTA `crank` of
@@ -245,6 +298,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
   const int num_k = (K + BLOCK_K - 1) / BLOCK_K;
   const bool grouped = (MODE == MODE_SCATTER) && args.n_prob > 0;
   const int num_tiles = grouped ? args.steps : num_m * num_n;  // steps of the tile loop (a grouped step may be empty)
+  const int num_items = num_tiles + (MODE == MODE_SPLIT ? args.split_tiles * (args.splits - 1) : 0);
   constexpr int GROUP_M = 16 / CG;  // 2048 rows of A share a column block of B through L2
 
   if (threadIdx.x == 0) {
@@ -303,14 +357,23 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
     return true;
   };
 
-  if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer (one per CTA)
-    if (lane == 0) {
-      uint32_t it = 0;
+  if (warp == 0 || (is_plain(MODE) && warp == 6)) {
+    // ------------------------------------------------------------ TMA producers
+    // Plain mode has two producers that take turns: waiting, announcing the bytes and issuing the copies of a K block cost
+    // one thread about 190 ns, which is more than the MMAs of a narrow tile take.  The number of stages is even, so
+    // producer j fills the stages of its parity.
+    constexpr int PRODUCERS = is_plain(MODE) ? 2 : 1;
+    static_assert(STAGES % PRODUCERS == 0 || PRODUCERS == 1, "every producer has its own stages");
+    const int producer = warp == 0 ? 0 : 1;
+    if (elect_one()) {
+      uint32_t s = producer, ph = 0;  // ring position: stage and how often (mod 2) the ring has gone round
+      int skip = producer;            // K blocks in front of this producer's next one
+      const uint32_t full_leader = CG == 2 ? mapa_shared(smem_u32(full), 0) : 0u;
       bool alive = true;
-      for (int t = unit; t < num_tiles && alive; t += nunits) {
+      for (int t = unit; t < num_items && alive; t += nunits) {
+        const WorkItem w = work_item<MODE>(args, t, num_k);
         int p, m0, n0;
-        if (!tile_coords(t, p, m0, n0)) continue;
+        if (!tile_coords(w.tile, p, m0, n0)) continue;
         const CUtensorMap* tma_a = &maps.a[p];
         const CUtensorMap* tma_b = &maps.b[p];
         const int N = grouped ? args.Np[p] : args.N;
@@ -336,9 +399,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
           if (!alive) break;
         }
         const int nb = n0 + (int)crank * B_ROWS;  // first B row this CTA holds
-        for (int kb = 0; kb < num_k; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
+        int kb = w.kb0 + skip;
+        for (; kb < w.kb1; kb += PRODUCERS) {
           if (!mbar_wait(&empty[s], ph ^ 1, 10)) { alive = false; break; }
           uint8_t* sa = smem + s * Cfg::STAGE_BYTES;
           uint8_t* sb = sa + Cfg::A_BYTES;
@@ -346,7 +408,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
           if (CG == 2) {
             // both CTAs' bytes are counted on the leader's barrier (the thread that issues the MMAs waits there)
             if (leader) mbar_expect_tx(&full[s], 2 * Cfg::STAGE_BYTES);
-            const uint32_t fb = mapa_shared(smem_u32(&full[s]), 0);
+            const uint32_t fb = full_leader + s * 8;
             if (!args.a_mn) {
               tma_load_2d_pair(sa, tma_a, fb, k0, m0);
             } else {
@@ -374,7 +436,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
               for (int j = 0; j < B_ROWS / 64; ++j) tma_load_2d(sb + j * (BLOCK_K * 128), tma_b, &full[s], nb + j * 64, k0);
             }
           }
+          s += PRODUCERS;
+          if (s >= STAGES) { s -= STAGES; ph ^= 1; }
         }
+        skip = kb - w.kb1;
       }
       if (!alive) {
         // give copies already in flight a bounded time to land before the CTA may exit
@@ -384,17 +449,23 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (pairs: the leader CTA issues for both)
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       const uint32_t idesc = umma_idesc_bf16(TILE_M, BLOCK_N, args.a_mn, args.b_mn);
-      const uint32_t a_lbo = args.a_mn ? BLOCK_K * 128 : 0, b_lbo = args.b_mn ? BLOCK_K * 128 : 0;
-      const uint32_t a_kstep = args.a_mn ? UMMA_K * 128 : UMMA_K * 2, b_kstep = args.b_mn ? UMMA_K * 128 : UMMA_K * 2;
-      uint32_t it = 0;
+      // Shared-memory descriptors: the upper words are constants, the lower ones advance by the stage and the K step (in
+      // units of 16 bytes; the whole of shared memory fits the address field).  One thread issues everything: what it
+      // computes per K block has to stay below the 256 to 512 cycles that the block's MMAs take.
+      const uint64_t a0 = umma_smem_desc_sw128(smem_u32(smem), args.a_mn ? BLOCK_K * 128 : 0, 1024);
+      const uint64_t b0 = umma_smem_desc_sw128(smem_u32(smem) + Cfg::A_BYTES, args.b_mn ? BLOCK_K * 128 : 0, 1024);
+      const uint32_t a_kstep = (args.a_mn ? UMMA_K * 128 : UMMA_K * 2) >> 4, b_kstep = (args.b_mn ? UMMA_K * 128 : UMMA_K * 2) >> 4;
+      const uint32_t empty_0 = CG == 2 ? mapa_shared(smem_u32(empty), 0) : 0u, empty_1 = CG == 2 ? mapa_shared(smem_u32(empty), 1) : 0u;
+      uint32_t s = 0, ph = 0;
       bool alive = true;
       int lt = 0;
-      for (int t = unit; t < num_tiles && alive; t += nunits) {
+      for (int t = unit; t < num_items && alive; t += nunits) {
+        const WorkItem w = work_item<MODE>(args, t, num_k);
         {
           int p, m0, n0;
-          if (!tile_coords(t, p, m0, n0)) continue;
+          if (!tile_coords(w.tile, p, m0, n0)) continue;
         }
         const int acc = lt & 1;
         const uint32_t acc_ph = (lt >> 1) & 1;
@@ -402,28 +473,25 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
         if (!mbar_wait(&tempty[acc], acc_ph ^ 1, 20)) { alive = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BLOCK_N;
-        for (int kb = 0; kb < num_k; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
+        uint32_t add = 0;  // the first MMA of an item overwrites the accumulator
+        for (int kb = w.kb0; kb < w.kb1; ++kb) {
           if (!mbar_wait(&full[s], ph, 21)) { alive = false; break; }
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + s * Cfg::STAGE_BYTES);
-          const uint32_t sb = sa + Cfg::A_BYTES;
+          const uint64_t a_desc = a0 + s * (Cfg::STAGE_BYTES >> 4), b_desc = b0 + s * (Cfg::STAGE_BYTES >> 4);
 #pragma unroll
           for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-            const uint64_t adesc = umma_smem_desc_sw128(sa + k * a_kstep, a_lbo, 1024);
-            const uint64_t bdesc = umma_smem_desc_sw128(sb + k * b_kstep, b_lbo, 1024);
-            if (CG == 2) tc_mma_bf16_pair(d_tmem, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
-            else tc_mma_bf16(d_tmem, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
+            if (CG == 2) tc_mma_bf16_pair(d_tmem, a_desc + k * a_kstep, b_desc + k * b_kstep, idesc, add);
+            else tc_mma_bf16(d_tmem, a_desc + k * a_kstep, b_desc + k * b_kstep, idesc, add);
+            add = 1;
           }
           // frees the stage (in both CTAs of a pair) once these MMAs have read it
           if (CG == 2) {
-            const uint32_t eb = smem_u32(&empty[s]);
-            tc_commit_pair(mapa_shared(eb, 0));
-            tc_commit_pair(mapa_shared(eb, 1));
+            tc_commit_pair(empty_0 + s * 8);
+            tc_commit_pair(empty_1 + s * 8);
           } else {
             tc_commit(&empty[s]);
           }
+          if (++s == STAGES) { s = 0; ph ^= 1; }
         }
         if (alive) {
           if (CG == 2) {
@@ -443,6 +511,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
     // ------------------------------------------------------------ epilogue (4 warps = 128 TMEM lanes)
     // TMEM -> registers -> 128-byte-swizzled staging block in shared memory -> TMA store (or TMA
     // reduce-add when accumulating): full 128-byte lines leave the SM, edges are clipped by the TMA unit.
+    // Every warp stages and stores its own 32 rows (two blocks of [32 rows x 128 bytes]), so the four warps run without
+    // barriers between them and hide each other's latencies.
     const int q = warp & 3;  // a warp may only touch TMEM lanes [32*(warp%4), +32)
     const int r_in_tile = q * 32 + lane;
     const bool store_thread = (threadIdx.x == 64);
@@ -452,9 +522,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
     int lt = 0;
     uint32_t chunk_ctr = 0;
     float ss = 0.f;  // sum of squares of this thread's outputs (rows / columns past the edges are exact zeros)
-    for (int t = unit; t < num_tiles && alive; t += nunits) {
+    for (int t = unit; t < num_items && alive; t += nunits) {
+      const WorkItem w = work_item<MODE>(args, t, num_k);
       int p, m0, n0;
-      if (!tile_coords(t, p, m0, n0)) continue;
+      if (!tile_coords(w.tile, p, m0, n0)) continue;
       const int M = grouped ? args.Mp[p] : args.M, N = grouped ? args.Np[p] : args.N;
       const long long c_flat_off = grouped ? args.flat_off[p] : fa.c_flat_off;
       const int acc = lt & 1;
@@ -553,12 +624,95 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
           tma_store_commit();
         }
       } else {
+      auto free_accumulator = [&]() {  // fully read: hand it back to the MMA warp (of the leader CTA)
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (CG == 2) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty[acc]), 0));
+          else mbar_arrive(&tempty[acc]);
+        }
+      };
+      // One range of a split tile: its sums go to its slot unless all other ranges are there already.  A slot holds float4
+      // column groups of 128 rows (512 contiguous bytes per warp and access).  The last range adds the others to its
+      // accumulator, in the order of the ranges, and carries on with the output as for a whole tile.
+      if (MODE == MODE_SPLIT && w.part >= 0) {
+        const bool rows_here = m0 + q * 32 < M;  // this warp's rows
+        const int cta_tile = w.tile * CG + (int)crank;
+        unsigned long long* ctr = args.counters + cta_tile;
+        float4* slot0 = reinterpret_cast<float4*>(args.slots) + (long long)cta_tile * args.splits * (BLOCK_M * BLOCK_N / 4) + r_in_tile;
+        bool last = named_bar_or(1, 128, store_thread && split_others_arrived(ctr, args.nonce, args.splits));
+        if (!last) {
+          float4* mine = slot0 + w.part * (BLOCK_M * BLOCK_N / 4);
+#pragma unroll 1
+          for (int c = 0; c < BLOCK_N / 32; ++c) {
+            uint32_t r[32];
+            tmem_ld32(taddr + c * 32, r);
+            tmem_ld_wait();
+            if (rows_here) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                __stcg(mine + (c * 8 + j) * BLOCK_M, make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                                                 __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3])));
+            }
+          }
+          named_bar_sync(1, 128);  // all 128 threads' sums are written before one of them publishes
+          if (store_thread) {
+            __threadfence();
+            last = split_arrive(ctr, args.nonce, args.splits);
+            __threadfence();
+          }
+          last = named_bar_or(1, 128, store_thread && last);
+        }
+        if (!last) {
+          free_accumulator();
+          continue;
+        }
+        if (store_thread) *ctr = 0ull;
+        // three 32-column pieces of other ranges in flight: of one block of columns, or with one other range of three blocks
+        const int others = args.splits - 1;
+        const int step = others == 1 ? 3 : 1;
+#pragma unroll 1
+        for (int c = 0; c < BLOCK_N / 32; c += step) {
+          float4 x[3][8];
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            const int range = others == 1 ? 1 - w.part : i + (i >= w.part ? 1 : 0), block = others == 1 ? c + i : c;
+            const bool there = rows_here && (others == 1 ? block < BLOCK_N / 32 : i < others);
+            const float4* src = slot0 + range * (BLOCK_M * BLOCK_N / 4) + block * 8 * BLOCK_M;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[i][j] = there ? __ldcg(src + j * BLOCK_M) : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+#pragma unroll
+          for (int b = 0; b < 3; ++b) {
+            if (b >= step || c + b >= BLOCK_N / 32) break;
+            uint32_t r[32];
+            tmem_ld32(taddr + (c + b) * 32, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const float own = __uint_as_float(r[j]);
+              auto at = [&](int i) { return (j & 3) == 0 ? x[i][j / 4].x : (j & 3) == 1 ? x[i][j / 4].y : (j & 3) == 2 ? x[i][j / 4].z : x[i][j / 4].w; };
+              float sum;
+              if (b > 0 || others == 1) {
+                sum = own + at(b);  // two terms: the same sum in either order
+              } else {  // in the order of the ranges, the own one is number w.part
+                sum = w.part == 0 ? own + at(0) : at(0) + (w.part == 1 ? own : at(1));
+                sum += w.part <= 1 ? at(1) : (w.part == 2 ? own : at(2));
+                sum += w.part <= 2 ? at(2) : own;
+              }
+              r[j] = __float_as_uint(sum);
+            }
+            tmem_st32(taddr + (c + b) * 32, r);
+          }
+        }
+        tmem_st_wait();
+      }
 #pragma unroll 1
       for (int c = 0; c < n_chunks; ++c, ++chunk_ctr) {
-        uint8_t* stg = staging + (chunk_ctr & 1) * 16384;
-        uint8_t* srow = stg + r_in_tile * 128;
-        if (store_thread) tma_store_wait_read1();  // the store that last read this block has finished reading
-        named_bar_sync(1, 128);
+        uint8_t* stg = staging + q * 8192 + (chunk_ctr & 1) * 4096;
+        uint8_t* srow = stg + lane * 128;
+        if (lane == 0) tma_store_wait_read1();  // the store that last read this block has finished reading
+        __syncwarp();
         if (args.out_f32) {
           uint32_t r[32];
           tmem_ld32(taddr + c * 32, r);
@@ -571,7 +725,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
             o.z = alpha * __uint_as_float(r[4 * j + 2]);
             o.w = alpha * __uint_as_float(r[4 * j + 3]);
             ss += o.x * o.x + o.y * o.y + o.z * o.z + o.w * o.w;
-            *reinterpret_cast<float4*>(srow + ((j ^ (r_in_tile & 7)) << 4)) = o;
+            *reinterpret_cast<float4*>(srow + ((j ^ (lane & 7)) << 4)) = o;
           }
         } else {
 #pragma unroll
@@ -598,32 +752,25 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
               for (int w = 0; w < 4; ++w)  // a bf16 pair: low half = even column
                 ow[w] = pack_bf16x2(fmaf(alpha, __uint_as_float(r[8 * j + 2 * w]), __uint_as_float(rw[w] << 16)),
                                     fmaf(alpha, __uint_as_float(r[8 * j + 2 * w + 1]), __uint_as_float(rw[w] & 0xffff0000u)));
-              *reinterpret_cast<uint4*>(srow + (((half * 4 + j) ^ (r_in_tile & 7)) << 4)) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+              *reinterpret_cast<uint4*>(srow + (((half * 4 + j) ^ (lane & 7)) << 4)) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
             }
           }
         }
-        if (c == n_chunks - 1) {  // accumulator fully read: hand it back to the MMA warp (of the leader CTA)
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            if (CG == 2) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty[acc]), 0));
-            else mbar_arrive(&tempty[acc]);
-          }
-        }
+        if (c == n_chunks - 1) free_accumulator();
         fence_proxy_async_smem();
-        named_bar_sync(1, 128);
-        if (store_thread) {
-          const int x = n0 + c * cols_per_chunk;
-          if (x < N && m0 < M) {
-            if (args.accumulate) tma_reduce_add_2d(&tma_c, stg, x, m0);
-            else tma_store_2d(&tma_c, stg, x, m0);
+        __syncwarp();
+        if (lane == 0) {
+          const int x = n0 + c * cols_per_chunk, y = m0 + q * 32;
+          if (x < N && y < M) {
+            if (args.accumulate) tma_reduce_add_2d(&tma_c, stg, x, y);
+            else tma_store_2d(&tma_c, stg, x, y);
           }
           tma_store_commit();
         }
       }
       }
     }
-    if (MODE == MODE_SCATTER || store_thread) tma_store_wait0();  // all of this thread's stores have completed
+    if (MODE == MODE_SCATTER || lane == 0) tma_store_wait0();  // all of this thread's stores have completed
     if (fa.sumsq != nullptr) {
       ss = warp_sum(ss);
       if (lane == 0) atomicAdd(fa.sumsq, ss);
@@ -663,6 +810,7 @@ struct Operands {
 
 template <int BLOCK_N, int CG, int MODE = MODE_PLAIN>
 int launch_gemm(const Operands* ops, int n_ops, GemmArgs args, const FusedArgs& fa, int sm_limit, cudaStream_t stream) {
+  // args.splits > 1: the caller's plan (tile shape, whole tiles, workspace) was made for this very configuration
   using Cfg = GemmCfg<BLOCK_N, CG, MODE>;
   if (n_ops < 1 || n_ops > MAX_GROUP) return -1;
   GroupMaps maps;
@@ -681,7 +829,7 @@ int launch_gemm(const Operands* ops, int n_ops, GemmArgs args, const FusedArgs& 
     maps.a[i] = maps.a[0];
     maps.b[i] = maps.b[0];
   }
-  const CUtensorMap* mc = yf_tensor_map_2d(args.C, args.N, args.M, args.ldc, args.out_f32 ? 32 : 64, BLOCK_M, args.out_f32 ? 4 : 2, 1);
+  const CUtensorMap* mc = yf_tensor_map_2d(args.C, args.N, args.M, args.ldc, args.out_f32 ? 32 : 64, 32, args.out_f32 ? 4 : 2, 1);
   if (!mc) return -2;
   static bool optin[64] = {};
   if (int rc = ensure_smem_optin(gemm_bf16_tcgen05_kernel<BLOCK_N, CG, MODE>, Cfg::SMEM_BYTES, optin)) return rc;
@@ -717,12 +865,13 @@ int launch_gemm(const Operands* ops, int n_ops, GemmArgs args, const FusedArgs& 
   if (units < 1) return -1;
   // never more CTAs than SMs (producers may wait on other CTAs' communication warps: all of them must be resident); the
   // gather mode keeps every SM's communication warp even when the GEMM has fewer tiles than that
-  if (num_tiles < units && MODE != MODE_GATHER) units = num_tiles;
+  const int items = num_tiles + (MODE == MODE_SPLIT ? args.split_tiles * (args.splits - 1) : 0);
+  if (items < units && MODE != MODE_GATHER) units = items;
   const int grid = units * CG;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(grid, 1, 1);
-  cfg.blockDim = dim3(MODE == MODE_GATHER ? GATHER_THREADS : GEMM_THREADS, 1, 1);
+  cfg.blockDim = dim3(MODE == MODE_SCATTER ? GEMM_THREADS : WIDE_THREADS, 1, 1);
   cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -744,8 +893,117 @@ int launch_gemm(const void* A, const void* B, const GemmArgs& args, const FusedA
   return launch_gemm<BLOCK_N, CG, MODE>(&one, 1, args, fa, sm_limit, stream);
 }
 
-// Tile shape for a problem: CTA pairs (256 x 256 tiles, half of B per CTA) whenever both extents fill such a tile; single
-// CTAs with 128 x 256 or 128 x 128 tiles for small or ragged problems.
+// ---- plain mode: tile shape and split of the last wave
+enum Tile : int { TILE_PAIR256 = 1, TILE_256 = 2, TILE_128 = 3, TILE_64 = 4, TILE_PAIR128 = 5 };
+struct Plan {
+  int tile, split_tiles, splits;
+  long long counters, bytes;  // workspace: counters (8 bytes each, rounded up to 256 bytes), then the slots
+};
+// Per tile shape, measured on one B200 in a stream of launches: us from launch to the end without main loop, and us per K
+// block of 64 with all units busy (and, for the wide tiles, the clock that the power cap leaves then).
+struct TileShape {
+  int cg, bn;
+  float fixed_us, kb_us;
+};
+constexpr TileShape TILE_SHAPES[6] = {{0, 0, 0.f, 0.f}, {2, 256, 7.f, 0.36f}, {1, 256, 6.f, 0.40f}, {1, 128, 4.8f, 0.225f}, {1, 64, 4.2f, 0.155f}, {2, 128, 6.f, 0.20f}};
+
+// Estimated time of a tile shape and split count.  A tile takes its K blocks or, where K is short, its epilogue (15 ns per
+// column of fp32 output, 10.5 ns of bf16); no shape gets more than 5.2 TB/s out of HBM on operands that are read once.
+// Splitting: an exchange of partial sums takes 6 to 18 us (a release and an acquire at GPU scope in an SM full of
+// asynchronous copies).  Whole tiles behind it hide it, unless a unit gets several ranges one after another.  Long GEMMs
+// run against the power cap, where idle units are not all lost, hence the factor of 1.1.
+//   [1337 x 4096 x 11008] 139 us whole, 96 us in three ranges; [999 x 5120 x 13824] 142 / 106 us in four;
+//   [2048 x 4096 x 22016] 250 / 258 us in four: stays whole.
+float plan_us(const TileShape& t, int M, int N, int K, int units, int splits, bool out_f32) {
+  const int tile_m = BLOCK_M * t.cg, num_k = (K + BLOCK_K - 1) / BLOCK_K;
+  const long long tiles = (long long)((M + tile_m - 1) / tile_m) * ((N + t.bn - 1) / t.bn);
+  const long long full = tiles / units, rest = tiles - full * units;
+  const float epi = (float)t.bn * (out_f32 ? 0.015f : 0.0105f), loop = (float)num_k * t.kb_us, tile_us = loop > epi ? loop : epi;
+  float us = (float)full * tile_us;
+  if (rest > 0 && splits == 1) us += tile_us;
+  if (rest > 0 && splits > 1) {
+    const float rounds = (float)((rest * splits + units - 1) / units), part = loop / (float)splits;
+    us += rounds * (rounds > 1.f && part < 9.f ? 9.f : part);
+    us += full > 0 ? 3.f : 2.f + 4.f * (float)splits;
+    us *= 1.1f;
+  }
+  const float read_us = ((float)M + (float)N) * (float)K * 2.f / 5.2e6f;
+  return t.fixed_us + (us > read_us ? us : read_us + 0.1f * us);
+}
+
+Plan make_plan(int M, int N, int K, bool out_f32, int sm_limit, bool may_split, int tile, int splits) {
+  int sms = yf_num_sms();
+  if (sm_limit > 0 && sm_limit < sms) sms = sm_limit;
+  const int num_k = (K + BLOCK_K - 1) / BLOCK_K;
+  Plan best = {0, 0, 1, 0, 0};
+  float best_c = 0.f;
+  for (int t = 1; t <= 5; ++t) {
+    if (tile > 0 && t != tile) continue;
+    const int units = sms / TILE_SHAPES[t].cg;
+    if (units < 1) continue;
+    for (int sp = 1; sp <= MAX_SPLITS; ++sp) {
+      if (sp > 1 && (!may_split || num_k < 4 * sp)) break;
+      if (splits > 0 && sp != splits && !(sp == 1 && num_k < 4 * splits)) continue;
+      const float c = plan_us(TILE_SHAPES[t], M, N, K, units, sp, out_f32);
+      if (best.tile == 0 || c < best_c) {
+        best.tile = t;
+        best.splits = sp;
+        best_c = c;
+      }
+    }
+  }
+  if (best.tile == 0) return best;
+  const TileShape& t = TILE_SHAPES[best.tile];
+  const int tile_m = BLOCK_M * t.cg, units = sms / t.cg;
+  const long long tiles = (long long)((M + tile_m - 1) / tile_m) * ((N + t.bn - 1) / t.bn);
+  best.split_tiles = (int)(tiles % units);
+  if (best.split_tiles == 0) best.splits = 1;
+  if (best.splits > 1) {
+    const long long ctas = (long long)best.split_tiles * t.cg;
+    best.counters = (ctas * 8 + 255) / 256 * 256;
+    best.bytes = best.counters + ctas * best.splits * BLOCK_M * t.bn * 4;
+  }
+  return best;
+}
+
+unsigned long long next_nonce() {  // 56 bits, never 0, different in every launch of this process
+  static std::atomic<unsigned long long> n{0};
+  unsigned long long z = n.fetch_add(1, std::memory_order_relaxed) + 1;
+  z *= 0x9E3779B97F4A7C15ull;  // odd: no two launches get the same word
+  return (z >> 8) | 1ull;
+}
+
+template <int MODE>
+int launch_tile(int tile, const void* A, const void* B, const GemmArgs& args, const FusedArgs& fa, long long lda, long long ldb, int sm_limit,
+                cudaStream_t s) {
+  switch (tile) {
+    case TILE_PAIR256: return launch_gemm<256, 2, MODE>(A, B, args, fa, lda, ldb, sm_limit, s);
+    case TILE_256: return launch_gemm<256, 1, MODE>(A, B, args, fa, lda, ldb, sm_limit, s);
+    case TILE_128: return launch_gemm<128, 1, MODE>(A, B, args, fa, lda, ldb, sm_limit, s);
+    case TILE_64: return launch_gemm<64, 1, MODE>(A, B, args, fa, lda, ldb, sm_limit, s);
+    default: return launch_gemm<128, 2, MODE>(A, B, args, fa, lda, ldb, sm_limit, s);
+  }
+}
+
+int launch_plain(const void* A, const void* B, GemmArgs args, const FusedArgs& fa, long long lda, long long ldb, int sm_limit,
+                 void* workspace, long long workspace_bytes, int tile, int splits, cudaStream_t s) {
+  const bool ws = workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255) == 0;
+  Plan p = make_plan(args.M, args.N, args.K, args.out_f32 != 0, sm_limit, ws, tile, splits);
+  if (p.bytes > workspace_bytes) p = make_plan(args.M, args.N, args.K, args.out_f32 != 0, sm_limit, false, tile, 1);
+  if (p.tile == 0) return -1;
+  args.splits = p.splits;
+  if (p.splits > 1) {
+    args.split_tiles = p.split_tiles;
+    args.nonce = next_nonce();
+    args.counters = static_cast<unsigned long long*>(workspace);
+    args.slots = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + p.counters);
+  }
+  if (p.splits > 1) return launch_tile<MODE_SPLIT>(p.tile, A, B, args, fa, lda, ldb, sm_limit, s);
+  return launch_tile<MODE_PLAIN>(p.tile, A, B, args, fa, lda, ldb, sm_limit, s);
+}
+
+// Tile shape of the fused modes: CTA pairs (256 x 256 tiles, half of B per CTA) whenever both extents fill such a tile;
+// single CTAs with 128 x 256 or 128 x 128 tiles for small or ragged problems.
 int dispatch_gemm(const void* A, const void* B, const GemmArgs& args, const FusedArgs& fa, long long lda, long long ldb, int sm_limit,
                   cudaStream_t s) {
   const int M = args.M, N = args.N;
@@ -765,8 +1023,7 @@ int dispatch_gemm(const void* A, const void* B, const GemmArgs& args, const Fuse
     return use256 ? launch_gemm<256, 1, MODE_SCATTER>(A, B, args, fa, lda, ldb, sm_limit, s)
                   : launch_gemm<128, 1, MODE_SCATTER>(A, B, args, fa, lda, ldb, sm_limit, s);
   }
-  if (pair_ok && force_cg != 1) return launch_gemm<256, 2>(A, B, args, fa, lda, ldb, sm_limit, s);
-  return use256 ? launch_gemm<256, 1>(A, B, args, fa, lda, ldb, sm_limit, s) : launch_gemm<128, 1>(A, B, args, fa, lda, ldb, sm_limit, s);
+  return launch_plain(A, B, args, fa, lda, ldb, sm_limit, nullptr, 0, force_cg == 1 ? (use256 ? TILE_256 : TILE_128) : 0, 0, s);
 }
 
 }  // namespace
@@ -833,6 +1090,40 @@ extern "C" int yf_gemm_bf16_residual(const void* A, const void* B, void* C, cons
   FusedArgs fa;
   memset(&fa, 0, sizeof(fa));
   return dispatch_gemm(A, B, args, fa, lda, ldb, sm_limit, reinterpret_cast<cudaStream_t>(stream));
+}
+
+// The general form of the entries above.  `workspace` (256-byte aligned device memory that no other launch uses meanwhile, its
+// contents do not matter) lets the last wave's tiles be split along K; yf_gemm_workspace says how much a problem wants, with
+// less (or none) no tile is split.  tile, splits: 0 = chosen from the shape; else a Tile and 1 to MAX_SPLITS.
+extern "C" int yf_gemm_workspace(int M, int N, int K, int out_f32, int sm_limit, int tile, int splits, long long* bytes) {
+  if (M <= 0 || N <= 0 || K <= 0 || bytes == nullptr || tile < 0 || tile > 5 || splits < 0 || splits > MAX_SPLITS) return -1;
+  *bytes = make_plan(M, N, K, out_f32 != 0, sm_limit, true, tile, splits).bytes;
+  return 0;
+}
+extern "C" int yf_gemm_bf16_ws(const void* A, const void* B, void* C, const void* R, int M, int N, int K, long long lda, long long ldb,
+                               long long ldc, long long ldr, int a_mn, int b_mn, int out_f32, int accumulate, float alpha, int sm_limit,
+                               float* sumsq, void* workspace, long long workspace_bytes, int tile, int splits, void* stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || tile < 0 || tile > 5 || splits < 0 || splits > MAX_SPLITS) return -1;
+  if (sumsq != nullptr && (!out_f32 || accumulate)) return -1;
+  if ((lda % 8) || (ldb % 8) || (ldc % (out_f32 ? 4 : 8))) return -1;
+  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15) return -1;
+  if (R != nullptr && (out_f32 || accumulate || (ldr % 8) || (N % 8) || (reinterpret_cast<uintptr_t>(R) & 15))) return -1;
+  GemmArgs args;
+  memset(&args, 0, sizeof(args));
+  args.C = C;
+  args.M = M; args.N = N; args.K = K;
+  args.ldc = ldc;
+  args.alpha = alpha;
+  args.a_mn = a_mn ? 1 : 0;
+  args.b_mn = b_mn ? 1 : 0;
+  args.out_f32 = out_f32 ? 1 : 0;
+  args.accumulate = accumulate ? 1 : 0;
+  args.R = R;
+  args.ldr = ldr;
+  FusedArgs fa;
+  memset(&fa, 0, sizeof(fa));
+  fa.sumsq = sumsq;
+  return launch_plain(A, B, args, fa, lda, ldb, sm_limit, workspace, workspace_bytes, tile, splits, reinterpret_cast<cudaStream_t>(stream));
 }
 
 // All-gather -> GEMM in one kernel.  C[M,N] = A[M,K] * B[N,K]^T where B (row-major, contiguous, K-major) is a

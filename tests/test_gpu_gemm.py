@@ -104,3 +104,36 @@ def test_gemm_residual_epilogue(m, n, k):
     kernels.gemm(a, b, residual=inplace, out=inplace)
     torch.cuda.synchronize()
     assert torch.equal(inplace, out)
+
+
+@pytest.mark.parametrize("tile", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("splits", [1, 2, 3, 4])
+@pytest.mark.parametrize("m,n,k,a_mn,b_mn", [(45, 1024, 1048, False, False), (264, 520, 1032, True, True), (1337, 2056, 1024, False, True),
+                                             (8, 8, 2048, False, False), (4096, 4104, 256, True, True)])
+def test_gemm_tile_shapes_and_split_last_wave(tile, splits, m, n, k, a_mn, b_mn):
+    """Every tile shape, whole and with its last wave's tiles split along K: fp32 output (plain, accumulating, with the squared
+    norm) and bf16 output with a residual.  fp32 sums of k products: a few sqrt(k) * 2^-24; a bf16 result: 2^-8."""
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(7)
+    a = torch.randn((k, m) if a_mn else (m, k), device="cuda", dtype=torch.bfloat16)
+    b = torch.randn((k, n) if b_mn else (n, k), device="cuda", dtype=torch.bfloat16)
+    res = torch.randn(m, n, device="cuda", dtype=torch.bfloat16)
+    ref = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+    kw = dict(a_mn_major=a_mn, b_mn_major=b_mn, tile=tile, splits=splits)
+    sq = torch.zeros(1, device="cuda")
+    f32 = kernels.gemm(a, b, out_dtype=torch.float32, sumsq=sq, **kw)
+    acc = kernels.gemm(a, b, out=torch.full_like(f32, 3.0), accumulate=True, **kw)
+    low = kernels.gemm(a, b, residual=res, **kw)
+    again = kernels.gemm(a, b, out_dtype=torch.float32, **kw)
+    torch.cuda.synchronize()
+    kernels.check_status()
+
+    def off(x, y):
+        return ((x.double() - y).norm() / y.norm()).item()
+
+    lim = 3.0 * k ** 0.5 * 2.0**-24
+    assert off(f32, ref) < lim and off(acc, ref + 3.0) < lim
+    assert abs(sq.item() / ref.pow(2).sum().item() - 1.0) < 2 * lim + 2.0**-16
+    assert off(low, ref + res.double()) < 2.0**-8
+    assert torch.equal(f32, again)  # the order of the sums does not depend on which range comes last

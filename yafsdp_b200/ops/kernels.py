@@ -10,6 +10,7 @@ error, and the autograd-level ops in :mod:`yafsdp_b200.ops.functional` choose be
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Any
 
 import torch
@@ -83,6 +84,8 @@ def gemm(
     sm_limit: int = 0,
     sumsq: torch.Tensor | None = None,
     residual: torch.Tensor | None = None,
+    tile: int = 0,
+    splits: int = 0,
 ) -> torch.Tensor:
     """``out[M,N] = alpha * A @ B^T (+ out)`` with bf16 inputs and fp32 accumulation (tcgen05).
 
@@ -91,6 +94,7 @@ def gemm(
     dimension); the row pitch may exceed the row length.  ``sumsq`` (fp32 output without accumulation only): a
     one-element fp32 tensor that receives ``+= sum(out**2)`` from the same kernel.  ``residual`` (bf16 output without
     accumulation only): a bf16 ``[M,N]`` tensor added in fp32 inside the epilogue, before the output is rounded.
+    ``tile`` (1-5) and ``splits`` (1-4): tile shape and K ranges of the last wave's tiles; 0 chooses them from the shape.
     """
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.is_cuda and b.is_cuda
     assert a.dim() == 2 and b.dim() == 2 and a.stride(1) == 1 and b.stride(1) == 1
@@ -110,19 +114,25 @@ def gemm(
     if residual is not None:
         assert out.dtype == torch.bfloat16 and not accumulate and sumsq is None
         assert residual.dtype == torch.bfloat16 and residual.shape == (m, n) and residual.stride(1) == 1
-        rc = _native.lib().yf_gemm_bf16_residual(
-            a.data_ptr(), b.data_ptr(), out.data_ptr(), residual.data_ptr(), m, n, k, a.stride(0), b.stride(0), out.stride(0),
-            residual.stride(0), int(a_mn_major), int(b_mn_major), float(alpha), int(sm_limit), _stream(),
-        )
-        _check(rc, "yf_gemm_bf16_residual")
-        return out
-    rc = _native.lib().yf_gemm_bf16_sumsq(
-        a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, a.stride(0), b.stride(0), out.stride(0),
-        int(a_mn_major), int(b_mn_major), int(out.dtype == torch.float32), int(accumulate), float(alpha),
-        int(sm_limit), _ptr(sumsq), _stream(),
+    nbytes = _gemm_workspace(m, n, k, int(out.dtype == torch.float32), sm_limit, tile, splits, a.device.index)
+    ws = torch.empty(nbytes, device=a.device, dtype=torch.uint8) if nbytes else None
+    rc = _native.lib().yf_gemm_bf16_ws(
+        a.data_ptr(), b.data_ptr(), out.data_ptr(), _ptr(residual), m, n, k, a.stride(0), b.stride(0), out.stride(0),
+        0 if residual is None else residual.stride(0), int(a_mn_major), int(b_mn_major), int(out.dtype == torch.float32),
+        int(accumulate), float(alpha), int(sm_limit), _ptr(sumsq), _ptr(ws), nbytes, tile, splits, _stream(),
     )
     _check(rc, "yf_gemm_bf16")
     return out
+
+
+@functools.lru_cache(maxsize=4096)
+def _gemm_workspace(m: int, n: int, k: int, out_f32: int, sm_limit: int, tile: int, splits: int, device: int | None) -> int:
+    """Workspace bytes that a GEMM wants (a function of its shape and the device's number of SMs)."""
+    nbytes = ctypes.c_longlong(0)
+    rc = _native.lib().yf_gemm_workspace(m, n, k, out_f32, int(sm_limit), tile, splits, ctypes.byref(nbytes))
+    if rc != 0:
+        raise RuntimeError(f"yf_gemm_workspace failed with code {rc}")
+    return nbytes.value
 
 
 def gemm_gathered(a: torch.Tensor, n: int, k: int, *, peer_in: Any, layer_buf: torch.Tensor, shard_bytes: int, b_byte_off: int,
