@@ -9,10 +9,12 @@
 // the three GEMMs of a linear layer (Y = X W^T, dX = dY W, dW = dY^T X) run without a transpose.
 // The fp32 output mode with accumulate writes weight gradients straight into a flat fp32 gradient
 // buffer (the cast and the micro-batch accumulation of a sharded-data-parallel step).
+#include <limits.h>
 #include <stdlib.h>
 #include <string.h>
 
 #include <atomic>
+#include <numeric>
 
 #include "common.cuh"
 #include "yafsdp_b200.h"
@@ -66,6 +68,10 @@ struct GemmArgs {
   // mode): a block's "x + proj(...)" costs no pass of its own over the activations
   const void* R;
   long long ldr;
+  // B in several pieces of memory (plain and split mode): parts[i] is where piece i ends, in rows of [N, K] storage (then no
+  // tile crosses a piece's end) or of [K, N] storage (no K block does).  n_parts <= 1: one piece.
+  int n_parts;
+  int parts[MAX_GROUP];
   // Split tiles (split mode).  The number of tiles modulo the number of units is what a last wave would leave most units
   // idle for: so many tiles, [0, split_tiles), are computed in `splits` K ranges each, the others whole.  Work items are
   // dealt round-robin: range 0 of every split tile, range 1 of every split tile, and so on - the units that run at the same
@@ -376,6 +382,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
         if (!tile_coords(w.tile, p, m0, n0)) continue;
         const CUtensorMap* tma_a = &maps.a[p];
         const CUtensorMap* tma_b = &maps.b[p];
+        int b_at = 0;  // first row of the current piece of B
+        if (is_plain(MODE) && args.n_parts > 1 && !args.b_mn)
+          for (int i = 0; n0 >= args.parts[i]; ++i) {
+            b_at = args.parts[i];
+            tma_b = &maps.b[i + 1];
+          }
         const int N = grouped ? args.Np[p] : args.N;
         if (MODE == MODE_GATHER) {
           // the rows [n0, n0 + BLOCK_N) of B must have landed in the local layer buffer: the column block's counter says so
@@ -398,13 +410,20 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
           }
           if (!alive) break;
         }
-        const int nb = n0 + (int)crank * B_ROWS;  // first B row this CTA holds
+        const int nb = n0 + (int)crank * B_ROWS - (args.b_mn ? 0 : b_at);  // first B row this CTA holds
+        const bool k_parts = is_plain(MODE) && args.n_parts > 1 && args.b_mn;
+        int piece = 0;
         int kb = w.kb0 + skip;
         for (; kb < w.kb1; kb += PRODUCERS) {
+          if (k_parts)
+            while (kb * BLOCK_K >= args.parts[piece]) {
+              b_at = args.parts[piece++];
+              tma_b = &maps.b[piece];
+            }
           if (!mbar_wait(&empty[s], ph ^ 1, 10)) { alive = false; break; }
           uint8_t* sa = smem + s * Cfg::STAGE_BYTES;
           uint8_t* sb = sa + Cfg::A_BYTES;
-          const int k0 = kb * BLOCK_K;
+          const int k0 = kb * BLOCK_K, kb0 = args.b_mn ? k0 - b_at : k0;
           if (CG == 2) {
             // both CTAs' bytes are counted on the leader's barrier (the thread that issues the MMAs waits there)
             if (leader) mbar_expect_tx(&full[s], 2 * Cfg::STAGE_BYTES);
@@ -416,10 +435,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
               for (int j = 0; j < BLOCK_M / 64; ++j) tma_load_2d_pair(sa + j * (BLOCK_K * 128), tma_a, fb, m0 + j * 64, k0);
             }
             if (!args.b_mn) {
-              tma_load_2d_pair(sb, tma_b, fb, k0, nb);
+              tma_load_2d_pair(sb, tma_b, fb, kb0, nb);
             } else {
 #pragma unroll
-              for (int j = 0; j < B_ROWS / 64; ++j) tma_load_2d_pair(sb + j * (BLOCK_K * 128), tma_b, fb, nb + j * 64, k0);
+              for (int j = 0; j < B_ROWS / 64; ++j) tma_load_2d_pair(sb + j * (BLOCK_K * 128), tma_b, fb, nb + j * 64, kb0);
             }
           } else {
             mbar_expect_tx(&full[s], Cfg::STAGE_BYTES);
@@ -430,10 +449,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
               for (int j = 0; j < BLOCK_M / 64; ++j) tma_load_2d(sa + j * (BLOCK_K * 128), tma_a, &full[s], m0 + j * 64, k0);
             }
             if (!args.b_mn) {
-              tma_load_2d(sb, tma_b, &full[s], k0, nb);
+              tma_load_2d(sb, tma_b, &full[s], kb0, nb);
             } else {
 #pragma unroll
-              for (int j = 0; j < B_ROWS / 64; ++j) tma_load_2d(sb + j * (BLOCK_K * 128), tma_b, &full[s], nb + j * 64, k0);
+              for (int j = 0; j < B_ROWS / 64; ++j) tma_load_2d(sb + j * (BLOCK_K * 128), tma_b, &full[s], nb + j * 64, kb0);
             }
           }
           s += PRODUCERS;
@@ -800,12 +819,13 @@ int ensure_smem_optin(KernelT kernel, int bytes, bool (&done)[64]) {
   return 0;
 }
 
-// One problem's operands (a grouped launch passes several).
+// One problem's operands (a grouped launch passes several); for B in pieces: N or K is that of the piece.
 struct Operands {
   const void* A;
   const void* B;
   long long lda, ldb;
   int M, N;
+  int K;
 };
 
 template <int BLOCK_N, int CG, int MODE = MODE_PLAIN>
@@ -819,8 +839,8 @@ int launch_gemm(const Operands* ops, int n_ops, GemmArgs args, const FusedArgs& 
     const Operands& o = ops[i];
     const CUtensorMap* ma = args.a_mn ? yf_tensor_map_2d(o.A, o.M, args.K, o.lda, 64, BLOCK_K, 2, 1)
                                       : yf_tensor_map_2d(o.A, args.K, o.M, o.lda, BLOCK_K, BLOCK_M, 2, 1);
-    const CUtensorMap* mb = args.b_mn ? yf_tensor_map_2d(o.B, o.N, args.K, o.ldb, 64, BLOCK_K, 2, 1)
-                                      : yf_tensor_map_2d(o.B, args.K, o.N, o.ldb, BLOCK_K, Cfg::B_ROWS, 2, 1);
+    const CUtensorMap* mb = args.b_mn ? yf_tensor_map_2d(o.B, o.N, o.K, o.ldb, 64, BLOCK_K, 2, 1)
+                                      : yf_tensor_map_2d(o.B, o.K, o.N, o.ldb, BLOCK_K, Cfg::B_ROWS, 2, 1);
     if (!ma || !mb) return -2;
     maps.a[i] = *ma;
     maps.b[i] = *mb;
@@ -889,7 +909,7 @@ int launch_gemm(const Operands* ops, int n_ops, GemmArgs args, const FusedArgs& 
 template <int BLOCK_N, int CG, int MODE = MODE_PLAIN>
 int launch_gemm(const void* A, const void* B, const GemmArgs& args, const FusedArgs& fa, long long lda, long long ldb, int sm_limit,
                 cudaStream_t stream) {
-  const Operands one = {A, B, lda, ldb, args.M, args.N};
+  const Operands one = {A, B, lda, ldb, args.M, args.N, args.K};
   return launch_gemm<BLOCK_N, CG, MODE>(&one, 1, args, fa, sm_limit, stream);
 }
 
@@ -931,7 +951,8 @@ float plan_us(const TileShape& t, int M, int N, int K, int units, int splits, bo
   return t.fixed_us + (us > read_us ? us : read_us + 0.1f * us);
 }
 
-Plan make_plan(int M, int N, int K, bool out_f32, int sm_limit, bool may_split, int tile, int splits) {
+// n_align > 0: tiles must end where multiples of n_align columns do (the pieces of B)
+Plan make_plan(int M, int N, int K, bool out_f32, int n_align, int sm_limit, bool may_split, int tile, int splits) {
   int sms = yf_num_sms();
   if (sm_limit > 0 && sm_limit < sms) sms = sm_limit;
   const int num_k = (K + BLOCK_K - 1) / BLOCK_K;
@@ -939,6 +960,7 @@ Plan make_plan(int M, int N, int K, bool out_f32, int sm_limit, bool may_split, 
   float best_c = 0.f;
   for (int t = 1; t <= 5; ++t) {
     if (tile > 0 && t != tile) continue;
+    if (n_align > 0 && n_align % TILE_SHAPES[t].bn != 0) continue;
     const int units = sms / TILE_SHAPES[t].cg;
     if (units < 1) continue;
     for (int sp = 1; sp <= MAX_SPLITS; ++sp) {
@@ -974,22 +996,33 @@ unsigned long long next_nonce() {  // 56 bits, never 0, different in every launc
 }
 
 template <int MODE>
-int launch_tile(int tile, const void* A, const void* B, const GemmArgs& args, const FusedArgs& fa, long long lda, long long ldb, int sm_limit,
-                cudaStream_t s) {
+int launch_tile(int tile, const Operands* ops, int n_ops, const GemmArgs& args, const FusedArgs& fa, int sm_limit, cudaStream_t s) {
   switch (tile) {
-    case TILE_PAIR256: return launch_gemm<256, 2, MODE>(A, B, args, fa, lda, ldb, sm_limit, s);
-    case TILE_256: return launch_gemm<256, 1, MODE>(A, B, args, fa, lda, ldb, sm_limit, s);
-    case TILE_128: return launch_gemm<128, 1, MODE>(A, B, args, fa, lda, ldb, sm_limit, s);
-    case TILE_64: return launch_gemm<64, 1, MODE>(A, B, args, fa, lda, ldb, sm_limit, s);
-    default: return launch_gemm<128, 2, MODE>(A, B, args, fa, lda, ldb, sm_limit, s);
+    case TILE_PAIR256: return launch_gemm<256, 2, MODE>(ops, n_ops, args, fa, sm_limit, s);
+    case TILE_256: return launch_gemm<256, 1, MODE>(ops, n_ops, args, fa, sm_limit, s);
+    case TILE_128: return launch_gemm<128, 1, MODE>(ops, n_ops, args, fa, sm_limit, s);
+    case TILE_64: return launch_gemm<64, 1, MODE>(ops, n_ops, args, fa, sm_limit, s);
+    default: return launch_gemm<128, 2, MODE>(ops, n_ops, args, fa, sm_limit, s);
   }
 }
 
-int launch_plain(const void* A, const void* B, GemmArgs args, const FusedArgs& fa, long long lda, long long ldb, int sm_limit,
-                 void* workspace, long long workspace_bytes, int tile, int splits, cudaStream_t s) {
+// n_ops > 1: the pieces of B (ops[i].N or ops[i].K rows each), every one with the same A
+int launch_plain(const Operands* ops, int n_ops, GemmArgs args, const FusedArgs& fa, int sm_limit, void* workspace,
+                 long long workspace_bytes, int tile, int splits, cudaStream_t s) {
+  int n_align = 0;
+  if (n_ops > 1) {
+    args.n_parts = n_ops;
+    int end = 0;
+    for (int i = 0; i < n_ops; ++i) {
+      if (i > 0 && !args.b_mn) n_align = std::gcd(n_align, end);
+      end += args.b_mn ? ops[i].K : ops[i].N;
+      args.parts[i] = end;
+    }
+    for (int i = n_ops - 1; i < MAX_GROUP; ++i) args.parts[i] = INT_MAX;  // searches stop at the last piece
+  }
   const bool ws = workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255) == 0;
-  Plan p = make_plan(args.M, args.N, args.K, args.out_f32 != 0, sm_limit, ws, tile, splits);
-  if (p.bytes > workspace_bytes) p = make_plan(args.M, args.N, args.K, args.out_f32 != 0, sm_limit, false, tile, 1);
+  Plan p = make_plan(args.M, args.N, args.K, args.out_f32 != 0, n_align, sm_limit, ws, tile, splits);
+  if (p.bytes > workspace_bytes) p = make_plan(args.M, args.N, args.K, args.out_f32 != 0, n_align, sm_limit, false, tile, 1);
   if (p.tile == 0) return -1;
   args.splits = p.splits;
   if (p.splits > 1) {
@@ -998,8 +1031,8 @@ int launch_plain(const void* A, const void* B, GemmArgs args, const FusedArgs& f
     args.counters = static_cast<unsigned long long*>(workspace);
     args.slots = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + p.counters);
   }
-  if (p.splits > 1) return launch_tile<MODE_SPLIT>(p.tile, A, B, args, fa, lda, ldb, sm_limit, s);
-  return launch_tile<MODE_PLAIN>(p.tile, A, B, args, fa, lda, ldb, sm_limit, s);
+  if (p.splits > 1) return launch_tile<MODE_SPLIT>(p.tile, ops, n_ops, args, fa, sm_limit, s);
+  return launch_tile<MODE_PLAIN>(p.tile, ops, n_ops, args, fa, sm_limit, s);
 }
 
 // Tile shape of the fused modes: CTA pairs (256 x 256 tiles, half of B per CTA) whenever both extents fill such a tile;
@@ -1023,7 +1056,8 @@ int dispatch_gemm(const void* A, const void* B, const GemmArgs& args, const Fuse
     return use256 ? launch_gemm<256, 1, MODE_SCATTER>(A, B, args, fa, lda, ldb, sm_limit, s)
                   : launch_gemm<128, 1, MODE_SCATTER>(A, B, args, fa, lda, ldb, sm_limit, s);
   }
-  return launch_plain(A, B, args, fa, lda, ldb, sm_limit, nullptr, 0, force_cg == 1 ? (use256 ? TILE_256 : TILE_128) : 0, 0, s);
+  const Operands one = {A, B, lda, ldb, M, N, args.K};
+  return launch_plain(&one, 1, args, fa, sm_limit, nullptr, 0, force_cg == 1 ? (use256 ? TILE_256 : TILE_128) : 0, 0, s);
 }
 
 }  // namespace
@@ -1095,9 +1129,9 @@ extern "C" int yf_gemm_bf16_residual(const void* A, const void* B, void* C, cons
 // The general form of the entries above.  `workspace` (256-byte aligned device memory that no other launch uses meanwhile, its
 // contents do not matter) lets the last wave's tiles be split along K; yf_gemm_workspace says how much a problem wants, with
 // less (or none) no tile is split.  tile, splits: 0 = chosen from the shape; else a Tile and 1 to MAX_SPLITS.
-extern "C" int yf_gemm_workspace(int M, int N, int K, int out_f32, int sm_limit, int tile, int splits, long long* bytes) {
-  if (M <= 0 || N <= 0 || K <= 0 || bytes == nullptr || tile < 0 || tile > 5 || splits < 0 || splits > MAX_SPLITS) return -1;
-  *bytes = make_plan(M, N, K, out_f32 != 0, sm_limit, true, tile, splits).bytes;
+extern "C" int yf_gemm_workspace(int M, int N, int K, int out_f32, int n_align, int sm_limit, int tile, int splits, long long* bytes) {
+  if (M <= 0 || N <= 0 || K <= 0 || n_align < 0 || bytes == nullptr || tile < 0 || tile > 5 || splits < 0 || splits > MAX_SPLITS) return -1;
+  *bytes = make_plan(M, N, K, out_f32 != 0, n_align, sm_limit, true, tile, splits).bytes;
   return 0;
 }
 extern "C" int yf_gemm_bf16_ws(const void* A, const void* B, void* C, const void* R, int M, int N, int K, long long lda, long long ldb,
@@ -1123,7 +1157,37 @@ extern "C" int yf_gemm_bf16_ws(const void* A, const void* B, void* C, const void
   FusedArgs fa;
   memset(&fa, 0, sizeof(fa));
   fa.sumsq = sumsq;
-  return launch_plain(A, B, args, fa, lda, ldb, sm_limit, workspace, workspace_bytes, tile, splits, reinterpret_cast<cudaStream_t>(stream));
+  const Operands one = {A, B, lda, ldb, M, N, K};
+  return launch_plain(&one, 1, args, fa, sm_limit, workspace, workspace_bytes, tile, splits, reinterpret_cast<cudaStream_t>(stream));
+}
+
+// C[M,N] = A * B^T (bf16 output) with B in n (2 to 4) pieces of memory, one below the other: rows[i] rows of its storage ([N,K], or
+// [K,N] with b_mn) at B[i], row pitch ldb[i].  Several weights of one layer act as one matrix without being copied together.
+// Every piece but the last has a multiple of 64 rows.  n_align of yf_gemm_workspace: the greatest common divisor of the
+// places where a piece of [N,K] storage starts; 0 with b_mn.
+extern "C" int yf_gemm_bf16_parts(const void* A, int n, const void* const* B, const int* rows, const long long* ldb, void* C, int M,
+                                  int N, int K, long long lda, long long ldc, int b_mn, void* workspace, long long workspace_bytes,
+                                  int tile, int splits, void* stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || n < 2 || n > MAX_GROUP || tile < 0 || tile > 5 || splits < 0 || splits > MAX_SPLITS) return -1;
+  if ((lda % 8) || (ldc % 8) || ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(C)) & 15)) return -1;
+  Operands ops[MAX_GROUP];
+  long long total = 0;
+  for (int i = 0; i < n; ++i) {
+    if (rows[i] <= 0 || (i + 1 < n && rows[i] % 64) || (ldb[i] % 8) || (reinterpret_cast<uintptr_t>(B[i]) & 15)) return -1;
+    total += rows[i];
+    ops[i] = {A, B[i], lda, ldb[i], M, b_mn ? N : rows[i], b_mn ? rows[i] : K};
+  }
+  if (total != (b_mn ? K : N)) return -1;
+  GemmArgs args;
+  memset(&args, 0, sizeof(args));
+  args.C = C;
+  args.M = M; args.N = N; args.K = K;
+  args.ldc = ldc;
+  args.alpha = 1.f;
+  args.b_mn = b_mn ? 1 : 0;
+  FusedArgs fa;
+  memset(&fa, 0, sizeof(fa));
+  return launch_plain(ops, n, args, fa, 0, workspace, workspace_bytes, tile, splits, reinterpret_cast<cudaStream_t>(stream));
 }
 
 // All-gather -> GEMM in one kernel.  C[M,N] = A[M,K] * B[N,K]^T where B (row-major, contiguous, K-major) is a
@@ -1230,7 +1294,7 @@ extern "C" int yf_gemm_bf16_scatter_grouped(int n, const void* const* A, const v
     if (flat_off[i] + (long long)M[i] * N[i] > shard_numel * world) return -1;
     if (i > 0 && flat_off[i] < flat_off[i - 1] + (long long)M[i - 1] * N[i - 1]) return -1;  // ascending, no overlap
     if ((reinterpret_cast<uintptr_t>(A[i]) | reinterpret_cast<uintptr_t>(B[i])) & 15) return -1;
-    ops[i] = {A[i], B[i], lda[i], ldb[i], M[i], N[i]};
+    ops[i] = {A[i], B[i], lda[i], ldb[i], M[i], N[i], K};
     args.Mp[i] = M[i];
     args.Np[i] = N[i];
     args.flat_off[i] = flat_off[i];

@@ -65,7 +65,8 @@ const CUtensorMap* encode(int rank, const void* base, const uint64_t* dims, cons
   auto it = g_maps.find(key);
   if (it != g_maps.end()) return it->second;
   EncodeTiledFn fn = get_encode_fn();
-  if (!fn) return nullptr;
+  // a driver call: a thread that has launched nothing yet (autograd's, at the start of a backward pass) has no context
+  if (!fn || cudaSetDevice(dev) != cudaSuccess) return nullptr;
   cuuint64_t gdim[3];
   cuuint64_t gstride[2];
   cuuint32_t gbox[3];
@@ -113,7 +114,8 @@ const CUtensorMap* yf_tensor_map_3d(const void* base, uint64_t d0, uint64_t d1, 
 int yf_tensor_map_3d_encode(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t pitch1_elems,
                             uint64_t pitch2_elems, uint32_t b0, uint32_t b1, uint32_t b2, int elem_bytes, int swizzle128) {
   EncodeTiledFn fn = get_encode_fn();
-  if (!fn) return -2;
+  int dev = 0;
+  if (!fn || cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return -2;
   cuuint64_t gdim[3] = {d0, d1, d2};
   cuuint64_t gstride[2] = {pitch1_elems * (uint64_t)elem_bytes, pitch2_elems * (uint64_t)elem_bytes};
   cuuint32_t gbox[3] = {b0, b1, b2};

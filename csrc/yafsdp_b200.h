@@ -26,10 +26,13 @@ int yf_gemm_bf16_residual(const void* A, const void* B, void* C, const void* R, 
                           long long ldc, long long ldr, int a_mn, int b_mn, float alpha, int sm_limit, void* stream);
 /* The general form: optional residual R, optional sumsq, a workspace for splitting the last wave along K (see gemm.cu), a tile
    shape and a split count (0 = chosen).  yf_gemm_workspace: the workspace bytes that a problem wants. */
-int yf_gemm_workspace(int M, int N, int K, int out_f32, int sm_limit, int tile, int splits, long long* bytes);
+int yf_gemm_workspace(int M, int N, int K, int out_f32, int n_align, int sm_limit, int tile, int splits, long long* bytes);
 int yf_gemm_bf16_ws(const void* A, const void* B, void* C, const void* R, int M, int N, int K, long long lda, long long ldb,
                     long long ldc, long long ldr, int a_mn, int b_mn, int out_f32, int accumulate, float alpha, int sm_limit,
                     float* sumsq, void* workspace, long long workspace_bytes, int tile, int splits, void* stream);
+/* bf16 C = A * B^T with B in n (2 to 4) pieces of memory, one below the other (see gemm.cu) */
+int yf_gemm_bf16_parts(const void* A, int n, const void* const* B, const int* rows, const long long* ldb, void* C, int M, int N, int K,
+                       long long lda, long long ldc, int b_mn, void* workspace, long long workspace_bytes, int tile, int splits, void* stream);
 // fused all-gather -> GEMM and GEMM -> reduce-scatter (same kernel, see gemm.cu for the argument contracts)
 int yf_gemm_bf16_gathered(const void* A, void* C, int M, int N, int K, long long lda, long long ldc, int a_mn, int out_f32,
                           void* const* peer_in, void* layer_buf, long long shard_bytes, long long b_byte_off, int rank, int world,

@@ -137,3 +137,23 @@ def test_gemm_tile_shapes_and_split_last_wave(tile, splits, m, n, k, a_mn, b_mn)
     assert abs(sq.item() / ref.pow(2).sum().item() - 1.0) < 2 * lim + 2.0**-16
     assert off(low, ref + res.double()) < 2.0**-8
     assert torch.equal(f32, again)  # the order of the sums does not depend on which range comes last
+
+
+@pytest.mark.parametrize("rows", [[512, 256, 256], [128, 64], [64, 64, 72], [192, 320, 256, 8]])
+@pytest.mark.parametrize("tile,splits", [(0, 0), (3, 1), (4, 2)])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_gemm_weight_in_pieces(rows, tile, splits, b_mn):
+    """A weight in several pieces of memory gives what the concatenated one gives, bit for bit (same tiles, same order)."""
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(8)
+    cols, m = 328, 200
+    parts = [torch.randn(r, cols, device="cuda").bfloat16() for r in rows]
+    whole = torch.cat(parts)
+    tile = 4 if not b_mn else tile  # the tile that every start of a piece is a multiple of
+    a = torch.randn(m, sum(rows) if b_mn else cols, device="cuda").bfloat16()
+    got = kernels.gemm_parts(a, parts, b_mn_major=b_mn, tile=tile, splits=splits)
+    want = kernels.gemm(a, whole, b_mn_major=b_mn, tile=tile, splits=splits)
+    torch.cuda.synchronize()
+    kernels.check_status()
+    assert torch.equal(got, want)

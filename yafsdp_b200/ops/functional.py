@@ -49,6 +49,21 @@ def _sink(p: torch.Tensor) -> Any:
 def fuse_adjacent(ts: list[torch.Tensor]) -> torch.Tensor:
     """One ``[sum(rows), cols]`` view over 2-D tensors that sit back to back in memory (consecutive
     parameters of a flat group buffer); a concatenated copy otherwise."""
+    fused = _adjacent_view(ts)
+    return torch.cat([t.detach() for t in ts], dim=0) if fused is None else fused
+
+
+def fuse_rows(ts: list[torch.Tensor]) -> "torch.Tensor | list[torch.Tensor]":
+    """The same matrix for :func:`_gemm_fused`, which takes weights that do not sit back to back as they are (parameters
+    of a module that ``fully_shard`` does not manage)."""
+    fused = _adjacent_view(ts)
+    if fused is not None:
+        return fused
+    parts = [t.detach() for t in ts]
+    return parts if kernels.can_be_parts(parts) else torch.cat(parts, dim=0)
+
+
+def _adjacent_view(ts: list[torch.Tensor]) -> torch.Tensor | None:
     first = ts[0]
     cols = first.shape[1]
     adjacent = all(t.is_contiguous() and t.shape[1] == cols and t.dtype == first.dtype for t in ts)
@@ -62,9 +77,15 @@ def fuse_adjacent(ts: list[torch.Tensor]) -> torch.Tensor:
                 break
             end += t.numel() * t.element_size()
     if not adjacent:
-        return torch.cat([t.detach() for t in ts], dim=0)
+        return None
     rows = sum(t.shape[0] for t in ts)
     return torch.as_strided(first.detach(), (rows, cols), (cols, 1))
+
+
+def _gemm_fused(a: torch.Tensor, w: "torch.Tensor | list[torch.Tensor]", b_mn_major: bool = False) -> torch.Tensor:
+    if isinstance(w, list):
+        return kernels.gemm_parts(a, w, b_mn_major=b_mn_major)
+    return kernels.gemm(a, w, b_mn_major=b_mn_major)
 
 
 class _WeightGrad:
@@ -205,24 +226,25 @@ class DecoderLayerFn(torch.autograd.Function):
                 cos_sin: torch.Tensor, dims: LayerDims) -> torch.Tensor:
         x = _c(x)
         hd, hq, hkv = dims.head_dim, dims.n_heads, dims.n_kv_heads
-        w_qkv = fuse_adjacent([wq, wk, wv])
-        w_gu = fuse_adjacent([wg, wu])
+        w_qkv = fuse_rows([wq, wk, wv])
+        w_gu = fuse_rows([wg, wu])
         n1, rstd1 = kernels.rmsnorm_fwd(x, w_n1.detach(), dims.eps)
         owner = getattr(wq, "_yf_group_index", None)
-        ticket = owner[0].take_in_kernel_gather(owner[1], w_qkv.shape[0]) if owner is not None else None
+        ticket = owner[0].take_in_kernel_gather(owner[1], wq.shape[0] + wk.shape[0] + wv.shape[0]) if owner is not None else None
         if ticket is not None:
+            assert isinstance(w_qkv, torch.Tensor)  # views of one gather buffer
             # this forward pass has not gathered the layer: the QKV GEMM pulls it from the peers while it computes
             qkv = kernels.gemm_gathered(n1, w_qkv.shape[0], w_qkv.shape[1], peer_in=ticket["peer_in"], layer_buf=ticket["layer_buf"],
                                         shard_bytes=ticket["shard_bytes"], b_byte_off=ticket["b_byte_off"], rank=ticket["rank"],
                                         world=ticket["world"], counters=ticket["counters"], epoch=ticket["epoch"])
         else:
-            qkv = kernels.gemm(n1, w_qkv)
+            qkv = _gemm_fused(n1, w_qkv)
         kernels.rope_(qkv, cos_sin, dims.seq, 0, hq + hkv, hd)
         q, k, v = qkv[:, : hq * hd], qkv[:, hq * hd : (hq + hkv) * hd], qkv[:, (hq + hkv) * hd :]
         att, lse = kernels.attn_fwd(q, k, v, dims.batch, dims.seq, hq, hkv, 1.0 / math.sqrt(hd), True)
         h = kernels.gemm(att, wo.detach(), residual=x)  # x + attention block: the residual is added in the GEMM's epilogue
         n2, rstd2 = kernels.rmsnorm_fwd(h, w_n2.detach(), dims.eps)
-        gu = kernels.gemm(n2, w_gu)
+        gu = _gemm_fused(n2, w_gu)
         a = kernels.swiglu_fwd(gu)
         out = kernels.gemm(a, wd.detach(), residual=h)
         ctx.save_for_backward(x, rstd1, n1, qkv, att, lse, h, rstd2, n2, gu, a, cos_sin)
@@ -238,15 +260,15 @@ class DecoderLayerFn(torch.autograd.Function):
         hd, hq, hkv = dims.head_dim, dims.n_heads, dims.n_kv_heads
         dout = _c(dout)
         # the weights are views of a rotating gather buffer: read them now, as gathered for this backward
-        w_qkv = fuse_adjacent([wq, wk, wv])
-        w_gu = fuse_adjacent([wg, wu])
+        w_qkv = fuse_rows([wq, wk, wv])
+        w_gu = fuse_rows([wg, wu])
         # ---- MLP
         pushed: list[tuple[Any, ...]] = []  # push mode: the four weight-gradient GEMMs run as one grouped launch at the end
         da = kernels.gemm(dout, wd.detach(), b_mn_major=True)
         (g_wd,) = _WeightGrad([wd]).run(dout, a, pushed)
         dgu = kernels.swiglu_bwd(gu, da)
         del da
-        dn2 = kernels.gemm(dgu, w_gu, b_mn_major=True)
+        dn2 = _gemm_fused(dgu, w_gu, b_mn_major=True)
         g_wg, g_wu = _WeightGrad([wg, wu]).run(dgu, n2, pushed)
         del dgu
         box: list[torch.Tensor] = []
@@ -260,7 +282,7 @@ class DecoderLayerFn(torch.autograd.Function):
         kernels.attn_bwd(q, k, v, att, datt, lse, dqkv[:, : hq * hd], dqkv[:, hq * hd : (hq + hkv) * hd],
                          dqkv[:, (hq + hkv) * hd :], dims.batch, dims.seq, hq, hkv, 1.0 / math.sqrt(hd), True)
         kernels.rope_(dqkv, cos_sin, dims.seq, 0, hq + hkv, hd, backward=True)
-        dn1 = kernels.gemm(dqkv, w_qkv, b_mn_major=True)
+        dn1 = _gemm_fused(dqkv, w_qkv, b_mn_major=True)
         g_wq, g_wk, g_wv = _WeightGrad([wq, wk, wv]).run(dqkv, n1, pushed)
         g_n1 = _norm_weight_grad(w_n1, lambda dw, z: box.append(kernels.rmsnorm_bwd(x, w_n1.detach(), dn1, rstd1, dw, dres=dh, zero_dw=z)), True)
         dx = box.pop()

@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import math
 from typing import Any
 
 import torch
@@ -114,7 +115,7 @@ def gemm(
     if residual is not None:
         assert out.dtype == torch.bfloat16 and not accumulate and sumsq is None
         assert residual.dtype == torch.bfloat16 and residual.shape == (m, n) and residual.stride(1) == 1
-    nbytes = _gemm_workspace(m, n, k, int(out.dtype == torch.float32), sm_limit, tile, splits, a.device.index)
+    nbytes = _gemm_workspace(m, n, k, int(out.dtype == torch.float32), 0, sm_limit, tile, splits, a.device.index)
     ws = torch.empty(nbytes, device=a.device, dtype=torch.uint8) if nbytes else None
     rc = _native.lib().yf_gemm_bf16_ws(
         a.data_ptr(), b.data_ptr(), out.data_ptr(), _ptr(residual), m, n, k, a.stride(0), b.stride(0), out.stride(0),
@@ -126,13 +127,42 @@ def gemm(
 
 
 @functools.lru_cache(maxsize=4096)
-def _gemm_workspace(m: int, n: int, k: int, out_f32: int, sm_limit: int, tile: int, splits: int, device: int | None) -> int:
+def _gemm_workspace(m: int, n: int, k: int, out_f32: int, n_align: int, sm_limit: int, tile: int, splits: int, device: int | None) -> int:
     """Workspace bytes that a GEMM wants (a function of its shape and the device's number of SMs)."""
     nbytes = ctypes.c_longlong(0)
-    rc = _native.lib().yf_gemm_workspace(m, n, k, out_f32, int(sm_limit), tile, splits, ctypes.byref(nbytes))
+    rc = _native.lib().yf_gemm_workspace(m, n, k, out_f32, n_align, int(sm_limit), tile, splits, ctypes.byref(nbytes))
     if rc != 0:
         raise RuntimeError(f"yf_gemm_workspace failed with code {rc}")
     return nbytes.value
+
+
+def gemm_parts(a: torch.Tensor, parts: "list[torch.Tensor]", *, b_mn_major: bool = False, tile: int = 0, splits: int = 0) -> torch.Tensor:
+    """:func:`gemm` (bf16 output) with ``b`` given as two to four tensors that lie one below the other: ``torch.cat(parts)``
+    without the copy.  Every part but the last has a multiple of 64 rows (:func:`can_be_parts`)."""
+    m, k = a.shape
+    rows = [p.shape[0] for p in parts]
+    cols = parts[0].shape[1]
+    n = cols if b_mn_major else sum(rows)
+    assert k == (sum(rows) if b_mn_major else cols) and a.dtype == torch.bfloat16 and a.stride(1) == 1
+    assert all(p.dtype == torch.bfloat16 and p.is_cuda and p.dim() == 2 and p.shape[1] == cols and p.stride(1) == 1 for p in parts)
+    out = torch.empty((m, n), device=a.device, dtype=torch.bfloat16)
+    align = 0 if b_mn_major else math.gcd(*(sum(rows[:i]) for i in range(1, len(rows))))
+    nbytes = _gemm_workspace(m, n, k, 0, align, 0, tile, splits, a.device.index)
+    ws = torch.empty(nbytes, device=a.device, dtype=torch.uint8) if nbytes else None
+    np_ = len(parts)
+    _check(_native.lib().yf_gemm_bf16_parts(
+        a.data_ptr(), np_, (ctypes.c_void_p * np_)(*[p.data_ptr() for p in parts]), (ctypes.c_int * np_)(*rows),
+        (ctypes.c_longlong * np_)(*[p.stride(0) for p in parts]), out.data_ptr(), m, n, k, a.stride(0), out.stride(0), int(b_mn_major),
+        _ptr(ws), nbytes, tile, splits, _stream()), "yf_gemm_bf16_parts")
+    return out
+
+
+def can_be_parts(ts: "list[torch.Tensor]") -> bool:
+    """Whether :func:`gemm_parts` takes these tensors."""
+    first = ts[0]
+    return 2 <= len(ts) <= 4 and all(
+        t.is_cuda and t.dtype == torch.bfloat16 and t.dim() == 2 and t.is_contiguous() and t.shape[1] == first.shape[1] and t.shape[1] % 8 == 0
+        and t.data_ptr() % 16 == 0 for t in ts) and all(t.shape[0] % 64 == 0 and t.shape[0] > 0 for t in ts)
 
 
 def gemm_gathered(a: torch.Tensor, n: int, k: int, *, peer_in: Any, layer_buf: torch.Tensor, shard_bytes: int, b_byte_off: int,
