@@ -944,11 +944,11 @@ float plan_us(const TileShape& t, int M, int N, int K, int units, int splits, bo
   if (rest > 0 && splits > 1) {
     const float rounds = (float)((rest * splits + units - 1) / units), part = loop / (float)splits;
     us += rounds * (rounds > 1.f && part < 9.f ? 9.f : part);
-    us += full > 0 ? 3.f : 2.f + 4.f * (float)splits;
     us *= 1.1f;
   }
+  const float exchange_us = rest == 0 || splits == 1 ? 0.f : (full > 0 ? 3.f : 2.f + 4.f * (float)splits);
   const float read_us = ((float)M + (float)N) * (float)K * 2.f / 5.2e6f;
-  return t.fixed_us + (us > read_us ? us : read_us + 0.1f * us);
+  return t.fixed_us + exchange_us + (us > read_us ? us + 0.1f * read_us : read_us + 0.1f * us);
 }
 
 // n_align > 0: tiles must end where multiples of n_align columns do (the pieces of B)

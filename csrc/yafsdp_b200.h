@@ -64,6 +64,9 @@ int yf_embedding_bwd(const void* dout, const long long* ids, float* dtable, long
 int yf_adamw(float* p, const float* g, float* m, float* v, void* p_bf16, const float* grad_scale_ptr, long long n,
              float lr, float beta1, float beta2, float eps, float weight_decay, int step, int max_ctas, void* stream);
 int yf_sumsq(const float* g, long long n, float* out, void* stream);
+/* one partial sum of squares per block (n_partials of them); x *= *coef.  Any start that is a multiple of four bytes. */
+int yf_sumsq_partials(const float* g, long long n, float* partials, int n_partials, void* stream);
+int yf_scale(float* x, long long n, const float* coef, void* stream);
 int yf_clip_coef(const float* total_sq, float max_norm, float* coef, float* norm_out, void* stream);
 int yf_cast_f32_to_bf16(const float* src, void* dst, long long n, void* stream);
 int yf_accum_bf16_to_f32(const void* src, float* dst, long long n, float scale, int accumulate, void* stream);

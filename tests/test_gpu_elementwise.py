@@ -158,3 +158,57 @@ def test_sumsq_clip_and_casts():
     assert torch.allclose(back, 1 + 0.5 * dst.float())
     s = kernels.add_bf16(dst, dst)
     assert torch.equal(s, (dst.float() * 2).bfloat16())
+
+
+@pytest.mark.parametrize("n,off", [(1, 0), (2, 3), (7, 1), (4096, 0), (100003, 2), (3_000_001, 1)])
+def test_sumsq_and_scale_of_flat_runs(n, off):
+    """Runs that start anywhere in a flat buffer: neighbours stay untouched; a coefficient of one changes nothing, NaN spreads."""
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(3)
+    flat = torch.randn(n + off + 5, device="cuda")
+    run = flat[off : off + n]
+    want = flat.clone()
+    other = torch.randn(77, device="cuda")[1:]
+    got = kernels.sumsq_runs([run, other])
+    ref = run.double().pow(2).sum() + other.double().pow(2).sum()
+    assert abs(got.item() / ref.item() - 1.0) < 1e-6  # fp32 partial sums of at most a few hundred terms each
+    assert torch.equal(got, kernels.sumsq_runs([run, other]))
+    kernels.scale_(run, torch.ones(1, device="cuda"))
+    assert torch.equal(flat, want)
+    kernels.scale_(run, torch.full((1,), 0.37, device="cuda"))
+    want[off : off + n] *= torch.full((1,), 0.37, device="cuda")
+    assert torch.equal(flat, want)
+    kernels.scale_(run, torch.full((1,), float("nan"), device="cuda"))
+    assert run.isnan().all() and not flat[off + n :].isnan().any() and not flat[:off].isnan().any()
+
+
+@pytest.mark.parametrize("max_norm", [1e-3, 1e9])
+def test_clip_grad_norm_of_adjacent_sharded_gradients(max_norm):
+    """Parameters of odd sizes behind each other in a group's flat gradient, against the norm and scale of each one."""
+    import torch.distributed as dist
+
+    from yafsdp_b200 import fully_shard
+    from yafsdp_b200.optim import clip_grad_norm_
+
+    torch.cuda.set_device(0)
+    created = not dist.is_initialized()
+    if created:
+        dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1)
+    try:
+        torch.manual_seed(4)
+        model = torch.nn.Sequential(torch.nn.Linear(33, 7, device="cuda"), torch.nn.Linear(7, 5, device="cuda"))
+        fully_shard(model[0])
+        fully_shard(model)
+        model(torch.randn(9, 33, device="cuda")).square().sum().backward()
+        grads = [p.grad._local_tensor for p in model.parameters()]
+        before = [g.clone() for g in grads]
+        norm = torch.stack([g.double().norm() for g in before]).norm()
+        got = clip_grad_norm_(model, max_norm)
+        assert abs(got.item() / norm.item() - 1.0) < 1e-6
+        coef = min(1.0, max_norm / (norm.item() + 1e-6))
+        for g, b in zip(grads, before):
+            assert torch.allclose(g, b * coef, rtol=1e-6, atol=0.0)
+    finally:
+        if created:
+            dist.destroy_process_group()

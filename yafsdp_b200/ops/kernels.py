@@ -317,6 +317,24 @@ def sumsq_(g: torch.Tensor, out: torch.Tensor) -> None:
     _check(_native.lib().yf_sumsq(g.data_ptr(), g.numel(), out.data_ptr(), _stream()), "yf_sumsq")
 
 
+def sumsq_runs(runs: "list[torch.Tensor]") -> torch.Tensor:
+    """``sum(g*g)`` over flat fp32 tensors of one device, without atomics (the same inputs give the same bits)."""
+    dev = runs[0].device
+    cap = torch.cuda.get_device_properties(dev).multi_processor_count * 8
+    ctas = [max(1, min(cap, r.numel() // 4096)) for r in runs]
+    partials = torch.empty(sum(ctas), device=dev, dtype=torch.float32)
+    at = 0
+    for r, n in zip(runs, ctas):
+        _check(_native.lib().yf_sumsq_partials(r.data_ptr(), r.numel(), partials.data_ptr() + 4 * at, n, _stream()), "yf_sumsq_partials")
+        at += n
+    return partials.sum()
+
+
+def scale_(x: torch.Tensor, coef: torch.Tensor) -> None:
+    """``x *= coef`` in place: flat fp32, ``coef`` one fp32 value on the same device."""
+    _check(_native.lib().yf_scale(x.data_ptr(), x.numel(), coef.data_ptr(), _stream()), "yf_scale")
+
+
 def clip_coef_(total_sq: torch.Tensor, max_norm: float, coef: torch.Tensor, norm_out: torch.Tensor | None) -> None:
     _check(_native.lib().yf_clip_coef(total_sq.data_ptr(), float(max_norm), coef.data_ptr(), _ptr(norm_out), _stream()), "yf_clip_coef")
 

@@ -262,6 +262,29 @@ class ShardedAdamW:
         self.step_count = int(sd.get("step", self.step_count))
 
 
+def _flat_runs(grads: list[torch.Tensor]) -> list[tuple[Any, torch.Tensor]] | None:
+    """The local pieces of sharded fp32 gradients as few flat tensors: pieces that follow each other in one buffer (the
+    parameters of a group) become one.  ``None`` when some gradient is of another kind: not sharded, not fp32, not contiguous
+    or on another device."""
+    runs: list[tuple[Any, torch.Tensor, int]] = []  # shard group, first piece, elements
+    for g in grads:
+        if not isinstance(g, RaggedShardDTensor):
+            return None
+        t = g._local_tensor
+        if type(t) is not torch.Tensor or t.dtype != torch.float32 or not t.is_contiguous() or t.device != grads[0].device:
+            return None
+        if not t.numel():
+            continue
+        pg = g._spec.group()
+        if runs:
+            last_pg, first, n = runs[-1]
+            if last_pg is pg and t.data_ptr() == first.data_ptr() + 4 * n and t.untyped_storage().data_ptr() == first.untyped_storage().data_ptr():
+                runs[-1] = (pg, first, n + t.numel())
+                continue
+        runs.append((pg, t, t.numel()))
+    return [(pg, torch.as_strided(t, (n,), (1,), t.storage_offset())) for pg, t, n in runs] or None
+
+
 def clip_grad_norm_(parameters: Iterable[torch.Tensor] | nn.Module, max_norm: float, norm_type: float = 2.0) -> torch.Tensor:
     """Global gradient-norm clipping for sharded (and plain) parameters; returns the total norm as a plain tensor.
 
@@ -283,12 +306,23 @@ def clip_grad_norm_(parameters: Iterable[torch.Tensor] | nn.Module, max_norm: fl
     # gradients (replicated or ignored parameters) are whole on every rank and enter once
     plain = torch.zeros((), device=dev, dtype=torch.float32)
     sharded: dict[Any, torch.Tensor] = {}
-    for g in grads:
-        if isinstance(g, RaggedShardDTensor):
-            pg = g._spec.group()
-            sharded[pg] = fold(sharded.get(pg, torch.zeros((), device=dev, dtype=torch.float32)), g._local_tensor)
-        else:
-            plain = fold(plain, g)
+    runs = _flat_runs(grads) if norm_type == 2.0 and dev.type == "cuda" else None
+    if runs is not None:
+        from .ops import kernels
+
+        with torch.cuda.device(dev):
+            for g in grads:  # a rank that holds nothing of a group's gradients takes part in its reduction all the same
+                pg = g._spec.group()  # type: ignore[attr-defined]
+                if pg not in sharded:
+                    mine = [r for p, r in runs if p is pg]
+                    sharded[pg] = kernels.sumsq_runs(mine) if mine else torch.zeros((), device=dev, dtype=torch.float32)
+    else:
+        for g in grads:
+            if isinstance(g, RaggedShardDTensor):
+                pg = g._spec.group()
+                sharded[pg] = fold(sharded.get(pg, torch.zeros((), device=dev, dtype=torch.float32)), g._local_tensor)
+            else:
+                plain = fold(plain, g)
     total = plain
     for pg, part in sharded.items():
         if pg is not None and pg.size() > 1:
@@ -297,6 +331,11 @@ def clip_grad_norm_(parameters: Iterable[torch.Tensor] | nn.Module, max_norm: fl
     if not inf:
         total = total.pow(1.0 / norm_type)
     coef = torch.clamp(max_norm / (total + 1e-6), max=1.0)
+    if runs is not None:
+        with torch.cuda.device(dev):
+            for _, r in runs:
+                kernels.scale_(r, coef)
+        return total
     for g in grads:
         (g._local_tensor if isinstance(g, RaggedShardDTensor) else g).mul_(coef)
     return total
