@@ -70,9 +70,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int jt = blockIdx.x;  // key tile
-  const int hk = blockIdx.y;
-  const int b = blockIdx.z;
+  const int jt = blockIdx.z;  // key tile: the slowest index, so that the tiles with the longest walks start first
+  const int hk = blockIdx.x;
+  const int b = blockIdx.y;
   const int group = args.Hq / args.Hkv;
   const int kv0 = jt * BKV;
   const int nq_tiles = (args.S + BQ - 1) / BQ;
@@ -105,7 +105,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 384;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(kv_full, 2 * TILE);
       tma_load_3d(sK, &tma_k, kv_full, hk * HD, kv0, b);
       tma_load_3d(sK + ATOM, &tma_k, kv_full, hk * HD + 64, kv0, b);
@@ -123,7 +123,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t id_kk = umma_idesc_bf16(128, 128, 0, 0);
       const uint32_t id_mm = umma_idesc_bf16(128, 128, 1, 1);
       const uint32_t id_km = umma_idesc_bf16(128, 128, 0, 1);
@@ -374,7 +374,7 @@ static int attn_bwd_launch(const CUtensorMap& mq, const CUtensorMap& mk, const C
   a.scale = scale;
   a.scale_log2 = scale * 1.4426950408889634f;
   a.causal = causal ? 1 : 0;
-  dim3 grid((S + BKV - 1) / BKV, Hkv, B);
+  dim3 grid(Hkv, B, (S + BKV - 1) / BKV);
   attn_bwd_kernel<<<grid, BWD_THREADS, BWD_SMEM, st>>>(mq, mk, mv, md, mdq, a);
   {
     const long long items = T * (Hq * HD / 8);
