@@ -1,14 +1,22 @@
 // Causal flash-attention backward for head_dim 128 on sm_100a (MHA and GQA).
 //
-// One CTA per (128-key tile, KV head, sequence); it walks the query tiles (and, for GQA, the query
-// heads of the group) that attend to those keys.  Per step five tcgen05 GEMMs:
-//   S  = Q K^T          dP = dO V^T                    (fp32 in TMEM, one query row per TMEM lane)
-//   P  = exp(S*scale - lse),  dS = P * (dP - D) * scale   (softmax warps; bf16 into swizzled smem)
-//   dV += P^T dO        dK += dS^T Q                   (accumulated in TMEM over the whole walk)
-//   dQ_part = dS K      -> staged in shared memory, added to a global fp32 dQ accumulator by TMA reduce-add
-// The P / dS tiles are stored once as [query][key] with the 128-byte swizzle and are read both as a
-// K-major operand (dQ) and as an MN-major operand (dV, dK): the two canonical layouts coincide.
-// D = rowsum(dO * O) comes from a small pre-pass; dQ is converted to bf16 by a post-pass.
+// One CTA per (128-key tile, KV head or part of its query heads, sequence); it walks the 64-row query tiles of its query
+// heads that attend to those keys.  Everything is computed with the keys in the TMEM lanes.  Per step five tcgen05 GEMMs:
+//   S^T = K Q^T         dP^T = V dO^T                  (fp32 in TMEM, one key per lane, one query per column)
+//   P^T = exp(S^T*scale - lse),  dS^T = P^T * (dP^T - D)   (softmax warps; bf16 back into TMEM, dS^T also into shared memory)
+//   dV += P^T dO        dK += dS^T Q                   (A operand from TMEM; accumulated in TMEM over the whole walk)
+//   dQ^T = K^T dS^T     -> TMEM -> shared memory -> added to a global fp32 dQ accumulator by TMA reduce-add
+// Roles:
+//   warps 0-3, 4-7   softmax of the even / odd steps, one thread per key
+//   warps 8-11       dQ^T: out of TMEM, transposed through shared memory, one TMA reduce-add per warp and step
+//   warp 12          TMA producer: K and V once, then Q and dO through a ring of three stages
+//   warp 13          MMA issuer
+//   warp 14          the query rows' statistics for the ring, read one step ahead
+// TMEM (512 columns): dV, dK (128 each) and two sets (even / odd steps) of [S^T | dP^T], 64 columns each: P^T and dS^T
+// (bf16, 32 columns each) replace S^T once it has been read, dQ^T replaces dP^T.  So the softmax of one step runs under
+// the MMAs of its neighbours.  Bound: about 1700 cycles of MMA per step (S^T, dP^T and dQ^T with N = 64 are limited by the
+// 128 bytes per cycle that shared memory delivers: 48 instead of 32 cycles per instruction).
+// D = rowsum(dO * O) comes from a small pre-pass; scale and bf16 of dQ are applied by a post-pass, of dK at the end.
 #include <stdio.h>
 
 #include "common.cuh"
@@ -19,21 +27,30 @@ YF_TU_STATUS()
 namespace {
 
 constexpr int HD = 128;
-constexpr int BQ = 128;
-constexpr int BKV = 128;
-constexpr int ATOM = 16384;
-constexpr int TILE = 2 * ATOM;
-constexpr int BWD_THREADS = 320;  // producer warp, MMA warp, eight softmax / epilogue warps
-constexpr int BWD_SMEM = 1024 + 7 * TILE + 256;  // K, V, Q, dO, P, dS and the dQ staging (two [128 x 32 fp32] blocks)
+constexpr int BQ = 64;    // query rows per step
+constexpr int BKV = 128;  // keys per CTA
+constexpr int ATOM = 16384;        // [128 rows x 64 bf16], 128-byte swizzle
+constexpr int TILE = 2 * ATOM;     // K or V: [128 x 128] bf16
+constexpr int QATOM = 8192;        // [64 rows x 64 bf16]
+constexpr int QTILE = 2 * QATOM;   // Q or dO of a step: [64 x 128] bf16
+constexpr int STAGES = 3;          // ring of Q, dO and statistics
+constexpr int BWD_THREADS = 480;
+constexpr int DS_BYTES = ATOM;     // dS^T of a step: [128 keys x 64 queries] bf16
+constexpr int DQ_BYTES = BQ * HD * 4;
+constexpr int STAT_FLOATS = 2 * BQ;  // per stage: -lse * log2(e), D
+constexpr int BWD_SMEM = 1024 + 2 * TILE + STAGES * 2 * QTILE + 2 * DS_BYTES + DQ_BYTES + STAGES * STAT_FLOATS * 4 + 256;
+static_assert(BWD_SMEM <= 232448, "shared memory of one CTA");
 
 struct BwdArgs {
   const float* lse;    // [B, Hq, S]
   const float* delta;  // [B, Hq, S]
-  float* dq_accum;     // [B*S, Hq*128] fp32, zeroed by the caller
   __nv_bfloat16* dk;   // rows dkv_stride apart, head hk at columns hk*128
   __nv_bfloat16* dv;
+  float* dkv_accum;    // head_parts > 1: fp32 sums [2 (dK without scale, dV)][B*S, Hkv*128], zero at the start; else null
   long long dkv_stride;
   int S, B, Hq, Hkv;
+  int head_group;      // order of the CTAs (head_group_order)
+  int head_parts;      // CTAs that share a key tile of a KV head, each with a part of its query heads
   float scale, scale_log2;
   int causal;
 };
@@ -44,6 +61,26 @@ YF_DEVINL void tma_reduce_add_3d(const CUtensorMap* m, const void* smem_src, int
                "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
                : "memory");
 }
+YF_DEVINL void red_add_v4(float* p, float a, float b, float c, float d) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+// Order of the CTAs: heads are taken in groups, within a group key tile by key tile with the heads fastest, so that all heads'
+// long walks start first.  One group holds all heads unless the dQ accumulator outgrows the L2 and there are heads for three
+// groups; then a group has two CTAs per SM, whose sums stay in the L2 (2 x 4096 tokens x 32 heads: 1235 us in one group,
+// 1036 us in groups of ten heads; 1 x 8192 x 32/8 heads, 1661 us in one group and 1772 us in two, stays whole).
+YF_DEVINL void head_group_order(int cta, int n_pos, int n_heads, int group, int& pos, int& head) {
+  const int per_group = n_pos * group;
+  const int g = cta / per_group;
+  const int r = cta - g * per_group;
+  const int size = min(group, n_heads - g * group);
+  pos = r / size;
+  head = g * group + r - pos * size;
+}
+int head_group_size(int n_pos, int n_heads, long long accum_bytes, int n_sms) {
+  const int group = (2 * n_sms + n_pos - 1) / n_pos;
+  return accum_bytes <= (64ll << 20) || group >= n_heads / 3 ? n_heads : group;
+}
 
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
@@ -53,48 +90,56 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sK = smem;
   uint8_t* sV = sK + TILE;
-  uint8_t* sQ = sV + TILE;
-  uint8_t* sdO = sQ + TILE;
-  uint8_t* sP = sdO + TILE;
-  uint8_t* sdS = sP + TILE;
-  uint8_t* sdQ = sdS + TILE;  // two 16 KB blocks, 128-byte swizzled rows, source of the TMA reduce-adds
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sdQ + TILE);
+  uint8_t* sRing = sV + TILE;                      // stage s: Q at sRing + s * 2 * QTILE, dO at + QTILE
+  uint8_t* sdS = sRing + STAGES * 2 * QTILE;       // even / odd steps
+  uint8_t* sdQ = sdS + 2 * DS_BYTES;               // warp w of the dQ warps: [64 queries x 32 dims] fp32 at w * 8192
+  float* sStat = reinterpret_cast<float*>(sdQ + DQ_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + STAGES * STAT_FLOATS);
   uint64_t* kv_full = bars;
-  uint64_t* qdo_full = bars + 1;
-  uint64_t* qdo_empty = bars + 2;
-  uint64_t* sdp_full = bars + 3;
-  uint64_t* pds_ready = bars + 4;
-  uint64_t* dq_full = bars + 5;
-  uint64_t* dq_read = bars + 6;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7);
+  uint64_t* q_full = bars + 1;              // [STAGES] TMA bytes + the statistics
+  uint64_t* q_empty = q_full + STAGES;      // [STAGES]
+  uint64_t* sdp_full = q_empty + STAGES;    // [2] even / odd steps, as all that follow
+  uint64_t* pds_ready = sdp_full + 2;
+  uint64_t* dq_full = pds_ready + 2;
+  uint64_t* vk_done = dq_full + 2;
+  uint64_t* dq_read = vk_done + 2;
+  uint64_t* all_done = dq_read + 2;         // every MMA of the walk (waiting two phases ahead on vk_done would not do)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(all_done + 1);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int jt = blockIdx.z;  // key tile: the slowest index, so that the tiles with the longest walks start first
-  const int hk = blockIdx.x;
-  const int b = blockIdx.y;
-  const int group = args.Hq / args.Hkv;
+  int jt, bh;  // key tile (under the causal mask the first ones have the longest walks), (sequence, KV head, part)
+  head_group_order((int)blockIdx.x, (args.S + BKV - 1) / BKV, args.B * args.Hkv * args.head_parts, args.head_group, jt, bh);
+  const int part = bh % args.head_parts, hk = (bh / args.head_parts) % args.Hkv, b = bh / (args.head_parts * args.Hkv);
+  const int heads = args.Hq / args.Hkv / args.head_parts;  // query heads of this CTA
+  const int h0 = hk * (args.Hq / args.Hkv) + part * heads;
   const int kv0 = jt * BKV;
-  const int nq_tiles = (args.S + BQ - 1) / BQ;
-  const int i_start = args.causal ? jt : 0;
-  const int per_head = nq_tiles - i_start;
-  const int n_it = per_head * group;
+  const int i_start = args.causal ? kv0 / BQ : 0;          // first query tile
+  const int per_head = (args.S + BQ - 1) / BQ - i_start;   // at least one: the tile that holds these keys' own rows
+  const int n_it = per_head * heads;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tma_q);
     tma_prefetch_desc(&tma_k);
     tma_prefetch_desc(&tma_v);
     tma_prefetch_desc(&tma_do);
+    tma_prefetch_desc(&tma_dq);
     mbar_init(kv_full, 1);
-    mbar_init(qdo_full, 1);
-    mbar_init(qdo_empty, 1);
-    mbar_init(sdp_full, 1);
-    mbar_init(pds_ready, 256);
-    mbar_init(dq_full, 1);
-    mbar_init(dq_read, 256);
+    mbar_init(all_done, 1);
+    for (int i = 0; i < STAGES; ++i) {
+      mbar_init(&q_full[i], 2);
+      mbar_init(&q_empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&sdp_full[i], 1);
+      mbar_init(&pds_ready[i], 4);
+      mbar_init(&dq_full[i], 1);
+      mbar_init(&vk_done[i], 1);
+      mbar_init(&dq_read[i], 4);
+    }
     mbar_fence_init();
   }
-  if (warp == 1) {
+  if (warp == 13) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
@@ -102,183 +147,267 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 384;
+  const uint32_t tdV = tmem_base + 256, tdK = tmem_base + 384;  // set p of S^T | dP^T: tmem_base + 128 p, + 64
 
-  if (warp == 0) {
+  if (warp == 12) {
     if (elect_one()) {
       mbar_expect_tx(kv_full, 2 * TILE);
       tma_load_3d(sK, &tma_k, kv_full, hk * HD, kv0, b);
       tma_load_3d(sK + ATOM, &tma_k, kv_full, hk * HD + 64, kv0, b);
       tma_load_3d(sV, &tma_v, kv_full, hk * HD, kv0, b);
       tma_load_3d(sV + ATOM, &tma_v, kv_full, hk * HD + 64, kv0, b);
-      for (int it = 0; it < n_it; ++it) {
-        const int h = hk * group + it / per_head;
-        const int q0 = (i_start + it % per_head) * BQ;
-        if (!mbar_wait(qdo_empty, (it & 1) ^ 1, 200)) break;
-        mbar_expect_tx(qdo_full, 2 * TILE);
-        tma_load_3d(sQ, &tma_q, qdo_full, h * HD, q0, b);
-        tma_load_3d(sQ + ATOM, &tma_q, qdo_full, h * HD + 64, q0, b);
-        tma_load_3d(sdO, &tma_do, qdo_full, h * HD, q0, b);
-        tma_load_3d(sdO + ATOM, &tma_do, qdo_full, h * HD + 64, q0, b);
+      int h = h0, i = 0;
+      for (int it = 0, st = 0, ph = 1; it < n_it; ++it) {
+        if (!mbar_wait(&q_empty[st], ph, 200)) break;
+        const int q0 = (i_start + i) * BQ;
+        uint8_t* sQ = sRing + st * 2 * QTILE;
+        uint8_t* sdO = sQ + QTILE;
+        mbar_expect_tx(&q_full[st], 2 * QTILE);
+        tma_load_3d(sQ, &tma_q, &q_full[st], h * HD, q0, b);
+        tma_load_3d(sQ + QATOM, &tma_q, &q_full[st], h * HD + 64, q0, b);
+        tma_load_3d(sdO, &tma_do, &q_full[st], h * HD, q0, b);
+        tma_load_3d(sdO + QATOM, &tma_do, &q_full[st], h * HD + 64, q0, b);
+        if (++i == per_head) { i = 0; ++h; }
+        if (++st == STAGES) { st = 0; ph ^= 1; }
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == 14) {
+    // statistics of a step's 64 query rows, read one step ahead; rows past the end of the sequence: a probability of zero
+    int h = h0, i = 0;
+    float nl[2], dl[2];
+    auto fetch = [&]() {
+      const int q0 = (i_start + i) * BQ;
+      const long long at = ((long long)b * args.Hq + h) * args.S + q0;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = lane + 32 * e;
+        const bool ok = q0 + r < args.S;
+        nl[e] = ok ? args.lse[at + r] * -1.4426950408889634f : -INFINITY;
+        dl[e] = ok ? args.delta[at + r] : 0.f;
+      }
+    };
+    fetch();
+    for (int it = 0, st = 0, ph = 1; it < n_it; ++it) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&q_empty[st], ph, 201))) break;
+      float* stat = sStat + st * STAT_FLOATS;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        stat[lane + 32 * e] = nl[e];
+        stat[BQ + lane + 32 * e] = dl[e];
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&q_full[st]);
+      if (++i == per_head) { i = 0; ++h; }
+      if (it + 1 < n_it) fetch();
+      if (++st == STAGES) { st = 0; ph ^= 1; }
+    }
+  } else if (warp == 13) {
     if (elect_one()) {
-      const uint32_t id_kk = umma_idesc_bf16(128, 128, 0, 0);
-      const uint32_t id_mm = umma_idesc_bf16(128, 128, 1, 1);
-      const uint32_t id_km = umma_idesc_bf16(128, 128, 0, 1);
-      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ = smem_u32(sQ), adO = smem_u32(sdO), aP = smem_u32(sP),
-                     adS = smem_u32(sdS);
-      bool alive = mbar_wait(kv_full, 0, 210);
+      const uint32_t id_s = umma_idesc_bf16(128, BQ, 0, 0);    // S^T, dP^T: both operands K-major (K = head dim)
+      const uint32_t id_g = umma_idesc_bf16(128, HD, 0, 1);    // dV, dK: A from TMEM (K = queries), dO / Q MN-major
+      const uint32_t id_q = umma_idesc_bf16(128, BQ, 1, 1);    // dQ^T: K tile MN-major (M = head dim), dS^T MN-major
+      const uint64_t kK = umma_smem_desc_sw128(smem_u32(sK), 0, 1024), kV = umma_smem_desc_sw128(smem_u32(sV), 0, 1024);
+      const uint64_t mK = umma_smem_desc_sw128(smem_u32(sK), ATOM, 1024);
+      const uint64_t kQ = umma_smem_desc_sw128(smem_u32(sRing), 0, 1024), mQ = umma_smem_desc_sw128(smem_u32(sRing), QATOM, 1024);
+      const uint64_t mS = umma_smem_desc_sw128(smem_u32(sdS), ATOM, 1024);
+      // descriptor addresses advance in units of 16 bytes
+      int st_s = 0, ph_s = 0;  // ring position of the next S^T, dP^T
+      // S^T and dP^T of step `it` into their set: S^T once dV and dK of step it - 2 have read P^T and dS^T there, dP^T once
+      // the dQ warps have read dQ^T
+      auto issue_sdp = [&](int it) -> bool {
+        const int p = it & 1, par = ((it >> 1) & 1) ^ 1;  // parity of step it - 2
+        if (!mbar_wait(&q_full[st_s], ph_s, 211)) return false;
+        if (it >= 2 && !mbar_wait(&vk_done[p], par, 212)) return false;
+        tc_fence_after();
+        const uint64_t q = kQ + st_s * (2 * QTILE >> 4);
+        const uint32_t t = tmem_base + p * 128;
+#pragma unroll
+        for (int e = 0; e < HD / 16; ++e)
+          tc_mma_bf16(t, kK + (((e >> 2) * ATOM + (e & 3) * 32) >> 4), q + (((e >> 2) * QATOM + (e & 3) * 32) >> 4), id_s, e != 0);
+        if (it >= 2 && !mbar_wait(&dq_read[p], par, 213)) return false;
+        tc_fence_after();
+#pragma unroll
+        for (int e = 0; e < HD / 16; ++e)
+          tc_mma_bf16(t + 64, kV + (((e >> 2) * ATOM + (e & 3) * 32) >> 4), q + ((QTILE + (e >> 2) * QATOM + (e & 3) * 32) >> 4), id_s,
+                      e != 0);
+        tc_commit(&sdp_full[p]);
+        if (++st_s == STAGES) { st_s = 0; ph_s ^= 1; }
+        return true;
+      };
+      bool alive = mbar_wait(kv_full, 0, 210) && issue_sdp(0) && (n_it < 2 || issue_sdp(1));
+      int st = 0;
       for (int it = 0; it < n_it && alive; ++it) {
-        if (!mbar_wait(qdo_full, it & 1, 211)) { alive = false; break; }
-        if (it > 0 && !mbar_wait(dq_read, (it - 1) & 1, 212)) { alive = false; break; }
+        const int p = it & 1;
+        if (!mbar_wait(&pds_ready[p], (it >> 1) & 1, 214)) break;
         tc_fence_after();
+        const uint32_t t = tmem_base + p * 128;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {  // S = Q K^T
-          const uint32_t off = (k >> 2) * ATOM + (k & 3) * 32;
-          tc_mma_bf16(tS, umma_smem_desc_sw128(aQ + off, 0, 1024), umma_smem_desc_sw128(aK + off, 0, 1024), id_kk, k != 0);
-        }
+        for (int e = 0; e < BKV / 16; ++e)  // dQ^T first: the dQ warps fetch it under dV and dK
+          tc_mma_bf16(t + 64, mK + e * (2048 >> 4), mS + ((p * DS_BYTES + e * 2048) >> 4), id_q, e != 0);
+        tc_commit(&dq_full[p]);
+        const uint64_t q = mQ + st * (2 * QTILE >> 4);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {  // dP = dO V^T
-          const uint32_t off = (k >> 2) * ATOM + (k & 3) * 32;
-          tc_mma_bf16(tdP, umma_smem_desc_sw128(adO + off, 0, 1024), umma_smem_desc_sw128(aV + off, 0, 1024), id_kk, k != 0);
-        }
-        tc_commit(sdp_full);
-        if (!mbar_wait(pds_ready, it & 1, 213)) { alive = false; break; }
-        tc_fence_after();
+        for (int e = 0; e < BQ / 16; ++e)  // 16 queries: 8 TMEM columns of P^T, 16 rows of dO
+          tc_mma_bf16_ts(tdV, t + e * 8, q + ((QTILE + e * 2048) >> 4), id_g, (it | e) != 0);
 #pragma unroll
-        for (int k = 0; k < 8; ++k)  // dV += P^T dO   (A = P read MN-major, B = dO MN-major; K = query rows)
-          tc_mma_bf16(tdV, umma_smem_desc_sw128(aP + k * 2048, ATOM, 1024), umma_smem_desc_sw128(adO + k * 2048, ATOM, 1024),
-                      id_mm, (it | k) != 0);
-#pragma unroll
-        for (int k = 0; k < 8; ++k)  // dK += dS^T Q
-          tc_mma_bf16(tdK, umma_smem_desc_sw128(adS + k * 2048, ATOM, 1024), umma_smem_desc_sw128(aQ + k * 2048, ATOM, 1024),
-                      id_mm, (it | k) != 0);
-#pragma unroll
-        for (int k = 0; k < 8; ++k)  // dQ_part = dS K   (A = dS K-major over keys, B = K tile MN-major)
-          tc_mma_bf16(tS, umma_smem_desc_sw128(adS + (k >> 2) * ATOM + (k & 3) * 32, 0, 1024),
-                      umma_smem_desc_sw128(aK + k * 2048, ATOM, 1024), id_km, k != 0);
-        tc_commit(dq_full);
-        tc_commit(qdo_empty);
+        for (int e = 0; e < BQ / 16; ++e)
+          tc_mma_bf16_ts(tdK, t + 32 + e * 8, q + (e * 2048 >> 4), id_g, (it | e) != 0);
+        tc_commit(&vk_done[p]);
+        tc_commit(&q_empty[st]);
+        if (++st == STAGES) st = 0;
+        if (it + 2 < n_it) alive = issue_sdp(it + 2);
+        if (it + 1 == n_it) tc_commit(all_done);
       }
     }
-  } else {
-    // eight warps: warp w owns TMEM lanes [32*(w%4), +32) (one query row per thread) and, of the four 32-column
-    // chunks of every tile, the two of its half ((w-2)/4): two threads share a row and split its columns
-    const int q = warp & 3;
-    const int row = q * 32 + lane;
-    const int c_begin = ((warp - 2) >> 2) * 2, c_end = c_begin + 2;
-    const uint32_t lane_off = (uint32_t)(q * 32) << 16;
+  } else if (warp < 8) {
+    const int p = warp >> 2;                  // even or odd steps
+    const int row = (warp & 3) * 32 + lane;   // key inside the tile == TMEM lane
+    const uint32_t t = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + p * 128;
+    const int key = kv0 + row;
     const float sl2 = args.scale_log2;
+    uint8_t* ds_row = sdS + p * DS_BYTES + row * 128;
     bool alive = true;
-    for (int it = 0; it < n_it && alive; ++it) {
-      const int h = hk * group + it / per_head;
-      const int q0 = (i_start + it % per_head) * BQ;
-      const int qrow = q0 + row;
-      const bool row_ok = qrow < args.S;
-      const long long stat_idx = ((long long)b * args.Hq + h) * args.S + qrow;
-      const float lse2 = row_ok ? args.lse[stat_idx] * 1.4426950408889634f : 0.f;
-      const float delta = row_ok ? args.delta[stat_idx] : 0.f;
-      // keys this query row may see: col <= limit
-      const int limit = row_ok ? (args.causal ? min(qrow, args.S - 1) : args.S - 1) : -1;
-      const bool need_mask = kv0 + BKV - 1 > limit;
-      if (!mbar_wait(sdp_full, it & 1, 220)) { alive = false; break; }
+    int st = p, ph = 0, i = p % per_head;     // ring stage and its parity, query tile of step p
+    for (int it = p; it < n_it; it += 2) {
+      const int q0 = (i_start + i) * BQ;
+      // a bounded wait that runs out ends the warp's work (the lanes decide together: TMEM accesses are warp-wide)
+      if (!__all_sync(0xffffffffu, mbar_wait(&q_full[st], ph, 220) && mbar_wait(&sdp_full[p], (it >> 1) & 1, 221))) { alive = false; break; }
       tc_fence_after();
-#pragma unroll 1
-      for (int c = c_begin; c < c_end; ++c) {
-        uint32_t rs[32], rp[32];
-        tmem_ld32(tS + lane_off + c * 32, rs);
-        tmem_ld32(tdP + lane_off + c * 32, rp);
-        tmem_ld_wait();
-        uint32_t pk[16], dk[16];
+      const float4* stat = reinterpret_cast<const float4*>(sStat + st * STAT_FLOATS);
+      uint32_t s[2][32];
+      tmem_ld32(t, s[0]);
+      tmem_ld32(t + 32, s[1]);
+      tmem_ld_wait();
 #pragma unroll
-        for (int t = 0; t < 32; t += 2) {
-          float p0 = fast_exp2(fmaf(__uint_as_float(rs[t]), sl2, -lse2));
-          float p1 = fast_exp2(fmaf(__uint_as_float(rs[t + 1]), sl2, -lse2));
-          if (need_mask) {  // only the tiles on the diagonal and the last one have masked keys
-            if (kv0 + c * 32 + t > limit) p0 = 0.f;
-            if (kv0 + c * 32 + t + 1 > limit) p1 = 0.f;
-          }
-          const float d0 = p0 * (__uint_as_float(rp[t]) - delta) * args.scale;
-          const float d1 = p1 * (__uint_as_float(rp[t + 1]) - delta) * args.scale;
-          pk[t >> 1] = pack_bf16x2(p0, p1);
-          dk[t >> 1] = pack_bf16x2(d0, d1);
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+          const float4 nl = stat[c * 8 + v];
+          s[c][4 * v + 0] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[c][4 * v + 0]), sl2, nl.x)));
+          s[c][4 * v + 1] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[c][4 * v + 1]), sl2, nl.y)));
+          s[c][4 * v + 2] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[c][4 * v + 2]), sl2, nl.z)));
+          s[c][4 * v + 3] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[c][4 * v + 3]), sl2, nl.w)));
         }
-        const int tile_off = (c >> 1) * ATOM + row * 128;
+      // queries [0, hidden) of the tile do not see this key: those in front of it, all when the key is past the end
+      const int hidden = key >= args.S ? BQ : (args.causal ? key - q0 : 0);
+      if (__any_sync(0xffffffffu, hidden > 0)) {
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const int chunk = (((c & 1) * 4 + t) ^ (row & 7)) << 4;
-          *reinterpret_cast<uint4*>(sP + tile_off + chunk) = make_uint4(pk[4 * t], pk[4 * t + 1], pk[4 * t + 2], pk[4 * t + 3]);
-          *reinterpret_cast<uint4*>(sdS + tile_off + chunk) = make_uint4(dk[4 * t], dk[4 * t + 1], dk[4 * t + 2], dk[4 * t + 3]);
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (c * 32 + e < hidden) s[c][e] = 0u;
+      }
+      {
+        uint32_t pk[32];
+#pragma unroll
+        for (int e = 0; e < 32; ++e)
+          pk[e] = pack_bf16x2(__uint_as_float(s[e >> 4][(2 * e) & 31]), __uint_as_float(s[e >> 4][(2 * e + 1) & 31]));
+        tmem_st32(t, pk);  // P^T over S^T, whose row is in registers
+      }
+      uint32_t dk[32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t dp[16];
+        tmem_ld16(t + 64 + c * 16, dp);
+        tmem_ld_wait();
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const float4 dl = stat[BQ / 4 + c * 4 + v];
+          const uint32_t* ps = &s[c >> 1][(c & 1) * 16 + 4 * v];
+          dk[c * 8 + 2 * v] = pack_bf16x2(__uint_as_float(ps[0]) * (__uint_as_float(dp[4 * v + 0]) - dl.x),
+                                          __uint_as_float(ps[1]) * (__uint_as_float(dp[4 * v + 1]) - dl.y));
+          dk[c * 8 + 2 * v + 1] = pack_bf16x2(__uint_as_float(ps[2]) * (__uint_as_float(dp[4 * v + 2]) - dl.z),
+                                              __uint_as_float(ps[3]) * (__uint_as_float(dp[4 * v + 3]) - dl.w));
         }
       }
+      tmem_st32(t + 32, dk);
+#pragma unroll
+      for (int v = 0; v < 8; ++v)
+        *reinterpret_cast<uint4*>(ds_row + ((v ^ (row & 7)) << 4)) = make_uint4(dk[4 * v], dk[4 * v + 1], dk[4 * v + 2], dk[4 * v + 3]);
+      tmem_st_wait();
       fence_proxy_async_smem();
       tc_fence_before();
-      mbar_arrive(pds_ready);
-      if (!mbar_wait(dq_full, it & 1, 221)) { alive = false; break; }
-      tc_fence_after();
-      // dQ_part: TMEM -> registers -> swizzled staging block -> one TMA reduce-add per [128 rows x 32 columns] block (full
-      // 128-byte lines reach the L2 reduction units; rows past the end of the sequence are clipped by the tensor map).
-      // The two column halves of the tile use one staging block each; two passes cover the four 32-column chunks.
-      const bool dq_thread = (threadIdx.x == 64 || threadIdx.x == 64 + 128);  // first thread of each half
-#pragma unroll 1
-      for (int pass = 0; pass < 2; ++pass) {
-        const int c = c_begin + pass;
-        uint8_t* blk = sdQ + (c_begin >> 1) * ATOM;  // half 0 -> block 0, half 1 -> block 1
-        uint32_t r[32];
-        tmem_ld32(tS + lane_off + c * 32, r);
-        tmem_ld_wait();
-        if (dq_thread) tma_store_wait_read0();  // the reduce that last read this block has finished reading
-        named_bar_sync(2 + (c_begin >> 1), 128);
-        uint8_t* srow = blk + row * 128;
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          *reinterpret_cast<uint4*>(srow + ((j ^ (row & 7)) << 4)) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-        fence_proxy_async_smem();
-        named_bar_sync(2 + (c_begin >> 1), 128);
-        if (dq_thread) {
-          tma_reduce_add_3d(&tma_dq, blk, h * HD + c * 32, q0, b);
-          tma_store_commit();
-        }
-      }
-      tc_fence_before();
-      mbar_arrive(dq_read);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&pds_ready[p]);
+      i += 2;
+      while (i >= per_head) i -= per_head;
+      st += 2;
+      if (st >= STAGES) { st -= STAGES; ph ^= 1; }
     }
-    if (threadIdx.x == 64 || threadIdx.x == 64 + 128) tma_store_wait0();  // this thread's dQ reduce-adds have completed
-    // dK, dV: TMEM lane == key row.  The last dq_full wait covers every MMA issued before it.
-    if (alive) {  // every lane issues the (warp-collective) TMEM loads; only the stores are predicated
-      const bool key_ok = kv0 + row < args.S;
-      const long long off = ((long long)b * args.S + kv0 + row) * args.dkv_stride + hk * HD;
+    // the results: the even steps' warps write dV, the odd steps' warps dK (TMEM lane == key)
+    if (alive && __all_sync(0xffffffffu, mbar_wait(all_done, 0, 222))) {
+      tc_fence_after();
+      const uint32_t src = (p == 0 ? tdV : tdK) + ((uint32_t)((warp & 3) * 32) << 16);
+      const float f = p == 0 ? 1.f : args.scale;
+      const long long token = (long long)b * args.S + key;
 #pragma unroll 1
-      for (int which = 0; which < 2; ++which) {
-        __nv_bfloat16* dst = (which == 0 ? args.dv : args.dk) + off;
-        const uint32_t tsrc = (which == 0 ? tdV : tdK) + lane_off;
-#pragma unroll 1
-        for (int c = c_begin; c < c_end; ++c) {
-          uint32_t r[32];
-          tmem_ld32(tsrc + c * 32, r);
-          tmem_ld_wait();
-          if (key_ok) {
+      for (int c = 0; c < 4; ++c) {
+        uint32_t r[32];
+        tmem_ld32(src + c * 32, r);
+        tmem_ld_wait();
+        if (key < args.S) {
+          if (args.dkv_accum != nullptr) {
+            float* dst = args.dkv_accum + ((p == 0 ? (long long)args.B * args.S : 0ll) + token) * args.Hkv * HD + hk * HD + c * 32;
+#pragma unroll
+            for (int v = 0; v < 8; ++v)
+              red_add_v4(dst + 4 * v, __uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]), __uint_as_float(r[4 * v + 2]),
+                         __uint_as_float(r[4 * v + 3]));
+          } else {
+            uint4* dst = reinterpret_cast<uint4*>((p == 0 ? args.dv : args.dk) + token * args.dkv_stride + hk * HD + c * 32);
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
               uint4 w;
-              w.x = pack_bf16x2(__uint_as_float(r[8 * v + 0]), __uint_as_float(r[8 * v + 1]));
-              w.y = pack_bf16x2(__uint_as_float(r[8 * v + 2]), __uint_as_float(r[8 * v + 3]));
-              w.z = pack_bf16x2(__uint_as_float(r[8 * v + 4]), __uint_as_float(r[8 * v + 5]));
-              w.w = pack_bf16x2(__uint_as_float(r[8 * v + 6]), __uint_as_float(r[8 * v + 7]));
-              reinterpret_cast<uint4*>(dst + c * 32)[v] = w;
+              w.x = pack_bf16x2(__uint_as_float(r[8 * v + 0]) * f, __uint_as_float(r[8 * v + 1]) * f);
+              w.y = pack_bf16x2(__uint_as_float(r[8 * v + 2]) * f, __uint_as_float(r[8 * v + 3]) * f);
+              w.z = pack_bf16x2(__uint_as_float(r[8 * v + 4]) * f, __uint_as_float(r[8 * v + 5]) * f);
+              w.w = pack_bf16x2(__uint_as_float(r[8 * v + 6]) * f, __uint_as_float(r[8 * v + 7]) * f);
+              dst[v] = w;
             }
           }
         }
       }
     }
     tc_fence_before();
+  } else if (warp < 12) {
+    const int w = warp & 3;                   // head dims [32 w, +32) == TMEM lanes
+    float* stg = reinterpret_cast<float*>(sdQ) + w * (BQ * 32);
+    int h = h0, i = 0;
+    for (int it = 0; it < n_it; ++it) {
+      const int p = it & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(&dq_full[p], (it >> 1) & 1, 230))) break;
+      tc_fence_after();
+      const uint32_t t = tmem_base + ((uint32_t)(w * 32) << 16) + p * 128 + 64;
+      uint32_t r[2][32];
+      tmem_ld32(t, r[0]);
+      tmem_ld32(t + 32, r[1]);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&dq_read[p]);
+        tma_store_wait_read0();  // the reduce of the step before has finished reading the block
+      }
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int e = 0; e < 32; ++e) stg[(c * 32 + e) * 32 + lane] = __uint_as_float(r[c][e]);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        // rows past the end of the sequence are clipped by the tensor map
+        tma_reduce_add_3d(&tma_dq, stg, h * HD + w * 32, (i_start + i) * BQ, b);
+        tma_store_commit();
+      }
+      if (++i == per_head) { i = 0; ++h; }
+    }
+    if (lane == 0) tma_store_wait0();  // this warp's reduce-adds have completed
+    tc_fence_before();
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 13) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
@@ -286,9 +415,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
 
 // delta[b,h,s] = sum_d dO * O, and the fp32 dQ accumulator of the same (token, head) cleared on the way (the main kernel
 // adds into it): sixteen lanes per (token, head), one 16-byte load of O and of dO and two 16-byte stores of zeros per lane.
+// The dK / dV accumulators of shared key tiles, where there are any, are cleared too.
 __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                                         float* __restrict__ delta, float* __restrict__ dq_zero, int B, int S, int Hq,
+                                                         float* __restrict__ delta, float* __restrict__ dq_zero, float4* __restrict__ dkv_zero,
+                                                         long long n_dkv_zero, int B, int S, int Hq,
                                                          long long o_stride, long long do_stride) {
+  if (dkv_zero != nullptr)
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n_dkv_zero; i += (long long)gridDim.x * blockDim.x)
+      dkv_zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   const long long total = (long long)B * S * Hq;
   const int sub = threadIdx.x & 15;
   const unsigned half_mask = 0xffffu << (threadIdx.x & 16);  // the two halves of a warp may leave the loop at different times
@@ -315,30 +449,55 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
   }
 }
 
-// dq (bf16, strided rows) = dq_accum (fp32, dense rows of `width`)
-__global__ void attn_dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long long T, int width,
-                                       long long dq_stride) {
-  const int vpr = width / 8;
+// dq (bf16, strided rows) = scale * dq_accum (fp32, dense rows of wq); with dkv_acc also dk = scale * its first half and
+// dv = its second half (dense rows of wkv)
+__global__ void attn_convert_kernel(const float* __restrict__ dq_acc, const float* __restrict__ dkv_acc, __nv_bfloat16* __restrict__ dq,
+                                    __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, long long T, int wq, int wkv,
+                                    long long dq_stride, long long dkv_stride, float scale) {
+  const int vpr = (wq + (dkv_acc != nullptr ? 2 * wkv : 0)) / 8;
   const long long total = T * vpr;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long t = i / vpr;
-    const int v = (int)(i % vpr);
-    const float4 a = reinterpret_cast<const float4*>(acc + t * width)[2 * v];
-    const float4 c = reinterpret_cast<const float4*>(acc + t * width)[2 * v + 1];
+    const int v = (int)(i - t * vpr) * 8;
+    const float* src = dq_acc + t * wq + v;
+    __nv_bfloat16* dst = dq + t * dq_stride + v;
+    float f = scale;
+    if (v >= wq) {
+      const int u = v - wq, is_v = u >= wkv ? 1 : 0, col = u - is_v * wkv;
+      src = dkv_acc + (is_v * T + t) * wkv + col;
+      dst = (is_v ? dv : dk) + t * dkv_stride + col;
+      if (is_v) f = 1.f;
+    }
+    const float4 a = reinterpret_cast<const float4*>(src)[0];
+    const float4 c = reinterpret_cast<const float4*>(src)[1];
     uint4 w;
-    w.x = pack_bf16x2(a.x, a.y);
-    w.y = pack_bf16x2(a.z, a.w);
-    w.z = pack_bf16x2(c.x, c.y);
-    w.w = pack_bf16x2(c.z, c.w);
-    *reinterpret_cast<uint4*>(dq + t * dq_stride + v * 8) = w;
+    w.x = pack_bf16x2(a.x * f, a.y * f);
+    w.y = pack_bf16x2(a.z * f, a.w * f);
+    w.z = pack_bf16x2(c.x * f, c.y * f);
+    w.w = pack_bf16x2(c.z * f, c.w * f);
+    *reinterpret_cast<uint4*>(dst) = w;
   }
+}
+
+// CTAs per key tile of a KV head.  With grouped-query attention a KV head's key tiles are few and their walks long (every
+// query head of the group): the walk is cut by query heads until there are three CTAs per SM to balance, at the price of
+// fp32 atomic sums of dK and dV.  Measured: see the figures at the top of the launch.
+int head_parts_for(int B, int S, int Hq, int Hkv) {
+  const int group = Hq / Hkv;
+  const long long tiles = (long long)((S + BKV - 1) / BKV) * Hkv * B;
+  int parts = 1;
+  while (parts < group && tiles * parts < 3ll * yf_num_sms()) {
+    ++parts;
+    while (group % parts) ++parts;
+  }
+  return parts;
 }
 
 }  // namespace
 
 // The three launches of one backward pass (delta pre-pass, main kernel, dQ conversion), shared by both entry points.
 // Allocates nothing: the tensor maps come by reference from the caller, the scratch by pointer.
-static int attn_bwd_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& md,
+static int attn_bwd_launch(int head_parts, float* dkv_accum, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& md,
                            const CUtensorMap& mdq, const void* out,
                            const void* dout, const float* lse, float* delta, float* dq_accum, void* dq, void* dk, void* dv, int B,
                            int S, int Hq, int Hkv, long long o_stride, long long do_stride, long long dq_stride,
@@ -360,13 +519,15 @@ static int attn_bwd_launch(const CUtensorMap& mq, const CUtensorMap& mk, const C
     const long long cap = (long long)yf_num_sms() * 8;
     if (blocks > cap) blocks = cap;
     attn_delta_kernel<<<(int)blocks, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(out),
-                                                  reinterpret_cast<const __nv_bfloat16*>(dout), delta, dq_accum, B, S, Hq, o_stride,
+                                                  reinterpret_cast<const __nv_bfloat16*>(dout), delta, dq_accum,
+                                                  reinterpret_cast<float4*>(dkv_accum), dkv_accum ? 2 * T * Hkv * (HD / 4) : 0, B, S, Hq, o_stride,
                                                   do_stride);
   }
   BwdArgs a;
   a.lse = lse;
   a.delta = delta;
-  a.dq_accum = dq_accum;
+  a.dkv_accum = dkv_accum;
+  a.head_parts = head_parts;
   a.dk = reinterpret_cast<__nv_bfloat16*>(dk);
   a.dv = reinterpret_cast<__nv_bfloat16*>(dv);
   a.dkv_stride = dkv_stride;
@@ -374,14 +535,19 @@ static int attn_bwd_launch(const CUtensorMap& mq, const CUtensorMap& mk, const C
   a.scale = scale;
   a.scale_log2 = scale * 1.4426950408889634f;
   a.causal = causal ? 1 : 0;
-  dim3 grid(Hkv, B, (S + BKV - 1) / BKV);
+  const int n_kt = (S + BKV - 1) / BKV;
+  a.head_group = head_group_size(n_kt, B * Hkv * head_parts, T * Hq * HD * 4, yf_num_sms());  // the dQ accumulator
+  const long long ctas = (long long)n_kt * B * Hkv * head_parts;
+  if (ctas > 0x7fffffffll) return -1;
+  const int grid = (int)ctas;
   attn_bwd_kernel<<<grid, BWD_THREADS, BWD_SMEM, st>>>(mq, mk, mv, md, mdq, a);
   {
-    const long long items = T * (Hq * HD / 8);
+    const long long items = T * ((Hq + (dkv_accum ? 2 * Hkv : 0)) * HD / 8);
     long long blocks = (items + 255) / 256;
     const long long cap = (long long)yf_num_sms() * 8;
     if (blocks > cap) blocks = cap;
-    attn_dq_convert_kernel<<<(int)blocks, 256, 0, st>>>(dq_accum, reinterpret_cast<__nv_bfloat16*>(dq), T, Hq * HD, dq_stride);
+    attn_convert_kernel<<<(int)blocks, 256, 0, st>>>(dq_accum, dkv_accum, reinterpret_cast<__nv_bfloat16*>(dq), a.dk, a.dv, T, Hq * HD, Hkv * HD, dq_stride, dkv_stride,
+                                                     scale);
   }
   return -(int)cudaGetLastError();
 }
@@ -390,25 +556,40 @@ static int attn_bwd_launch(const CUtensorMap& mq, const CUtensorMap& mk, const C
 // o_stride apart); lse from the forward.  Scratch supplied by the caller: delta [B,Hq,S] fp32 and
 // dq_accum [B*S, Hq*128] fp32 (zeroed here).  Results: dq (rows dq_stride apart), dk/dv (rows
 // dkv_stride apart), all bf16; they may be column blocks of one fused d(QKV) buffer.
-extern "C" int yf_attn_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout, const float* lse,
-                           float* delta, float* dq_accum, void* dq, void* dk, void* dv, int B, int S, int Hq, int Hkv,
-                           long long q_stride, long long kv_stride, long long o_stride, long long do_stride,
-                           long long dq_stride, long long dkv_stride, float scale, int causal, void* stream) {
+// The general form: `dkv_accum` ([2][B*S, Hkv*128] fp32 scratch, cleared here) lets `head_parts` CTAs (a divisor of Hq / Hkv) share
+// a key tile of a KV head; yf_attn_bwd_head_parts says how many a problem wants.  head_parts == 1 needs no dkv_accum.
+extern "C" int yf_attn_bwd_head_parts(int B, int S, int Hq, int Hkv) {
   if (B <= 0 || S <= 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv)) return -1;
+  return head_parts_for(B, S, Hq, Hkv);
+}
+extern "C" int yf_attn_bwd_parts(const void* q, const void* k, const void* v, const void* out, const void* dout, const float* lse,
+                                 float* delta, float* dq_accum, float* dkv_accum, int head_parts, void* dq, void* dk, void* dv, int B,
+                                 int S, int Hq, int Hkv, long long q_stride, long long kv_stride, long long o_stride,
+                                 long long do_stride, long long dq_stride, long long dkv_stride, float scale, int causal, void* stream) {
+  if (B <= 0 || S <= 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv)) return -1;
+  if (head_parts < 1 || (Hq / Hkv) % head_parts || (head_parts > 1) != (dkv_accum != nullptr)) return -1;
   if ((q_stride % 8) || (kv_stride % 8) || (o_stride % 8) || (do_stride % 8) || (dq_stride % 8) || (dkv_stride % 8)) return -1;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
        reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(dq) |
-       reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv) | reinterpret_cast<uintptr_t>(dq_accum)) & 15)
+       reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv) | reinterpret_cast<uintptr_t>(dq_accum) |
+       reinterpret_cast<uintptr_t>(dkv_accum)) & 15)
     return -1;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const CUtensorMap* mq = yf_tensor_map_3d(q, (uint64_t)Hq * HD, S, B, q_stride, (uint64_t)S * q_stride, 64, BQ, 1, 2, 1);
   const CUtensorMap* mk = yf_tensor_map_3d(k, (uint64_t)Hkv * HD, S, B, kv_stride, (uint64_t)S * kv_stride, 64, BKV, 1, 2, 1);
   const CUtensorMap* mv = yf_tensor_map_3d(v, (uint64_t)Hkv * HD, S, B, kv_stride, (uint64_t)S * kv_stride, 64, BKV, 1, 2, 1);
   const CUtensorMap* md = yf_tensor_map_3d(dout, (uint64_t)Hq * HD, S, B, do_stride, (uint64_t)S * do_stride, 64, BQ, 1, 2, 1);
-  const CUtensorMap* mdq = yf_tensor_map_3d(dq_accum, (uint64_t)Hq * HD, S, B, (uint64_t)Hq * HD, (uint64_t)S * Hq * HD, 32, BQ, 1, 4, 1);
+  const CUtensorMap* mdq = yf_tensor_map_3d(dq_accum, (uint64_t)Hq * HD, S, B, (uint64_t)Hq * HD, (uint64_t)S * Hq * HD, 32, BQ, 1, 4, 0);
   if (!mq || !mk || !mv || !md || !mdq) return -2;
-  return attn_bwd_launch(*mq, *mk, *mv, *md, *mdq, out, dout, lse, delta, dq_accum, dq, dk, dv, B, S, Hq, Hkv, o_stride, do_stride, dq_stride,
-                         dkv_stride, scale, causal, st);
+  return attn_bwd_launch(head_parts, dkv_accum, *mq, *mk, *mv, *md, *mdq, out, dout, lse, delta, dq_accum, dq, dk, dv, B, S, Hq, Hkv,
+                         o_stride, do_stride, dq_stride, dkv_stride, scale, causal, st);
+}
+extern "C" int yf_attn_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout, const float* lse,
+                           float* delta, float* dq_accum, void* dq, void* dk, void* dv, int B, int S, int Hq, int Hkv,
+                           long long q_stride, long long kv_stride, long long o_stride, long long do_stride,
+                           long long dq_stride, long long dkv_stride, float scale, int causal, void* stream) {
+  return yf_attn_bwd_parts(q, k, v, out, dout, lse, delta, dq_accum, nullptr, 1, dq, dk, dv, B, S, Hq, Hkv, q_stride, kv_stride, o_stride,
+                           do_stride, dq_stride, dkv_stride, scale, causal, stream);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -488,8 +669,8 @@ extern "C" int yf_attn_bwd_noalloc(const void* q, const void* k, const void* v, 
       yf_tensor_map_3d_encode(&mk, k, (uint64_t)Hkv * HD, S, B, kv_stride, (uint64_t)S * kv_stride, 64, BKV, 1, 2, 1) != 0 ||
       yf_tensor_map_3d_encode(&mv, v, (uint64_t)Hkv * HD, S, B, kv_stride, (uint64_t)S * kv_stride, 64, BKV, 1, 2, 1) != 0 ||
       yf_tensor_map_3d_encode(&md, dout, (uint64_t)Hq * HD, S, B, do_stride, (uint64_t)S * do_stride, 64, BQ, 1, 2, 1) != 0 ||
-      yf_tensor_map_3d_encode(&mdq, dq_accum, (uint64_t)Hq * HD, S, B, (uint64_t)Hq * HD, (uint64_t)S * Hq * HD, 32, BQ, 1, 4, 1) != 0)
+      yf_tensor_map_3d_encode(&mdq, dq_accum, (uint64_t)Hq * HD, S, B, (uint64_t)Hq * HD, (uint64_t)S * Hq * HD, 32, BQ, 1, 4, 0) != 0)
     return -2;
-  return attn_bwd_launch(mq, mk, mv, md, mdq, out, dout, lse, delta, dq_accum, dq, dk, dv, B, S, Hq, Hkv, o_stride, do_stride, dq_stride,
+  return attn_bwd_launch(1, nullptr, mq, mk, mv, md, mdq, out, dout, lse, delta, dq_accum, dq, dk, dv, B, S, Hq, Hkv, o_stride, do_stride, dq_stride,
                          dkv_stride, scale, causal, st);
 }

@@ -85,3 +85,33 @@ def test_attention_forward_with_growing_scores():
     att = torch.einsum("bqhd,bkhd->bhqk", q.float().view(b, s, hq, d), k.float().view(b, s, hkv, d).repeat_interleave(hq // hkv, dim=2)) / math.sqrt(d)
     att = att.masked_fill(~torch.ones(s, s, device="cuda", dtype=torch.bool).tril(), float("-inf"))
     assert torch.allclose(lse, att.logsumexp(-1), atol=2e-2, rtol=1e-3)
+
+
+@pytest.mark.parametrize("b,s,hq,hkv", [(1, 300, 8, 2), (2, 129, 4, 1), (1, 64, 6, 1), (3, 45, 8, 8)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_attention_bwd_shared_key_tiles(b, s, hq, hkv, causal):
+    """The query heads of a KV head dealt to one or several CTAs: the same gradients but for the order of fp32 sums, which may
+    move a bf16 result by one rounding (2^-8 of it)."""
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(5)
+    t, d = b * s, 128
+    qkv = torch.randn(t, (hq + 2 * hkv) * d, device="cuda").bfloat16()
+    q, k, v = qkv[:, : hq * d], qkv[:, hq * d : (hq + hkv) * d], qkv[:, (hq + hkv) * d :]
+    scale = 1.0 / math.sqrt(d)
+    out, lse = kernels.attn_fwd(q, k, v, b, s, hq, hkv, scale, causal)
+    dout = torch.randn_like(out)
+    got = []
+    for parts in [p for p in range(1, hq // hkv + 1) if (hq // hkv) % p == 0]:
+        g = torch.full_like(qkv, float("nan"))
+        kernels.attn_bwd(q, k, v, out, dout, lse, g[:, : hq * d], g[:, hq * d : (hq + hkv) * d], g[:, (hq + hkv) * d :], b, s, hq, hkv,
+                         scale, causal, head_parts=parts)
+        got.append(g)
+    torch.cuda.synchronize()
+    kernels.check_status()
+    for g in got[1:]:
+        assert torch.allclose(g.float(), got[0].float(), rtol=2.0**-7, atol=1e-5)
+    qf, kf, vf = (x.double().view(b, s, -1, d).requires_grad_(True) for x in (q, k, v))
+    _ref(qf, kf, vf, causal).backward(dout.double().view(b, s, hq, d))
+    want = torch.cat([x.grad.reshape(t, -1) for x in (qf, kf, vf)], dim=1)
+    assert ((got[0].double() - want).norm() / want.norm()).item() < 2.0**-7  # P, dS and the results are rounded to bf16
