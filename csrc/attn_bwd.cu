@@ -13,7 +13,7 @@
 //   warp 13          MMA issuer
 //   warp 14          the query rows' statistics for the ring, read one step ahead
 // TMEM (512 columns): dV, dK (128 each) and two sets (even / odd steps) of [S^T | dP^T], 64 columns each: P^T and dS^T
-// (bf16, 32 columns each) replace S^T once it has been read, dQ^T replaces dP^T.  So the softmax of one step runs under
+// (bf16, 16 + 16 columns per 32 queries) replace S^T once it has been read, dQ^T replaces dP^T.  So the softmax of one step runs under
 // the MMAs of its neighbours.  Bound: about 1700 cycles of MMA per step (S^T, dP^T and dQ^T with N = 64 are limited by the
 // 128 bytes per cycle that shared memory delivers: 48 instead of 32 cycles per instruction).
 // D = rowsum(dO * O) comes from a small pre-pass; scale and bf16 of dQ are applied by a post-pass, of dK at the end.
@@ -248,10 +248,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         const uint64_t q = mQ + st * (2 * QTILE >> 4);
 #pragma unroll
         for (int e = 0; e < BQ / 16; ++e)  // 16 queries: 8 TMEM columns of P^T, 16 rows of dO
-          tc_mma_bf16_ts(tdV, t + e * 8, q + ((QTILE + e * 2048) >> 4), id_g, (it | e) != 0);
+          tc_mma_bf16_ts(tdV, t + (e >> 1) * 32 + (e & 1) * 8, q + ((QTILE + e * 2048) >> 4), id_g, (it | e) != 0);
 #pragma unroll
         for (int e = 0; e < BQ / 16; ++e)
-          tc_mma_bf16_ts(tdK, t + 32 + e * 8, q + (e * 2048 >> 4), id_g, (it | e) != 0);
+          tc_mma_bf16_ts(tdK, t + (e >> 1) * 32 + 16 + (e & 1) * 8, q + (e * 2048 >> 4), id_g, (it | e) != 0);
         tc_commit(&vk_done[p]);
         tc_commit(&q_empty[st]);
         if (++st == STAGES) st = 0;
@@ -274,56 +274,38 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       if (!__all_sync(0xffffffffu, mbar_wait(&q_full[st], ph, 220) && mbar_wait(&sdp_full[p], (it >> 1) & 1, 221))) { alive = false; break; }
       tc_fence_after();
       const float4* stat = reinterpret_cast<const float4*>(sStat + st * STAT_FLOATS);
-      uint32_t s[2][32];
-      tmem_ld32(t, s[0]);
-      tmem_ld32(t + 32, s[1]);
-      tmem_ld_wait();
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int v = 0; v < 8; ++v) {
-          const float4 nl = stat[c * 8 + v];
-          s[c][4 * v + 0] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[c][4 * v + 0]), sl2, nl.x)));
-          s[c][4 * v + 1] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[c][4 * v + 1]), sl2, nl.y)));
-          s[c][4 * v + 2] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[c][4 * v + 2]), sl2, nl.z)));
-          s[c][4 * v + 3] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[c][4 * v + 3]), sl2, nl.w)));
-        }
       // queries [0, hidden) of the tile do not see this key: those in front of it, all when the key is past the end
       const int hidden = key >= args.S ? BQ : (args.causal ? key - q0 : 0);
-      if (__any_sync(0xffffffffu, hidden > 0)) {
+      const bool any_hidden = __any_sync(0xffffffffu, hidden > 0);
+      // 32 queries at a time: everything stays in registers (a spill goes to the L2: shared memory leaves no L1)
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (c * 32 + e < hidden) s[c][e] = 0u;
-      }
-      {
-        uint32_t pk[32];
-#pragma unroll
-        for (int e = 0; e < 32; ++e)
-          pk[e] = pack_bf16x2(__uint_as_float(s[e >> 4][(2 * e) & 31]), __uint_as_float(s[e >> 4][(2 * e + 1) & 31]));
-        tmem_st32(t, pk);  // P^T over S^T, whose row is in registers
-      }
-      uint32_t dk[32];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t dp[16];
-        tmem_ld16(t + 64 + c * 16, dp);
+      for (int c = 0; c < 2; ++c) {
+        uint32_t s[32], dp[32], pk[16], dk[16];
+        tmem_ld32(t + c * 32, s);
+        tmem_ld32(t + 64 + c * 32, dp);
         tmem_ld_wait();
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const float4 dl = stat[BQ / 4 + c * 4 + v];
-          const uint32_t* ps = &s[c >> 1][(c & 1) * 16 + 4 * v];
-          dk[c * 8 + 2 * v] = pack_bf16x2(__uint_as_float(ps[0]) * (__uint_as_float(dp[4 * v + 0]) - dl.x),
-                                          __uint_as_float(ps[1]) * (__uint_as_float(dp[4 * v + 1]) - dl.y));
-          dk[c * 8 + 2 * v + 1] = pack_bf16x2(__uint_as_float(ps[2]) * (__uint_as_float(dp[4 * v + 2]) - dl.z),
-                                              __uint_as_float(ps[3]) * (__uint_as_float(dp[4 * v + 3]) - dl.w));
-        }
-      }
-      tmem_st32(t + 32, dk);
+        for (int v = 0; v < 8; ++v) {
+          const float4 nl = stat[c * 8 + v], dl = stat[BQ / 4 + c * 8 + v];
+          float x[4] = {fast_exp2(fmaf(__uint_as_float(s[4 * v + 0]), sl2, nl.x)), fast_exp2(fmaf(__uint_as_float(s[4 * v + 1]), sl2, nl.y)),
+                        fast_exp2(fmaf(__uint_as_float(s[4 * v + 2]), sl2, nl.z)), fast_exp2(fmaf(__uint_as_float(s[4 * v + 3]), sl2, nl.w))};
+          if (any_hidden) {
 #pragma unroll
-      for (int v = 0; v < 8; ++v)
-        *reinterpret_cast<uint4*>(ds_row + ((v ^ (row & 7)) << 4)) = make_uint4(dk[4 * v], dk[4 * v + 1], dk[4 * v + 2], dk[4 * v + 3]);
+            for (int e = 0; e < 4; ++e)
+              if (c * 32 + 4 * v + e < hidden) x[e] = 0.f;
+          }
+          pk[2 * v] = pack_bf16x2(x[0], x[1]);
+          pk[2 * v + 1] = pack_bf16x2(x[2], x[3]);
+          dk[2 * v] = pack_bf16x2(x[0] * (__uint_as_float(dp[4 * v + 0]) - dl.x), x[1] * (__uint_as_float(dp[4 * v + 1]) - dl.y));
+          dk[2 * v + 1] = pack_bf16x2(x[2] * (__uint_as_float(dp[4 * v + 2]) - dl.z), x[3] * (__uint_as_float(dp[4 * v + 3]) - dl.w));
+        }
+        // over the half of S^T that has been read: P^T, then dS^T
+        tmem_st16(t + c * 32, pk);
+        tmem_st16(t + c * 32 + 16, dk);
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          *reinterpret_cast<uint4*>(ds_row + (((c * 4 + v) ^ (row & 7)) << 4)) = make_uint4(dk[4 * v], dk[4 * v + 1], dk[4 * v + 2], dk[4 * v + 3]);
+      }
       tmem_st_wait();
       fence_proxy_async_smem();
       tc_fence_before();
