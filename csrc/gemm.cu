@@ -32,8 +32,9 @@ constexpr int WIDE_THREADS = 224;  // one more warp: plain mode's second TMA pro
 // MODE_PLAIN: C is stored locally through TMA; MODE_SPLIT: so too, and the last wave's tiles are split along K (an
 // instantiation of its own: the exchange's code alone costs the plain kernel 0.3 us per tile).  MODE_SCATTER: GEMM -> reduce-scatter, the fp32 rows of C are pushed to the
 // ranks that own them.  MODE_GATHER: all-gather -> GEMM, the kernel also gathers the layer that B is part of (see FusedArgs).
-constexpr int MODE_PLAIN = 0, MODE_SCATTER = 1, MODE_GATHER = 2, MODE_SPLIT = 3;
-__host__ __device__ constexpr bool is_plain(int mode) { return mode == MODE_PLAIN || mode == MODE_SPLIT; }
+// MODE_SWIGLU: the gate and up projections of an MLP with their activation (see GemmArgs).
+constexpr int MODE_PLAIN = 0, MODE_SCATTER = 1, MODE_GATHER = 2, MODE_SPLIT = 3, MODE_SWIGLU = 4;
+__host__ __device__ constexpr bool is_plain(int mode) { return mode != MODE_SCATTER && mode != MODE_GATHER; }
 constexpr int SCATTER_COLS = 64;                         // columns per pushed row piece: 256 bytes of fp32
 constexpr int SCATTER_PITCH = SCATTER_COLS * 4 + 16;     // row pitch of the staging block (16 B of padding: no bank conflicts)
 
@@ -63,11 +64,16 @@ struct GemmArgs {
   int M, N, K;
   long long ldc;
   float alpha;
+  const float* alpha_ptr;  // optional: one fp32 on the device that alpha is multiplied by
   int a_mn, b_mn, out_f32, accumulate;
   // optional bf16 residual [M, N] with row pitch ldr, added in fp32 before the bf16 output is rounded (bf16 output, plain
   // mode): a block's "x + proj(...)" costs no pass of its own over the activations
   const void* R;
   long long ldr;
+  // MODE_SWIGLU: B is two matrices of N / 2 rows, gate (maps.b[0]) and up (maps.b[1]); a tile is 128 columns of each, and the
+  // epilogue writes silu(gate) * up, of the values as rounded to bf16, through maps.a[1] and, with store_gu, gate and up into
+  // the halves of C.
+  int store_gu;
   // B in several pieces of memory (plain and split mode): parts[i] is where piece i ends, in rows of [N, K] storage (then no
   // tile crosses a piece's end) or of [K, N] storage (no K block does).  n_parts <= 1: one piece.
   int n_parts;
@@ -97,6 +103,9 @@ struct GemmArgs {
   int own_start[MAX_RANKS + 1];
   int steps;   // world * (largest number of tiles of one owner)
 };
+
+// the factor of A * B^T, possibly with a device scalar in it
+YF_DEVINL float alpha_of(const GemmArgs& args) { return args.alpha_ptr != nullptr ? args.alpha * __ldg(args.alpha_ptr) : args.alpha; }
 
 // one piece of work of a unit: K blocks [kb0, kb1) of a tile; part < 0: all of them
 struct WorkItem {
@@ -410,7 +419,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
           }
           if (!alive) break;
         }
-        const int nb = n0 + (int)crank * B_ROWS - (args.b_mn ? 0 : b_at);  // first B row this CTA holds
+        int nb = n0 + (int)crank * B_ROWS - (args.b_mn ? 0 : b_at);  // first B row this CTA holds
+        if (MODE == MODE_SWIGLU) {  // a pair: its leader holds gate rows, the other CTA the same rows of up
+          nb = n0 / 2;
+          tma_b = &maps.b[crank];
+        }
         const bool k_parts = is_plain(MODE) && args.n_parts > 1 && args.b_mn;
         int piece = 0;
         int kb = w.kb0 + skip;
@@ -559,7 +572,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
       }
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BLOCK_N;
-      const float alpha = args.alpha;
+      const float alpha = alpha_of(args);
       if constexpr (MODE == MODE_SCATTER) {
         // GEMM -> reduce-scatter.  Every thread owns one row of the accumulator: it moves 64 columns at a time from its
         // TMEM lane into its own row of a staging block and sends that 256-byte piece with one bulk store (two where the
@@ -726,6 +739,53 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
         }
         tmem_st_wait();
       }
+      if constexpr (MODE == MODE_SWIGLU) {
+        // 64 columns of one output: 32 packed pairs of this thread's row -> this warp's staging block -> TMA store
+        auto store64 = [&](const CUtensorMap* map, int x, const uint32_t (&v)[32]) {  // (F is a multiple of a tile's 128)
+          uint8_t* stg = staging + q * 8192 + (chunk_ctr & 1) * 4096;
+          ++chunk_ctr;
+          if (lane == 0) tma_store_wait_read1();
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<uint4*>(stg + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            const int y = m0 + q * 32;
+            if (y < M) tma_store_2d(map, stg, x, y);
+            tma_store_commit();
+          }
+        };
+        auto load64 = [&](int col, uint32_t (&v)[32]) {  // 64 accumulator columns of this thread's row, rounded to bf16
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            uint32_t r[32];
+            tmem_ld32(taddr + col + half * 32, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[half * 16 + j] = pack_bf16x2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+          }
+        };
+        const int F = N / 2;
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+          const int x = n0 / 2 + c * 64;
+          uint32_t g[32], u[32];
+          load64(c * 64, g);
+          if (args.store_gu) store64(&tma_c, x, g);
+          load64(128 + c * 64, u);
+          if (c == 1) free_accumulator();
+          if (args.store_gu) store64(&tma_c, F + x, u);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const float2 gf = unpack_bf16x2(g[j]), uf = unpack_bf16x2(u[j]);
+            g[j] = pack_bf16x2(gf.x / (1.f + __expf(-gf.x)) * uf.x, gf.y / (1.f + __expf(-gf.y)) * uf.y);
+          }
+          store64(&maps.a[1], x, g);
+        }
+        continue;
+      }
 #pragma unroll 1
       for (int c = 0; c < n_chunks; ++c, ++chunk_ctr) {
         uint8_t* stg = staging + q * 8192 + (chunk_ctr & 1) * 4096;
@@ -845,11 +905,18 @@ int launch_gemm(const Operands* ops, int n_ops, GemmArgs args, const FusedArgs& 
     maps.a[i] = *ma;
     maps.b[i] = *mb;
   }
+  if (MODE == MODE_SWIGLU) {  // the activation's store map
+    const CUtensorMap* mact = yf_tensor_map_2d(args.R, args.N / 2, args.M, args.ldr, 64, 32, 2, 1);
+    if (!mact) return -2;
+    maps.a[1] = *mact;
+    n_ops = 2;
+  }
   for (int i = n_ops; i < MAX_GROUP; ++i) {  // unused entries hold a valid descriptor all the same
     maps.a[i] = maps.a[0];
     maps.b[i] = maps.b[0];
   }
-  const CUtensorMap* mc = yf_tensor_map_2d(args.C, args.N, args.M, args.ldc, args.out_f32 ? 32 : 64, 32, args.out_f32 ? 4 : 2, 1);
+  const int c_cols = MODE == MODE_SWIGLU && !args.store_gu ? args.N / 2 : args.N;
+  const CUtensorMap* mc = yf_tensor_map_2d(args.C, c_cols, args.M, args.ldc, args.out_f32 ? 32 : 64, 32, args.out_f32 ? 4 : 2, 1);
   if (!mc) return -2;
   static bool optin[64] = {};
   if (int rc = ensure_smem_optin(gemm_bf16_tcgen05_kernel<BLOCK_N, CG, MODE>, Cfg::SMEM_BYTES, optin)) return rc;
@@ -1136,7 +1203,7 @@ extern "C" int yf_gemm_workspace(int M, int N, int K, int out_f32, int n_align, 
 }
 extern "C" int yf_gemm_bf16_ws(const void* A, const void* B, void* C, const void* R, int M, int N, int K, long long lda, long long ldb,
                                long long ldc, long long ldr, int a_mn, int b_mn, int out_f32, int accumulate, float alpha, int sm_limit,
-                               float* sumsq, void* workspace, long long workspace_bytes, int tile, int splits, void* stream) {
+                               const float* alpha_ptr, float* sumsq, void* workspace, long long workspace_bytes, int tile, int splits, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0 || tile < 0 || tile > 5 || splits < 0 || splits > MAX_SPLITS) return -1;
   if (sumsq != nullptr && (!out_f32 || accumulate)) return -1;
   if ((lda % 8) || (ldb % 8) || (ldc % (out_f32 ? 4 : 8))) return -1;
@@ -1152,6 +1219,7 @@ extern "C" int yf_gemm_bf16_ws(const void* A, const void* B, void* C, const void
   args.b_mn = b_mn ? 1 : 0;
   args.out_f32 = out_f32 ? 1 : 0;
   args.accumulate = accumulate ? 1 : 0;
+  args.alpha_ptr = alpha_ptr;
   args.R = R;
   args.ldr = ldr;
   FusedArgs fa;
@@ -1188,6 +1256,50 @@ extern "C" int yf_gemm_bf16_parts(const void* A, int n, const void* const* B, co
   FusedArgs fa;
   memset(&fa, 0, sizeof(fa));
   return launch_plain(ops, n, args, fa, 0, workspace, workspace_bytes, tile, splits, reinterpret_cast<cudaStream_t>(stream));
+}
+
+// act[M,F] = silu(X Wg^T) * (X Wu^T) with Wg, Wu [F,K] (row pitches ldg, ldu); gu [M,2F] (may be null: not wanted) receives both
+// products.  F a multiple of 128.
+extern "C" int yf_gemm_swiglu(const void* X, const void* Wg, const void* Wu, void* gu, void* act, int M, int F, int K, long long ldx,
+                              long long ldg, long long ldu, long long ldgu, long long ldact, void* stream) {
+  if (M <= 0 || F <= 0 || K <= 0 || (F % 128) || (ldx % 8) || (ldg % 8) || (ldu % 8) || (ldact % 8) || (gu && (ldgu % 8))) return -1;
+  if ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Wg) | reinterpret_cast<uintptr_t>(Wu) | reinterpret_cast<uintptr_t>(gu) |
+       reinterpret_cast<uintptr_t>(act)) & 15)
+    return -1;
+  GemmArgs args;
+  memset(&args, 0, sizeof(args));
+  args.C = gu ? gu : act;  // without gu only a store map that nothing uses
+  args.M = M; args.N = 2 * F; args.K = K;
+  args.ldc = gu ? ldgu : ldact;
+  args.alpha = 1.f;
+  args.R = act;
+  args.ldr = ldact;
+  args.store_gu = gu != nullptr;
+  FusedArgs fa;
+  memset(&fa, 0, sizeof(fa));
+  const Operands ops[2] = {{X, Wg, ldx, ldg, M, F, K}, {X, Wu, ldx, ldu, M, F, K}};
+  return launch_gemm<256, 2, MODE_SWIGLU>(ops, 2, args, fa, 0, reinterpret_cast<cudaStream_t>(stream));
+}
+// Whether that is estimated to be faster than the best plain GEMM and a separate activation kernel (6 bytes per element of act
+// at 4 TB/s, 3 us): the epilogue of a tile takes some 15 us (exponentials, divisions and three stores in four warps), which
+// the next tile's main loop hides, but not the last one's and not where K is short.  Measured, F 11008, K 4096 (GEMM +
+// activation / fused, us): 2048 tokens 239 + 33 / 251, 8192 tokens 922 + 166 / 973, 1337 tokens 198 + 21 / 196; 300 tokens 65 + 6 /
+// 127, 512 x 1408 x 512 7 + 3 / 26: those stay separate.
+extern "C" int yf_gemm_swiglu_pays(int M, int F, int K) {
+  if (M <= 0 || F <= 0 || K <= 0) return -1;
+  if (F % 128) return 0;
+  const int sms = yf_num_sms(), num_k = (K + BLOCK_K - 1) / BLOCK_K;
+  float best = 1e30f;
+  for (int t = 1; t <= 5; ++t)
+    for (int sp = 1; sp <= MAX_SPLITS && (sp == 1 || num_k >= 4 * sp); ++sp) {
+      const float us = plan_us(TILE_SHAPES[t], M, 2 * F, K, sms / TILE_SHAPES[t].cg, sp, false);
+      if (us < best) best = us;
+    }
+  const TileShape& t = TILE_SHAPES[TILE_PAIR256];
+  const long long tiles = (long long)((M + 255) / 256) * (F / 128), units = sms / 2;
+  const float loop = (float)num_k * t.kb_us;
+  const float fused = t.fixed_us + 10.f + (float)((tiles + units - 1) / units) * (loop > 15.f ? loop : 15.f);
+  return fused <= best + 3.f + (float)M * (float)F * 6.f / 4e6f ? 1 : 0;
 }
 
 // All-gather -> GEMM in one kernel.  C[M,N] = A[M,K] * B[N,K]^T where B (row-major, contiguous, K-major) is a

@@ -29,7 +29,11 @@ int yf_gemm_bf16_residual(const void* A, const void* B, void* C, const void* R, 
 int yf_gemm_workspace(int M, int N, int K, int out_f32, int n_align, int sm_limit, int tile, int splits, long long* bytes);
 int yf_gemm_bf16_ws(const void* A, const void* B, void* C, const void* R, int M, int N, int K, long long lda, long long ldb,
                     long long ldc, long long ldr, int a_mn, int b_mn, int out_f32, int accumulate, float alpha, int sm_limit,
-                    float* sumsq, void* workspace, long long workspace_bytes, int tile, int splits, void* stream);
+                    const float* alpha_ptr, float* sumsq, void* workspace, long long workspace_bytes, int tile, int splits, void* stream);
+/* SwiGLU as the epilogue of the gate / up GEMM, and whether that pays (see gemm.cu) */
+int yf_gemm_swiglu(const void* X, const void* Wg, const void* Wu, void* gu, void* act, int M, int F, int K, long long ldx, long long ldg,
+                   long long ldu, long long ldgu, long long ldact, void* stream);
+int yf_gemm_swiglu_pays(int M, int F, int K);
 /* bf16 C = A * B^T with B in n (2 to 4) pieces of memory, one below the other (see gemm.cu) */
 int yf_gemm_bf16_parts(const void* A, int n, const void* const* B, const int* rows, const long long* ldb, void* C, int M, int N, int K,
                        long long lda, long long ldc, int b_mn, void* workspace, long long workspace_bytes, int tile, int splits, void* stream);

@@ -157,3 +157,39 @@ def test_gemm_weight_in_pieces(rows, tile, splits, b_mn):
     torch.cuda.synchronize()
     kernels.check_status()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("t,f,k", [(1, 128, 64), (200, 384, 136), (300, 1408, 512), (777, 256, 1032), (2048, 1408, 512)])
+@pytest.mark.parametrize("keep", [True, False])
+def test_gemm_swiglu_epilogue(t, f, k, keep):
+    """Gate, up and their activation from one kernel, against the separate kernels (same rounding points) and fp64 (results
+    rounded to bf16: 2^-8)."""
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(9)
+    x = torch.randn(t, k, device="cuda").bfloat16()
+    wg, wu = (torch.randn(f, k, device="cuda").bfloat16() * k**-0.5 for _ in range(2))
+    gu, a = kernels.gemm_swiglu(x, wg, wu, keep_gu=keep)
+    want_gu = torch.cat([x.double() @ wg.double().t(), x.double() @ wu.double().t()], dim=1)
+    if keep:
+        assert ((gu.double() - want_gu).norm() / want_gu.norm()).item() < 2.0**-8
+        assert torch.equal(a, kernels.swiglu_fwd(gu))
+    else:
+        assert gu is None
+        gu = torch.cat([kernels.gemm(x, wg), kernels.gemm(x, wu)], dim=1)
+        want = kernels.swiglu_fwd(gu).double()
+        assert ((a.double() - want).norm() / want.norm()).item() < 2.0**-8
+    torch.cuda.synchronize()
+    kernels.check_status()
+
+
+def test_gemm_alpha_from_device():
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(10)
+    a, b = torch.randn(300, 1032, device="cuda").bfloat16(), torch.randn(520, 1032, device="cuda").bfloat16()
+    alpha = torch.tensor(0.37, device="cuda")
+    for splits in (1, 3):
+        got = kernels.gemm(a, b, out_dtype=torch.float32, alpha=2.0, alpha_tensor=alpha, tile=3, splits=splits)
+        want = kernels.gemm(a, b, out_dtype=torch.float32, tile=3, splits=splits) * (2.0 * alpha)
+        assert torch.allclose(got, want, rtol=2.0**-22, atol=0.0)

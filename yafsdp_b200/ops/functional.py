@@ -97,11 +97,14 @@ class _WeightGrad:
         self.sinks = [_sink(p) for p in params]
         self.use_sinks = all(s is not None for s in self.sinks)
 
-    def run(self, dy: torch.Tensor, x: torch.Tensor, deferred: "list[tuple[Any, ...]] | None" = None) -> list[torch.Tensor | None]:
-        """dW = dy^T x for the fused weight; returns per-parameter gradients (None when sunk).  ``deferred``: in push mode
-        the GEMM is not launched but recorded there, for one grouped launch at the end of the layer's backward
-        (:func:`flush_pushed`)."""
+    def run(self, dy: torch.Tensor, x: torch.Tensor, deferred: "list[tuple[Any, ...]] | None" = None,
+            scale: torch.Tensor | None = None) -> list[torch.Tensor | None]:
+        """dW = dy^T x (times ``scale``, one fp32 value on the device) for the fused weight; returns per-parameter gradients
+        (None when sunk).  ``deferred``: in push mode the GEMM is not launched but recorded there, for one grouped launch at
+        the end of the layer's backward (:func:`flush_pushed`)."""
         if self.use_sinks and all(s.pushes() for s in self.sinks):
+            if scale is not None:
+                x = x * scale.to(x.dtype)
             # fused GEMM -> reduce-scatter: parameters that follow each other in the flat gradient are one GEMM
             i, r0 = 0, 0
             while i < len(self.sinks):
@@ -123,14 +126,15 @@ class _WeightGrad:
             fused = fuse_adjacent(list(views)) if len(views) > 1 else views[0]
             targets = [s.norm_target(acc) for s, acc in zip(self.sinks, accs)]
             if len(views) == 1 or (fused.data_ptr() == views[0].data_ptr() and len(set(accs)) == 1):
-                kernels.gemm(dy, x, a_mn_major=True, b_mn_major=True, out=fused, accumulate=accs[0], sumsq=targets[0])
+                kernels.gemm(dy, x, a_mn_major=True, b_mn_major=True, out=fused, accumulate=accs[0], sumsq=targets[0], alpha_tensor=scale)
             else:
                 r0 = 0
                 for v, acc, tgt in zip(views, accs, targets):
-                    kernels.gemm(dy[:, r0 : r0 + v.shape[0]], x, a_mn_major=True, b_mn_major=True, out=v, accumulate=acc, sumsq=tgt)
+                    kernels.gemm(dy[:, r0 : r0 + v.shape[0]], x, a_mn_major=True, b_mn_major=True, out=v, accumulate=acc, sumsq=tgt,
+                                 alpha_tensor=scale)
                     r0 += v.shape[0]
             return [None] * len(self.params)
-        dw = kernels.gemm(dy, x, a_mn_major=True, b_mn_major=True)
+        dw = kernels.gemm(dy, x, a_mn_major=True, b_mn_major=True, alpha_tensor=scale)
         out: list[torch.Tensor | None] = []
         r0 = 0
         for p in self.params:
@@ -223,11 +227,11 @@ class DecoderLayerFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx: Any, x: torch.Tensor, w_n1: torch.Tensor, wq: torch.Tensor, wk: torch.Tensor, wv: torch.Tensor,  # type: ignore[override]
                 wo: torch.Tensor, w_n2: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, wd: torch.Tensor,
-                cos_sin: torch.Tensor, dims: LayerDims) -> torch.Tensor:
+                cos_sin: torch.Tensor, dims: LayerDims, keep: bool = True) -> torch.Tensor:
+        """``keep``: the values that the backward pass reads are wanted."""
         x = _c(x)
         hd, hq, hkv = dims.head_dim, dims.n_heads, dims.n_kv_heads
         w_qkv = fuse_rows([wq, wk, wv])
-        w_gu = fuse_rows([wg, wu])
         n1, rstd1 = kernels.rmsnorm_fwd(x, w_n1.detach(), dims.eps)
         owner = getattr(wq, "_yf_group_index", None)
         ticket = owner[0].take_in_kernel_gather(owner[1], wq.shape[0] + wk.shape[0] + wv.shape[0]) if owner is not None else None
@@ -244,10 +248,15 @@ class DecoderLayerFn(torch.autograd.Function):
         att, lse = kernels.attn_fwd(q, k, v, dims.batch, dims.seq, hq, hkv, 1.0 / math.sqrt(hd), True)
         h = kernels.gemm(att, wo.detach(), residual=x)  # x + attention block: the residual is added in the GEMM's epilogue
         n2, rstd2 = kernels.rmsnorm_fwd(h, w_n2.detach(), dims.eps)
-        gu = _gemm_fused(n2, w_gu)
-        a = kernels.swiglu_fwd(gu)
+        t, d, f = n2.shape[0], n2.shape[1], wg.shape[0]
+        if wg.is_contiguous() and wu.is_contiguous() and kernels.swiglu_pays(t, f, d, n2.device.index):
+            gu, a = kernels.gemm_swiglu(n2, wg.detach(), wu.detach(), keep_gu=keep)
+        else:
+            gu = _gemm_fused(n2, fuse_rows([wg, wu]))
+            a = kernels.swiglu_fwd(gu)
         out = kernels.gemm(a, wd.detach(), residual=h)
-        ctx.save_for_backward(x, rstd1, n1, qkv, att, lse, h, rstd2, n2, gu, a, cos_sin)
+        if keep:
+            ctx.save_for_backward(x, rstd1, n1, qkv, att, lse, h, rstd2, n2, gu, a, cos_sin)
         ctx.weights = (w_n1, wq, wk, wv, wo, w_n2, wg, wu, wd)
         ctx.dims = dims
         return out
@@ -287,7 +296,7 @@ class DecoderLayerFn(torch.autograd.Function):
         g_n1 = _norm_weight_grad(w_n1, lambda dw, z: box.append(kernels.rmsnorm_bwd(x, w_n1.detach(), dn1, rstd1, dw, dres=dh, zero_dw=z)), True)
         dx = box.pop()
         flush_pushed(pushed)
-        return dx, g_n1, g_wq, g_wk, g_wv, g_wo, g_n2, g_wg, g_wu, g_wd, None, None
+        return dx, g_n1, g_wq, g_wk, g_wv, g_wo, g_n2, g_wg, g_wu, g_wd, None, None, None
 
 
 # ------------------------------------------------------------------------------------- final norm + head + loss
@@ -311,11 +320,10 @@ class HeadLossFn(torch.autograd.Function):
     def backward(ctx: Any, dloss: torch.Tensor) -> Any:  # type: ignore[override]
         h, rstd, n, dlogits = ctx.saved_tensors
         w_norm, w_head = ctx.weights
-        # the incoming gradient of the loss (a device scalar) scales the two small [T, d] operands instead of a pass over
-        # the [T, vocab] gradient: dn = dloss * (dlogits W), dW = dlogits^T (dloss * n)
-        dn = kernels.gemm(dlogits, w_head.detach(), b_mn_major=True)
-        dn.mul_(dloss.to(dn.dtype))
-        (g_head,) = _WeightGrad([w_head]).run(dlogits, n * dloss.to(n.dtype))
+        # the incoming gradient of the loss (a device scalar) is a factor of the two products: the GEMMs read it themselves
+        scale = dloss.float()
+        dn = kernels.gemm(dlogits, w_head.detach(), b_mn_major=True, alpha_tensor=scale)
+        (g_head,) = _WeightGrad([w_head]).run(dlogits, n, scale=scale)
         box: list[torch.Tensor] = []
         g_norm = _norm_weight_grad(w_norm, lambda dw, z: box.append(kernels.rmsnorm_bwd(h, w_norm.detach(), dn, rstd, dw, zero_dw=z)), True)
         return box.pop(), g_norm, g_head, None, None
@@ -379,7 +387,7 @@ def decoder_layer_ref(x: torch.Tensor, w_n1: torch.Tensor, wq: torch.Tensor, wk:
 def decoder_layer(x: torch.Tensor, *weights_and_table: Any) -> torch.Tensor:
     """``x [B*S, d]`` through one decoder layer (arguments as ``DecoderLayerFn.forward``)."""
     if x.is_cuda:
-        return DecoderLayerFn.apply(x, *weights_and_table)
+        return DecoderLayerFn.apply(x, *weights_and_table, torch.is_grad_enabled())
     return decoder_layer_ref(x, *weights_and_table)
 
 

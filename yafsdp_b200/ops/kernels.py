@@ -87,6 +87,7 @@ def gemm(
     residual: torch.Tensor | None = None,
     tile: int = 0,
     splits: int = 0,
+    alpha_tensor: torch.Tensor | None = None,
 ) -> torch.Tensor:
     """``out[M,N] = alpha * A @ B^T (+ out)`` with bf16 inputs and fp32 accumulation (tcgen05).
 
@@ -96,6 +97,7 @@ def gemm(
     one-element fp32 tensor that receives ``+= sum(out**2)`` from the same kernel.  ``residual`` (bf16 output without
     accumulation only): a bf16 ``[M,N]`` tensor added in fp32 inside the epilogue, before the output is rounded.
     ``tile`` (1-5) and ``splits`` (1-4): tile shape and K ranges of the last wave's tiles; 0 chooses them from the shape.
+    ``alpha_tensor``: one fp32 value on the device that ``alpha`` is multiplied by (read by the kernel).
     """
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.is_cuda and b.is_cuda
     assert a.dim() == 2 and b.dim() == 2 and a.stride(1) == 1 and b.stride(1) == 1
@@ -115,12 +117,13 @@ def gemm(
     if residual is not None:
         assert out.dtype == torch.bfloat16 and not accumulate and sumsq is None
         assert residual.dtype == torch.bfloat16 and residual.shape == (m, n) and residual.stride(1) == 1
+    assert alpha_tensor is None or (alpha_tensor.dtype == torch.float32 and alpha_tensor.numel() == 1 and alpha_tensor.device == a.device)
     nbytes = _gemm_workspace(m, n, k, int(out.dtype == torch.float32), 0, sm_limit, tile, splits, a.device.index)
     ws = torch.empty(nbytes, device=a.device, dtype=torch.uint8) if nbytes else None
     rc = _native.lib().yf_gemm_bf16_ws(
         a.data_ptr(), b.data_ptr(), out.data_ptr(), _ptr(residual), m, n, k, a.stride(0), b.stride(0), out.stride(0),
         0 if residual is None else residual.stride(0), int(a_mn_major), int(b_mn_major), int(out.dtype == torch.float32),
-        int(accumulate), float(alpha), int(sm_limit), _ptr(sumsq), _ptr(ws), nbytes, tile, splits, _stream(),
+        int(accumulate), float(alpha), int(sm_limit), _ptr(alpha_tensor), _ptr(sumsq), _ptr(ws), nbytes, tile, splits, _stream(),
     )
     _check(rc, "yf_gemm_bf16")
     return out
@@ -163,6 +166,23 @@ def can_be_parts(ts: "list[torch.Tensor]") -> bool:
     return 2 <= len(ts) <= 4 and all(
         t.is_cuda and t.dtype == torch.bfloat16 and t.dim() == 2 and t.is_contiguous() and t.shape[1] == first.shape[1] and t.shape[1] % 8 == 0
         and t.data_ptr() % 16 == 0 for t in ts) and all(t.shape[0] % 64 == 0 and t.shape[0] > 0 for t in ts)
+
+
+@functools.lru_cache(maxsize=4096)
+def swiglu_pays(t: int, f: int, k: int, device: int | None) -> bool:
+    """Whether :func:`gemm_swiglu` takes this shape and is expected to beat the two separate kernels."""
+    return _native.lib().yf_gemm_swiglu_pays(t, f, k) == 1
+
+
+def gemm_swiglu(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, keep_gu: bool = True) -> tuple[torch.Tensor | None, torch.Tensor]:
+    """``(gu, a)``: ``gu = [x wg^T | x wu^T]`` (``None`` unless kept) and ``a = silu(gate) * up`` from one kernel."""
+    (t, k), f = x.shape, wg.shape[0]
+    assert x.dtype == wg.dtype == wu.dtype == torch.bfloat16 and wg.shape == wu.shape == (f, k) and x.stride(1) == wg.stride(1) == wu.stride(1) == 1
+    gu = torch.empty((t, 2 * f), device=x.device, dtype=torch.bfloat16) if keep_gu else None
+    act = torch.empty((t, f), device=x.device, dtype=torch.bfloat16)
+    _check(_native.lib().yf_gemm_swiglu(x.data_ptr(), wg.data_ptr(), wu.data_ptr(), _ptr(gu), act.data_ptr(), t, f, k, x.stride(0), wg.stride(0),
+                                        wu.stride(0), 2 * f, f, _stream()), "yf_gemm_swiglu")
+    return gu, act
 
 
 def gemm_gathered(a: torch.Tensor, n: int, k: int, *, peer_in: Any, layer_buf: torch.Tensor, shard_bytes: int, b_byte_off: int,
