@@ -473,6 +473,28 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   }
 }
 
+// The loss's two scalars, one block each: bound by the latency of a launch.  (As comparison, sum, clamp, cast and reciprocal, and as
+// sum and product, they were seven launches of 2 to 4 us.)
+constexpr int ONE_BLOCK = 1024;
+__global__ void __launch_bounds__(ONE_BLOCK) inv_valid_labels_kernel(const long long* __restrict__ labels, long long n, float* __restrict__ out) {
+  __shared__ int count;
+  if (threadIdx.x == 0) count = 0;
+  __syncthreads();
+  int c = 0;
+  for (long long i = threadIdx.x; i < n; i += ONE_BLOCK) c += labels[i] >= 0 ? 1 : 0;
+  c = __reduce_add_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&count, c);
+  __syncthreads();
+  if (threadIdx.x == 0) *out = 1.f / (float)max(count, 1);
+}
+__global__ void __launch_bounds__(ONE_BLOCK) scaled_sum_kernel(const float* __restrict__ x, long long n, const float* __restrict__ scale, float* __restrict__ out) {
+  __shared__ float red[32];
+  float s = 0.f;
+  for (long long i = threadIdx.x; i < n; i += ONE_BLOCK) s += x[i];
+  s = block_sum<ONE_BLOCK>(s, red);
+  if (threadIdx.x == 0) *out = s * *scale;
+}
+
 // ------------------------------------------------------------------ embedding
 __global__ void embedding_fwd_kernel(const __nv_bfloat16* __restrict__ table, const long long* __restrict__ ids,
                                      __nv_bfloat16* __restrict__ out, long long T, int D, int V) {
@@ -768,6 +790,16 @@ extern "C" int yf_cross_entropy(void* logits, const long long* labels, float* lo
   const int grid = T < yf_num_sms() * 4 ? T : yf_num_sms() * 4;
   cross_entropy_kernel<<<grid, CE_THREADS, 0, YF_STREAM(stream)>>>((__nv_bfloat16*)logits, labels, loss_rows, T, V, ldl, grad_scale,
                                                                    scale_ptr, write_grad);
+  YF_LAUNCH_RET();
+}
+extern "C" int yf_inv_valid_labels(const long long* labels, long long n, float* out, void* stream) {
+  if (n < 0 || n > 0x7fffffffll) return -1;
+  inv_valid_labels_kernel<<<1, ONE_BLOCK, 0, YF_STREAM(stream)>>>(labels, n, out);
+  YF_LAUNCH_RET();
+}
+extern "C" int yf_scaled_sum(const float* x, long long n, const float* scale, float* out, void* stream) {
+  if (n < 0) return -1;
+  scaled_sum_kernel<<<1, ONE_BLOCK, 0, YF_STREAM(stream)>>>(x, n, scale, out);
   YF_LAUNCH_RET();
 }
 extern "C" int yf_embedding_fwd(const void* table, const long long* ids, void* out, long long T, int D, int V, void* stream) {

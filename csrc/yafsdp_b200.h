@@ -63,6 +63,9 @@ int yf_swiglu_fwd(const void* gu, void* h, long long T, int F, void* stream);
 int yf_swiglu_bwd(const void* gu, const void* dh, void* dgu, long long T, int F, void* stream);
 int yf_cross_entropy(void* logits, const long long* labels, float* loss_rows, int T, int V, long long ldl,
                      float grad_scale, const float* scale_ptr, int write_grad, void* stream);
+/* *out = 1 / max(1, number of labels >= 0); *out = sum(x) * *scale in a fixed order: one block each */
+int yf_inv_valid_labels(const long long* labels, long long n, float* out, void* stream);
+int yf_scaled_sum(const float* x, long long n, const float* scale, float* out, void* stream);
 int yf_embedding_fwd(const void* table, const long long* ids, void* out, long long T, int D, int V, void* stream);
 int yf_embedding_bwd(const void* dout, const long long* ids, float* dtable, long long T, int D, int V, void* stream);
 int yf_adamw(float* p, const float* g, float* m, float* v, void* p_bf16, const float* grad_scale_ptr, long long n,

@@ -5,6 +5,7 @@ Parity: ``ya_fsdp/_common.py:13-74``.
 
 from __future__ import annotations
 
+import contextlib
 import enum
 import logging
 import traceback
@@ -16,6 +17,16 @@ import torch.distributed as dist
 from torch.distributed.device_mesh import DeviceMesh
 
 logger = logging.getLogger("yafsdp_b200")
+
+_NO_LABEL = contextlib.nullcontext()
+
+
+def phase_label(name: str, of: str = "") -> Any:
+    """``record_function`` range ``name (of)`` while a profiler is active, nothing otherwise: entering and leaving a range costs
+    4 to 8 us of host time, 35 times in a step of a two-layer model."""
+    if not torch.autograd._profiler_enabled():  # type: ignore[attr-defined]
+        return _NO_LABEL
+    return torch.profiler.record_function(f"{name} ({of})" if of else name)
 
 
 class TrainingState(enum.Enum):

@@ -31,11 +31,10 @@ from typing import Any, Callable, Iterator, NamedTuple
 import torch
 import torch.distributed as dist
 import torch.nn as nn
-from torch.profiler import record_function
 
 from .api import MixedPrecisionPolicy
 from .comm.backends import CommBackend, TorchBackend, gradient_divide_factors
-from .common import ShardMeshInfo, TrainingState, is_backward_running, logger
+from .common import ShardMeshInfo, TrainingState, is_backward_running, logger, phase_label
 from .layout import FlatLayout, ParamPlacement
 from .tensor import RaggedShard, RaggedShardDTensor, RaggedSpec, _contiguous_stride
 
@@ -688,7 +687,7 @@ class ParamGroup:
         st = cc.streams
         assert st is not None
         logger.debug("unshard %s", self._module_fqn)
-        with record_function(self._with_fqn("YaFSDP::all_gather")):
+        with phase_label("YaFSDP::all_gather", self._module_fqn):
             if self._alias_data:
                 self.wait_optimizer()
                 self._refresh_gather_input()
@@ -782,7 +781,7 @@ class ParamGroup:
     # ------------------------------------------------------------------ forward
     def pre_forward(self) -> None:
         logger.debug("pre_forward %s", self._module_fqn)
-        with record_function(self._with_fqn("YaFSDP::pre_forward")):
+        with phase_label("YaFSDP::pre_forward", self._module_fqn):
             self._training_state = TrainingState.FORWARD
             if self._can_gather_in_kernel():
                 self._begin_in_kernel_gather()
@@ -844,7 +843,7 @@ class ParamGroup:
             self._in_kernel_gather = None
             raise RuntimeError(f"{self._module_fqn}: fused_gather is set but the module's forward never gathered its parameters "
                                "(only modules that call take_in_kernel_gather may use it)")
-        with record_function(self._with_fqn("YaFSDP::post_forward")):
+        with phase_label("YaFSDP::post_forward", self._module_fqn):
             if not is_backward_running():  # inside backward (checkpoint recompute) the backward owns the buffer
                 if self.reshard_after_forward:
                     self.reshard()
@@ -866,7 +865,7 @@ class ParamGroup:
         if self._training_state == TrainingState.PRE_BACKWARD:
             return
         logger.debug("pre_backward %s", self._module_fqn)
-        with record_function(self._with_fqn("YaFSDP::pre_backward")):
+        with phase_label("YaFSDP::pre_backward", self._module_fqn):
             self._training_state = TrainingState.PRE_BACKWARD
             self._kept_after_forward = False
             if self._norm_sq is not None and self._alias_grad and not self._has_sharded_grads():
@@ -903,7 +902,7 @@ class ParamGroup:
         ctx = target.data_ctx
         if not target._alias_data and ctx is not None and ctx.owner is not None and ctx.owner is not target._owner:
             return  # the buffer is not free yet: the target gathers itself when its turn comes
-        with record_function(target._with_fqn(f"YaFSDP::{pass_type}_prefetch")):
+        with phase_label(f"YaFSDP::{pass_type}_prefetch", target._module_fqn):
             old = target._training_state
             target._training_state = state
             target.unshard(target.unshard_async_op)
@@ -940,7 +939,7 @@ class ParamGroup:
         self._training_state = TrainingState.POST_BACKWARD
         assert self.comm_ctx is not None and self.comm_ctx.streams is not None
         st = self.comm_ctx.streams
-        with record_function(self._with_fqn("YaFSDP::post_backward_accumulate")):
+        with phase_label("YaFSDP::post_backward_accumulate", self._module_fqn):
             with_grad: list[ShardedParam] = []
             for sp in self.params:
                 up = sp.unsharded_param
@@ -953,10 +952,10 @@ class ParamGroup:
                 return
             if self._pushed:
                 self._finish_pushes()
-                with record_function(self._with_fqn("YaFSDP::post_backward_reshard")):
+                with phase_label("YaFSDP::post_backward_reshard", self._module_fqn):
                     if self.reshard_after_backward:
                         self.reshard()
-                with record_function(self._with_fqn("YaFSDP::post_backward_reduce")):
+                with phase_label("YaFSDP::post_backward_reduce", self._module_fqn):
                     self._reduce([sp for sp in self.params if sp.requires_grad], st)
                 return
             self._acquire_grad_buffer()
@@ -990,14 +989,14 @@ class ParamGroup:
                 if dsts_add:
                     torch._foreach_add_([d for d, _ in dsts_add], [s.to(d.dtype) if s.dtype != d.dtype else s for d, s in dsts_add])
         if not self.reduce_grads:
-            with record_function(self._with_fqn("YaFSDP::post_backward_reshard")):
+            with phase_label("YaFSDP::post_backward_reshard", self._module_fqn):
                 if self.reshard_after_backward:
                     self.reshard()
             return  # keeps the grad buffer: the unsharded accumulated gradients live there
-        with record_function(self._with_fqn("YaFSDP::post_backward_reshard")):
+        with phase_label("YaFSDP::post_backward_reshard", self._module_fqn):
             if self.reshard_after_backward:
                 self.reshard()
-        with record_function(self._with_fqn("YaFSDP::post_backward_reduce")):
+        with phase_label("YaFSDP::post_backward_reduce", self._module_fqn):
             self._reduce(with_grad, st)
 
     def _finish_pushes(self) -> None:
@@ -1243,9 +1242,6 @@ class ParamGroup:
         return self.world_size == 1 and self.reduce_scatter_dtype == self.orig_dtype
 
     # ------------------------------------------------------------------ misc
-    def _with_fqn(self, label: str) -> str:
-        return f"{label} ({self._module_fqn})" if self._module_fqn else label
-
     def __repr__(self) -> str:
         return f"ParamGroup(fqn={self._module_fqn!r}, {self.layout})"
 

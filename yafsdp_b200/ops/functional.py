@@ -310,11 +310,12 @@ class HeadLossFn(torch.autograd.Function):
         n, rstd = kernels.rmsnorm_fwd(h, w_norm.detach(), eps)
         logits = kernels.gemm(n, w_head.detach())
         # the mean's 1 / (number of valid labels) goes into the gradient that the loss kernel leaves in place of the logits
-        inv_valid = (labels >= 0).sum().clamp_(min=1).to(torch.float32).reciprocal_().reshape(1)
+        labels = _c(labels)
+        inv_valid = kernels.inv_valid_labels(labels)
         loss_rows = kernels.cross_entropy_(logits, labels, 1.0, write_grad=True, scale=inv_valid)
         ctx.save_for_backward(h, rstd, n, logits)
         ctx.weights = (w_norm, w_head)
-        return (loss_rows.sum() * inv_valid).reshape(())
+        return kernels.scaled_sum(loss_rows, inv_valid)
 
     @staticmethod
     def backward(ctx: Any, dloss: torch.Tensor) -> Any:  # type: ignore[override]

@@ -31,7 +31,8 @@ def reset_launch_count() -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # torch.cuda.current_stream() without the Stream object around it (some 5 us a call)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())  # type: ignore[no-any-return]
 
 
 def _check(rc: int, name: str) -> None:
@@ -305,6 +306,22 @@ def cross_entropy_(logits: torch.Tensor, labels: torch.Tensor, grad_scale: float
     _check(_native.lib().yf_cross_entropy(logits.data_ptr(), labels.data_ptr(), loss_rows.data_ptr(), t, v, logits.stride(0),
                                           float(grad_scale), _ptr(scale), int(write_grad), _stream()), "yf_cross_entropy")
     return loss_rows
+
+
+def inv_valid_labels(labels: torch.Tensor) -> torch.Tensor:
+    """``1 / max(1, number of labels that are not negative)`` as one fp32 value on the device."""
+    assert labels.dtype == torch.int64 and labels.is_contiguous()
+    out = torch.empty(1, device=labels.device, dtype=torch.float32)
+    _check(_native.lib().yf_inv_valid_labels(labels.data_ptr(), labels.numel(), out.data_ptr(), _stream()), "yf_inv_valid_labels")
+    return out
+
+
+def scaled_sum(x: torch.Tensor, scale: torch.Tensor) -> torch.Tensor:
+    """``x.sum() * scale`` (fp32, 0-dimensional) in a fixed order."""
+    assert x.dtype == scale.dtype == torch.float32 and x.is_contiguous()
+    out = torch.empty((), device=x.device, dtype=torch.float32)
+    _check(_native.lib().yf_scaled_sum(x.data_ptr(), x.numel(), scale.data_ptr(), out.data_ptr(), _stream()), "yf_scaled_sum")
+    return out
 
 
 def embedding_fwd(table: torch.Tensor, ids: torch.Tensor) -> torch.Tensor:

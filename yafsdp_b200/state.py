@@ -21,12 +21,11 @@ import torch
 import torch.nn as nn
 from torch.autograd import Variable
 from torch.autograd.graph import register_multi_grad_hook
-from torch.profiler import record_function
 from torch.utils._pytree import tree_flatten, tree_map, tree_unflatten
 
 from .api import MixedPrecisionPolicy
 from .comm.backends import CommBackend, make_backend
-from .common import TrainingState, cast_fp_tensor, logger
+from .common import TrainingState, cast_fp_tensor, logger, phase_label
 from .group import BufferContext, CommContext, ParamGroup, RegisterPostBackwardFunction
 
 __all__ = ["FSDPState", "StateContext", "get_module_state"]
@@ -120,7 +119,7 @@ class FSDPState:
             from .ops import kernels
 
             kernels.poll_status()  # a bounded device-side wait that ran out during the previous step surfaces here
-        with record_function("YaFSDP::root_pre_forward"):
+        with phase_label("YaFSDP::root_pre_forward"):
             st = self._comm_ctx.streams
             assert st is not None
             # a previous forward that was never followed by a backward left its last groups gathered: release them
@@ -140,7 +139,7 @@ class FSDPState:
                 st.wait_stream(self._comm_ctx.all_gather_stream, st.current())
             self._comm_ctx.sync_gather_inputs(self._comm_ctx.all_gather_stream)
             if self._device.type == "cuda":
-                with record_function("YaFSDP::inputs_to_device"):
+                with phase_label("YaFSDP::inputs_to_device"):
                     args, kwargs = tree_map(lambda x: x.to(self._device, non_blocking=True) if isinstance(x, torch.Tensor) and x.device.type == "cpu" else x, (args, kwargs))
         return args, kwargs
 
@@ -329,7 +328,7 @@ class FSDPState:
         if self._is_root is None or self._is_root:
             args, kwargs = self._root_pre_forward(module, args, kwargs)
         if self._mp_policy.cast_forward_inputs and self._mp_policy.param_dtype:
-            with record_function("YaFSDP::cast_forward_inputs"):
+            with phase_label("YaFSDP::cast_forward_inputs"):
                 cast = functools.partial(cast_fp_tensor, self._mp_policy.param_dtype)
                 args, kwargs = tree_map(cast, args), tree_map(cast, kwargs)
         g = self._param_group
@@ -358,7 +357,7 @@ class FSDPState:
                         s._param_group.reshard()
                 self._comm_ctx.post_forward_order.clear()
         if self._mp_policy.output_dtype is not None:
-            with record_function("YaFSDP::cast_forward_outputs"):
+            with phase_label("YaFSDP::cast_forward_outputs"):
                 output = tree_map(functools.partial(cast_fp_tensor, self._mp_policy.output_dtype), output)
         return output
 
@@ -408,7 +407,7 @@ class FSDPState:
 
     def _root_post_backward_final_callback(self) -> None:
         logger.debug("root post-backward final callback")
-        with record_function("YaFSDP::root_post_backward_callback"):
+        with phase_label("YaFSDP::root_post_backward_callback"):
             ctx = self._state_ctx
             for state in ctx.all_states:
                 g = state._param_group
