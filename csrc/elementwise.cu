@@ -105,68 +105,12 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_fwd_kernel(const __nv_bflo
   }
 }
 
-// Backward in two kernels.  (1) dx = r * (dy*w - xhat * mean(dy*w*xhat)) (+ dres, the gradient arriving
-// through the residual branch, fused to save a pass): one CTA per row, the row stays in registers.
-// (2) dw[j] += sum_rows dy * xhat: a column reduction over the token dimension, tiled [64 columns x a slice of
-// rows] per CTA with one fp32 atomic per column per CTA.
-__global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ x,
-                                                                    const __nv_bfloat16* __restrict__ w,
-                                                                    const __nv_bfloat16* __restrict__ dy,
-                                                                    const float* __restrict__ rstd,
-                                                                    const __nv_bfloat16* __restrict__ dres,
-                                                                    __nv_bfloat16* __restrict__ dx, int T, int D) {
-  __shared__ float red[32];
-  const int nvec = D / 8;
-  for (int row = blockIdx.x; row < T; row += gridDim.x) {
-    const __nv_bfloat16* xr = x + (size_t)row * D;
-    const __nv_bfloat16* dyr = dy + (size_t)row * D;
-    const float r = rstd[row];
-    float xh[RN_MAXV][8], g[RN_MAXV][8];
-    float dot = 0.f;
-#pragma unroll
-    for (int i = 0; i < RN_MAXV; ++i) {
-      const int v = threadIdx.x + i * RN_THREADS;
-      if (v < nvec) {
-        float xv[8], dv[8], wv[8];
-        load8(xr + v * 8, xv);
-        load8(dyr + v * 8, dv);
-        load8(w + v * 8, wv);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          xh[i][j] = xv[j] * r;
-          g[i][j] = dv[j] * wv[j];
-          dot += g[i][j] * xh[i][j];
-        }
-      }
-    }
-    dot = block_sum<RN_THREADS>(dot, red) / (float)D;
-    __nv_bfloat16* dxr = dx + (size_t)row * D;
-#pragma unroll
-    for (int i = 0; i < RN_MAXV; ++i) {
-      const int v = threadIdx.x + i * RN_THREADS;
-      if (v < nvec) {
-        float o[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = r * (g[i][j] - xh[i][j] * dot);
-        if (dres) {
-          float e[8];
-          load8(dres + (size_t)row * D + v * 8, e);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += e[j];
-        }
-        store8(dxr + v * 8, o);
-      }
-    }
-  }
-}
-
-// G warps per row (G = 1, 2 or 4; D <= 32 * G * 8 * RNW_NV forward, RNW_NV_B backward), four warps per CTA: the row stays in registers as packed bf16,
+// G warps per row (G = 1, 2 or 4; D <= 32 * G * 8 * RNW_NV), four warps per CTA: the row stays in registers as packed bf16,
 // every operand of a row is requested before anything is reduced (one exposed memory latency per row, not one per pass),
 // and the only synchronisation is a named barrier among the G warps of the row.  Thread t of a row's group holds the
 // vectors t, t + 32 G, ... of the row (contiguous 512 G bytes per load instruction).
 constexpr int RNW_WARPS = 4;
-constexpr int RNW_NV = 8;    // forward: vectors of a row per thread
-constexpr int RNW_NV_B = 4;  // backward (three operands per row in registers)
+constexpr int RNW_NV = 8;  // vectors of a row per thread
 YF_DEVINL void unpack8(const uint4& v, float (&f)[8]) {
   float2 a = unpack_bf16x2(v.x), b = unpack_bf16x2(v.y), c = unpack_bf16x2(v.z), d = unpack_bf16x2(v.w);
   f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
@@ -230,105 +174,141 @@ __global__ void __launch_bounds__(RNW_WARPS * 32) rmsnorm_fwd_warp_kernel(const 
   }
 }
 
-// dx of the same form; CTA 0 also clears the weight gradient when `dw_zero` is given (the column-reduction kernel that
-// accumulates into it is launched after this one on the same stream).
-template <int G>
-__global__ void __launch_bounds__(RNW_WARPS * 32, 6) rmsnorm_bwd_dx_warp_kernel(const __nv_bfloat16* __restrict__ x,
-                                                                                const __nv_bfloat16* __restrict__ w,
-                                                                                const __nv_bfloat16* __restrict__ dy,
-                                                                                const float* __restrict__ rstd,
-                                                                                const __nv_bfloat16* __restrict__ dres,
-                                                                                __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_zero,
-                                                                                int T, int D) {
-  __shared__ float red[RNW_WARPS];
-  if (dw_zero != nullptr && blockIdx.x == 0)
-    for (int i = threadIdx.x; i < D; i += RNW_WARPS * 32) dw_zero[i] = 0.f;
-  constexpr int ROWS = RNW_WARPS / G, TPR = 32 * G;
-  const int row_in_cta = threadIdx.x / TPR, tr = threadIdx.x % TPR;
-  const int row = blockIdx.x * ROWS + row_in_cta;
-  if (row >= T) return;
+// Backward: dx = r * (dy*w - xhat * mean(dy*w*xhat)) (+ dres, the gradient arriving through the residual branch) and
+// dw = sum_rows dy * xhat.  TPR threads per row (D <= 32 TPR), 256 threads = 256 / TPR rows at a time, two CTAs per SM that walk
+// over the rows: a thread holds the same columns of every row, so dw is summed in registers on the way and x and dy are read once
+// (a column reduction of its own read both again).  The row groups of a CTA meet in shared memory at the end (unless all
+// of them together are below 2 MB); the sums go to rows of `partials`, added up in a fixed order by rmsnorm_bwd_dw_kernel, or, without
+// partials, atomically to dw.
+// Bound by HBM: 8 bytes per element with dres.  With dres, both kernels: 2048 x 4096 23 us, 8192 x 4096 57 us,
+// 2048 x 8192 34 us (the dx and column kernels before: 27, 90 and 56 us).
+constexpr int RNB_NV = 4;  // vectors of 8 per thread
+constexpr int RNB_THREADS = 256;
+template <int TPR>
+__global__ void __launch_bounds__(RNB_THREADS, 2) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                                     const __nv_bfloat16* __restrict__ dy, const float* __restrict__ rstd,
+                                                                     const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+                                                                     float* __restrict__ partials, float* __restrict__ dw, int T, int D, int combine) {
+  constexpr int ROWS = RNB_THREADS / TPR;
+  __shared__ float red[2][RNB_THREADS / 32];
+  __shared__ float sums[ROWS > 1 ? TPR * RNB_NV * 8 : 1];
+  const int group = threadIdx.x / TPR, tr = threadIdx.x % TPR;
   const int nvec = D / 8;
-  const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * D);
-  const uint4* dyr = reinterpret_cast<const uint4*>(dy + (size_t)row * D);
-  const uint4* er = reinterpret_cast<const uint4*>(dres ? dres + (size_t)row * D : x);
   const uint4* wr = reinterpret_cast<const uint4*>(w);
-  uint4 xv[RNW_NV_B], dv[RNW_NV_B], ev[RNW_NV_B];
+  float acc[RNB_NV][8];
 #pragma unroll
-  for (int i = 0; i < RNW_NV_B; ++i) {
-    const int v = tr + TPR * i;
-    const bool in = v < nvec;
-    xv[i] = in ? xr[v] : make_uint4(0u, 0u, 0u, 0u);
-    dv[i] = in ? dyr[v] : make_uint4(0u, 0u, 0u, 0u);
-    ev[i] = (in && dres) ? er[v] : make_uint4(0u, 0u, 0u, 0u);
-  }
-  const float r = rstd[row];
-  // g = dy * w replaces dy in registers (fp32 products rounded to bf16 would lose bits: keep dy and w apart instead and
-  // multiply twice; w comes from L1 both times)
-  float dot = 0.f;
+  for (int i = 0; i < RNB_NV; ++i)
 #pragma unroll
-  for (int i = 0; i < RNW_NV_B; ++i) {
-    const int v = tr + TPR * i;
-    if (v < nvec) {
-      float xf[8], df[8], wf[8];
-      unpack8(xv[i], xf);
-      unpack8(dv[i], df);
-      unpack8(__ldg(wr + v), wf);
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  int parity = 0;
+  for (int row = blockIdx.x * ROWS + group; row < T; row += gridDim.x * ROWS, parity ^= 1) {
+    const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * D);
+    const uint4* dyr = reinterpret_cast<const uint4*>(dy + (size_t)row * D);
+    const uint4* er = reinterpret_cast<const uint4*>(dres ? dres + (size_t)row * D : x);
+    uint4 xv[RNB_NV], dv[RNB_NV], ev[RNB_NV];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) dot += df[j] * wf[j] * (xf[j] * r);
+    for (int i = 0; i < RNB_NV; ++i) {
+      const int v = tr + TPR * i;
+      const bool in = v < nvec;
+      xv[i] = in ? xr[v] : make_uint4(0u, 0u, 0u, 0u);
+      dv[i] = in ? dyr[v] : make_uint4(0u, 0u, 0u, 0u);
+      ev[i] = (in && dres) ? er[v] : make_uint4(0u, 0u, 0u, 0u);
+    }
+    const float r = rstd[row];
+    float dot = 0.f;
+#pragma unroll
+    for (int i = 0; i < RNB_NV; ++i) {
+      const int v = tr + TPR * i;
+      if (v < nvec) {  // w comes from the L1 both times: its registers would cost the second CTA
+        float xf[8], df[8], wf[8];
+        unpack8(xv[i], xf);
+        unpack8(dv[i], df);
+        unpack8(__ldg(wr + v), wf);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float p = df[j] * (xf[j] * r);
+          dot += p * wf[j];
+          acc[i][j] += p;
+        }
+      }
+    }
+    dot = warp_sum(dot);
+    if (TPR > 32) {  // the row's warps; two sets of slots, so one barrier per row is enough
+      if ((threadIdx.x & 31) == 0) red[parity][threadIdx.x >> 5] = dot;
+      if (group == 0) named_bar_sync(1, TPR);  // literal barrier numbers: a computed one reserves all sixteen
+      else if (group == 1) named_bar_sync(2, TPR);
+      else if (group == 2) named_bar_sync(3, TPR);
+      else named_bar_sync(4, TPR);
+      dot = 0.f;
+#pragma unroll
+      for (int g = 0; g < TPR / 32; ++g) dot += red[parity][group * (TPR / 32) + g];
+    }
+    dot /= (float)D;
+    __nv_bfloat16* dxr = dx + (size_t)row * D;
+#pragma unroll
+    for (int i = 0; i < RNB_NV; ++i) {
+      const int v = tr + TPR * i;
+      if (v < nvec) {
+        float xf[8], df[8], wf[8], ef[8], o[8];
+        unpack8(xv[i], xf);
+        unpack8(dv[i], df);
+        unpack8(ev[i], ef);
+        unpack8(__ldg(wr + v), wf);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = r * (df[j] * wf[j] - xf[j] * r * dot) + ef[j];
+        store8(dxr + v * 8, o);
+      }
     }
   }
-  dot = row_group_sum<G>(dot, red, row_in_cta) / (float)D;
-  __nv_bfloat16* dxr = dx + (size_t)row * D;
+  if (dw == nullptr) return;
+  int part_row = blockIdx.x * ROWS + group;
+  if (ROWS > 1 && combine) {  // sum the row groups: the last one ends up with the total
+#pragma unroll 1
+    for (int g = 0; g < ROWS; ++g) {
+      if (group == g) {
 #pragma unroll
-  for (int i = 0; i < RNW_NV_B; ++i) {
+        for (int i = 0; i < RNB_NV; ++i) {
+          float* at = sums + (tr + TPR * i) * 8;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            if (g > 0) acc[i][j] += at[j];
+            at[j] = acc[i][j];
+          }
+        }
+      }
+      __syncthreads();
+    }
+    if (group != ROWS - 1) return;
+    part_row = blockIdx.x;
+  }
+#pragma unroll
+  for (int i = 0; i < RNB_NV; ++i) {
     const int v = tr + TPR * i;
     if (v < nvec) {
-      float xf[8], df[8], wf[8], ef[8], o[8];
-      unpack8(xv[i], xf);
-      unpack8(dv[i], df);
-      unpack8(ev[i], ef);
-      unpack8(__ldg(wr + v), wf);
+      if (partials != nullptr) {
+        float4* at = reinterpret_cast<float4*>(partials + (size_t)part_row * D + v * 8);
+        at[0] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        at[1] = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+      } else {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = r * (df[j] * wf[j] - xf[j] * r * dot) + ef[j];
-      store8(dxr + v * 8, o);
+        for (int j = 0; j < 8; ++j) atomicAdd(dw + v * 8 + j, acc[i][j]);
+      }
     }
   }
 }
-
-constexpr int RN_DW_COLS = 64;     // columns per CTA (8 threads x 8 bf16)
-constexpr int RN_DW_ROWLANES = 32; // row lanes per CTA (256 threads / 8)
-__global__ void __launch_bounds__(256) rmsnorm_bwd_dw_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
-                                                             const float* __restrict__ rstd, float* __restrict__ dw, int T, int D,
-                                                             int rows_per_cta) {
-  __shared__ float part[RN_DW_ROWLANES][RN_DW_COLS + 1];
-  const int c8 = threadIdx.x & 7;
-  const int rl = threadIdx.x >> 3;
-  const int col = blockIdx.x * RN_DW_COLS + c8 * 8;
-  const int row0 = blockIdx.y * rows_per_cta;
-  const int row1 = min(T, row0 + rows_per_cta);
-  float acc[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-  if (col < D) {
-    for (int row = row0 + rl; row < row1; row += RN_DW_ROWLANES) {
-      float xv[8], dv[8];
-      load8(x + (size_t)row * D + col, xv);
-      load8(dy + (size_t)row * D + col, dv);
-      const float r = rstd[row];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] += dv[j] * xv[j] * r;
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) part[rl][c8 * 8 + j] = acc[j];
+// dw (= or +=) column sums of partials [n, D]: 32 columns per CTA, 32 row lanes
+__global__ void __launch_bounds__(1024) rmsnorm_bwd_dw_kernel(const float* __restrict__ partials, float* __restrict__ dw, int n, int D, int add) {
+  __shared__ float part[32][33];
+  const int c = threadIdx.x & 31, lane_row = threadIdx.x >> 5;
+  const int col = blockIdx.x * 32 + c;
+  float s = 0.f;
+  if (col < D)
+    for (int i = lane_row; i < n; i += 32) s += partials[(size_t)i * D + col];
+  part[lane_row][c] = s;
   __syncthreads();
-  if (threadIdx.x < RN_DW_COLS) {
-    float s = 0.f;
-#pragma unroll
-    for (int r = 0; r < RN_DW_ROWLANES; ++r) s += part[r][threadIdx.x];
-    const int c = blockIdx.x * RN_DW_COLS + threadIdx.x;
-    if (c < D) atomicAdd(dw + c, s);
-  }
+  s = warp_sum(part[c][lane_row]);  // warp lane_row sums column blockIdx.x * 32 + lane_row over the row lanes
+  const int mine = blockIdx.x * 32 + lane_row;
+  if (c == 0 && mine < D) dw[mine] = add ? dw[mine] + s : s;
 }
 
 // ------------------------------------------------------------------ RoPE (rotate-half pairing, in place)
@@ -404,6 +384,10 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __
 // logits [T, V] bf16 (row pitch ldl) are replaced in place by dlogits = (softmax - onehot) * grad_scale, where grad_scale is
 // the host value times *scale_ptr when that device pointer is given (e.g. 1 / number of valid labels, counted on the device);
 // loss_rows[t] = logsumexp - logit[label] (0 for ignored rows, label < 0).  One CTA per row.
+// A row is read twice: the grid is kept so small that all rows in flight together stay in the L2, where the second read finds
+// them, and four loads per thread are in flight.  8192 x 128256: 1075 us (592 CTAs, 152 MB in flight, one load at a time: 1300 us);
+// 2048 x 32000: 73 us (82 us); there the exponentials and conversions are the bound: holding the row in registers, one read
+// for both passes, took 86 us.
 constexpr int CE_THREADS = 512;
 __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16* __restrict__ logits,
                                                                    const long long* __restrict__ labels,
@@ -427,6 +411,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
     }
     // online max / sum-exp
     float m = -INFINITY, s = 0.f;
+#pragma unroll 4
     for (int v = threadIdx.x; v < nvec; v += CE_THREADS) {
       float f[8];
       load8(lr + v * 8, f);
@@ -453,6 +438,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
     if (threadIdx.x == 0) loss_rows[row] = lse - __bfloat162float(lr[label]);
     if (write_grad) {
       __syncthreads();  // the label logit was read above before anyone overwrites it
+#pragma unroll 4
       for (int v = threadIdx.x; v < nvec; v += CE_THREADS) {
         float f[8], o[8];
         load8(lr + v * 8, f);
@@ -509,9 +495,10 @@ __global__ void embedding_fwd_kernel(const __nv_bfloat16* __restrict__ table, co
     *reinterpret_cast<uint4*>(out + t * D + v * 8) = val;
   }
 }
-// dtable[ids[t], :] += dout[t, :]  (fp32 table gradient, atomics: token ids repeat)
+// dtable[ids[t], :] += dout[t, :]  (fp32 table gradient; token ids repeat: atomics, four floats each).  `owner` (optional, V ints
+// that need no initial value): one of the tokens with id i is left in owner[i].
 __global__ void embedding_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const long long* __restrict__ ids,
-                                     float* __restrict__ dtable, long long T, int D, int V) {
+                                     float* __restrict__ dtable, int* __restrict__ owner, long long T, int D, int V, int aligned) {
   const int vpr = D / 8;
   const long long total = T * vpr;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -522,9 +509,30 @@ __global__ void embedding_bwd_kernel(const __nv_bfloat16* __restrict__ dout, con
     float f[8];
     load8(dout + t * D + v * 8, f);
     float* dst = dtable + id * D + v * 8;
+    if (aligned) {
+      asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(f[0]), "f"(f[1]), "f"(f[2]), "f"(f[3]) : "memory");
+      asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4), "f"(f[4]), "f"(f[5]), "f"(f[6]), "f"(f[7]) : "memory");
+    } else {  // a table that starts anywhere in a flat buffer
 #pragma unroll
-    for (int j = 0; j < 8; ++j) atomicAdd(dst + j, f[j]);
+      for (int j = 0; j < 8; ++j) atomicAdd(dst + j, f[j]);
+    }
+    if (v == 0 && owner != nullptr) atomicExch(owner + id, (int)t);  // any of them will do
   }
+}
+// *out += sum of squares of the rows that some token touched, each row once: the token that owner[] names reads it.  The other
+// rows of a gradient that started from zeros are zero: 32000 x 4096 after 2048 tokens, 33 MB instead of 524 MB.
+__global__ void __launch_bounds__(256) embedding_sumsq_kernel(const float* __restrict__ dtable, const long long* __restrict__ ids,
+                                                              const int* __restrict__ owner, float* __restrict__ out, long long T, int D, int V) {
+  __shared__ float red[32];
+  float acc = 0.f;
+  for (long long t = blockIdx.x; t < T; t += gridDim.x) {
+    const long long id = ids[t];
+    if (id < 0 || id >= V || owner[id] != (int)t) continue;
+    const float* row = dtable + id * D;
+    for (int v = threadIdx.x; v < D; v += 256) acc += row[v] * row[v];
+  }
+  acc = block_sum<256>(acc, red);
+  if (threadIdx.x == 0) atomicAdd(out, acc);
 }
 
 // ------------------------------------------------------------------ AdamW on the flat fp32 master shard
@@ -596,8 +604,8 @@ __global__ void __launch_bounds__(256) sumsq_kernel(const float* __restrict__ g,
 // ------------------------------------------------------------------ clipping a flat run of fp32 gradients
 // Bound by HBM: one read for the norm, one read and write for the scaling.  The run may start at any element (a
 // parameter's place in a flat buffer): up to three elements in front of the first 16-byte boundary are taken singly.
-// Every thread keeps four 16-byte loads in flight.  Measured on 90 M elements: sum of squares 57 us = 6.3 TB/s (as abs, pow
-// and sum, three kernels with fp32 tensors in between: 210 us), scaling 116 us = 6.2 TB/s (a broadcast multiplication: 160 us).
+// Every thread keeps four 16-byte loads in flight.  Measured on 90 M elements: sum of squares 61 us = 5.9 TB/s (as abs, pow
+// and sum, three kernels with fp32 tensors in between: 303 us), scaling 124 us = 5.8 TB/s (a broadcast multiplication: 220 us).
 YF_DEVINL long long run_head(const float* p, long long n) {
   const long long h = (long long)((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15) / 4;
   return h < n ? h : n;
@@ -730,40 +738,40 @@ extern "C" int yf_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd
                                                                  (__nv_bfloat16*)y, rstd, T, D, eps);
   YF_LAUNCH_RET();
 }
+static int rmsnorm_bwd_tpr(int D) { return D <= 1024 ? 32 : (D <= 2048 ? 64 : (D <= 4096 ? 128 : 256)); }
+static int rmsnorm_bwd_ctas(int T, int D) {
+  const int rows = RNB_THREADS / rmsnorm_bwd_tpr(D), need = (T + rows - 1) / rows, cap = 2 * yf_num_sms();
+  return need < cap ? need : cap;
+}
+static bool rmsnorm_bwd_combines(int T, int D) {
+  return (long long)rmsnorm_bwd_ctas(T, D) * (RNB_THREADS / rmsnorm_bwd_tpr(D)) * D * 4 > (2ll << 20);
+}
+// rows of yf_rmsnorm_bwd_ws's partials
+extern "C" int yf_rmsnorm_bwd_partials(int T, int D) {
+  if (T <= 0 || D <= 0 || (D % 8) || D > RNB_THREADS * 8 * RNB_NV) return -1;
+  return rmsnorm_bwd_ctas(T, D) * (rmsnorm_bwd_combines(T, D) ? 1 : RNB_THREADS / rmsnorm_bwd_tpr(D));
+}
+extern "C" int yf_rmsnorm_bwd_ws(const void* x, const void* w, const void* dy, const float* rstd, const void* dres, void* dx, float* dw,
+                                 int zero_dw, float* partials, int T, int D, void* stream) {
+  if (T <= 0 || D <= 0 || (D % 8) || D > RNB_THREADS * 8 * RNB_NV) return -1;
+  if (!aligned16(x) || !aligned16(w) || !aligned16(dy) || !aligned16(dx) || (dres && !aligned16(dres)) || (partials && !aligned16(partials))) return -1;
+  if ((zero_dw || partials) && !dw) return -1;
+  cudaStream_t st = YF_STREAM(stream);
+  if (zero_dw && !partials && cudaMemsetAsync(dw, 0, (size_t)D * sizeof(float), st) != cudaSuccess) return -2;
+  const __nv_bfloat16 *xp = (const __nv_bfloat16*)x, *wp = (const __nv_bfloat16*)w, *dyp = (const __nv_bfloat16*)dy, *ep = (const __nv_bfloat16*)dres;
+  __nv_bfloat16* dxp = (__nv_bfloat16*)dx;
+  const int ctas = rmsnorm_bwd_ctas(T, D), combine = !partials || rmsnorm_bwd_combines(T, D) ? 1 : 0;
+  if (D <= 1024) rmsnorm_bwd_kernel<32><<<ctas, RNB_THREADS, 0, st>>>(xp, wp, dyp, rstd, ep, dxp, partials, dw, T, D, combine);
+  else if (D <= 2048) rmsnorm_bwd_kernel<64><<<ctas, RNB_THREADS, 0, st>>>(xp, wp, dyp, rstd, ep, dxp, partials, dw, T, D, combine);
+  else if (D <= 4096) rmsnorm_bwd_kernel<128><<<ctas, RNB_THREADS, 0, st>>>(xp, wp, dyp, rstd, ep, dxp, partials, dw, T, D, combine);
+  else rmsnorm_bwd_kernel<256><<<ctas, RNB_THREADS, 0, st>>>(xp, wp, dyp, rstd, ep, dxp, partials, dw, T, D, combine);
+  if (partials) rmsnorm_bwd_dw_kernel<<<(D + 31) / 32, 1024, 0, st>>>(partials, dw, yf_rmsnorm_bwd_partials(T, D), D,
+                                                                        zero_dw ? 0 : 1);
+  YF_LAUNCH_RET();
+}
 extern "C" int yf_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float* rstd, const void* dres, void* dx,
                               float* dw, int zero_dw, int T, int D, void* stream) {
-  if (T <= 0 || D <= 0 || (D % 8) || D > RN_THREADS * 8 * RN_MAXV) return -1;
-  if (!aligned16(x) || !aligned16(w) || !aligned16(dy) || !aligned16(dx) || (dres && !aligned16(dres))) return -1;
-  if (zero_dw && !dw) return -1;
-  if (D <= 32 * 4 * 8 * RNW_NV_B) {  // G warps per row
-    const __nv_bfloat16 *xp = (const __nv_bfloat16*)x, *wp = (const __nv_bfloat16*)w, *dyp = (const __nv_bfloat16*)dy,
-                        *ep = (const __nv_bfloat16*)dres;
-    __nv_bfloat16* dxp = (__nv_bfloat16*)dx;
-    float* dwz = zero_dw ? dw : nullptr;
-    const int g = D <= 32 * 8 * RNW_NV_B ? 1 : (D <= 64 * 8 * RNW_NV_B ? 2 : 4);
-    const int rows = RNW_WARPS / g, ctas = (T + rows - 1) / rows;
-    if (g == 1) rmsnorm_bwd_dx_warp_kernel<1><<<ctas, RNW_WARPS * 32, 0, YF_STREAM(stream)>>>(xp, wp, dyp, rstd, ep, dxp, dwz, T, D);
-    else if (g == 2) rmsnorm_bwd_dx_warp_kernel<2><<<ctas, RNW_WARPS * 32, 0, YF_STREAM(stream)>>>(xp, wp, dyp, rstd, ep, dxp, dwz, T, D);
-    else rmsnorm_bwd_dx_warp_kernel<4><<<ctas, RNW_WARPS * 32, 0, YF_STREAM(stream)>>>(xp, wp, dyp, rstd, ep, dxp, dwz, T, D);
-  } else {
-    if (zero_dw && cudaMemsetAsync(dw, 0, (size_t)D * sizeof(float), YF_STREAM(stream)) != cudaSuccess) return -2;
-    const int grid = T < yf_num_sms() * 8 ? T : yf_num_sms() * 8;
-    rmsnorm_bwd_dx_kernel<<<grid, RN_THREADS, 0, YF_STREAM(stream)>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
-                                                                      (const __nv_bfloat16*)dy, rstd, (const __nv_bfloat16*)dres,
-                                                                      (__nv_bfloat16*)dx, T, D);
-  }
-  if (dw) {
-    const int col_blocks = (D + RN_DW_COLS - 1) / RN_DW_COLS;
-    int splits = (yf_num_sms() * 6 + col_blocks - 1) / col_blocks;  // about six CTAs per SM in total
-    const int max_splits = (T + RN_DW_ROWLANES - 1) / RN_DW_ROWLANES;
-    if (splits > max_splits) splits = max_splits;
-    if (splits < 1) splits = 1;
-    const int rows_per_cta = (T + splits - 1) / splits;
-    dim3 g2(col_blocks, (T + rows_per_cta - 1) / rows_per_cta);
-    rmsnorm_bwd_dw_kernel<<<g2, 256, 0, YF_STREAM(stream)>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, rstd, dw, T, D,
-                                                             rows_per_cta);
-  }
-  YF_LAUNCH_RET();
+  return yf_rmsnorm_bwd_ws(x, w, dy, rstd, dres, dx, dw, zero_dw, nullptr, T, D, stream);
 }
 extern "C" int yf_rope(void* qkv, const float* cos_sin, int T, int seq_len, long long row_stride, int col0, int n_heads,
                        int head_dim, int backward, void* stream) {
@@ -787,7 +795,10 @@ extern "C" int yf_swiglu_bwd(const void* gu, const void* dh, void* dgu, long lon
 extern "C" int yf_cross_entropy(void* logits, const long long* labels, float* loss_rows, int T, int V, long long ldl,
                                 float grad_scale, const float* scale_ptr, int write_grad, void* stream) {
   if (T <= 0 || V <= 0 || (ldl % 8) || !aligned16(logits)) return -1;
-  const int grid = T < yf_num_sms() * 4 ? T : yf_num_sms() * 4;
+  // one to four CTAs per SM, rows in flight of at most 80 MB
+  const long long row_bytes = (long long)V * 2 * yf_num_sms();
+  const int per_sm = row_bytes * 4 <= (80ll << 20) ? 4 : (row_bytes * 2 <= (80ll << 20) ? 2 : 1);
+  const int grid = T < yf_num_sms() * per_sm ? T : yf_num_sms() * per_sm;
   cross_entropy_kernel<<<grid, CE_THREADS, 0, YF_STREAM(stream)>>>((__nv_bfloat16*)logits, labels, loss_rows, T, V, ldl, grad_scale,
                                                                    scale_ptr, write_grad);
   YF_LAUNCH_RET();
@@ -808,10 +819,17 @@ extern "C" int yf_embedding_fwd(const void* table, const long long* ids, void* o
                                                                                       (__nv_bfloat16*)out, T, D, V);
   YF_LAUNCH_RET();
 }
-extern "C" int yf_embedding_bwd(const void* dout, const long long* ids, float* dtable, long long T, int D, int V, void* stream) {
-  if (T <= 0 || (D % 8) || !aligned16(dout)) return -1;
-  embedding_bwd_kernel<<<grid_for(T * (D / 8), 256, 8), 256, 0, YF_STREAM(stream)>>>((const __nv_bfloat16*)dout, ids, dtable, T, D, V);
+extern "C" int yf_embedding_bwd_norm(const void* dout, const long long* ids, float* dtable, int* owner, float* sumsq, long long T, int D, int V,
+                                     void* stream) {
+  if (T <= 0 || T > 0x7fffffffll || (D % 8) || !aligned16(dout) || (sumsq != nullptr && owner == nullptr)) return -1;
+  embedding_bwd_kernel<<<grid_for(T * (D / 8), 256, 8), 256, 0, YF_STREAM(stream)>>>((const __nv_bfloat16*)dout, ids, dtable, owner, T, D, V,
+                                                                                      aligned16(dtable) ? 1 : 0);
+  if (sumsq != nullptr)
+    embedding_sumsq_kernel<<<(int)(T < yf_num_sms() * 8 ? T : yf_num_sms() * 8), 256, 0, YF_STREAM(stream)>>>(dtable, ids, owner, sumsq, T, D, V);
   YF_LAUNCH_RET();
+}
+extern "C" int yf_embedding_bwd(const void* dout, const long long* ids, float* dtable, long long T, int D, int V, void* stream) {
+  return yf_embedding_bwd_norm(dout, ids, dtable, nullptr, nullptr, T, D, V, stream);
 }
 extern "C" int yf_adamw(float* p, const float* g, float* m, float* v, void* p_bf16, const float* grad_scale_ptr, long long n,
                         float lr, float beta1, float beta2, float eps, float weight_decay, int step, int max_ctas, void* stream) {

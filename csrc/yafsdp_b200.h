@@ -57,6 +57,10 @@ int yf_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int T, in
 /* dx (+ dres) and dw += column sums of dy * xhat; zero_dw: dw is cleared first, inside the dx kernel (no fill launch) */
 int yf_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float* rstd, const void* dres, void* dx,
                    float* dw, int zero_dw, int T, int D, void* stream);
+/* the same with the weight gradient summed in a fixed order: partials [yf_rmsnorm_bwd_partials(T, D), D] fp32 scratch */
+int yf_rmsnorm_bwd_partials(int T, int D);
+int yf_rmsnorm_bwd_ws(const void* x, const void* w, const void* dy, const float* rstd, const void* dres, void* dx, float* dw, int zero_dw,
+                      float* partials, int T, int D, void* stream);
 int yf_rope(void* qkv, const float* cos_sin, int T, int seq_len, long long row_stride, int col0, int n_heads,
             int head_dim, int backward, void* stream);
 int yf_swiglu_fwd(const void* gu, void* h, long long T, int F, void* stream);
@@ -68,6 +72,9 @@ int yf_inv_valid_labels(const long long* labels, long long n, float* out, void* 
 int yf_scaled_sum(const float* x, long long n, const float* scale, float* out, void* stream);
 int yf_embedding_fwd(const void* table, const long long* ids, void* out, long long T, int D, int V, void* stream);
 int yf_embedding_bwd(const void* dout, const long long* ids, float* dtable, long long T, int D, int V, void* stream);
+/* the same, and *sumsq += the squares of the touched rows (dtable zero before); owner: scratch of V ints */
+int yf_embedding_bwd_norm(const void* dout, const long long* ids, float* dtable, int* owner, float* sumsq, long long T, int D, int V,
+                          void* stream);
 int yf_adamw(float* p, const float* g, float* m, float* v, void* p_bf16, const float* grad_scale_ptr, long long n,
              float lr, float beta1, float beta2, float eps, float weight_decay, int step, int max_ctas, void* stream);
 int yf_sumsq(const float* g, long long n, float* out, void* stream);

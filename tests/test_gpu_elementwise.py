@@ -212,3 +212,72 @@ def test_clip_grad_norm_of_adjacent_sharded_gradients(max_norm):
     finally:
         if created:
             dist.destroy_process_group()
+
+
+@pytest.mark.parametrize("t,d", [(1, 8), (7, 1024), (700, 1032), (601, 2048), (1200, 4096), (297, 4104), (599, 8192)])
+def test_rmsnorm_bwd_weight_gradient_over_many_rows(t, d):
+    """Every width class of the row walk, more rows than a wave holds: the weight gradient in a fixed order, cleared or added to,
+    against fp64 sums (fp32 sums of t terms)."""
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(6)
+    x, dy = (torch.randn(t, d, device="cuda").bfloat16() for _ in range(2))
+    w = (1 + 0.1 * torch.randn(d, device="cuda")).bfloat16()
+    _, rstd = kernels.rmsnorm_fwd(x, w, 1e-5)
+    want = (dy.double() * x.double() * rstd.double()[:, None]).sum(0)
+    got = torch.full((d,), 3.0, device="cuda")
+    dx = kernels.rmsnorm_bwd(x, w, dy, rstd, got, zero_dw=True)
+    again = torch.empty_like(got)
+    dx2 = kernels.rmsnorm_bwd(x, w, dy, rstd, again, zero_dw=True)
+    assert torch.equal(got, again) and torch.equal(dx, dx2)
+    lim = 4.0 * t**0.5 * 2.0**-24 * (dy.double() * x.double() * rstd.double()[:, None]).abs().sum(0).max().item() + 1e-7
+    assert (got.double() - want).abs().max().item() < lim
+    kernels.rmsnorm_bwd(x, w, dy, rstd, again)
+    assert (again.double() - 2 * want).abs().max().item() < 2 * lim
+
+
+@pytest.mark.parametrize("v", [8, 1024, 32000, 32768, 32776, 1001, 128256])
+@pytest.mark.parametrize("t", [3, 700])
+def test_cross_entropy_row_lengths(v, t):
+    """Rows held in registers, longer ones, odd ones; ignored labels; logits at -inf."""
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(11)
+    pitch = (v + 7) // 8 * 8
+    logits = (3 * torch.randn(t, pitch, device="cuda")).bfloat16()[:, :v]
+    labels = torch.randint(0, v, (t,), device="cuda")
+    labels[1] = -100
+    if v > 8:
+        logits[0, 1:5] = -math.inf
+        labels[0] = 0
+    ref = logits.double().requires_grad_(True)
+    rows = torch.nn.functional.cross_entropy(ref, labels, ignore_index=-100, reduction="none")
+    (rows.sum() * 0.25).backward()
+    work = torch.empty(t, pitch, device="cuda", dtype=torch.bfloat16)[:, :v]
+    work.copy_(logits)
+    got = kernels.cross_entropy_(work, labels, 0.25)
+    assert torch.allclose(got.double(), rows, rtol=1e-5, atol=1e-5)  # fast exponentials of up to 2^17 terms in fp32
+    assert torch.allclose(work.double(), ref.grad, rtol=2.0**-7, atol=1e-6)
+
+
+def test_loss_scalars_and_embedding_norm():
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(12)
+    labels = torch.randint(-100, 50, (5003,), device="cuda")
+    inv = kernels.inv_valid_labels(labels)
+    assert abs(inv.item() * max(1, int((labels >= 0).sum())) - 1.0) < 1e-6
+    assert kernels.inv_valid_labels(torch.full((7,), -100, device="cuda")).item() == 1.0
+    x = torch.rand(5003, device="cuda")
+    assert abs(kernels.scaled_sum(x, inv).item() / (x.double().sum() * inv.double()).item() - 1.0) < 1e-6
+    for off in (0, 1):  # a table gradient that starts anywhere in a flat buffer
+        flat = torch.zeros(off + 300 * 264, device="cuda")
+        table = flat[off:].view(300, 264)
+        ids = torch.randint(0, 300, (900,), device="cuda")
+        ids[:200] = 17
+        dout = torch.randn(900, 264, device="cuda").bfloat16()
+        sq = torch.zeros(1, device="cuda")
+        kernels.embedding_bwd_(dout, ids, table, sq)
+        want = torch.zeros(300, 264, device="cuda", dtype=torch.float64).index_add_(0, ids, dout.double())
+        assert torch.allclose(table.double(), want, rtol=1e-4, atol=1e-4)  # up to 200 fp32 additions in any order
+        assert abs(sq.item() / table.double().pow(2).sum().item() - 1.0) < 1e-5

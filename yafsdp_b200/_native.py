@@ -148,6 +148,8 @@ def _declare(l: ctypes.CDLL) -> None:
         "yf_gemm_bf16": [_P, _P, _P, _I, _I, _I, _L, _L, _L, _I, _I, _I, _I, _F, _I, _P],
         "yf_rmsnorm_fwd": [_P, _P, _P, _P, _I, _I, _F, _P],
         "yf_rmsnorm_bwd": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _P],
+        "yf_rmsnorm_bwd_partials": [_I, _I],
+        "yf_rmsnorm_bwd_ws": [_P, _P, _P, _P, _P, _P, _P, _I, _P, _I, _I, _P],
         "yf_rope": [_P, _P, _I, _I, _L, _I, _I, _I, _I, _P],
         "yf_swiglu_fwd": [_P, _P, _L, _I, _P],
         "yf_swiglu_bwd": [_P, _P, _P, _L, _I, _P],
@@ -156,6 +158,7 @@ def _declare(l: ctypes.CDLL) -> None:
         "yf_scaled_sum": [_P, _L, _P, _P, _P],
         "yf_embedding_fwd": [_P, _P, _P, _L, _I, _I, _P],
         "yf_embedding_bwd": [_P, _P, _P, _L, _I, _I, _P],
+        "yf_embedding_bwd_norm": [_P, _P, _P, _P, _P, _L, _I, _I, _P],
         "yf_adamw": [_P, _P, _P, _P, _P, _P, _L, _F, _F, _F, _F, _F, _I, _I, _P],
         "yf_sumsq": [_P, _L, _P, _P],
         "yf_sumsq_partials": [_P, _L, _P, _I, _P],

@@ -161,9 +161,10 @@ def flush_pushed(deferred: "list[tuple[Any, ...]]") -> None:
     deferred.clear()
 
 
-def _norm_weight_grad(w: torch.Tensor, fn: Any, self_zeroing: bool = False) -> torch.Tensor | None:
-    """Run ``fn(dw_fp32)`` (a kernel that atomically accumulates into dw); returns the gradient unless sunk.
-    ``self_zeroing``: the kernel can clear its target itself and is called as ``fn(dw, zero)``."""
+def _norm_weight_grad(w: torch.Tensor, fn: Any, self_zeroing: bool = False, self_norm: bool = False) -> torch.Tensor | None:
+    """Run ``fn(dw_fp32)`` (a kernel that accumulates into dw); returns the gradient unless sunk.
+    ``self_zeroing``: the kernel can clear its target itself and is called as ``fn(dw, zero)``.  ``self_norm``: the kernel can
+    sum the squares of a gradient that starts from zeros and is called as ``fn(dw, target or None)``."""
     s = _sink(w)
     if s is not None and s.pushes():
         dw = torch.empty(w.shape, device=w.device, dtype=torch.float32) if self_zeroing else torch.zeros(w.shape, device=w.device, dtype=torch.float32)
@@ -172,6 +173,10 @@ def _norm_weight_grad(w: torch.Tensor, fn: Any, self_zeroing: bool = False) -> t
         return None
     if s is not None and s.local_ok:
         zeroed_now = not s.would_accumulate()
+        if self_norm:
+            view, _ = s.begin(zero=True)
+            fn(view, s.norm_target(not zeroed_now))
+            return None
         if self_zeroing:
             view, _ = s.begin(zero=False)
             fn(view, zeroed_now)
@@ -210,7 +215,7 @@ class EmbeddingFn(torch.autograd.Function):
         (ids,) = ctx.saved_tensors
         table = ctx.table
         dout2 = _c(dout).view(-1, table.shape[1])
-        grad = _norm_weight_grad(table, lambda dw: kernels.embedding_bwd_(dout2, ids.reshape(-1), dw))
+        grad = _norm_weight_grad(table, lambda dw, sumsq=None: kernels.embedding_bwd_(dout2, ids.reshape(-1), dw, sumsq), self_norm=True)
         return None, grad
 
 

@@ -267,9 +267,18 @@ def rmsnorm_bwd(x: torch.Tensor, w: torch.Tensor, dy: torch.Tensor, rstd: torch.
     t, d = x.shape
     dx = torch.empty_like(x)
     assert dw_f32.dtype == torch.float32 and dw_f32.numel() == d
-    _check(_native.lib().yf_rmsnorm_bwd(x.data_ptr(), w.data_ptr(), dy.data_ptr(), rstd.data_ptr(), _ptr(dres), dx.data_ptr(),
-                                        dw_f32.data_ptr(), int(zero_dw), t, d, _stream()), "yf_rmsnorm_bwd")
+    partials = torch.empty(_rmsnorm_bwd_partials(t, d, x.device.index) * d, device=x.device, dtype=torch.float32)
+    _check(_native.lib().yf_rmsnorm_bwd_ws(x.data_ptr(), w.data_ptr(), dy.data_ptr(), rstd.data_ptr(), _ptr(dres), dx.data_ptr(),
+                                           dw_f32.data_ptr(), int(zero_dw), partials.data_ptr(), t, d, _stream()), "yf_rmsnorm_bwd")
     return dx
+
+
+@functools.lru_cache(maxsize=4096)
+def _rmsnorm_bwd_partials(t: int, d: int, device: int | None) -> int:
+    rows = _native.lib().yf_rmsnorm_bwd_partials(t, d)
+    if rows < 1:
+        raise RuntimeError(f"yf_rmsnorm_bwd failed with code {rows}")
+    return rows
 
 
 def rope_(qkv: torch.Tensor, cos_sin: torch.Tensor, seq_len: int, col0: int, n_heads: int, head_dim: int,
@@ -332,10 +341,12 @@ def embedding_fwd(table: torch.Tensor, ids: torch.Tensor) -> torch.Tensor:
     return out
 
 
-def embedding_bwd_(dout: torch.Tensor, ids: torch.Tensor, dtable_f32: torch.Tensor) -> None:
+def embedding_bwd_(dout: torch.Tensor, ids: torch.Tensor, dtable_f32: torch.Tensor, sumsq: torch.Tensor | None = None) -> None:
+    """``dtable[ids[t]] += dout[t]``.  ``sumsq`` (only where ``dtable`` was all zeros before): ``+= sum(dtable**2)``."""
     v, d = dtable_f32.shape
-    _check(_native.lib().yf_embedding_bwd(dout.data_ptr(), ids.data_ptr(), dtable_f32.data_ptr(), ids.numel(), d, v, _stream()),
-           "yf_embedding_bwd")
+    owner = torch.empty(v, device=dout.device, dtype=torch.int32) if sumsq is not None else None
+    _check(_native.lib().yf_embedding_bwd_norm(dout.data_ptr(), ids.data_ptr(), dtable_f32.data_ptr(), _ptr(owner), _ptr(sumsq), ids.numel(),
+                                               d, v, _stream()), "yf_embedding_bwd")
 
 
 def adamw_(p: torch.Tensor, g: torch.Tensor, m: torch.Tensor, v: torch.Tensor, p_bf16: torch.Tensor | None,
