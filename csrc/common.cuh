@@ -143,6 +143,7 @@ YF_DEVINL void tma_reduce_add_2d(const CUtensorMap* m, const void* smem_src, int
                "r"(smem_u32(smem_src)), "r"(x), "r"(y)
                : "memory");
 }
+YF_DEVINL void tma_store_wait_read3() { asm volatile("cp.async.bulk.wait_group.read 3;" ::: "memory"); }
 YF_DEVINL void tma_store_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 YF_DEVINL void named_bar_sync(int id, int nthreads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory"); }
 // named barrier that also ORs a predicate over its participants: every thread learns whether ANY of them raised it.  Used

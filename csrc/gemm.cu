@@ -15,6 +15,7 @@
 
 #include <atomic>
 #include <numeric>
+#include <utility>
 
 #include "common.cuh"
 #include "yafsdp_b200.h"
@@ -33,7 +34,8 @@ constexpr int WIDE_THREADS = 224;  // one more warp: plain mode's second TMA pro
 // instantiation of its own: the exchange's code alone costs the plain kernel 0.3 us per tile).  MODE_SCATTER: GEMM -> reduce-scatter, the fp32 rows of C are pushed to the
 // ranks that own them.  MODE_GATHER: all-gather -> GEMM, the kernel also gathers the layer that B is part of (see FusedArgs).
 // MODE_SWIGLU: the gate and up projections of an MLP with their activation (see GemmArgs).
-constexpr int MODE_PLAIN = 0, MODE_SCATTER = 1, MODE_GATHER = 2, MODE_SPLIT = 3, MODE_SWIGLU = 4;
+// MODE_SWAP: C is stored transposed: A is the weight, B the tokens, whose tile is any multiple of 16 wide (see GemmArgs::bn).
+constexpr int MODE_PLAIN = 0, MODE_SCATTER = 1, MODE_GATHER = 2, MODE_SPLIT = 3, MODE_SWIGLU = 4, MODE_SWAP = 5;
 __host__ __device__ constexpr bool is_plain(int mode) { return mode != MODE_SCATTER && mode != MODE_GATHER; }
 constexpr int SCATTER_COLS = 64;                         // columns per pushed row piece: 256 bytes of fp32
 constexpr int SCATTER_PITCH = SCATTER_COLS * 4 + 16;     // row pitch of the staging block (16 B of padding: no bank conflicts)
@@ -74,7 +76,11 @@ struct GemmArgs {
   // epilogue writes silu(gate) * up, of the values as rounded to bf16, through maps.a[1] and, with store_gu, gate and up into
   // the halves of C.
   int store_gu;
-  // B in several pieces of memory (plain and split mode): parts[i] is where piece i ends, in rows of [N, K] storage (then no
+  // MODE_SWAP: M counts the output's columns (rows of the weight, operand A) and N its rows (tokens, operand B), so that the
+  // padding of a ragged number of tokens shrinks from a multiple of 256 to one of 16 and the width of a tile can be chosen for
+  // full waves.  bn: tokens per tile, half of them in each CTA of the pair.
+  int bn;
+  // B (MODE_SWAP: A) in several pieces of memory (plain modes): parts[i] is where piece i ends, in rows of [N, K] storage (then no
   // tile crosses a piece's end) or of [K, N] storage (no K block does).  n_parts <= 1: one piece.
   int n_parts;
   int parts[MAX_GROUP];
@@ -309,7 +315,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
   const int lane = threadIdx.x & 31;
   const int K = args.K;
   const int num_m = (args.M + TILE_M - 1) / TILE_M;
-  const int num_n = (args.N + BLOCK_N - 1) / BLOCK_N;
+  const int bn = MODE == MODE_SWAP ? args.bn : BLOCK_N;
+  const int num_n = (args.N + bn - 1) / bn;
   const int num_k = (K + BLOCK_K - 1) / BLOCK_K;
   const bool grouped = (MODE == MODE_SCATTER) && args.n_prob > 0;
   const int num_tiles = grouped ? args.steps : num_m * num_n;  // steps of the tile loop (a grouped step may be empty)
@@ -368,7 +375,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
     const int gsize = min(GROUP_M, num_m - first_m);
     const int r = t - g * per_group;
     m0 = (first_m + r % gsize) * TILE_M + (int)crank * BLOCK_M;
-    n0 = (r / gsize) * BLOCK_N;
+    n0 = (r / gsize) * bn;
     return true;
   };
 
@@ -391,12 +398,17 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
         if (!tile_coords(w.tile, p, m0, n0)) continue;
         const CUtensorMap* tma_a = &maps.a[p];
         const CUtensorMap* tma_b = &maps.b[p];
-        int b_at = 0;  // first row of the current piece of B
-        if (is_plain(MODE) && args.n_parts > 1 && !args.b_mn)
-          for (int i = 0; n0 >= args.parts[i]; ++i) {
-            b_at = args.parts[i];
-            tma_b = &maps.b[i + 1];
-          }
+        // the weight may lie in pieces: B, or A in the swapped form; w_at: first row of the current one
+        constexpr bool SWAP = MODE == MODE_SWAP;
+        const bool w_mn = SWAP ? args.a_mn : args.b_mn;
+        int w_at = 0;
+        auto next_piece = [&](int i) {
+          w_at = args.parts[i];
+          if (SWAP) tma_a = &maps.a[i + 1];
+          else tma_b = &maps.b[i + 1];
+        };
+        if (is_plain(MODE) && args.n_parts > 1 && !w_mn)
+          for (int i = 0; (SWAP ? m0 : n0) >= args.parts[i]; ++i) next_piece(i);
         const int N = grouped ? args.Np[p] : args.N;
         if (MODE == MODE_GATHER) {
           // the rows [n0, n0 + BLOCK_N) of B must have landed in the local layer buffer: the column block's counter says so
@@ -419,33 +431,32 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
           }
           if (!alive) break;
         }
-        int nb = n0 + (int)crank * B_ROWS - (args.b_mn ? 0 : b_at);  // first B row this CTA holds
+        int nb = n0 + (int)crank * (SWAP ? bn / 2 : B_ROWS) - (!SWAP && !args.b_mn ? w_at : 0);  // first B row this CTA holds
+        const int ma = m0 - (SWAP && !args.a_mn ? w_at : 0);
+        const uint32_t stage_tx = SWAP ? Cfg::A_BYTES + bn / 2 * (BLOCK_K * 2) : Cfg::STAGE_BYTES;  // bytes that land in a CTA's stage
         if (MODE == MODE_SWIGLU) {  // a pair: its leader holds gate rows, the other CTA the same rows of up
           nb = n0 / 2;
           tma_b = &maps.b[crank];
         }
-        const bool k_parts = is_plain(MODE) && args.n_parts > 1 && args.b_mn;
+        const bool k_parts = is_plain(MODE) && args.n_parts > 1 && w_mn;
         int piece = 0;
         int kb = w.kb0 + skip;
         for (; kb < w.kb1; kb += PRODUCERS) {
           if (k_parts)
-            while (kb * BLOCK_K >= args.parts[piece]) {
-              b_at = args.parts[piece++];
-              tma_b = &maps.b[piece];
-            }
+            while (kb * BLOCK_K >= args.parts[piece]) next_piece(piece++);
           if (!mbar_wait(&empty[s], ph ^ 1, 10)) { alive = false; break; }
           uint8_t* sa = smem + s * Cfg::STAGE_BYTES;
           uint8_t* sb = sa + Cfg::A_BYTES;
-          const int k0 = kb * BLOCK_K, kb0 = args.b_mn ? k0 - b_at : k0;
+          const int k0 = kb * BLOCK_K, ka0 = SWAP && args.a_mn ? k0 - w_at : k0, kb0 = !SWAP && args.b_mn ? k0 - w_at : k0;
           if (CG == 2) {
             // both CTAs' bytes are counted on the leader's barrier (the thread that issues the MMAs waits there)
-            if (leader) mbar_expect_tx(&full[s], 2 * Cfg::STAGE_BYTES);
+            if (leader) mbar_expect_tx(&full[s], 2 * stage_tx);
             const uint32_t fb = full_leader + s * 8;
             if (!args.a_mn) {
-              tma_load_2d_pair(sa, tma_a, fb, k0, m0);
+              tma_load_2d_pair(sa, tma_a, fb, ka0, ma);
             } else {
 #pragma unroll
-              for (int j = 0; j < BLOCK_M / 64; ++j) tma_load_2d_pair(sa + j * (BLOCK_K * 128), tma_a, fb, m0 + j * 64, k0);
+              for (int j = 0; j < BLOCK_M / 64; ++j) tma_load_2d_pair(sa + j * (BLOCK_K * 128), tma_a, fb, ma + j * 64, ka0);
             }
             if (!args.b_mn) {
               tma_load_2d_pair(sb, tma_b, fb, kb0, nb);
@@ -454,12 +465,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
               for (int j = 0; j < B_ROWS / 64; ++j) tma_load_2d_pair(sb + j * (BLOCK_K * 128), tma_b, fb, nb + j * 64, kb0);
             }
           } else {
-            mbar_expect_tx(&full[s], Cfg::STAGE_BYTES);
+            mbar_expect_tx(&full[s], stage_tx);
             if (!args.a_mn) {
-              tma_load_2d(sa, tma_a, &full[s], k0, m0);
+              tma_load_2d(sa, tma_a, &full[s], ka0, ma);
             } else {
 #pragma unroll
-              for (int j = 0; j < BLOCK_M / 64; ++j) tma_load_2d(sa + j * (BLOCK_K * 128), tma_a, &full[s], m0 + j * 64, k0);
+              for (int j = 0; j < BLOCK_M / 64; ++j) tma_load_2d(sa + j * (BLOCK_K * 128), tma_a, &full[s], ma + j * 64, ka0);
             }
             if (!args.b_mn) {
               tma_load_2d(sb, tma_b, &full[s], kb0, nb);
@@ -482,7 +493,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (pairs: the leader CTA issues for both)
     if (leader && elect_one()) {
-      const uint32_t idesc = umma_idesc_bf16(TILE_M, BLOCK_N, args.a_mn, args.b_mn);
+      const uint32_t idesc = umma_idesc_bf16(TILE_M, bn, args.a_mn, args.b_mn);
       // Shared-memory descriptors: the upper words are constants, the lower ones advance by the stage and the K step (in
       // units of 16 bytes; the whole of shared memory fits the address field).  One thread issues everything: what it
       // computes per K block has to stay below the 256 to 512 cycles that the block's MMAs take.
@@ -739,6 +750,42 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
         }
         tmem_st_wait();
       }
+      if constexpr (MODE == MODE_SWAP) {
+        // a thread owns an output column (weight row), TMEM columns are tokens: 32 tokens at a time through a block of
+        // [32 tokens x 32 columns] bf16 (a warp's stores fill one 64-byte row each), two TMA stores of 16 tokens
+        const int col = m0 + r_in_tile;
+#pragma unroll 1
+        for (int c = 0; c < bn; c += 32, ++chunk_ctr) {
+          uint8_t* stg = staging + q * 8192 + (chunk_ctr & 3) * 2048;
+          if (lane == 0) tma_store_wait_read3();  // the stores that last read this block have finished reading
+          __syncwarp();
+          unsigned short res[32];
+          if (args.R != nullptr) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              res[j] = col < M && n0 + c + j < N ? __ldg(static_cast<const unsigned short*>(args.R) + (long long)(n0 + c + j) * args.ldr + col) : 0;
+          }
+          uint32_t r[32];
+          tmem_ld32(taddr + c, r);
+          tmem_ld_wait();
+          if (c + 32 >= bn) free_accumulator();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            float v = alpha * __uint_as_float(r[j]);
+            if (args.R != nullptr) v = fmaf(alpha, __uint_as_float(r[j]), __uint_as_float((uint32_t)res[j] << 16));
+            *reinterpret_cast<__nv_bfloat16*>(stg + j * 64 + lane * 2) = __float2bfloat16_rn(v);
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            const int x = m0 + q * 32;
+            if (x < M && n0 + c < N) tma_store_2d(&tma_c, stg, x, n0 + c);
+            if (x < M && c + 16 < bn && n0 + c + 16 < N) tma_store_2d(&tma_c, stg + 1024, x, n0 + c + 16);
+            tma_store_commit();
+          }
+        }
+        continue;
+      }
       if constexpr (MODE == MODE_SWIGLU) {
         // 64 columns of one output: 32 packed pairs of this thread's row -> this warp's staging block -> TMA store
         auto store64 = [&](const CUtensorMap* map, int x, const uint32_t (&v)[32]) {  // (F is a multiple of a tile's 128)
@@ -897,10 +944,12 @@ int launch_gemm(const Operands* ops, int n_ops, GemmArgs args, const FusedArgs& 
   memset(&maps, 0, sizeof(maps));
   for (int i = 0; i < n_ops; ++i) {
     const Operands& o = ops[i];
-    const CUtensorMap* ma = args.a_mn ? yf_tensor_map_2d(o.A, o.M, args.K, o.lda, 64, BLOCK_K, 2, 1)
-                                      : yf_tensor_map_2d(o.A, args.K, o.M, o.lda, BLOCK_K, BLOCK_M, 2, 1);
-    const CUtensorMap* mb = args.b_mn ? yf_tensor_map_2d(o.B, o.N, o.K, o.ldb, 64, BLOCK_K, 2, 1)
-                                      : yf_tensor_map_2d(o.B, o.K, o.N, o.ldb, BLOCK_K, Cfg::B_ROWS, 2, 1);
+    constexpr bool SWAP = MODE == MODE_SWAP;
+    const int ka = SWAP ? o.K : args.K, kb = SWAP ? args.K : o.K, b_rows = SWAP ? args.bn / 2 : Cfg::B_ROWS;
+    const CUtensorMap* ma = args.a_mn ? yf_tensor_map_2d(o.A, o.M, ka, o.lda, 64, BLOCK_K, 2, 1)
+                                      : yf_tensor_map_2d(o.A, ka, o.M, o.lda, BLOCK_K, BLOCK_M, 2, 1);
+    const CUtensorMap* mb = args.b_mn ? yf_tensor_map_2d(o.B, o.N, kb, o.ldb, 64, BLOCK_K, 2, 1)
+                                      : yf_tensor_map_2d(o.B, kb, o.N, o.ldb, BLOCK_K, b_rows, 2, 1);
     if (!ma || !mb) return -2;
     maps.a[i] = *ma;
     maps.b[i] = *mb;
@@ -916,7 +965,8 @@ int launch_gemm(const Operands* ops, int n_ops, GemmArgs args, const FusedArgs& 
     maps.b[i] = maps.b[0];
   }
   const int c_cols = MODE == MODE_SWIGLU && !args.store_gu ? args.N / 2 : args.N;
-  const CUtensorMap* mc = yf_tensor_map_2d(args.C, c_cols, args.M, args.ldc, args.out_f32 ? 32 : 64, 32, args.out_f32 ? 4 : 2, 1);
+  const CUtensorMap* mc = MODE == MODE_SWAP ? yf_tensor_map_2d(args.C, args.M, args.N, args.ldc, 32, 16, 2, 0)
+                                            : yf_tensor_map_2d(args.C, c_cols, args.M, args.ldc, args.out_f32 ? 32 : 64, 32, args.out_f32 ? 4 : 2, 1);
   if (!mc) return -2;
   static bool optin[64] = {};
   if (int rc = ensure_smem_optin(gemm_bf16_tcgen05_kernel<BLOCK_N, CG, MODE>, Cfg::SMEM_BYTES, optin)) return rc;
@@ -944,7 +994,8 @@ int launch_gemm(const Operands* ops, int n_ops, GemmArgs args, const FusedArgs& 
     args.steps = most * fa.world;
     num_tiles = args.steps;
   } else {
-    num_tiles = ((args.M + tile_m - 1) / tile_m) * ((args.N + BLOCK_N - 1) / BLOCK_N);
+    const int bn = MODE == MODE_SWAP ? args.bn : BLOCK_N;
+    num_tiles = ((args.M + tile_m - 1) / tile_m) * ((args.N + bn - 1) / bn);
   }
   int sms = yf_num_sms();
   if (sm_limit > 0 && sm_limit < sms) sms = sm_limit;
@@ -981,9 +1032,9 @@ int launch_gemm(const void* A, const void* B, const GemmArgs& args, const FusedA
 }
 
 // ---- plain mode: tile shape and split of the last wave
-enum Tile : int { TILE_PAIR256 = 1, TILE_256 = 2, TILE_128 = 3, TILE_64 = 4, TILE_PAIR128 = 5 };
+enum Tile : int { TILE_PAIR256 = 1, TILE_256 = 2, TILE_128 = 3, TILE_64 = 4, TILE_PAIR128 = 5, TILE_SWAP = 6 };
 struct Plan {
-  int tile, split_tiles, splits;
+  int tile, split_tiles, splits, bn;  // bn: tokens per tile of TILE_SWAP
   long long counters, bytes;  // workspace: counters (8 bytes each, rounded up to 256 bytes), then the slots
 };
 // Per tile shape, measured on one B200 in a stream of launches: us from launch to the end without main loop, and us per K
@@ -1018,12 +1069,38 @@ float plan_us(const TileShape& t, int M, int N, int K, int units, int splits, bo
   return t.fixed_us + exchange_us + (us > read_us ? us + 0.1f * read_us : read_us + 0.1f * us);
 }
 
+// The swapped form: pairs of 256 weight rows x bn tokens, for every number of token tiles.  A K block takes its MMAs (1.55 ns per
+// token with all units busy, a little more than the unswapped form: the epilogue transposes) or its loads (128 + bn / 2 rows at
+// 122 GB/s per SM), an epilogue 12 ns per token.  Best unswapped / swapped, us:
+//   [333 x 27648 x 5120] 98 / 84, [777 x 8192 x 22016] 265 / 218, [777 x 8192 x 8192] 96 / 84, [1337 x 22016 x 4096] 179 / 166,
+//   [1337 x 4096 x 4096] 42 / 38; [2048 x 22016 x 4096] 243 / 270 and [999 x 27648 x 5120] 199 / 209 stay unswapped.
+float swap_us(int M, int N, int K, int units, int* bn) {
+  const int num_k = (K + BLOCK_K - 1) / BLOCK_K, rows = (N + 255) / 256, least = (M + 255) / 256;
+  const float read_us = ((float)M + (float)N) * (float)K * 2.f / 5.2e6f;
+  float best = 1e30f;
+  for (int nt = least; nt < least + 10; ++nt) {
+    const int w = ((M + nt - 1) / nt + 15) / 16 * 16;
+    if (w > 256 || w < 16) continue;
+    const long long tiles = (long long)rows * ((M + w - 1) / w), waves = (tiles + units - 1) / units;
+    const float mma = 0.00155f * (float)w, load = (128.f + 0.5f * (float)w) * 0.00105f, loop = (float)num_k * (mma > load ? mma : load);
+    const float epi = 0.012f * (float)w, us = (float)waves * (loop > epi ? loop : epi);
+    const float t = 7.f + (us > read_us ? us + 0.1f * read_us : read_us + 0.1f * us);
+    if (t < best) {
+      best = t;
+      *bn = w;
+    }
+  }
+  return best;
+}
+
 // n_align > 0: tiles must end where multiples of n_align columns do (the pieces of B)
-Plan make_plan(int M, int N, int K, bool out_f32, int n_align, int sm_limit, bool may_split, int tile, int splits) {
+// kind: 0 bf16 output that may be computed swapped, 1 fp32 output, 2 any other
+Plan make_plan(int M, int N, int K, int kind, int n_align, int sm_limit, bool may_split, int tile, int splits, float* us = nullptr) {
+  const bool out_f32 = kind == 1;
   int sms = yf_num_sms();
   if (sm_limit > 0 && sm_limit < sms) sms = sm_limit;
   const int num_k = (K + BLOCK_K - 1) / BLOCK_K;
-  Plan best = {0, 0, 1, 0, 0};
+  Plan best = {0, 0, 1, 0, 0, 0};
   float best_c = 0.f;
   for (int t = 1; t <= 5; ++t) {
     if (tile > 0 && t != tile) continue;
@@ -1041,7 +1118,16 @@ Plan make_plan(int M, int N, int K, bool out_f32, int n_align, int sm_limit, boo
       }
     }
   }
-  if (best.tile == 0) return best;
+  if (kind == 0 && (tile == 0 || tile == TILE_SWAP) && splits <= 1 && n_align % 256 == 0 && sms >= 2) {
+    int bn = 0;
+    const float c = swap_us(M, N, K, sms / 2, &bn);
+    if (bn > 0 && (best.tile == 0 || c < best_c)) {
+      best = {TILE_SWAP, 0, 1, bn, 0, 0};
+      best_c = c;
+    }
+  }
+  if (us != nullptr) *us = best_c;
+  if (best.tile == 0 || best.tile == TILE_SWAP) return best;
   const TileShape& t = TILE_SHAPES[best.tile];
   const int tile_m = BLOCK_M * t.cg, units = sms / t.cg;
   const long long tiles = (long long)((M + tile_m - 1) / tile_m) * ((N + t.bn - 1) / t.bn);
@@ -1088,17 +1174,27 @@ int launch_plain(const Operands* ops, int n_ops, GemmArgs args, const FusedArgs&
     for (int i = n_ops - 1; i < MAX_GROUP; ++i) args.parts[i] = INT_MAX;  // searches stop at the last piece
   }
   const bool ws = workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255) == 0;
-  Plan p = make_plan(args.M, args.N, args.K, args.out_f32 != 0, n_align, sm_limit, ws, tile, splits);
-  if (p.bytes > workspace_bytes) p = make_plan(args.M, args.N, args.K, args.out_f32 != 0, n_align, sm_limit, false, tile, 1);
+  const int kind = args.out_f32 ? 1 : (args.a_mn || args.accumulate ? 2 : 0);
+  Plan p = make_plan(args.M, args.N, args.K, kind, n_align, sm_limit, ws, tile, splits);
+  if (p.bytes > workspace_bytes) p = make_plan(args.M, args.N, args.K, kind, n_align, sm_limit, false, tile, 1);
   if (p.tile == 0) return -1;
   args.splits = p.splits;
+  if (p.tile == TILE_SWAP) {
+    Operands swapped[MAX_GROUP];
+    for (int i = 0; i < n_ops; ++i) swapped[i] = {ops[i].B, ops[i].A, ops[i].ldb, ops[i].lda, ops[i].N, ops[i].M, ops[i].K};
+    std::swap(args.M, args.N);
+    args.a_mn = args.b_mn;
+    args.b_mn = 0;
+    args.bn = p.bn;
+    return launch_gemm<256, 2, MODE_SWAP>(swapped, n_ops, args, fa, sm_limit, s);
+  }
   if (p.splits > 1) {
     args.split_tiles = p.split_tiles;
     args.nonce = next_nonce();
     args.counters = static_cast<unsigned long long*>(workspace);
     args.slots = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + p.counters);
+    return launch_tile<MODE_SPLIT>(p.tile, ops, n_ops, args, fa, sm_limit, s);
   }
-  if (p.splits > 1) return launch_tile<MODE_SPLIT>(p.tile, ops, n_ops, args, fa, sm_limit, s);
   return launch_tile<MODE_PLAIN>(p.tile, ops, n_ops, args, fa, sm_limit, s);
 }
 
@@ -1195,16 +1291,17 @@ extern "C" int yf_gemm_bf16_residual(const void* A, const void* B, void* C, cons
 
 // The general form of the entries above.  `workspace` (256-byte aligned device memory that no other launch uses meanwhile, its
 // contents do not matter) lets the last wave's tiles be split along K; yf_gemm_workspace says how much a problem wants, with
-// less (or none) no tile is split.  tile, splits: 0 = chosen from the shape; else a Tile and 1 to MAX_SPLITS.
-extern "C" int yf_gemm_workspace(int M, int N, int K, int out_f32, int n_align, int sm_limit, int tile, int splits, long long* bytes) {
-  if (M <= 0 || N <= 0 || K <= 0 || n_align < 0 || bytes == nullptr || tile < 0 || tile > 5 || splits < 0 || splits > MAX_SPLITS) return -1;
-  *bytes = make_plan(M, N, K, out_f32 != 0, n_align, sm_limit, true, tile, splits).bytes;
+// less (or none) no tile is split.  kind: 0 bf16 output of a K-major A, 1 fp32 output, 2 any other.  tile, splits: 0 = chosen from the shape; else a Tile (TILE_SWAP with
+// kind 0 only) and 1 to MAX_SPLITS.
+extern "C" int yf_gemm_workspace(int M, int N, int K, int kind, int n_align, int sm_limit, int tile, int splits, long long* bytes) {
+  if (M <= 0 || N <= 0 || K <= 0 || kind < 0 || kind > 2 || n_align < 0 || bytes == nullptr || tile < 0 || tile > 6 || splits < 0 || splits > MAX_SPLITS) return -1;
+  *bytes = make_plan(M, N, K, kind, n_align, sm_limit, true, tile, splits).bytes;
   return 0;
 }
 extern "C" int yf_gemm_bf16_ws(const void* A, const void* B, void* C, const void* R, int M, int N, int K, long long lda, long long ldb,
                                long long ldc, long long ldr, int a_mn, int b_mn, int out_f32, int accumulate, float alpha, int sm_limit,
                                const float* alpha_ptr, float* sumsq, void* workspace, long long workspace_bytes, int tile, int splits, void* stream) {
-  if (M <= 0 || N <= 0 || K <= 0 || tile < 0 || tile > 5 || splits < 0 || splits > MAX_SPLITS) return -1;
+  if (M <= 0 || N <= 0 || K <= 0 || tile < 0 || tile > 6 || splits < 0 || splits > MAX_SPLITS) return -1;
   if (sumsq != nullptr && (!out_f32 || accumulate)) return -1;
   if ((lda % 8) || (ldb % 8) || (ldc % (out_f32 ? 4 : 8))) return -1;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15) return -1;
@@ -1236,7 +1333,7 @@ extern "C" int yf_gemm_bf16_ws(const void* A, const void* B, void* C, const void
 extern "C" int yf_gemm_bf16_parts(const void* A, int n, const void* const* B, const int* rows, const long long* ldb, void* C, int M,
                                   int N, int K, long long lda, long long ldc, int b_mn, void* workspace, long long workspace_bytes,
                                   int tile, int splits, void* stream) {
-  if (M <= 0 || N <= 0 || K <= 0 || n < 2 || n > MAX_GROUP || tile < 0 || tile > 5 || splits < 0 || splits > MAX_SPLITS) return -1;
+  if (M <= 0 || N <= 0 || K <= 0 || n < 2 || n > MAX_GROUP || tile < 0 || tile > 6 || splits < 0 || splits > MAX_SPLITS) return -1;
   if ((lda % 8) || (ldc % 8) || ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(C)) & 15)) return -1;
   Operands ops[MAX_GROUP];
   long long total = 0;
@@ -1289,12 +1386,8 @@ extern "C" int yf_gemm_swiglu_pays(int M, int F, int K) {
   if (M <= 0 || F <= 0 || K <= 0) return -1;
   if (F % 128) return 0;
   const int sms = yf_num_sms(), num_k = (K + BLOCK_K - 1) / BLOCK_K;
-  float best = 1e30f;
-  for (int t = 1; t <= 5; ++t)
-    for (int sp = 1; sp <= MAX_SPLITS && (sp == 1 || num_k >= 4 * sp); ++sp) {
-      const float us = plan_us(TILE_SHAPES[t], M, 2 * F, K, sms / TILE_SHAPES[t].cg, sp, false);
-      if (us < best) best = us;
-    }
+  float best = 0.f;
+  make_plan(M, 2 * F, K, 0, 0, 0, true, 0, 0, &best);
   const TileShape& t = TILE_SHAPES[TILE_PAIR256];
   const long long tiles = (long long)((M + 255) / 256) * (F / 128), units = sms / 2;
   const float loop = (float)num_k * t.kb_us;

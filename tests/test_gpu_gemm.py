@@ -193,3 +193,33 @@ def test_gemm_alpha_from_device():
         got = kernels.gemm(a, b, out_dtype=torch.float32, alpha=2.0, alpha_tensor=alpha, tile=3, splits=splits)
         want = kernels.gemm(a, b, out_dtype=torch.float32, tile=3, splits=splits) * (2.0 * alpha)
         assert torch.allclose(got, want, rtol=2.0**-22, atol=0.0)
+
+
+@pytest.mark.parametrize("m", [1, 16, 45, 208, 250, 257, 333, 777, 1337])
+@pytest.mark.parametrize("n,k", [(8, 72), (256, 1032), (1000, 264), (2056, 512)])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_gemm_swapped_form(m, n, k, b_mn):
+    """Tokens as the narrow operand: every width of a tile, ragged edges on both sides, residual and alpha (bf16 results: 2^-8),
+    and the weight in pieces."""
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(13)
+    a = torch.randn(m, k, device="cuda").bfloat16()
+    b = torch.randn((k, n) if b_mn else (n, k), device="cuda").bfloat16()
+    res = torch.randn(m, n, device="cuda").bfloat16()
+    big = torch.full((m + 2, n + 8), 7.0, device="cuda").bfloat16()
+    ref = a.double() @ (b.double() if b_mn else b.double().t())
+    got = kernels.gemm(a, b, b_mn_major=b_mn, tile=6, out=big[1 : m + 1, :n])
+    with_res = kernels.gemm(a, b, b_mn_major=b_mn, tile=6, residual=res, alpha=0.5)
+    if b_mn:
+        parts = [b[: k // 128 * 64], b[k // 128 * 64 :]] if k >= 128 else None
+    else:
+        parts = [b[:256], b[256:]] if n > 256 else None
+    torch.cuda.synchronize()
+    kernels.check_status()
+    assert ((got.double() - ref).norm() / ref.norm()).item() < 2.0**-8
+    assert (big[0] == 7).all() and (big[m + 1] == 7).all() and (big[1 : m + 1, n:] == 7).all()
+    want = 0.5 * ref + res.double()
+    assert ((with_res.double() - want).norm() / want.norm()).item() < 2.0**-8
+    if parts is not None:
+        assert torch.equal(kernels.gemm_parts(a, parts, b_mn_major=b_mn, tile=6), got)

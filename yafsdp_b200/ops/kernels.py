@@ -97,7 +97,7 @@ def gemm(
     dimension); the row pitch may exceed the row length.  ``sumsq`` (fp32 output without accumulation only): a
     one-element fp32 tensor that receives ``+= sum(out**2)`` from the same kernel.  ``residual`` (bf16 output without
     accumulation only): a bf16 ``[M,N]`` tensor added in fp32 inside the epilogue, before the output is rounded.
-    ``tile`` (1-5) and ``splits`` (1-4): tile shape and K ranges of the last wave's tiles; 0 chooses them from the shape.
+    ``tile`` (1-6) and ``splits`` (1-4): tile shape and K ranges of the last wave's tiles; 0 chooses them from the shape.
     ``alpha_tensor``: one fp32 value on the device that ``alpha`` is multiplied by (read by the kernel).
     """
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.is_cuda and b.is_cuda
@@ -119,7 +119,8 @@ def gemm(
         assert out.dtype == torch.bfloat16 and not accumulate and sumsq is None
         assert residual.dtype == torch.bfloat16 and residual.shape == (m, n) and residual.stride(1) == 1
     assert alpha_tensor is None or (alpha_tensor.dtype == torch.float32 and alpha_tensor.numel() == 1 and alpha_tensor.device == a.device)
-    nbytes = _gemm_workspace(m, n, k, int(out.dtype == torch.float32), 0, sm_limit, tile, splits, a.device.index)
+    kind = 1 if out.dtype == torch.float32 else (2 if a_mn_major or accumulate else 0)
+    nbytes = _gemm_workspace(m, n, k, kind, 0, sm_limit, tile, splits, a.device.index)
     ws = torch.empty(nbytes, device=a.device, dtype=torch.uint8) if nbytes else None
     rc = _native.lib().yf_gemm_bf16_ws(
         a.data_ptr(), b.data_ptr(), out.data_ptr(), _ptr(residual), m, n, k, a.stride(0), b.stride(0), out.stride(0),
@@ -131,10 +132,10 @@ def gemm(
 
 
 @functools.lru_cache(maxsize=4096)
-def _gemm_workspace(m: int, n: int, k: int, out_f32: int, n_align: int, sm_limit: int, tile: int, splits: int, device: int | None) -> int:
+def _gemm_workspace(m: int, n: int, k: int, kind: int, n_align: int, sm_limit: int, tile: int, splits: int, device: int | None) -> int:
     """Workspace bytes that a GEMM wants (a function of its shape and the device's number of SMs)."""
     nbytes = ctypes.c_longlong(0)
-    rc = _native.lib().yf_gemm_workspace(m, n, k, out_f32, n_align, int(sm_limit), tile, splits, ctypes.byref(nbytes))
+    rc = _native.lib().yf_gemm_workspace(m, n, k, kind, n_align, int(sm_limit), tile, splits, ctypes.byref(nbytes))
     if rc != 0:
         raise RuntimeError(f"yf_gemm_workspace failed with code {rc}")
     return nbytes.value
