@@ -1061,7 +1061,7 @@ float plan_us(const TileShape& t, int M, int N, int K, int units, int splits, bo
   if (rest > 0 && splits == 1) us += tile_us;
   if (rest > 0 && splits > 1) {
     const float rounds = (float)((rest * splits + units - 1) / units), part = loop / (float)splits;
-    us += rounds * (rounds > 1.f && part < 9.f ? 9.f : part);
+    us += rounds * ((rounds > 1.f && part < 9.f ? 9.f : part) + 4.f);
     us *= 1.1f;
   }
   const float exchange_us = rest == 0 || splits == 1 ? 0.f : (full > 0 ? 3.f : 2.f + 4.f * (float)splits);

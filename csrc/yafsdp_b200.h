@@ -57,10 +57,10 @@ int yf_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int T, in
 /* dx (+ dres) and dw += column sums of dy * xhat; zero_dw: dw is cleared first, inside the dx kernel (no fill launch) */
 int yf_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float* rstd, const void* dres, void* dx,
                    float* dw, int zero_dw, int T, int D, void* stream);
-/* the same with the weight gradient summed in a fixed order: partials [yf_rmsnorm_bwd_partials(T, D), D] fp32 scratch */
+/* the same with the weight gradient summed in a fixed order and, optionally, *sumsq += its squares: partials [yf_rmsnorm_bwd_partials(T, D), D] fp32 scratch */
 int yf_rmsnorm_bwd_partials(int T, int D);
 int yf_rmsnorm_bwd_ws(const void* x, const void* w, const void* dy, const float* rstd, const void* dres, void* dx, float* dw, int zero_dw,
-                      float* partials, int T, int D, void* stream);
+                      float* partials, float* sumsq, int T, int D, void* stream);
 int yf_rope(void* qkv, const float* cos_sin, int T, int seq_len, long long row_stride, int col0, int n_heads,
             int head_dim, int backward, void* stream);
 int yf_swiglu_fwd(const void* gu, void* h, long long T, int F, void* stream);
@@ -69,6 +69,8 @@ int yf_cross_entropy(void* logits, const long long* labels, float* loss_rows, in
                      float grad_scale, const float* scale_ptr, int write_grad, void* stream);
 /* *out = 1 / max(1, number of labels >= 0); *out = sum(x) * *scale in a fixed order: one block each */
 int yf_inv_valid_labels(const long long* labels, long long n, float* out, void* stream);
+/* next-token labels: out[b][s] = labels[b][s + 1] (row pitch ld), -100 at the end of a row */
+int yf_shift_labels(const long long* labels, long long* out, long long batch, int seq, long long ld, void* stream);
 int yf_scaled_sum(const float* x, long long n, const float* scale, float* out, void* stream);
 int yf_embedding_fwd(const void* table, const long long* ids, void* out, long long T, int D, int V, void* stream);
 int yf_embedding_bwd(const void* dout, const long long* ids, float* dtable, long long T, int D, int V, void* stream);
@@ -84,6 +86,8 @@ int yf_scale(float* x, long long n, const float* coef, void* stream);
 int yf_clip_coef(const float* total_sq, float max_norm, float* coef, float* norm_out, void* stream);
 int yf_cast_f32_to_bf16(const float* src, void* dst, long long n, void* stream);
 int yf_accum_bf16_to_f32(const void* src, float* dst, long long n, float scale, int accumulate, void* stream);
+/* dst[i] (=, or += with accumulate) src[i] for count tensors of n[i] elements, in as few launches as fit */
+int yf_accum_bf16_to_f32_multi(int count, const void* const* src, float* const* dst, const long long* n, int accumulate, void* stream);
 int yf_add_bf16(const void* a, const void* b, void* y, long long n, void* stream);
 
 // ---- flash attention, head_dim 128 (attn_fwd.cu, attn_bwd.cu)

@@ -281,3 +281,37 @@ def test_loss_scalars_and_embedding_norm():
         want = torch.zeros(300, 264, device="cuda", dtype=torch.float64).index_add_(0, ids, dout.double())
         assert torch.allclose(table.double(), want, rtol=1e-4, atol=1e-4)  # up to 200 fp32 additions in any order
         assert abs(sq.item() / table.double().pow(2).sum().item() - 1.0) < 1e-5
+
+
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_accumulate_many_bf16_tensors(accumulate):
+    """Tensors of odd sizes at odd places of one flat buffer, more of them than fit a launch, some empty."""
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(14)
+    sizes = [1, 0, 7, 8, 16384, 16385, 40000, 3] * 8
+    flat = torch.randn(sum(sizes) + 1, device="cuda")
+    want, pairs, at = flat.clone(), [], 1
+    for n in sizes:
+        src = torch.randn(n, device="cuda").bfloat16()
+        pairs.append((flat[at : at + n], src))
+        want[at : at + n] = want[at : at + n] + src.float() if accumulate else src.float()
+        at += n
+    kernels.accum_bf16_to_f32_multi_(pairs, accumulate)
+    assert torch.equal(flat, want)
+
+
+def test_shift_labels_and_rmsnorm_weight_norm():
+    from yafsdp_b200.ops import kernels
+
+    labels = torch.arange(30, device="cuda").view(3, 10)
+    for x in (labels, labels[:, 2:7], labels[:, :1]):
+        want = torch.cat([x[:, 1:], x.new_full((3, 1), -100)], dim=1)
+        assert torch.equal(kernels.shift_labels(x), want)
+    torch.manual_seed(15)
+    x, dy = (torch.randn(50, 1032, device="cuda").bfloat16() for _ in range(2))
+    w = torch.ones(1032, device="cuda").bfloat16()
+    _, rstd = kernels.rmsnorm_fwd(x, w, 1e-5)
+    dw, sq = torch.randn(1032, device="cuda"), torch.full((1,), 2.0, device="cuda")
+    kernels.rmsnorm_bwd(x, w, dy, rstd, dw, zero_dw=True, sumsq=sq)
+    assert abs((sq.item() - 2.0) / dw.double().pow(2).sum().item() - 1.0) < 1e-5

@@ -149,12 +149,13 @@ def _declare(l: ctypes.CDLL) -> None:
         "yf_rmsnorm_fwd": [_P, _P, _P, _P, _I, _I, _F, _P],
         "yf_rmsnorm_bwd": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _P],
         "yf_rmsnorm_bwd_partials": [_I, _I],
-        "yf_rmsnorm_bwd_ws": [_P, _P, _P, _P, _P, _P, _P, _I, _P, _I, _I, _P],
+        "yf_rmsnorm_bwd_ws": [_P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _P],
         "yf_rope": [_P, _P, _I, _I, _L, _I, _I, _I, _I, _P],
         "yf_swiglu_fwd": [_P, _P, _L, _I, _P],
         "yf_swiglu_bwd": [_P, _P, _P, _L, _I, _P],
         "yf_cross_entropy": [_P, _P, _P, _I, _I, _L, _F, _P, _I, _P],
         "yf_inv_valid_labels": [_P, _L, _P, _P],
+        "yf_shift_labels": [_P, _P, _L, _I, _L, _P],
         "yf_scaled_sum": [_P, _L, _P, _P, _P],
         "yf_embedding_fwd": [_P, _P, _P, _L, _I, _I, _P],
         "yf_embedding_bwd": [_P, _P, _P, _L, _I, _I, _P],
@@ -166,6 +167,7 @@ def _declare(l: ctypes.CDLL) -> None:
         "yf_clip_coef": [_P, _F, _P, _P, _P],
         "yf_cast_f32_to_bf16": [_P, _P, _L, _P],
         "yf_accum_bf16_to_f32": [_P, _P, _L, _F, _I, _P],
+        "yf_accum_bf16_to_f32_multi": [_I, _P, _P, _P, _I, _P],
         "yf_add_bf16": [_P, _P, _P, _L, _P],
         "yf_attn_fwd": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _L, _L, _L, _F, _I, _P],
         "yf_attn_bwd": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _L, _L, _L, _L, _L, _L, _F, _I, _P],

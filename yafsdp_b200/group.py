@@ -984,6 +984,8 @@ class ParamGroup:
                 if not self._alias_grad and self.layout.padded_numel > self.layout.total_numel:
                     # padding tail: never written by any gradient, must not carry another layer's bytes into the reduction
                     self._grad_flat[self.layout.total_numel :].zero_()
+                dsts_copy = self._accumulate_natively(dsts_copy, False)
+                dsts_add = self._accumulate_natively(dsts_add, True)
                 if dsts_copy:
                     torch._foreach_copy_([d for d, _ in dsts_copy], [s for _, s in dsts_copy])
                 if dsts_add:
@@ -998,6 +1000,23 @@ class ParamGroup:
                 self.reshard()
         with phase_label("YaFSDP::post_backward_reduce", self._module_fqn):
             self._reduce(with_grad, st)
+
+    def _accumulate_natively(self, pairs: list[tuple[torch.Tensor, torch.Tensor]], accumulate: bool) -> list[tuple[torch.Tensor, torch.Tensor]]:
+        """The plain bf16 gradients among ``(place in the flat gradient, gradient)`` pairs into their fp32 places, in one launch;
+        returns the others."""
+        if self.device.type != "cuda":
+            return pairs
+        mine, rest = [], []
+        for d, s in pairs:
+            plain = (type(s) is torch.Tensor and s.dtype == torch.bfloat16 and d.dtype == torch.float32 and s.is_contiguous()
+                     and d.is_contiguous() and s.device == d.device and s.shape == d.shape)
+            (mine if plain else rest).append((d, s))
+        if mine:
+            from .ops import kernels
+
+            with torch.cuda.device(self.device):
+                kernels.accum_bf16_to_f32_multi_(mine, accumulate)
+        return rest
 
     def _finish_pushes(self) -> None:
         """End of a backward pass in push mode: gradients that autograd produced (``.grad``) are pushed now, parameters

@@ -213,7 +213,7 @@ class LlamaForCausalLM(nn.Module):
             x = layer(x, cos_sin, b, s)
         if labels is not None:
             if shift_labels:
-                labels = torch.cat([labels[:, 1:], labels.new_full((b, 1), -100)], dim=1)
+                labels = Fn.shift_labels(labels)
             return self.head(x, labels.reshape(-1))
         return self.head(x, None).view(b, s, -1)
 

@@ -164,7 +164,8 @@ def flush_pushed(deferred: "list[tuple[Any, ...]]") -> None:
 def _norm_weight_grad(w: torch.Tensor, fn: Any, self_zeroing: bool = False, self_norm: bool = False) -> torch.Tensor | None:
     """Run ``fn(dw_fp32)`` (a kernel that accumulates into dw); returns the gradient unless sunk.
     ``self_zeroing``: the kernel can clear its target itself and is called as ``fn(dw, zero)``.  ``self_norm``: the kernel can
-    sum the squares of a gradient that starts from zeros and is called as ``fn(dw, target or None)``."""
+    sum the squares of a gradient that starts from zeros and is called as ``fn(dw, target or None)``; with both,
+    ``fn(dw, zero, target or None)``."""
     s = _sink(w)
     if s is not None and s.pushes():
         dw = torch.empty(w.shape, device=w.device, dtype=torch.float32) if self_zeroing else torch.zeros(w.shape, device=w.device, dtype=torch.float32)
@@ -174,8 +175,9 @@ def _norm_weight_grad(w: torch.Tensor, fn: Any, self_zeroing: bool = False, self
     if s is not None and s.local_ok:
         zeroed_now = not s.would_accumulate()
         if self_norm:
-            view, _ = s.begin(zero=True)
-            fn(view, s.norm_target(not zeroed_now))
+            view, _ = s.begin(zero=not self_zeroing)
+            target = s.norm_target(not zeroed_now)
+            fn(view, zeroed_now, target) if self_zeroing else fn(view, target)
             return None
         if self_zeroing:
             view, _ = s.begin(zero=False)
@@ -286,7 +288,7 @@ class DecoderLayerFn(torch.autograd.Function):
         g_wg, g_wu = _WeightGrad([wg, wu]).run(dgu, n2, pushed)
         del dgu
         box: list[torch.Tensor] = []
-        g_n2 = _norm_weight_grad(w_n2, lambda dw, z: box.append(kernels.rmsnorm_bwd(h, w_n2.detach(), dn2, rstd2, dw, dres=dout, zero_dw=z)), True)
+        g_n2 = _norm_weight_grad(w_n2, lambda dw, z, sq=None: box.append(kernels.rmsnorm_bwd(h, w_n2.detach(), dn2, rstd2, dw, dres=dout, zero_dw=z, sumsq=sq)), True, True)
         dh = box.pop()
         # ---- attention
         datt = kernels.gemm(dh, wo.detach(), b_mn_major=True)
@@ -298,7 +300,7 @@ class DecoderLayerFn(torch.autograd.Function):
         kernels.rope_(dqkv, cos_sin, dims.seq, 0, hq + hkv, hd, backward=True)
         dn1 = _gemm_fused(dqkv, w_qkv, b_mn_major=True)
         g_wq, g_wk, g_wv = _WeightGrad([wq, wk, wv]).run(dqkv, n1, pushed)
-        g_n1 = _norm_weight_grad(w_n1, lambda dw, z: box.append(kernels.rmsnorm_bwd(x, w_n1.detach(), dn1, rstd1, dw, dres=dh, zero_dw=z)), True)
+        g_n1 = _norm_weight_grad(w_n1, lambda dw, z, sq=None: box.append(kernels.rmsnorm_bwd(x, w_n1.detach(), dn1, rstd1, dw, dres=dh, zero_dw=z, sumsq=sq)), True, True)
         dx = box.pop()
         flush_pushed(pushed)
         return dx, g_n1, g_wq, g_wk, g_wv, g_wo, g_n2, g_wg, g_wu, g_wd, None, None, None
@@ -331,7 +333,7 @@ class HeadLossFn(torch.autograd.Function):
         dn = kernels.gemm(dlogits, w_head.detach(), b_mn_major=True, alpha_tensor=scale)
         (g_head,) = _WeightGrad([w_head]).run(dlogits, n, scale=scale)
         box: list[torch.Tensor] = []
-        g_norm = _norm_weight_grad(w_norm, lambda dw, z: box.append(kernels.rmsnorm_bwd(h, w_norm.detach(), dn, rstd, dw, zero_dw=z)), True)
+        g_norm = _norm_weight_grad(w_norm, lambda dw, z, sq=None: box.append(kernels.rmsnorm_bwd(h, w_norm.detach(), dn, rstd, dw, zero_dw=z, sumsq=sq)), True, True)
         return box.pop(), g_norm, g_head, None, None
 
 
@@ -354,7 +356,7 @@ class HeadLogitsFn(torch.autograd.Function):
         dn = kernels.gemm(dlogits, w_head.detach(), b_mn_major=True)
         (g_head,) = _WeightGrad([w_head]).run(dlogits, n)
         box: list[torch.Tensor] = []
-        g_norm = _norm_weight_grad(w_norm, lambda dw, z: box.append(kernels.rmsnorm_bwd(h, w_norm.detach(), dn, rstd, dw, zero_dw=z)), True)
+        g_norm = _norm_weight_grad(w_norm, lambda dw, z, sq=None: box.append(kernels.rmsnorm_bwd(h, w_norm.detach(), dn, rstd, dw, zero_dw=z, sumsq=sq)), True, True)
         return box.pop(), g_norm, g_head, None
 
 
@@ -395,6 +397,13 @@ def decoder_layer(x: torch.Tensor, *weights_and_table: Any) -> torch.Tensor:
     if x.is_cuda:
         return DecoderLayerFn.apply(x, *weights_and_table, torch.is_grad_enabled())
     return decoder_layer_ref(x, *weights_and_table)
+
+
+def shift_labels(labels: torch.Tensor) -> torch.Tensor:
+    """``labels [B, S]`` moved one to the left, -100 (ignored) at the end of every row."""
+    if labels.is_cuda and labels.dtype == torch.int64 and labels.stride(1) == 1:
+        return kernels.shift_labels(labels)
+    return torch.cat([labels[:, 1:], labels.new_full((labels.shape[0], 1), -100)], dim=1)
 
 
 def head_loss(h: torch.Tensor, w_norm: torch.Tensor, w_head: torch.Tensor, labels: torch.Tensor, eps: float) -> torch.Tensor:

@@ -262,15 +262,15 @@ def rmsnorm_fwd(x: torch.Tensor, w: torch.Tensor, eps: float) -> tuple[torch.Ten
 
 
 def rmsnorm_bwd(x: torch.Tensor, w: torch.Tensor, dy: torch.Tensor, rstd: torch.Tensor, dw_f32: torch.Tensor,
-                dres: torch.Tensor | None = None, zero_dw: bool = False) -> torch.Tensor:
+                dres: torch.Tensor | None = None, zero_dw: bool = False, sumsq: torch.Tensor | None = None) -> torch.Tensor:
     """Returns dx (+ dres when given); accumulates the weight gradient into the fp32 tensor ``dw_f32`` (``zero_dw``: the
-    kernel clears it first, which saves the caller a fill launch)."""
+    kernel clears it first, which saves the caller a fill launch; ``sumsq``: ``+= sum(dw_f32**2)`` of the result)."""
     t, d = x.shape
     dx = torch.empty_like(x)
     assert dw_f32.dtype == torch.float32 and dw_f32.numel() == d
     partials = torch.empty(_rmsnorm_bwd_partials(t, d, x.device.index) * d, device=x.device, dtype=torch.float32)
     _check(_native.lib().yf_rmsnorm_bwd_ws(x.data_ptr(), w.data_ptr(), dy.data_ptr(), rstd.data_ptr(), _ptr(dres), dx.data_ptr(),
-                                           dw_f32.data_ptr(), int(zero_dw), partials.data_ptr(), t, d, _stream()), "yf_rmsnorm_bwd")
+                                           dw_f32.data_ptr(), int(zero_dw), partials.data_ptr(), _ptr(sumsq), t, d, _stream()), "yf_rmsnorm_bwd")
     return dx
 
 
@@ -323,6 +323,15 @@ def inv_valid_labels(labels: torch.Tensor) -> torch.Tensor:
     assert labels.dtype == torch.int64 and labels.is_contiguous()
     out = torch.empty(1, device=labels.device, dtype=torch.float32)
     _check(_native.lib().yf_inv_valid_labels(labels.data_ptr(), labels.numel(), out.data_ptr(), _stream()), "yf_inv_valid_labels")
+    return out
+
+
+def shift_labels(labels: torch.Tensor) -> torch.Tensor:
+    """Next-token labels of ``labels [B, S]``: moved one to the left, -100 at the end of every row."""
+    b, s = labels.shape
+    assert labels.dtype == torch.int64 and labels.stride(1) == 1
+    out = torch.empty((b, s), device=labels.device, dtype=torch.int64)
+    _check(_native.lib().yf_shift_labels(labels.data_ptr(), out.data_ptr(), b, s, labels.stride(0), _stream()), "yf_shift_labels")
     return out
 
 
@@ -397,6 +406,14 @@ def accum_bf16_to_f32_(src: torch.Tensor, dst: torch.Tensor, scale: float = 1.0,
     assert src.numel() == dst.numel()
     _check(_native.lib().yf_accum_bf16_to_f32(src.data_ptr(), dst.data_ptr(), src.numel(), float(scale), int(accumulate), _stream()),
            "yf_accum_bf16_to_f32")
+
+
+def accum_bf16_to_f32_multi_(pairs: "list[tuple[torch.Tensor, torch.Tensor]]", accumulate: bool) -> None:
+    """``dst (+)= src`` for ``(dst fp32, src bf16)`` pairs of contiguous tensors of one device, in one launch."""
+    n = len(pairs)
+    _check(_native.lib().yf_accum_bf16_to_f32_multi(
+        n, (ctypes.c_void_p * n)(*[s.data_ptr() for _, s in pairs]), (ctypes.c_void_p * n)(*[d.data_ptr() for d, _ in pairs]),
+        (ctypes.c_longlong * n)(*[d.numel() for d, _ in pairs]), int(accumulate), _stream()), "yf_accum_bf16_to_f32_multi")
 
 
 def add_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
