@@ -47,6 +47,7 @@ struct BwdArgs {
   __nv_bfloat16* dk;   // rows dkv_stride apart, head hk at columns hk*128
   __nv_bfloat16* dv;
   float* dkv_accum;    // head_parts > 1: fp32 sums [2 (dK without scale, dV)][B*S, Hkv*128], zero at the start; else null
+  const float* rope;   // optional [S, 64, 2] (cos, sin): dK goes back through the rotation of K (head dims j and j + 64)
   long long dkv_stride;
   int S, B, Hq, Hkv;
   int head_group;      // order of the CTAs (head_group_order)
@@ -322,6 +323,31 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       const uint32_t src = (p == 0 ? tdV : tdK) + ((uint32_t)((warp & 3) * 32) << 16);
       const float f = p == 0 ? 1.f : args.scale;
       const long long token = (long long)b * args.S + key;
+      if (p == 1 && args.rope != nullptr && args.dkv_accum == nullptr) {
+        const float4* cs = reinterpret_cast<const float4*>(args.rope + (long long)min(key, args.S - 1) * HD);  // two dims each
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {  // 16 dims and their partners
+          uint32_t a[16], z[16];
+          tmem_ld16(src + c * 16, a);
+          tmem_ld16(src + 64 + c * 16, z);
+          tmem_ld_wait();
+          if (key < args.S) {
+            uint32_t lo[8], hi[8];
+#pragma unroll
+            for (int v = 0; v < 8; ++v) {
+              const float4 t4 = __ldg(cs + c * 8 + v);
+              const float a0 = __uint_as_float(a[2 * v]), a1 = __uint_as_float(a[2 * v + 1]), z0 = __uint_as_float(z[2 * v]), z1 = __uint_as_float(z[2 * v + 1]);
+              lo[v] = pack_bf16x2((a0 * t4.x + z0 * t4.y) * f, (a1 * t4.z + z1 * t4.w) * f);
+              hi[v] = pack_bf16x2((z0 * t4.x - a0 * t4.y) * f, (z1 * t4.z - a1 * t4.w) * f);
+            }
+            uint4* dst = reinterpret_cast<uint4*>(args.dk + token * args.dkv_stride + hk * HD + c * 16);
+            dst[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            dst[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+            dst[8] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            dst[9] = make_uint4(hi[4], hi[5], hi[6], hi[7]);
+          }
+        }
+      } else
 #pragma unroll 1
       for (int c = 0; c < 4; ++c) {
         uint32_t r[32];
@@ -431,33 +457,62 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
   }
 }
 
-// dq (bf16, strided rows) = scale * dq_accum (fp32, dense rows of wq); with dkv_acc also dk = scale * its first half and
-// dv = its second half (dense rows of wkv)
-__global__ void attn_convert_kernel(const float* __restrict__ dq_acc, const float* __restrict__ dkv_acc, __nv_bfloat16* __restrict__ dq,
-                                    __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, long long T, int wq, int wkv,
-                                    long long dq_stride, long long dkv_stride, float scale) {
-  const int vpr = (wq + (dkv_acc != nullptr ? 2 * wkv : 0)) / 8;
-  const long long total = T * vpr;
+// dq (bf16, strided rows) = scale * dq_accum (fp32, dense rows of 128 Hq); with dkv_acc also dk = scale * its first half and
+// dv = its second half (dense rows of 128 Hkv).  With `rope` ([S, 64, 2]: cos, sin) dq and dk go back through the rotation on the
+// way: a thread holds eight head dims and their partners 64 further on.
+__global__ void attn_convert_kernel(const float* __restrict__ dq_acc, const float* __restrict__ dkv_acc, const float* __restrict__ rope,
+                                    __nv_bfloat16* __restrict__ dq, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, long long T,
+                                    int S, int Hq, int Hkv, long long dq_stride, long long dkv_stride, float scale) {
+  const int per_token = (Hq + (dkv_acc != nullptr ? 2 * Hkv : 0)) * 8;
+  const long long total = T * per_token;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / vpr;
-    const int v = (int)(i - t * vpr) * 8;
-    const float* src = dq_acc + t * wq + v;
-    __nv_bfloat16* dst = dq + t * dq_stride + v;
+    const long long t = i / per_token;
+    const int u = (int)(i - t * per_token), v = (u & 7) * 8;
+    int h = u >> 3;
+    const float* src;
+    __nv_bfloat16* dst;
     float f = scale;
-    if (v >= wq) {
-      const int u = v - wq, is_v = u >= wkv ? 1 : 0, col = u - is_v * wkv;
-      src = dkv_acc + (is_v * T + t) * wkv + col;
-      dst = (is_v ? dv : dk) + t * dkv_stride + col;
-      if (is_v) f = 1.f;
+    bool rotate = rope != nullptr;
+    if (h < Hq) {
+      src = dq_acc + (t * Hq + h) * HD + v;
+      dst = dq + t * dq_stride + h * HD + v;
+    } else {
+      h -= Hq;
+      const int is_v = h >= Hkv ? 1 : 0;
+      h -= is_v * Hkv;
+      src = dkv_acc + ((is_v * T + t) * Hkv + h) * HD + v;
+      dst = (is_v ? dv : dk) + t * dkv_stride + h * HD + v;
+      if (is_v) {
+        f = 1.f;
+        rotate = false;
+      }
     }
-    const float4 a = reinterpret_cast<const float4*>(src)[0];
-    const float4 c = reinterpret_cast<const float4*>(src)[1];
+    float a[8], z[8];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float4 x = reinterpret_cast<const float4*>(src)[j], y = reinterpret_cast<const float4*>(src + 64)[j];
+      a[4 * j] = x.x; a[4 * j + 1] = x.y; a[4 * j + 2] = x.z; a[4 * j + 3] = x.w;
+      z[4 * j] = y.x; z[4 * j + 1] = y.y; z[4 * j + 2] = y.z; z[4 * j + 3] = y.w;
+    }
+    if (rotate) {
+      const float4* cs = reinterpret_cast<const float4*>(rope + ((long long)(int)(t % S) * 64 + v) * 2);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float4 c = __ldg(cs + j);
+        const float a0 = a[2 * j], a1 = a[2 * j + 1];
+        a[2 * j] = a0 * c.x + z[2 * j] * c.y;
+        a[2 * j + 1] = a1 * c.z + z[2 * j + 1] * c.w;
+        z[2 * j] = z[2 * j] * c.x - a0 * c.y;
+        z[2 * j + 1] = z[2 * j + 1] * c.z - a1 * c.w;
+      }
+    }
     uint4 w;
-    w.x = pack_bf16x2(a.x * f, a.y * f);
-    w.y = pack_bf16x2(a.z * f, a.w * f);
-    w.z = pack_bf16x2(c.x * f, c.y * f);
-    w.w = pack_bf16x2(c.z * f, c.w * f);
+    w.x = pack_bf16x2(a[0] * f, a[1] * f); w.y = pack_bf16x2(a[2] * f, a[3] * f);
+    w.z = pack_bf16x2(a[4] * f, a[5] * f); w.w = pack_bf16x2(a[6] * f, a[7] * f);
     *reinterpret_cast<uint4*>(dst) = w;
+    w.x = pack_bf16x2(z[0] * f, z[1] * f); w.y = pack_bf16x2(z[2] * f, z[3] * f);
+    w.z = pack_bf16x2(z[4] * f, z[5] * f); w.w = pack_bf16x2(z[6] * f, z[7] * f);
+    *reinterpret_cast<uint4*>(dst + 64) = w;
   }
 }
 
@@ -479,7 +534,7 @@ int head_parts_for(int B, int S, int Hq, int Hkv) {
 
 // The three launches of one backward pass (delta pre-pass, main kernel, dQ conversion), shared by both entry points.
 // Allocates nothing: the tensor maps come by reference from the caller, the scratch by pointer.
-static int attn_bwd_launch(int head_parts, float* dkv_accum, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& md,
+static int attn_bwd_launch(int head_parts, float* dkv_accum, const float* rope, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& md,
                            const CUtensorMap& mdq, const void* out,
                            const void* dout, const float* lse, float* delta, float* dq_accum, void* dq, void* dk, void* dv, int B,
                            int S, int Hq, int Hkv, long long o_stride, long long do_stride, long long dq_stride,
@@ -509,6 +564,7 @@ static int attn_bwd_launch(int head_parts, float* dkv_accum, const CUtensorMap& 
   a.lse = lse;
   a.delta = delta;
   a.dkv_accum = dkv_accum;
+  a.rope = rope;
   a.head_parts = head_parts;
   a.dk = reinterpret_cast<__nv_bfloat16*>(dk);
   a.dv = reinterpret_cast<__nv_bfloat16*>(dv);
@@ -524,12 +580,12 @@ static int attn_bwd_launch(int head_parts, float* dkv_accum, const CUtensorMap& 
   const int grid = (int)ctas;
   attn_bwd_kernel<<<grid, BWD_THREADS, BWD_SMEM, st>>>(mq, mk, mv, md, mdq, a);
   {
-    const long long items = T * ((Hq + (dkv_accum ? 2 * Hkv : 0)) * HD / 8);
+    const long long items = T * (Hq + (dkv_accum ? 2 * Hkv : 0)) * 8;
     long long blocks = (items + 255) / 256;
     const long long cap = (long long)yf_num_sms() * 8;
     if (blocks > cap) blocks = cap;
-    attn_convert_kernel<<<(int)blocks, 256, 0, st>>>(dq_accum, dkv_accum, reinterpret_cast<__nv_bfloat16*>(dq), a.dk, a.dv, T, Hq * HD, Hkv * HD, dq_stride, dkv_stride,
-                                                     scale);
+    attn_convert_kernel<<<(int)blocks, 256, 0, st>>>(dq_accum, dkv_accum, rope, reinterpret_cast<__nv_bfloat16*>(dq), a.dk, a.dv, T, S, Hq, Hkv,
+                                                     dq_stride, dkv_stride, scale);
   }
   return -(int)cudaGetLastError();
 }
@@ -539,13 +595,14 @@ static int attn_bwd_launch(int head_parts, float* dkv_accum, const CUtensorMap& 
 // dq_accum [B*S, Hq*128] fp32 (zeroed here).  Results: dq (rows dq_stride apart), dk/dv (rows
 // dkv_stride apart), all bf16; they may be column blocks of one fused d(QKV) buffer.
 // The general form: `dkv_accum` ([2][B*S, Hkv*128] fp32 scratch, cleared here) lets `head_parts` CTAs (a divisor of Hq / Hkv) share
-// a key tile of a KV head; yf_attn_bwd_head_parts says how many a problem wants.  head_parts == 1 needs no dkv_accum.
+// a key tile of a KV head; yf_attn_bwd_head_parts says how many a problem wants.  head_parts == 1 needs no dkv_accum.  `rope` (may be
+// null; [S, 64, 2] fp32 cos, sin, 16-byte aligned): q and k are rotated, dq and dk are wanted with respect to what was rotated.
 extern "C" int yf_attn_bwd_head_parts(int B, int S, int Hq, int Hkv) {
   if (B <= 0 || S <= 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv)) return -1;
   return head_parts_for(B, S, Hq, Hkv);
 }
 extern "C" int yf_attn_bwd_parts(const void* q, const void* k, const void* v, const void* out, const void* dout, const float* lse,
-                                 float* delta, float* dq_accum, float* dkv_accum, int head_parts, void* dq, void* dk, void* dv, int B,
+                                 float* delta, float* dq_accum, float* dkv_accum, int head_parts, const float* rope, void* dq, void* dk, void* dv, int B,
                                  int S, int Hq, int Hkv, long long q_stride, long long kv_stride, long long o_stride,
                                  long long do_stride, long long dq_stride, long long dkv_stride, float scale, int causal, void* stream) {
   if (B <= 0 || S <= 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv)) return -1;
@@ -554,7 +611,7 @@ extern "C" int yf_attn_bwd_parts(const void* q, const void* k, const void* v, co
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
        reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(dq) |
        reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv) | reinterpret_cast<uintptr_t>(dq_accum) |
-       reinterpret_cast<uintptr_t>(dkv_accum)) & 15)
+       reinterpret_cast<uintptr_t>(dkv_accum) | reinterpret_cast<uintptr_t>(rope)) & 15)
     return -1;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const CUtensorMap* mq = yf_tensor_map_3d(q, (uint64_t)Hq * HD, S, B, q_stride, (uint64_t)S * q_stride, 64, BQ, 1, 2, 1);
@@ -563,14 +620,14 @@ extern "C" int yf_attn_bwd_parts(const void* q, const void* k, const void* v, co
   const CUtensorMap* md = yf_tensor_map_3d(dout, (uint64_t)Hq * HD, S, B, do_stride, (uint64_t)S * do_stride, 64, BQ, 1, 2, 1);
   const CUtensorMap* mdq = yf_tensor_map_3d(dq_accum, (uint64_t)Hq * HD, S, B, (uint64_t)Hq * HD, (uint64_t)S * Hq * HD, 32, BQ, 1, 4, 0);
   if (!mq || !mk || !mv || !md || !mdq) return -2;
-  return attn_bwd_launch(head_parts, dkv_accum, *mq, *mk, *mv, *md, *mdq, out, dout, lse, delta, dq_accum, dq, dk, dv, B, S, Hq, Hkv,
+  return attn_bwd_launch(head_parts, dkv_accum, rope, *mq, *mk, *mv, *md, *mdq, out, dout, lse, delta, dq_accum, dq, dk, dv, B, S, Hq, Hkv,
                          o_stride, do_stride, dq_stride, dkv_stride, scale, causal, st);
 }
 extern "C" int yf_attn_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout, const float* lse,
                            float* delta, float* dq_accum, void* dq, void* dk, void* dv, int B, int S, int Hq, int Hkv,
                            long long q_stride, long long kv_stride, long long o_stride, long long do_stride,
                            long long dq_stride, long long dkv_stride, float scale, int causal, void* stream) {
-  return yf_attn_bwd_parts(q, k, v, out, dout, lse, delta, dq_accum, nullptr, 1, dq, dk, dv, B, S, Hq, Hkv, q_stride, kv_stride, o_stride,
+  return yf_attn_bwd_parts(q, k, v, out, dout, lse, delta, dq_accum, nullptr, 1, nullptr, dq, dk, dv, B, S, Hq, Hkv, q_stride, kv_stride, o_stride,
                            do_stride, dq_stride, dkv_stride, scale, causal, stream);
 }
 
@@ -653,6 +710,6 @@ extern "C" int yf_attn_bwd_noalloc(const void* q, const void* k, const void* v, 
       yf_tensor_map_3d_encode(&md, dout, (uint64_t)Hq * HD, S, B, do_stride, (uint64_t)S * do_stride, 64, BQ, 1, 2, 1) != 0 ||
       yf_tensor_map_3d_encode(&mdq, dq_accum, (uint64_t)Hq * HD, S, B, (uint64_t)Hq * HD, (uint64_t)S * Hq * HD, 32, BQ, 1, 4, 0) != 0)
     return -2;
-  return attn_bwd_launch(1, nullptr, mq, mk, mv, md, mdq, out, dout, lse, delta, dq_accum, dq, dk, dv, B, S, Hq, Hkv, o_stride, do_stride, dq_stride,
+  return attn_bwd_launch(1, nullptr, nullptr, mq, mk, mv, md, mdq, out, dout, lse, delta, dq_accum, dq, dk, dv, B, S, Hq, Hkv, o_stride, do_stride, dq_stride,
                          dkv_stride, scale, causal, st);
 }

@@ -115,3 +115,26 @@ def test_attention_bwd_shared_key_tiles(b, s, hq, hkv, causal):
     _ref(qf, kf, vf, causal).backward(dout.double().view(b, s, hq, d))
     want = torch.cat([x.grad.reshape(t, -1) for x in (qf, kf, vf)], dim=1)
     assert ((got[0].double() - want).norm() / want.norm()).item() < 2.0**-7  # P, dS and the results are rounded to bf16
+
+
+@pytest.mark.parametrize("b,s,hq,hkv,parts", [(2, 200, 4, 2, 1), (1, 333, 4, 1, 4), (2, 64, 2, 2, 1)])
+def test_attention_bwd_through_rotation(b, s, hq, hkv, parts):
+    """dq and dk straight back through RoPE, against the rotation kernel on the rounded gradients (one bf16 rounding less)."""
+    from yafsdp_b200.ops import kernels
+    from yafsdp_b200.ops.functional import rope_table
+
+    torch.manual_seed(16)
+    t, d = b * s, 128
+    qkv = torch.randn(t, (hq + 2 * hkv) * d, device="cuda").bfloat16()
+    q, k, v = qkv[:, : hq * d], qkv[:, hq * d : (hq + hkv) * d], qkv[:, (hq + hkv) * d :]
+    scale, table = 1.0 / math.sqrt(d), rope_table(s + 5, d, 10000.0, "cuda")
+    out, lse = kernels.attn_fwd(q, k, v, b, s, hq, hkv, scale, True)
+    dout = torch.randn_like(out)
+    got, want = torch.empty_like(qkv), torch.empty_like(qkv)
+    for g, rope in ((got, table), (want, None)):
+        kernels.attn_bwd(q, k, v, out, dout, lse, g[:, : hq * d], g[:, hq * d : (hq + hkv) * d], g[:, (hq + hkv) * d :], b, s, hq, hkv,
+                         scale, True, head_parts=parts, rope=rope)
+    kernels.rope_(want, table, s, 0, hq + hkv, d, backward=True)
+    torch.cuda.synchronize()
+    kernels.check_status()
+    assert ((got.double() - want.double()).norm() / want.double().norm()).item() < 2.0**-8

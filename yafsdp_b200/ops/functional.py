@@ -294,10 +294,14 @@ class DecoderLayerFn(torch.autograd.Function):
         datt = kernels.gemm(dh, wo.detach(), b_mn_major=True)
         (g_wo,) = _WeightGrad([wo]).run(dh, att, pushed)
         dqkv = torch.empty_like(qkv)
+        # the attention kernels turn dq and dk back themselves, given a table that 16-byte loads can read
+        rotates = cos_sin.is_contiguous() and cos_sin.numel() >= dims.seq * hd and cos_sin.data_ptr() % 16 == 0
         q, k, v = qkv[:, : hq * hd], qkv[:, hq * hd : (hq + hkv) * hd], qkv[:, (hq + hkv) * hd :]
         kernels.attn_bwd(q, k, v, att, datt, lse, dqkv[:, : hq * hd], dqkv[:, hq * hd : (hq + hkv) * hd],
-                         dqkv[:, (hq + hkv) * hd :], dims.batch, dims.seq, hq, hkv, 1.0 / math.sqrt(hd), True)
-        kernels.rope_(dqkv, cos_sin, dims.seq, 0, hq + hkv, hd, backward=True)
+                         dqkv[:, (hq + hkv) * hd :], dims.batch, dims.seq, hq, hkv, 1.0 / math.sqrt(hd), True,
+                         rope=cos_sin if rotates else None)
+        if not rotates:
+            kernels.rope_(dqkv, cos_sin, dims.seq, 0, hq + hkv, hd, backward=True)
         dn1 = _gemm_fused(dqkv, w_qkv, b_mn_major=True)
         g_wq, g_wk, g_wv = _WeightGrad([wq, wk, wv]).run(dqkv, n1, pushed)
         g_n1 = _norm_weight_grad(w_n1, lambda dw, z, sq=None: box.append(kernels.rmsnorm_bwd(x, w_n1.detach(), dn1, rstd1, dw, dres=dh, zero_dw=z, sumsq=sq)), True, True)

@@ -449,9 +449,11 @@ def _attn_bwd_head_parts(batch: int, seq: int, n_heads: int, n_kv_heads: int, de
 
 def attn_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor, dout: torch.Tensor, lse: torch.Tensor,
              dq: torch.Tensor, dk: torch.Tensor, dv: torch.Tensor, batch: int, seq: int, n_heads: int, n_kv_heads: int,
-             scale: float, causal: bool = True, head_parts: int = 0) -> None:
+             scale: float, causal: bool = True, head_parts: int = 0, rope: torch.Tensor | None = None) -> None:
     """Flash attention backward into the given ``dq``/``dk``/``dv`` views (bf16, unit column stride).  ``head_parts``: CTAs that
-    share a key tile of a KV head (a divisor of the group; 0 = chosen from the shape)."""
+    share a key tile of a KV head (a divisor of the group; 0 = chosen from the shape).  ``rope``: the ``[seq, 64, 2]`` table that
+    ``q`` and ``k`` were rotated with; ``dq`` and ``dk`` are then the gradients of what was rotated."""
+    assert rope is None or (rope.dtype == torch.float32 and rope.is_contiguous() and rope.numel() >= seq * 128)
     t = batch * seq
     assert dout.stride(1) == 1 and out.stride(1) == 1 and dq.stride(1) == 1 and dk.stride(1) == 1 and dv.stride(1) == 1
     assert dk.stride(0) == dv.stride(0)
@@ -461,7 +463,7 @@ def attn_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tenso
     dkv_acc = torch.empty((2, t, n_kv_heads * 128), device=q.device, dtype=torch.float32) if parts > 1 else None
     global _launches
     _check(_native.lib().yf_attn_bwd_parts(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(),
-                                           delta.data_ptr(), dq_acc.data_ptr(), _ptr(dkv_acc), parts, dq.data_ptr(), dk.data_ptr(),
+                                           delta.data_ptr(), dq_acc.data_ptr(), _ptr(dkv_acc), parts, _ptr(rope), dq.data_ptr(), dk.data_ptr(),
                                            dv.data_ptr(), batch, seq, n_heads, n_kv_heads, q.stride(0), k.stride(0), out.stride(0),
                                            dout.stride(0), dq.stride(0), dk.stride(0), float(scale), int(causal), _stream()),
            "yf_attn_bwd")
