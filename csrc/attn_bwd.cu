@@ -518,7 +518,8 @@ __global__ void attn_convert_kernel(const float* __restrict__ dq_acc, const floa
 
 // CTAs per key tile of a KV head.  With grouped-query attention a KV head's key tiles are few and their walks long (every
 // query head of the group): the walk is cut by query heads until there are three CTAs per SM to balance, at the price of
-// fp32 atomic sums of dK and dV.  Measured: see the figures at the top of the launch.
+// fp32 atomic sums of dK and dV.  1 x 2048 tokens, 64 / 8 heads: 617 us whole, 276 us in four parts; 1 x 777, 64 / 8: 266 us whole, 83 us in
+// eight.
 int head_parts_for(int B, int S, int Hq, int Hkv) {
   const int group = Hq / Hkv;
   const long long tiles = (long long)((S + BKV - 1) / BKV) * Hkv * B;

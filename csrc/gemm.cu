@@ -1,8 +1,8 @@
 // bf16 GEMM family for sm_100a: C[M,N] = alpha * A[M,K] * B[N,K]^T (+ C), fp32 accumulation in TMEM.
 //
 // Persistent, warp-specialised kernel, one CTA per SM:
-//   warp 0     TMA producer  (cp.async.bulk.tensor, 128-byte swizzle, no multicast); plain mode: warps 0 and 6 in turn
-//   warp 1     MMA issuer    (tcgen05.mma cta_group::1, M=128, N=BLOCK_N, K=16 per instruction)
+//   warp 0     TMA producer  (cp.async.bulk.tensor, 128-byte swizzle, no multicast); plain modes: warps 0 and 6 in turn
+//   warp 1     MMA issuer    (tcgen05.mma, 128 rows per CTA, cta_group::1 or one instruction for a pair of CTAs, K=16)
 //   warps 2-5  epilogue      (tcgen05.ld 32x32b, convert, store; overlaps the next tile's main loop
 //                             through two TMEM accumulators)
 // Either operand may be K-major (rows of K contiguous) or MN-major (the M/N index contiguous), so
@@ -31,8 +31,9 @@ constexpr int GEMM_THREADS = 192;
 constexpr int WIDE_THREADS = 224;  // one more warp: plain mode's second TMA producer, gather mode's communication role
 
 // MODE_PLAIN: C is stored locally through TMA; MODE_SPLIT: so too, and the last wave's tiles are split along K (an
-// instantiation of its own: the exchange's code alone costs the plain kernel 0.3 us per tile).  MODE_SCATTER: GEMM -> reduce-scatter, the fp32 rows of C are pushed to the
-// ranks that own them.  MODE_GATHER: all-gather -> GEMM, the kernel also gathers the layer that B is part of (see FusedArgs).
+// instantiation of its own: the exchange's code alone costs the plain kernel 0.3 us per tile).
+// MODE_SCATTER: GEMM -> reduce-scatter, the fp32 rows of C are pushed to the ranks that own them.  MODE_GATHER: all-gather ->
+// GEMM, the kernel also gathers the layer that B is part of (see FusedArgs).
 // MODE_SWIGLU: the gate and up projections of an MLP with their activation (see GemmArgs).
 // MODE_SWAP: C is stored transposed: A is the weight, B the tokens, whose tile is any multiple of 16 wide (see GemmArgs::bn).
 constexpr int MODE_PLAIN = 0, MODE_SCATTER = 1, MODE_GATHER = 2, MODE_SPLIT = 3, MODE_SWIGLU = 4, MODE_SWAP = 5;
@@ -1102,8 +1103,12 @@ Plan make_plan(int M, int N, int K, int kind, int n_align, int sm_limit, bool ma
   const int num_k = (K + BLOCK_K - 1) / BLOCK_K;
   Plan best = {0, 0, 1, 0, 0, 0};
   float best_c = 0.f;
+  static const bool single_ctas = [] {
+    const char* v = getenv("YAFSDP_GEMM_CTA_GROUP");
+    return v && atoi(v) == 1;
+  }();
   for (int t = 1; t <= 5; ++t) {
-    if (tile > 0 && t != tile) continue;
+    if ((tile > 0 && t != tile) || (tile == 0 && single_ctas && TILE_SHAPES[t].cg == 2)) continue;
     if (n_align > 0 && n_align % TILE_SHAPES[t].bn != 0) continue;
     const int units = sms / TILE_SHAPES[t].cg;
     if (units < 1) continue;
@@ -1118,7 +1123,7 @@ Plan make_plan(int M, int N, int K, int kind, int n_align, int sm_limit, bool ma
       }
     }
   }
-  if (kind == 0 && (tile == 0 || tile == TILE_SWAP) && splits <= 1 && n_align % 256 == 0 && sms >= 2) {
+  if (kind == 0 && ((tile == 0 && !single_ctas) || tile == TILE_SWAP) && splits <= 1 && n_align % 256 == 0 && sms >= 2) {
     int bn = 0;
     const float c = swap_us(M, N, K, sms / 2, &bn);
     if (bn > 0 && (best.tile == 0 || c < best_c)) {

@@ -264,14 +264,15 @@ class ShardedAdamW:
 
 def _flat_runs(grads: list[torch.Tensor]) -> list[tuple[Any, torch.Tensor]] | None:
     """The local pieces of sharded fp32 gradients as few flat tensors: pieces that follow each other in one buffer (the
-    parameters of a group) become one.  ``None`` when some gradient is of another kind: not sharded, not fp32, not contiguous
-    or on another device."""
+    parameters of a group) become one.  ``None`` when some gradient is of another kind: not sharded, not fp32, not contiguous,
+    part of a graph or on another device."""
     runs: list[tuple[Any, torch.Tensor, int]] = []  # shard group, first piece, elements
     for g in grads:
         if not isinstance(g, RaggedShardDTensor):
             return None
         t = g._local_tensor
-        if type(t) is not torch.Tensor or t.dtype != torch.float32 or not t.is_contiguous() or t.device != grads[0].device:
+        if (type(t) is not torch.Tensor or t.dtype != torch.float32 or not t.is_contiguous() or t.device != grads[0].device
+                or g.requires_grad or t.requires_grad):
             return None
         if not t.numel():
             continue
@@ -335,6 +336,7 @@ def clip_grad_norm_(parameters: Iterable[torch.Tensor] | nn.Module, max_norm: fl
         with torch.cuda.device(dev):
             for _, r in runs:
                 kernels.scale_(r, coef)
+                torch.autograd.graph.increment_version(r)  # changed in place, behind autograd's back
         return total
     for g in grads:
         (g._local_tensor if isinstance(g, RaggedShardDTensor) else g).mul_(coef)
