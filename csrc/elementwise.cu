@@ -396,11 +396,21 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __
 // logits [T, V] bf16 (row pitch ldl) are replaced in place by dlogits = (softmax - onehot) * grad_scale, where grad_scale is
 // the host value times *scale_ptr when that device pointer is given (e.g. 1 / number of valid labels, counted on the device);
 // loss_rows[t] = logsumexp - logit[label] (0 for ignored rows, label < 0).  One CTA per row.
-// A row is read twice: the grid is kept so small that all rows in flight together stay in the L2, where the second read finds
-// them, and four loads per thread are in flight.  8192 x 128256: 1075 us (592 CTAs, 152 MB in flight, one load at a time: 1300 us);
-// 2048 x 32000: 73 us (82 us); there the exponentials and conversions are the bound: holding the row in registers, one read
-// for both passes, took 86 us.
-constexpr int CE_THREADS = 512;
+// A row is read twice, and the rows in flight together stay in the L2, where the second read finds them.  The exponentials and the
+// instructions around them bound it as much as the memory: two ex2 per logit (one instruction each, differences scaled by log2 e),
+// the maximum of a batch of four vectors on packed bf16 with one rescale for all of them, and the label's term set apart.
+// 8192 x 128256: 875 us (with a rescale per vector, __expf's guarded sequence and a label test per logit: 1075 us); 2048 x 32000: 62 us
+// (73 us); 999 x 32000: 29 us.  Batches of two vectors: 1040 and 69 us; 256 threads: 960 and 57 us; 1024 threads: 940 and 81 us.
+constexpr int CE_THREADS = 512, CE_BATCH = 4;
+constexpr float LOG2E = 1.4426950408889634f;
+// probabilities are computed 2^16 times too large: fast_exp2 flushes results below 2^-126, bf16 goes down to 2^-133
+constexpr float CE_SHIFT = 16.f, CE_UNSHIFT = 1.f / 65536.f;
+constexpr uint32_t BF16X2_NEG_INF = 0xff80ff80u;
+YF_DEVINL uint32_t max_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
 __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16* __restrict__ logits,
                                                                    const long long* __restrict__ labels,
                                                                    float* __restrict__ loss_rows, int T, int V,
@@ -421,49 +431,83 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
       }
       continue;
     }
-    // online max / sum-exp
+    // online max / sum-exp, CE_BATCH vectors at a time: one rescale for all of them
     float m = -INFINITY, s = 0.f;
-#pragma unroll 4
-    for (int v = threadIdx.x; v < nvec; v += CE_THREADS) {
-      float f[8];
-      load8(lr + v * 8, f);
-      float lm = f[0];
+    for (int v0 = threadIdx.x; v0 < nvec; v0 += CE_BATCH * CE_THREADS) {
+      uint4 x[CE_BATCH];
 #pragma unroll
-      for (int j = 1; j < 8; ++j) lm = fmaxf(lm, f[j]);
-      const float nm = fmaxf(m, lm);
+      for (int i = 0; i < CE_BATCH; ++i) {
+        const int v = v0 + i * CE_THREADS;
+        x[i] = v < nvec ? *reinterpret_cast<const uint4*>(lr + v * 8) : make_uint4(BF16X2_NEG_INF, BF16X2_NEG_INF, BF16X2_NEG_INF, BF16X2_NEG_INF);
+      }
+      uint32_t mx = max_bf16x2(max_bf16x2(x[0].x, x[0].y), max_bf16x2(x[0].z, x[0].w));
+#pragma unroll
+      for (int i = 1; i < CE_BATCH; ++i)
+        mx = max_bf16x2(mx, max_bf16x2(max_bf16x2(x[i].x, x[i].y), max_bf16x2(x[i].z, x[i].w)));
+      const float2 pair = unpack_bf16x2(mx);
+      const float nm = fmaxf(m, fmaxf(pair.x, pair.y));
+      const float ref = nm == -INFINITY ? 0.f : nm;  // nothing but -inf so far: every term is zero
       float acc = 0.f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc += __expf(f[j] - nm);
-      s = s * __expf(m - nm) + acc;
+      for (int i = 0; i < CE_BATCH; ++i) {
+        if (v0 + i * CE_THREADS >= nvec) break;
+        const uint32_t u[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = unpack_bf16x2(u[j]);
+          acc += fast_exp2((f.x - ref) * LOG2E);
+          acc += fast_exp2((f.y - ref) * LOG2E);
+        }
+      }
+      s = s * fast_exp2((m - ref) * LOG2E) + acc;
       m = nm;
     }
     for (int j = nvec * 8 + threadIdx.x; j < V; j += CE_THREADS) {
       const float f = __bfloat162float(lr[j]);
       const float nm = fmaxf(m, f);
-      s = s * __expf(m - nm) + __expf(f - nm);
+      const float ref = nm == -INFINITY ? 0.f : nm;
+      s = s * fast_exp2((m - ref) * LOG2E) + fast_exp2((f - ref) * LOG2E);
       m = nm;
     }
     const float gm = block_max<CE_THREADS>(m, red);
     const float contrib = (m == -INFINITY) ? 0.f : s * __expf(m - gm);
     const float gs = block_sum<CE_THREADS>(contrib, red);
-    const float lse = gm + __logf(gs);
-    if (threadIdx.x == 0) loss_rows[row] = lse - __bfloat162float(lr[label]);
+    // differences to the maximum first: they are exact, logsumexp itself would be rounded at its own size
+    const float log_gs = __logf(gs);
+    if (threadIdx.x == 0) loss_rows[row] = (gm - __bfloat162float(lr[label])) + log_gs;
     if (write_grad) {
       __syncthreads();  // the label logit was read above before anyone overwrites it
-#pragma unroll 4
-      for (int v = threadIdx.x; v < nvec; v += CE_THREADS) {
-        float f[8], o[8];
-        load8(lr + v * 8, f);
+      const float shift = CE_SHIFT - __log2f(gs), unshift = grad_scale * CE_UNSHIFT;
+      const int label_vec = (int)(label >> 3), label_elem = (int)(label & 7);
+      for (int v0 = threadIdx.x; v0 < nvec; v0 += CE_BATCH * CE_THREADS) {
+        uint4 x[CE_BATCH];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          float p = __expf(f[j] - lse);
-          if (v * 8 + j == label) p -= 1.f;
-          o[j] = p * grad_scale;
+        for (int i = 0; i < CE_BATCH; ++i)
+          if (v0 + i * CE_THREADS < nvec) x[i] = *reinterpret_cast<const uint4*>(lr + (v0 + i * CE_THREADS) * 8);
+#pragma unroll
+        for (int i = 0; i < CE_BATCH; ++i) {
+          const int v = v0 + i * CE_THREADS;
+          if (v >= nvec) break;
+          const uint32_t u[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+          float o[8];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 f = unpack_bf16x2(u[j]);
+            o[2 * j] = fast_exp2(fmaf(f.x - gm, LOG2E, shift)) * unshift;
+            o[2 * j + 1] = fast_exp2(fmaf(f.y - gm, LOG2E, shift)) * unshift;
+          }
+          if (v == label_vec) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float2 f = unpack_bf16x2(u[j / 2]);
+              if (j == label_elem) o[j] = (__expf(((j & 1 ? f.y : f.x) - gm) - log_gs) - 1.f) * grad_scale;
+            }
+          }
+          store8(lr + v * 8, o);
         }
-        store8(lr + v * 8, o);
       }
       for (int j = nvec * 8 + threadIdx.x; j < V; j += CE_THREADS) {
-        float p = __expf(__bfloat162float(lr[j]) - lse);
+        float p = __expf((__bfloat162float(lr[j]) - gm) - log_gs);
         if (j == label) p -= 1.f;
         lr[j] = __float2bfloat16_rn(p * grad_scale);
       }
@@ -714,8 +758,8 @@ __global__ void accum_bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ src, 
 }
 // The same for many tensors in one launch (the gradients of a group's parameters, which autograd left in bf16, into their places
 // of the flat fp32 gradient): blocks are dealt by chunks of 16384 elements.  A place may start anywhere: without 16-byte
-// alignment on both sides a tensor's elements are taken singly.  90 M elements in four matrices and vectors: 93 us = 5.8 TB/s
-// (a foreach copy: 136 us).
+// alignment on both sides a tensor's elements are taken singly.  90 M elements in four matrices and two vectors: 95 us =
+// 5.6 TB/s, added to what is there 142 us = 6.3 TB/s (foreach copy and add: 151 and 317 us).
 constexpr int MULTI_MAX = 48, MULTI_CHUNK = 16384;
 struct MultiAccum {
   const __nv_bfloat16* src[MULTI_MAX];
@@ -857,9 +901,9 @@ extern "C" int yf_swiglu_bwd(const void* gu, const void* dh, void* dgu, long lon
 extern "C" int yf_cross_entropy(void* logits, const long long* labels, float* loss_rows, int T, int V, long long ldl,
                                 float grad_scale, const float* scale_ptr, int write_grad, void* stream) {
   if (T <= 0 || V <= 0 || (ldl % 8) || !aligned16(logits)) return -1;
-  // one to four CTAs per SM, rows in flight of at most 80 MB
-  const long long row_bytes = (long long)V * 2 * yf_num_sms();
-  const int per_sm = row_bytes * 4 <= (80ll << 20) ? 4 : (row_bytes * 2 <= (80ll << 20) ? 2 : 1);
+  // Registers let two CTAs reside on an SM; twice as many are launched, so that an SM that is done early takes more rows (1024 x
+  // 128256: 116 us, with two per SM 128 us).  One per SM where the rows in flight of two would exceed 80 MB of the L2.
+  const int per_sm = (long long)V * 2 * yf_num_sms() * 2 <= (80ll << 20) ? 4 : 1;
   const int grid = T < yf_num_sms() * per_sm ? T : yf_num_sms() * per_sm;
   cross_entropy_kernel<<<grid, CE_THREADS, 0, YF_STREAM(stream)>>>((__nv_bfloat16*)logits, labels, loss_rows, T, V, ldl, grad_scale,
                                                                    scale_ptr, write_grad);

@@ -239,7 +239,7 @@ def test_rmsnorm_bwd_weight_gradient_over_many_rows(t, d):
 @pytest.mark.parametrize("v", [8, 1024, 32000, 32768, 32776, 1001, 128256])
 @pytest.mark.parametrize("t", [3, 700])
 def test_cross_entropy_row_lengths(v, t):
-    """Rows held in registers, longer ones, odd ones; ignored labels; logits at -inf."""
+    """Short, long and odd rows; ignored labels; logits at -inf."""
     from yafsdp_b200.ops import kernels
 
     torch.manual_seed(11)
@@ -315,3 +315,35 @@ def test_shift_labels_and_rmsnorm_weight_norm():
     dw, sq = torch.randn(1032, device="cuda"), torch.full((1,), 2.0, device="cuda")
     kernels.rmsnorm_bwd(x, w, dy, rstd, dw, zero_dw=True, sumsq=sq)
     assert abs((sq.item() - 2.0) / dw.double().pow(2).sum().item() - 1.0) < 1e-5
+
+
+@pytest.mark.parametrize("v", [1024, 32000, 50257, 128256])
+def test_cross_entropy_extreme_logits(v):
+    """Masks of the type's lowest value and of -inf over whole batches of loads, sure predictions, the smallest probabilities."""
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(13)
+    pitch = (v + 7) // 8 * 8
+    logits = torch.randn(5, pitch, device="cuda").bfloat16()[:, :v]
+    lowest = torch.finfo(torch.bfloat16).min
+    logits[0] = lowest
+    logits[1, : v - 100] = lowest
+    logits[2, : v - 100] = -math.inf
+    logits[3] -= 84.0
+    logits[3, 7] = 5.0
+    logits[4, v - 1] = 25.0
+    labels = torch.tensor([3, v - 5, v - 1, 7, v - 1], device="cuda")
+    ref = logits.double().requires_grad_(True)
+    rows = torch.nn.functional.cross_entropy(ref, labels, reduction="none")
+    rows.sum().backward()
+    work = torch.empty(5, pitch, device="cuda", dtype=torch.bfloat16)[:, :v]
+    work.copy_(logits)
+    got = kernels.cross_entropy_(work, labels, 1.0)
+    # the sum's fp32 rounding, relative to logsumexp <= 25 and to the loss
+    assert torch.allclose(got.double(), rows, rtol=1e-5, atol=1e-5)
+    grad, want = work.double(), ref.grad
+    rest = torch.ones(5, v, dtype=torch.bool, device="cuda")
+    rest[torch.arange(5), labels] = False
+    # probabilities: bf16's 2^-9 and the exponentials' error; 2^-133 is the smallest bf16 (half of it for rounding)
+    assert torch.allclose(grad[rest], want[rest], rtol=2.0**-8, atol=2.0**-133)
+    assert torch.allclose(grad[~rest], want[~rest], rtol=2.0**-8, atol=4e-6)  # p - 1: p to fp32's precision of logsumexp
