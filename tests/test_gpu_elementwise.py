@@ -214,6 +214,40 @@ def test_clip_grad_norm_of_adjacent_sharded_gradients(max_norm):
             dist.destroy_process_group()
 
 
+@pytest.mark.parametrize("max_norm", [1e-3, 1e9])
+@pytest.mark.parametrize("form", ["float64", "float64 on the CPU", "float64 vector", "float16 on the CPU", "int64"])
+def test_clip_grad_norm_with_a_tensor_as_limit(max_norm, form):
+    """``max_norm`` as a tensor of another type than the gradients, below and above their norm: what multiplying each gradient
+    by the coefficient gives."""
+    import torch.distributed as dist
+
+    from yafsdp_b200 import fully_shard
+    from yafsdp_b200.optim import clip_grad_norm_
+
+    dtype = getattr(torch, form.split()[0])
+    if dtype in (torch.float16, torch.int64):
+        max_norm = min(max(max_norm, 2.0 if dtype == torch.int64 else 0.0), 1000.0)
+    limit = torch.tensor([max_norm] if "vector" in form else max_norm, dtype=dtype, device="cpu" if "CPU" in form else "cuda")
+    torch.cuda.set_device(0)
+    created = not dist.is_initialized()
+    if created:
+        dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1)
+    try:
+        torch.manual_seed(4)
+        model = torch.nn.Sequential(torch.nn.Linear(33, 7, device="cuda"), torch.nn.Linear(7, 5, device="cuda"))
+        fully_shard(model)
+        model(torch.randn(9, 33, device="cuda")).square().sum().backward()
+        grads = [p.grad._local_tensor for p in model.parameters()]
+        before = [g.clone() for g in grads]
+        got = clip_grad_norm_(model, limit)
+        coef = torch.clamp(limit / (got + 1e-6), max=1.0)
+        for g, b in zip(grads, before):
+            assert torch.equal(g, b.clone().mul_(coef))
+    finally:
+        if created:
+            dist.destroy_process_group()
+
+
 @pytest.mark.parametrize("t,d", [(1, 8), (7, 1024), (700, 1032), (601, 2048), (1200, 4096), (297, 4104), (599, 8192)])
 def test_rmsnorm_bwd_weight_gradient_over_many_rows(t, d):
     """Every width class of the row walk, more rows than a wave holds: the weight gradient in a fixed order, cleared or added to,

@@ -378,6 +378,7 @@ def sumsq_(g: torch.Tensor, out: torch.Tensor) -> None:
 def sumsq_runs(runs: "list[torch.Tensor]") -> torch.Tensor:
     """``sum(g*g)`` over flat fp32 tensors of one device, without atomics (the same inputs give the same bits)."""
     dev = runs[0].device
+    assert all(r.is_cuda and r.dtype == torch.float32 and r.is_contiguous() and r.device == dev for r in runs)
     cap = torch.cuda.get_device_properties(dev).multi_processor_count * 8
     ctas = [max(1, min(cap, r.numel() // 4096)) for r in runs]
     partials = torch.empty(sum(ctas), device=dev, dtype=torch.float32)
@@ -390,6 +391,8 @@ def sumsq_runs(runs: "list[torch.Tensor]") -> torch.Tensor:
 
 def scale_(x: torch.Tensor, coef: torch.Tensor) -> None:
     """``x *= coef`` in place: flat fp32, ``coef`` one fp32 value on the same device."""
+    assert x.is_cuda and x.dtype == torch.float32 and x.is_contiguous()
+    assert coef.dtype == torch.float32 and coef.numel() == 1 and coef.device == x.device
     _check(_native.lib().yf_scale(x.data_ptr(), x.numel(), coef.data_ptr(), _stream()), "yf_scale")
 
 
@@ -411,6 +414,8 @@ def accum_bf16_to_f32_(src: torch.Tensor, dst: torch.Tensor, scale: float = 1.0,
 def accum_bf16_to_f32_multi_(pairs: "list[tuple[torch.Tensor, torch.Tensor]]", accumulate: bool) -> None:
     """``dst (+)= src`` for ``(dst fp32, src bf16)`` pairs of contiguous tensors of one device, in one launch."""
     n = len(pairs)
+    assert all(d.is_cuda and d.dtype == torch.float32 and s.dtype == torch.bfloat16 and d.is_contiguous() and s.is_contiguous()
+               and d.numel() == s.numel() and d.device == s.device == pairs[0][0].device for d, s in pairs)
     _check(_native.lib().yf_accum_bf16_to_f32_multi(
         n, (ctypes.c_void_p * n)(*[s.data_ptr() for _, s in pairs]), (ctypes.c_void_p * n)(*[d.data_ptr() for d, _ in pairs]),
         (ctypes.c_longlong * n)(*[d.numel() for d, _ in pairs]), int(accumulate), _stream()), "yf_accum_bf16_to_f32_multi")

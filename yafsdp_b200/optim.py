@@ -332,7 +332,9 @@ def clip_grad_norm_(parameters: Iterable[torch.Tensor] | nn.Module, max_norm: fl
     if not inf:
         total = total.pow(1.0 / norm_type)
     coef = torch.clamp(max_norm / (total + 1e-6), max=1.0)
-    if runs is not None:
+    if runs is not None and coef.dim() == 0:
+        # a max_norm that is a tensor gives the coefficient its type; a 0-dimensional one multiplies fp32 gradients as fp32
+        coef = coef.to(device=dev, dtype=torch.float32)
         with torch.cuda.device(dev):
             for _, r in runs:
                 kernels.scale_(r, coef)
