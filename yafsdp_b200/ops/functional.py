@@ -256,7 +256,7 @@ class DecoderLayerFn(torch.autograd.Function):
         h = kernels.gemm(att, wo.detach(), residual=x)  # x + attention block: the residual is added in the GEMM's epilogue
         n2, rstd2 = kernels.rmsnorm_fwd(h, w_n2.detach(), dims.eps)
         t, d, f = n2.shape[0], n2.shape[1], wg.shape[0]
-        if wg.is_contiguous() and wu.is_contiguous() and kernels.swiglu_pays(t, f, d, n2.device.index):
+        if kernels.swiglu_pays(t, f, d, n2.device.index) and kernels.can_fuse_swiglu(wg, wu):
             gu, a = kernels.gemm_swiglu(n2, wg.detach(), wu.detach(), keep_gu=keep)
         else:
             gu = _gemm_fused(n2, fuse_rows([wg, wu]))

@@ -176,6 +176,12 @@ def swiglu_pays(t: int, f: int, k: int, device: int | None) -> bool:
     return _native.lib().yf_gemm_swiglu_pays(t, f, k) == 1
 
 
+def can_fuse_swiglu(wg: torch.Tensor, wu: torch.Tensor) -> bool:
+    """Whether :func:`gemm_swiglu` takes these weights where they are (TMA: 16-byte aligned addresses and rows).  What it does not
+    take goes through the separate kernels, on a concatenated copy if need be."""
+    return wg.shape == wu.shape and can_be_parts([wg, wu])
+
+
 def gemm_swiglu(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, keep_gu: bool = True) -> tuple[torch.Tensor | None, torch.Tensor]:
     """``(gu, a)``: ``gu = [x wg^T | x wu^T]`` (``None`` unless kept) and ``a = silu(gate) * up`` from one kernel."""
     (t, k), f = x.shape, wg.shape[0]
