@@ -1094,6 +1094,15 @@ float swap_us(int M, int N, int K, int units, int* bn) {
   return best;
 }
 
+// YAFSDP_GEMM_CTA_GROUP=1 in the environment: no CTA pairs where a single CTA can do the work
+bool single_ctas_only() {
+  static const bool single = [] {
+    const char* v = getenv("YAFSDP_GEMM_CTA_GROUP");
+    return v && atoi(v) == 1;
+  }();
+  return single;
+}
+
 // n_align > 0: tiles must end where multiples of n_align columns do (the pieces of B)
 // kind: 0 bf16 output that may be computed swapped, 1 fp32 output, 2 any other
 Plan make_plan(int M, int N, int K, int kind, int n_align, int sm_limit, bool may_split, int tile, int splits, float* us = nullptr) {
@@ -1103,10 +1112,7 @@ Plan make_plan(int M, int N, int K, int kind, int n_align, int sm_limit, bool ma
   const int num_k = (K + BLOCK_K - 1) / BLOCK_K;
   Plan best = {0, 0, 1, 0, 0, 0};
   float best_c = 0.f;
-  static const bool single_ctas = [] {
-    const char* v = getenv("YAFSDP_GEMM_CTA_GROUP");
-    return v && atoi(v) == 1;
-  }();
+  const bool single_ctas = single_ctas_only();
   for (int t = 1; t <= 5; ++t) {
     if ((tile > 0 && t != tile) || (tile == 0 && single_ctas && TILE_SHAPES[t].cg == 2)) continue;
     if (n_align > 0 && n_align % TILE_SHAPES[t].bn != 0) continue;
@@ -1209,23 +1215,20 @@ int dispatch_gemm(const void* A, const void* B, const GemmArgs& args, const Fuse
                   cudaStream_t s) {
   const int M = args.M, N = args.N;
   const bool use256 = (N >= 256) && ((N % 256 == 0) || (N % 256 > 128) || N >= 2048);
-  static const int force_cg = [] {
-    const char* v = getenv("YAFSDP_GEMM_CTA_GROUP");
-    return v ? atoi(v) : 0;
-  }();
+  const bool single_ctas = single_ctas_only();
   const bool pair_ok = use256 && M >= 256 && (M % 256 == 0 || M % 256 > 128 || M >= 2048);
   if (fa.gather) {
-    if (pair_ok && force_cg != 1) return launch_gemm<256, 2, MODE_GATHER>(A, B, args, fa, lda, ldb, sm_limit, s);
+    if (pair_ok && !single_ctas) return launch_gemm<256, 2, MODE_GATHER>(A, B, args, fa, lda, ldb, sm_limit, s);
     return use256 ? launch_gemm<256, 1, MODE_GATHER>(A, B, args, fa, lda, ldb, sm_limit, s)
                   : launch_gemm<128, 1, MODE_GATHER>(A, B, args, fa, lda, ldb, sm_limit, s);
   }
   if (fa.scatter) {
-    if (pair_ok && force_cg != 1) return launch_gemm<256, 2, MODE_SCATTER>(A, B, args, fa, lda, ldb, sm_limit, s);
+    if (pair_ok && !single_ctas) return launch_gemm<256, 2, MODE_SCATTER>(A, B, args, fa, lda, ldb, sm_limit, s);
     return use256 ? launch_gemm<256, 1, MODE_SCATTER>(A, B, args, fa, lda, ldb, sm_limit, s)
                   : launch_gemm<128, 1, MODE_SCATTER>(A, B, args, fa, lda, ldb, sm_limit, s);
   }
   const Operands one = {A, B, lda, ldb, M, N, args.K};
-  return launch_plain(&one, 1, args, fa, sm_limit, nullptr, 0, force_cg == 1 ? (use256 ? TILE_256 : TILE_128) : 0, 0, s);
+  return launch_plain(&one, 1, args, fa, sm_limit, nullptr, 0, single_ctas ? (use256 ? TILE_256 : TILE_128) : 0, 0, s);
 }
 
 }  // namespace
@@ -1389,7 +1392,7 @@ extern "C" int yf_gemm_swiglu(const void* X, const void* Wg, const void* Wu, voi
 // 127, 512 x 1408 x 512 7 + 3 / 26: those stay separate.
 extern "C" int yf_gemm_swiglu_pays(int M, int F, int K) {
   if (M <= 0 || F <= 0 || K <= 0) return -1;
-  if (F % 128) return 0;
+  if ((F % 128) || single_ctas_only()) return 0;  // the fused kernel has CTA pairs only
   const int sms = yf_num_sms(), num_k = (K + BLOCK_K - 1) / BLOCK_K;
   float best = 0.f;
   make_plan(M, 2 * F, K, 0, 0, 0, true, 0, 0, &best);
