@@ -1186,8 +1186,8 @@ int launch_plain(const Operands* ops, int n_ops, GemmArgs args, const FusedArgs&
   }
   const bool ws = workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255) == 0;
   const int kind = args.out_f32 ? 1 : (args.a_mn || args.accumulate ? 2 : 0);
-  Plan p = make_plan(args.M, args.N, args.K, kind, n_align, sm_limit, ws, tile, splits);
-  if (p.bytes > workspace_bytes) p = make_plan(args.M, args.N, args.K, kind, n_align, sm_limit, false, tile, 1);
+  Plan p = make_plan(args.M, args.N, args.K, kind, n_align, sm_limit, true, tile, splits);
+  if (p.splits > 1 && (!ws || p.bytes > workspace_bytes)) p = make_plan(args.M, args.N, args.K, kind, n_align, sm_limit, false, tile, 1);
   if (p.tile == 0) return -1;
   args.splits = p.splits;
   if (p.tile == TILE_SWAP) {

@@ -223,3 +223,26 @@ def test_gemm_swapped_form(m, n, k, b_mn):
     assert ((with_res.double() - want).norm() / want.norm()).item() < 2.0**-8
     if parts is not None:
         assert torch.equal(kernels.gemm_parts(a, parts, b_mn_major=b_mn, tile=6), got)
+
+
+@pytest.mark.parametrize("tile,splits", [(0, 0), (0, 3), (3, 3), (1, 2)])
+@pytest.mark.parametrize("given", ["none", "short", "unaligned"])
+def test_gemm_without_a_usable_workspace(tile, splits, given):
+    """No workspace, one that is too short or one at an odd address: no tile is split, whether or not a split was asked for."""
+    from yafsdp_b200 import _native
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(17)
+    m, n, k = 300, 520, 4096
+    a, b = torch.randn(m, k, device="cuda").bfloat16(), torch.randn(n, k, device="cuda").bfloat16()
+    out = torch.empty(m, n, device="cuda")
+    ws = torch.empty(1 << 24, device="cuda", dtype=torch.uint8)
+    at, nbytes = {"none": (None, 0), "short": (ws.data_ptr(), 256), "unaligned": (ws.data_ptr() + 128, (1 << 24) - 128)}[given]
+    rc = _native.lib().yf_gemm_bf16_ws(a.data_ptr(), b.data_ptr(), out.data_ptr(), None, m, n, k, k, k, n, 0, 0, 0, 1, 0, 1.0, 0, None, None,
+                                       at, nbytes, tile, splits, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    want = kernels.gemm(a, b, out_dtype=torch.float32, tile=tile, splits=1)
+    torch.cuda.synchronize()
+    kernels.check_status()
+    # the same plan as for a caller that asks for whole tiles
+    assert torch.equal(out, want)
