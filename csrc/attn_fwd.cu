@@ -188,7 +188,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     const int qrow = q0 + i * BQ + q * 32 + lane;
     const uint32_t lane_off = (uint32_t)(q * 32) << 16;
     const uint32_t tS = tmem_base + lane_off + i * 128, tO = tmem_base + lane_off + 256 + i * 128;
-    float m_run = -INFINITY, l_run = 0.f;    // m_run: reference maximum of the exponent
+    float m_run = -INFINITY;                 // reference maximum of the exponent
+    float l_run[2] = {0.f, 0.f};             // row sums of the even and the odd 64 keys of all blocks, each in the order of the keys
     const float sl2 = args.scale_log2;
     constexpr float RESCALE_LOG2 = 8.f;      // move the reference maximum when a row's maximum exceeds it by 2^8
     // keys allowed for this row: col <= limit
@@ -235,25 +236,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
             for (int t = 0; t < 32; ++t) r[t] = __float_as_uint(__uint_as_float(r[t]) * alpha);
             tmem_st32(tO + c * 32, r);
           }
-          l_run *= alpha;
+          l_run[0] *= alpha;
+          l_run[1] *= alpha;
         }
         m_run = m_new;
       }
       const float neg_ms = (m_run == -INFINITY) ? 0.f : -m_run * sl2;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int c = 0; c < 2; ++c) {  // 64 keys: 32 TMEM columns of packed bf16 pairs
         uint32_t packed[32];
+        float sum = 0.f;
 #pragma unroll
         for (int t = 0; t < 32; ++t) {
           const float p0 = fast_exp2(fmaf(__uint_as_float(sc[2 * c + (t >> 4)][(2 * t) & 31]), sl2, neg_ms));
           const float p1 = fast_exp2(fmaf(__uint_as_float(sc[2 * c + (t >> 4)][(2 * t + 1) & 31]), sl2, neg_ms));
-          sum4[t & 3] += p0 + p1;
+          sum += p0 + p1;  // one chain: an addition takes less than the two exponentials next to it
           packed[t] = pack_bf16x2(p0, p1);
         }
         tmem_st32(tS + c * 32, packed);
+        l_run[c] += sum;
       }
-      l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -262,7 +264,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     // the output of the last block
     if (n > 0 && alive && __all_sync(0xffffffffu, mbar_wait(&o_full[i], (n - 1) & 1, 124 + i))) {
       tc_fence_after();
-      const float inv = (l_run > 0.f) ? 1.f / l_run : 0.f;
+      const float l = l_run[0] + l_run[1];
+      const float inv = (l > 0.f) ? 1.f / l : 0.f;
       __nv_bfloat16* dst = args.out + ((long long)b * args.S + qrow) * args.out_stride + h * HD;
 #pragma unroll 1
       for (int c = 0; c < 4; ++c) {
@@ -282,7 +285,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         }
       }
       if (qrow < args.S)
-        args.lse[((long long)b * args.Hq + h) * args.S + qrow] = (l_run > 0.f) ? (m_run * args.scale + logf(l_run)) : -INFINITY;
+        args.lse[((long long)b * args.Hq + h) * args.S + qrow] = (l > 0.f) ? (m_run * args.scale + logf(l)) : -INFINITY;
     }
     tc_fence_before();
   }

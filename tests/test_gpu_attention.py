@@ -138,3 +138,19 @@ def test_attention_bwd_through_rotation(b, s, hq, hkv, parts):
     torch.cuda.synchronize()
     kernels.check_status()
     assert ((got.double() - want.double()).norm() / want.double().norm()).item() < 2.0**-8
+
+
+def test_attention_fwd_adds_row_sums_in_the_order_of_the_keys():
+    """The sums of a row's even and odd groups of 64 keys run through the keys one pair after the other, so that the results of
+    ordinary rows repeat bit for bit from version to version.  One weight of 1 and 127 of 2^-25 tell the orders apart: every pair
+    of small ones is lost next to the 1 (2^-24, ties to even), while those of the other group add up to 2^-19."""
+    from yafsdp_b200.ops import kernels
+
+    s, d, scale = 128, 128, 0.6931471824645996  # scale * log2(e) is 1 in fp32
+    qkv = torch.zeros(s, 3 * d, device="cuda").bfloat16()
+    qkv[:, 0] = 1.0
+    qkv[1:, d] = -25.0
+    _, lse = kernels.attn_fwd(qkv[:, :d], qkv[:, d : 2 * d], qkv[:, 2 * d :], 1, s, 1, 1, scale, False)
+    torch.cuda.synchronize()
+    kernels.check_status()
+    assert (lse.double() - math.log1p(2.0**-19)).abs().max().item() < 2.0**-24  # the next sum is 2^-20 away
