@@ -46,7 +46,7 @@ struct BwdArgs {
   const float* delta;  // [B, Hq, S]
   __nv_bfloat16* dk;   // rows dkv_stride apart, head hk at columns hk*128
   __nv_bfloat16* dv;
-  float* dkv_accum;    // head_parts > 1: fp32 sums [2 (dK without scale, dV)][B*S, Hkv*128], zero at the start; else null
+  float4* dkv_parts;   // head_parts > 1: every part's own fp32 sums (part_tile), dK without scale; else null
   const float* rope;   // optional [S, 64, 2] (cos, sin): dK goes back through the rotation of K (head dims j and j + 64)
   long long dkv_stride;
   int S, B, Hq, Hkv;
@@ -62,8 +62,13 @@ YF_DEVINL void tma_reduce_add_3d(const CUtensorMap* m, const void* smem_src, int
                "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
                : "memory");
 }
-YF_DEVINL void red_add_v4(float* p, float a, float b, float c, float d) {
-  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+
+// Where a CTA that shares its key tile leaves dK (is_v = 0) and dV: [head_parts][B][key tiles][Hkv][2] blocks of 32 groups of four head
+// dims x 128 keys, so that a warp, one key per lane, stores 512 contiguous bytes at a time (rows of 128 dims: 16 bytes in each of
+// 32 lines).
+constexpr int PART_TILE = BKV * HD / 4;  // float4s of a block
+__host__ __device__ inline long long part_tile(int part, int B, int b, int n_kt, int jt, int Hkv, int hk, int is_v) {
+  return (((((long long)part * B + b) * n_kt + jt) * Hkv + hk) * 2 + is_v) * PART_TILE;
 }
 
 // Order of the CTAs: heads are taken in groups, within a group key tile by key tile with the heads fastest, so that all heads'
@@ -83,6 +88,8 @@ int head_group_size(int n_pos, int n_heads, long long accum_bytes, int n_sms) {
   return accum_bytes <= (64ll << 20) || group >= n_heads / 3 ? n_heads : group;
 }
 
+// SHARED: head_parts > 1 (an instantiation of its own: the parts' addresses cost the other one registers it does not have)
+template <bool SHARED>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
                 const __grid_constant__ CUtensorMap tma_v, const __grid_constant__ CUtensorMap tma_do,
@@ -110,9 +117,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   int jt, bh;  // key tile (under the causal mask the first ones have the longest walks), (sequence, KV head, part)
-  head_group_order((int)blockIdx.x, (args.S + BKV - 1) / BKV, args.B * args.Hkv * args.head_parts, args.head_group, jt, bh);
-  const int part = bh % args.head_parts, hk = (bh / args.head_parts) % args.Hkv, b = bh / (args.head_parts * args.Hkv);
-  const int heads = args.Hq / args.Hkv / args.head_parts;  // query heads of this CTA
+  const int head_parts = SHARED ? args.head_parts : 1;
+  head_group_order((int)blockIdx.x, (args.S + BKV - 1) / BKV, args.B * args.Hkv * head_parts, args.head_group, jt, bh);
+  const int part = bh % head_parts, hk = (bh / head_parts) % args.Hkv, b = bh / (head_parts * args.Hkv);
+  const int heads = args.Hq / args.Hkv / head_parts;  // query heads of this CTA
   const int h0 = hk * (args.Hq / args.Hkv) + part * heads;
   const int kv0 = jt * BKV;
   const int i_start = args.causal ? kv0 / BQ : 0;          // first query tile
@@ -323,7 +331,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       const uint32_t src = (p == 0 ? tdV : tdK) + ((uint32_t)((warp & 3) * 32) << 16);
       const float f = p == 0 ? 1.f : args.scale;
       const long long token = (long long)b * args.S + key;
-      if (p == 1 && args.rope != nullptr && args.dkv_accum == nullptr) {
+      if (!SHARED && p == 1 && args.rope != nullptr) {
         const float4* cs = reinterpret_cast<const float4*>(args.rope + (long long)min(key, args.S - 1) * HD);  // two dims each
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {  // 16 dims and their partners
@@ -354,12 +362,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         tmem_ld32(src + c * 32, r);
         tmem_ld_wait();
         if (key < args.S) {
-          if (args.dkv_accum != nullptr) {
-            float* dst = args.dkv_accum + ((p == 0 ? (long long)args.B * args.S : 0ll) + token) * args.Hkv * HD + hk * HD + c * 32;
+          if (SHARED) {
+            float4* dst = args.dkv_parts + part_tile(part, args.B, b, (args.S + BKV - 1) / BKV, jt, args.Hkv, hk, p == 0 ? 1 : 0) + row;
 #pragma unroll
             for (int v = 0; v < 8; ++v)
-              red_add_v4(dst + 4 * v, __uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]), __uint_as_float(r[4 * v + 2]),
-                         __uint_as_float(r[4 * v + 3]));
+              dst[(c * 8 + v) * BKV] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]), __uint_as_float(r[4 * v + 2]),
+                                                   __uint_as_float(r[4 * v + 3]));
           } else {
             uint4* dst = reinterpret_cast<uint4*>((p == 0 ? args.dv : args.dk) + token * args.dkv_stride + hk * HD + c * 32);
 #pragma unroll
@@ -423,14 +431,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
 
 // delta[b,h,s] = sum_d dO * O, and the fp32 dQ accumulator of the same (token, head) cleared on the way (the main kernel
 // adds into it): sixteen lanes per (token, head), one 16-byte load of O and of dO and two 16-byte stores of zeros per lane.
-// The dK / dV accumulators of shared key tiles, where there are any, are cleared too.
 __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                                         float* __restrict__ delta, float* __restrict__ dq_zero, float4* __restrict__ dkv_zero,
-                                                         long long n_dkv_zero, int B, int S, int Hq,
+                                                         float* __restrict__ delta, float* __restrict__ dq_zero, int B, int S, int Hq,
                                                          long long o_stride, long long do_stride) {
-  if (dkv_zero != nullptr)
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n_dkv_zero; i += (long long)gridDim.x * blockDim.x)
-      dkv_zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   const long long total = (long long)B * S * Hq;
   const int sub = threadIdx.x & 15;
   const unsigned half_mask = 0xffffu << (threadIdx.x & 16);  // the two halves of a warp may leave the loop at different times
@@ -457,68 +460,88 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
   }
 }
 
-// dq (bf16, strided rows) = scale * dq_accum (fp32, dense rows of 128 Hq); with dkv_acc also dk = scale * its first half and
-// dv = its second half (dense rows of 128 Hkv).  With `rope` ([S, 64, 2]: cos, sin) dq and dk go back through the rotation on the
-// way: a thread holds eight head dims and their partners 64 further on.
-__global__ void attn_convert_kernel(const float* __restrict__ dq_acc, const float* __restrict__ dkv_acc, const float* __restrict__ rope,
-                                    __nv_bfloat16* __restrict__ dq, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, long long T,
+// dst, dst + 64 (bf16) = f * (a, z): eight head dims and their partners 64 further on.  With `cs` (cos, sin of the eight dims) they
+// go back through the rotation on the way.
+YF_DEVINL void store_gradient(__nv_bfloat16* dst, float (&a)[8], float (&z)[8], const float4* cs, float f) {
+  if (cs != nullptr) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float4 c = __ldg(cs + j);
+      const float a0 = a[2 * j], a1 = a[2 * j + 1];
+      a[2 * j] = a0 * c.x + z[2 * j] * c.y;
+      a[2 * j + 1] = a1 * c.z + z[2 * j + 1] * c.w;
+      z[2 * j] = z[2 * j] * c.x - a0 * c.y;
+      z[2 * j + 1] = z[2 * j + 1] * c.z - a1 * c.w;
+    }
+  }
+  uint4 w;
+  w.x = pack_bf16x2(a[0] * f, a[1] * f); w.y = pack_bf16x2(a[2] * f, a[3] * f);
+  w.z = pack_bf16x2(a[4] * f, a[5] * f); w.w = pack_bf16x2(a[6] * f, a[7] * f);
+  *reinterpret_cast<uint4*>(dst) = w;
+  w.x = pack_bf16x2(z[0] * f, z[1] * f); w.y = pack_bf16x2(z[2] * f, z[3] * f);
+  w.z = pack_bf16x2(z[4] * f, z[5] * f); w.w = pack_bf16x2(z[6] * f, z[7] * f);
+  *reinterpret_cast<uint4*>(dst + 64) = w;
+}
+YF_DEVINL const float4* rope_at(const float* rope, int pos, int dim) {
+  return rope == nullptr ? nullptr : reinterpret_cast<const float4*>(rope + ((long long)pos * 64 + dim) * 2);
+}
+
+// dq (bf16, strided rows) = scale * dq_accum (fp32, dense rows of 128 Hq); with dkv_parts also dk = scale * the sum of the parts' dK and
+// dv = that of their dV, in the order of the parts.  `rope` ([S, 64, 2]: cos, sin): dq and dk go back through the rotation.
+__global__ void __launch_bounds__(256) attn_convert_kernel(const float* __restrict__ dq_acc, const float4* __restrict__ dkv_parts, int parts, const float* __restrict__ rope,
+                                    __nv_bfloat16* __restrict__ dq, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, int B,
                                     int S, int Hq, int Hkv, long long dq_stride, long long dkv_stride, float scale) {
-  const int per_token = (Hq + (dkv_acc != nullptr ? 2 * Hkv : 0)) * 8;
-  const long long total = T * per_token;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / per_token;
-    const int u = (int)(i - t * per_token), v = (u & 7) * 8;
-    int h = u >> 3;
-    const float* src;
-    __nv_bfloat16* dst;
-    float f = scale;
-    bool rotate = rope != nullptr;
-    if (h < Hq) {
-      src = dq_acc + (t * Hq + h) * HD + v;
-      dst = dq + t * dq_stride + h * HD + v;
-    } else {
-      h -= Hq;
-      const int is_v = h >= Hkv ? 1 : 0;
-      h -= is_v * Hkv;
-      src = dkv_acc + ((is_v * T + t) * Hkv + h) * HD + v;
-      dst = (is_v ? dv : dk) + t * dkv_stride + h * HD + v;
-      if (is_v) {
-        f = 1.f;
-        rotate = false;
-      }
-    }
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  const long long n_dq = (long long)B * S * Hq * 8;
+  const int n_kt = (S + BKV - 1) / BKV;
+  const long long blocks = dkv_parts == nullptr ? 0 : (long long)B * n_kt * Hkv * 2;  // of a part
+  const long long total = n_dq + blocks * (BKV * 8);
+  for (long long i = first; i < total; i += step) {
     float a[8], z[8];
+    if (i < n_dq) {
+      const long long t = i / (Hq * 8);
+      const int u = (int)(i - t * (Hq * 8)), h = u >> 3, v = (u & 7) * 8;
+      const float4* src = reinterpret_cast<const float4*>(dq_acc + (t * Hq + h) * HD + v);
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const float4 x = reinterpret_cast<const float4*>(src)[j], y = reinterpret_cast<const float4*>(src + 64)[j];
-      a[4 * j] = x.x; a[4 * j + 1] = x.y; a[4 * j + 2] = x.z; a[4 * j + 3] = x.w;
-      z[4 * j] = y.x; z[4 * j + 1] = y.y; z[4 * j + 2] = y.z; z[4 * j + 3] = y.w;
-    }
-    if (rotate) {
-      const float4* cs = reinterpret_cast<const float4*>(rope + ((long long)(int)(t % S) * 64 + v) * 2);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float4 c = __ldg(cs + j);
-        const float a0 = a[2 * j], a1 = a[2 * j + 1];
-        a[2 * j] = a0 * c.x + z[2 * j] * c.y;
-        a[2 * j + 1] = a1 * c.z + z[2 * j + 1] * c.w;
-        z[2 * j] = z[2 * j] * c.x - a0 * c.y;
-        z[2 * j + 1] = z[2 * j + 1] * c.z - a1 * c.w;
+      for (int j = 0; j < 2; ++j) {
+        const float4 x = src[j], y = src[16 + j];
+        a[4 * j] = x.x; a[4 * j + 1] = x.y; a[4 * j + 2] = x.z; a[4 * j + 3] = x.w;
+        z[4 * j] = y.x; z[4 * j + 1] = y.y; z[4 * j + 2] = y.z; z[4 * j + 3] = y.w;
       }
+      store_gradient(dq + t * dq_stride + h * HD + v, a, z, rope_at(rope, (int)(t % S), v), scale);
+    } else {  // a warp: eight keys x four groups of dims (whole lines read, 64 contiguous bytes per key written)
+      const long long k = i - n_dq, block = k >> 10;
+      const int v = ((int)k & 3) + ((int)(k >> 5) & 1) * 4, row = ((int)(k >> 2) & 7) + ((int)(k >> 6) & 15) * 8, is_v = (int)(block & 1);
+      const long long bj = (block >> 1) / Hkv;
+      const int hk = (int)((block >> 1) - bj * Hkv), s = (int)(bj % n_kt) * BKV + row;
+      if (s >= S) continue;
+      const float4* src = dkv_parts + block * PART_TILE + 2 * v * BKV + row;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a[j] = z[j] = 0.f;
+      for (int p0 = 0; p0 < parts; p0 += 4, src += 4 * blocks * PART_TILE) {  // four parts in flight
+        float4 x[4][4];
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            x[p][j] = p0 + p < parts ? __ldcg(src + p * blocks * PART_TILE + ((j & 1) + (j >> 1) * 16) * BKV) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            a[4 * j] += x[p][j].x; a[4 * j + 1] += x[p][j].y; a[4 * j + 2] += x[p][j].z; a[4 * j + 3] += x[p][j].w;
+            z[4 * j] += x[p][2 + j].x; z[4 * j + 1] += x[p][2 + j].y; z[4 * j + 2] += x[p][2 + j].z; z[4 * j + 3] += x[p][2 + j].w;
+          }
+      }
+      __nv_bfloat16* dst = (is_v ? dv : dk) + ((bj / n_kt) * S + s) * dkv_stride + hk * HD + v * 8;
+      store_gradient(dst, a, z, is_v ? nullptr : rope_at(rope, s, v * 8), is_v ? 1.f : scale);
     }
-    uint4 w;
-    w.x = pack_bf16x2(a[0] * f, a[1] * f); w.y = pack_bf16x2(a[2] * f, a[3] * f);
-    w.z = pack_bf16x2(a[4] * f, a[5] * f); w.w = pack_bf16x2(a[6] * f, a[7] * f);
-    *reinterpret_cast<uint4*>(dst) = w;
-    w.x = pack_bf16x2(z[0] * f, z[1] * f); w.y = pack_bf16x2(z[2] * f, z[3] * f);
-    w.z = pack_bf16x2(z[4] * f, z[5] * f); w.w = pack_bf16x2(z[6] * f, z[7] * f);
-    *reinterpret_cast<uint4*>(dst + 64) = w;
   }
 }
 
 // CTAs per key tile of a KV head.  With grouped-query attention a KV head's key tiles are few and their walks long (every
 // query head of the group): the walk is cut by query heads until there are three CTAs per SM to balance, at the price of
-// fp32 atomic sums of dK and dV.  1 x 2048 tokens, 64 / 8 heads: 617 us whole, 276 us in four parts; 1 x 777, 64 / 8: 266 us whole, 83 us in
+// sums of dK and dV that go through memory in fp32 (131 KB per CTA).  1 x 2048 tokens, 64 / 8 heads: 617 us whole, 276 us in four parts; 1 x 777, 64 / 8: 266 us whole, 83 us in
 // eight.
 int head_parts_for(int B, int S, int Hq, int Hkv) {
   const int group = Hq / Hkv;
@@ -535,18 +558,20 @@ int head_parts_for(int B, int S, int Hq, int Hkv) {
 
 // The three launches of one backward pass (delta pre-pass, main kernel, dQ conversion), shared by both entry points.
 // Allocates nothing: the tensor maps come by reference from the caller, the scratch by pointer.
-static int attn_bwd_launch(int head_parts, float* dkv_accum, const float* rope, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& md,
+static int attn_bwd_launch(int head_parts, float* dkv_parts, const float* rope, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& md,
                            const CUtensorMap& mdq, const void* out,
                            const void* dout, const float* lse, float* delta, float* dq_accum, void* dq, void* dk, void* dv, int B,
                            int S, int Hq, int Hkv, long long o_stride, long long do_stride, long long dq_stride,
                            long long dkv_stride, float scale, int causal, cudaStream_t st) {
-  static bool optin[64] = {};  // the shared-memory opt-in is a per-device attribute
+  const auto kernel = dkv_parts != nullptr ? attn_bwd_kernel<true> : attn_bwd_kernel<false>;
+  static bool optin[2][64] = {};  // the shared-memory opt-in is a per-device attribute
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
-  if (!optin[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM);
+  bool& done = optin[dkv_parts != nullptr ? 1 : 0][dev];
+  if (!done) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM);
     if (e != cudaSuccess) return -(int)e;
-    optin[dev] = true;
+    done = true;
   }
   if (int rc = yf_tu_bind_status()) return rc;
   const long long T = (long long)B * S;
@@ -557,14 +582,13 @@ static int attn_bwd_launch(int head_parts, float* dkv_accum, const float* rope, 
     const long long cap = (long long)yf_num_sms() * 8;
     if (blocks > cap) blocks = cap;
     attn_delta_kernel<<<(int)blocks, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(out),
-                                                  reinterpret_cast<const __nv_bfloat16*>(dout), delta, dq_accum,
-                                                  reinterpret_cast<float4*>(dkv_accum), dkv_accum ? 2 * T * Hkv * (HD / 4) : 0, B, S, Hq, o_stride,
-                                                  do_stride);
+                                                  reinterpret_cast<const __nv_bfloat16*>(dout), delta, dq_accum, B, S, Hq,
+                                                  o_stride, do_stride);
   }
   BwdArgs a;
   a.lse = lse;
   a.delta = delta;
-  a.dkv_accum = dkv_accum;
+  a.dkv_parts = reinterpret_cast<float4*>(dkv_parts);
   a.rope = rope;
   a.head_parts = head_parts;
   a.dk = reinterpret_cast<__nv_bfloat16*>(dk);
@@ -579,13 +603,13 @@ static int attn_bwd_launch(int head_parts, float* dkv_accum, const float* rope, 
   const long long ctas = (long long)n_kt * B * Hkv * head_parts;
   if (ctas > 0x7fffffffll) return -1;
   const int grid = (int)ctas;
-  attn_bwd_kernel<<<grid, BWD_THREADS, BWD_SMEM, st>>>(mq, mk, mv, md, mdq, a);
+  kernel<<<grid, BWD_THREADS, BWD_SMEM, st>>>(mq, mk, mv, md, mdq, a);
   {
-    const long long items = T * (Hq + (dkv_accum ? 2 * Hkv : 0)) * 8;
+    const long long items = T * Hq * 8 + (dkv_parts ? (long long)B * n_kt * Hkv * 2 * BKV * 8 : 0);
     long long blocks = (items + 255) / 256;
     const long long cap = (long long)yf_num_sms() * 8;
     if (blocks > cap) blocks = cap;
-    attn_convert_kernel<<<(int)blocks, 256, 0, st>>>(dq_accum, dkv_accum, rope, reinterpret_cast<__nv_bfloat16*>(dq), a.dk, a.dv, T, S, Hq, Hkv,
+    attn_convert_kernel<<<(int)blocks, 256, 0, st>>>(dq_accum, a.dkv_parts, head_parts, rope, reinterpret_cast<__nv_bfloat16*>(dq), a.dk, a.dv, B, S, Hq, Hkv,
                                                      dq_stride, dkv_stride, scale);
   }
   return -(int)cudaGetLastError();
@@ -595,24 +619,26 @@ static int attn_bwd_launch(int head_parts, float* dkv_accum, const float* rope, 
 // o_stride apart); lse from the forward.  Scratch supplied by the caller: delta [B,Hq,S] fp32 and
 // dq_accum [B*S, Hq*128] fp32 (zeroed here).  Results: dq (rows dq_stride apart), dk/dv (rows
 // dkv_stride apart), all bf16; they may be column blocks of one fused d(QKV) buffer.
-// The general form: `dkv_accum` ([2][B*S, Hkv*128] fp32 scratch, cleared here) lets `head_parts` CTAs (a divisor of Hq / Hkv) share
-// a key tile of a KV head; yf_attn_bwd_head_parts says how many a problem wants.  head_parts == 1 needs no dkv_accum.  `rope` (may be
+// The general form: `dkv_parts` (scratch of head_parts * 2 * B * S rounded up to 128 * Hkv * 128 floats, whose contents do not matter; dkv_floats says
+// how many there are) lets `head_parts` CTAs (a divisor of Hq / Hkv) share a key tile of a KV head; yf_attn_bwd_head_parts says how many a
+// problem wants.  head_parts == 1 takes none.  dK and dV do not vary from run to run (dQ's atomic sums may).  `rope` (may be
 // null; [S, 64, 2] fp32 cos, sin, 16-byte aligned): q and k are rotated, dq and dk are wanted with respect to what was rotated.
 extern "C" int yf_attn_bwd_head_parts(int B, int S, int Hq, int Hkv) {
   if (B <= 0 || S <= 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv)) return -1;
   return head_parts_for(B, S, Hq, Hkv);
 }
 extern "C" int yf_attn_bwd_parts(const void* q, const void* k, const void* v, const void* out, const void* dout, const float* lse,
-                                 float* delta, float* dq_accum, float* dkv_accum, int head_parts, const float* rope, void* dq, void* dk, void* dv, int B,
+                                 float* delta, float* dq_accum, float* dkv_parts, long long dkv_floats, int head_parts, const float* rope, void* dq, void* dk, void* dv, int B,
                                  int S, int Hq, int Hkv, long long q_stride, long long kv_stride, long long o_stride,
                                  long long do_stride, long long dq_stride, long long dkv_stride, float scale, int causal, void* stream) {
   if (B <= 0 || S <= 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv)) return -1;
-  if (head_parts < 1 || (Hq / Hkv) % head_parts || (head_parts > 1) != (dkv_accum != nullptr)) return -1;
+  if (head_parts < 1 || (Hq / Hkv) % head_parts || (head_parts > 1) != (dkv_parts != nullptr)) return -1;
+  if (dkv_parts != nullptr && dkv_floats < 4 * part_tile(head_parts, B, 0, (S + BKV - 1) / BKV, 0, Hkv, 0, 0)) return -1;
   if ((q_stride % 8) || (kv_stride % 8) || (o_stride % 8) || (do_stride % 8) || (dq_stride % 8) || (dkv_stride % 8)) return -1;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
        reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(dq) |
        reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv) | reinterpret_cast<uintptr_t>(dq_accum) |
-       reinterpret_cast<uintptr_t>(dkv_accum) | reinterpret_cast<uintptr_t>(rope)) & 15)
+       reinterpret_cast<uintptr_t>(dkv_parts) | reinterpret_cast<uintptr_t>(rope)) & 15)
     return -1;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const CUtensorMap* mq = yf_tensor_map_3d(q, (uint64_t)Hq * HD, S, B, q_stride, (uint64_t)S * q_stride, 64, BQ, 1, 2, 1);
@@ -621,14 +647,14 @@ extern "C" int yf_attn_bwd_parts(const void* q, const void* k, const void* v, co
   const CUtensorMap* md = yf_tensor_map_3d(dout, (uint64_t)Hq * HD, S, B, do_stride, (uint64_t)S * do_stride, 64, BQ, 1, 2, 1);
   const CUtensorMap* mdq = yf_tensor_map_3d(dq_accum, (uint64_t)Hq * HD, S, B, (uint64_t)Hq * HD, (uint64_t)S * Hq * HD, 32, BQ, 1, 4, 0);
   if (!mq || !mk || !mv || !md || !mdq) return -2;
-  return attn_bwd_launch(head_parts, dkv_accum, rope, *mq, *mk, *mv, *md, *mdq, out, dout, lse, delta, dq_accum, dq, dk, dv, B, S, Hq, Hkv,
+  return attn_bwd_launch(head_parts, dkv_parts, rope, *mq, *mk, *mv, *md, *mdq, out, dout, lse, delta, dq_accum, dq, dk, dv, B, S, Hq, Hkv,
                          o_stride, do_stride, dq_stride, dkv_stride, scale, causal, st);
 }
 extern "C" int yf_attn_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout, const float* lse,
                            float* delta, float* dq_accum, void* dq, void* dk, void* dv, int B, int S, int Hq, int Hkv,
                            long long q_stride, long long kv_stride, long long o_stride, long long do_stride,
                            long long dq_stride, long long dkv_stride, float scale, int causal, void* stream) {
-  return yf_attn_bwd_parts(q, k, v, out, dout, lse, delta, dq_accum, nullptr, 1, nullptr, dq, dk, dv, B, S, Hq, Hkv, q_stride, kv_stride, o_stride,
+  return yf_attn_bwd_parts(q, k, v, out, dout, lse, delta, dq_accum, nullptr, 0, 1, nullptr, dq, dk, dv, B, S, Hq, Hkv, q_stride, kv_stride, o_stride,
                            do_stride, dq_stride, dkv_stride, scale, causal, stream);
 }
 

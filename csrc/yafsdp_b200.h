@@ -97,12 +97,12 @@ int yf_attn_bwd(const void* q, const void* k, const void* v, const void* out, co
                 float* delta, float* dq_accum, void* dq, void* dk, void* dv, int B, int S, int Hq, int Hkv,
                 long long q_stride, long long kv_stride, long long o_stride, long long do_stride, long long dq_stride,
                 long long dkv_stride, float scale, int causal, void* stream);
-/* The same with `head_parts` CTAs per key tile of a KV head (a divisor of Hq / Hkv), whose dK and dV meet in dkv_accum
-   ([2][B*S, Hkv*128] fp32 scratch); yf_attn_bwd_head_parts: how many a problem wants.  rope: optional, dq and dk go back through
+/* The same with `head_parts` CTAs per key tile of a KV head (a divisor of Hq / Hkv), each with its own sums of dK and dV in dkv_parts
+   (scratch of dkv_floats >= head_parts * 2 * B * S rounded up to 128 * Hkv*128 floats); yf_attn_bwd_head_parts: how many a problem wants.  rope: optional, dq and dk go back through
    the rotation of q and k (see attn_bwd.cu). */
 int yf_attn_bwd_head_parts(int B, int S, int Hq, int Hkv);
 int yf_attn_bwd_parts(const void* q, const void* k, const void* v, const void* out, const void* dout, const float* lse,
-                      float* delta, float* dq_accum, float* dkv_accum, int head_parts, const float* rope, void* dq, void* dk, void* dv, int B, int S, int Hq,
+                      float* delta, float* dq_accum, float* dkv_parts, long long dkv_floats, int head_parts, const float* rope, void* dq, void* dk, void* dv, int B, int S, int Hq,
                       int Hkv, long long q_stride, long long kv_stride, long long o_stride, long long do_stride, long long dq_stride,
                       long long dkv_stride, float scale, int causal, void* stream);
 

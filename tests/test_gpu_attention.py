@@ -140,6 +140,43 @@ def test_attention_bwd_through_rotation(b, s, hq, hkv, parts):
     assert ((got.double() - want.double()).norm() / want.double().norm()).item() < 2.0**-8
 
 
+@pytest.mark.parametrize("b,s,hq,hkv,parts", [(1, 777, 16, 2, 8), (1, 2048, 16, 2, 4), (2, 300, 14, 2, 7), (1, 640, 8, 8, 1)])
+@pytest.mark.parametrize("rotated", [False, True])
+def test_attention_bwd_key_gradients_repeat(b, s, hq, hkv, parts, rotated):
+    """dk and dv do not vary from run to run, however many CTAs share a key tile: every part's sums have a place of their own."""
+    from yafsdp_b200.ops import kernels
+    from yafsdp_b200.ops.functional import rope_table
+
+    torch.manual_seed(18)
+    t, d = b * s, 128
+    qkv = torch.randn(t, (hq + 2 * hkv) * d, device="cuda").bfloat16()
+    q, k, v = qkv[:, : hq * d], qkv[:, hq * d : (hq + hkv) * d], qkv[:, (hq + hkv) * d :]
+    scale, table = 1.0 / math.sqrt(d), rope_table(s, d, 10000.0, "cuda") if rotated else None
+    out, lse = kernels.attn_fwd(q, k, v, b, s, hq, hkv, scale, True)
+    dout = torch.randn_like(out)
+    runs = []
+    for _ in range(6):
+        g = torch.empty_like(qkv)
+        kernels.attn_bwd(q, k, v, out, dout, lse, g[:, : hq * d], g[:, hq * d : (hq + hkv) * d], g[:, (hq + hkv) * d :], b, s, hq, hkv,
+                         scale, True, head_parts=parts, rope=table)
+        runs.append(g[:, hq * d :])
+    torch.cuda.synchronize()
+    kernels.check_status()
+    assert all(torch.equal(r, runs[0]) for r in runs[1:])
+
+
+def test_attention_bwd_refuses_short_scratch():
+    from yafsdp_b200 import _native
+
+    b, s, hq, hkv, d = 1, 64, 4, 1, 128
+    x = torch.zeros(s, hq * d, device="cuda").bfloat16()
+    f = torch.zeros(s * hq * d, device="cuda")
+    p, fp = x.data_ptr(), f.data_ptr()
+    for parts, floats in ((2, 2 * 2 * 128 * d - 1), (4, 2 * 2 * 128 * d), (2, 0)):
+        assert _native.lib().yf_attn_bwd_parts(p, p, p, p, p, fp, fp, fp, fp, floats, parts, None, p, p, p, b, s, hq, hkv, hq * d, d, hq * d, hq * d,
+                                               hq * d, d, 0.1, 1, torch.cuda.current_stream().cuda_stream) == -1
+
+
 def test_attention_fwd_adds_row_sums_in_the_order_of_the_keys():
     """The sums of a row's even and odd groups of 64 keys run through the keys one pair after the other, so that the results of
     ordinary rows repeat bit for bit from version to version.  One weight of 1 and 127 of 2^-25 tell the orders apart: every pair

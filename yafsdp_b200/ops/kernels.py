@@ -471,10 +471,10 @@ def attn_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tenso
     delta = torch.empty((batch, n_heads, seq), device=q.device, dtype=torch.float32)
     dq_acc = torch.empty((t, n_heads * 128), device=q.device, dtype=torch.float32)
     parts = _attn_bwd_head_parts(batch, seq, n_heads, n_kv_heads, q.device.index) if head_parts == 0 else head_parts
-    dkv_acc = torch.empty((2, t, n_kv_heads * 128), device=q.device, dtype=torch.float32) if parts > 1 else None
+    dkv_parts = torch.empty((parts, 2, batch, (seq + 127) // 128 * 128, n_kv_heads * 128), device=q.device, dtype=torch.float32) if parts > 1 else None
     global _launches
     _check(_native.lib().yf_attn_bwd_parts(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(),
-                                           delta.data_ptr(), dq_acc.data_ptr(), _ptr(dkv_acc), parts, _ptr(rope), dq.data_ptr(), dk.data_ptr(),
+                                           delta.data_ptr(), dq_acc.data_ptr(), _ptr(dkv_parts), 0 if dkv_parts is None else dkv_parts.numel(), parts, _ptr(rope), dq.data_ptr(), dk.data_ptr(),
                                            dv.data_ptr(), batch, seq, n_heads, n_kv_heads, q.stride(0), k.stride(0), out.stride(0),
                                            dout.stride(0), dq.stride(0), dk.stride(0), float(scale), int(causal), _stream()),
            "yf_attn_bwd")
