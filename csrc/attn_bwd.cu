@@ -540,18 +540,31 @@ __global__ void __launch_bounds__(256) attn_convert_kernel(const float* __restri
 }
 
 // CTAs per key tile of a KV head.  With grouped-query attention a KV head's key tiles are few and their walks long (every
-// query head of the group): the walk is cut by query heads until there are three CTAs per SM to balance, at the price of
-// sums of dK and dV that go through memory in fp32 (131 KB per CTA).  1 x 2048 tokens, 64 / 8 heads: 617 us whole, 276 us in four parts; 1 x 777, 64 / 8: 266 us whole, 83 us in
-// eight.
+// query head of the group): the walk is cut by query heads where that is estimated to end sooner.  The main kernel takes its longest
+// walk or its share of all steps, 1.5 us a step and 8 us a CTA (start, end, first loads); the parts' sums (131 KB a CTA) are read at
+// 3.7 TB/s.  Measured, the whole backward pass, us, in 1 / 2 / 4 / 8 parts (* the choice):
+//   1 x 333 tokens, 64 / 8 heads 88 / 56 / 42 / 42*;  1 x 777, 64 / 8 166 / 103 / 72* / 92;  1 x 2048, 64 / 8 396 / 253* / 290 / 331;
+//   1 x 8192, 64 / 8 3422* / 3335 / 3455 / 3457;  8 x 300, 32 / 8 85* / 97 / 121;  4 x 1024, 32 / 8 162* / 204 / 255;
+//   1 x 4096, 32 / 8 455 / 479* / 542;  1 x 4096, 28 / 4 653 whole, 432* in seven.
+// (Cut until there were three CTAs per SM, 8 x 300 took 113, 4 x 1024 204 and 1 x 777 92 us.)
 int head_parts_for(int B, int S, int Hq, int Hkv) {
-  const int group = Hq / Hkv;
-  const long long tiles = (long long)((S + BKV - 1) / BKV) * Hkv * B;
-  int parts = 1;
-  while (parts < group && tiles * parts < 3ll * yf_num_sms()) {
-    ++parts;
-    while (group % parts) ++parts;
+  const int group = Hq / Hkv, n_kt = (S + BKV - 1) / BKV, n_qt = (S + BQ - 1) / BQ;
+  const float sms = (float)yf_num_sms(), walks = (float)n_kt * (float)Hkv * (float)B;
+  // steps of all walks, under the causal mask (key tile j starts at query tile 2 j)
+  const float longest = (float)n_qt * (float)group;
+  const float steps = (float)n_kt * (float)(n_qt - n_kt + 1) * (float)Hq * (float)B;
+  int best = 1;
+  float best_us = 0.f;
+  for (int parts = 1; parts <= group; ++parts) {
+    if (group % parts) continue;
+    const float walk = longest / (float)parts * 1.5f + 8.f, share = (steps * 1.5f + walks * (float)parts * 8.f) / sms;
+    const float us = (walk > share ? walk : share) + (parts > 1 ? walks * (float)parts * (131072.f / 3.7e6f) : 0.f);
+    if (parts == 1 || us < best_us) {
+      best = parts;
+      best_us = us;
+    }
   }
-  return parts;
+  return best;
 }
 
 }  // namespace
