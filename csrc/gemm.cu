@@ -825,10 +825,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_co
           load64(128 + c * 64, u);
           if (c == 1) free_accumulator();
           if (args.store_gu) store64(&tma_c, F + x, u);
+          if (m0 + r_in_tile < M) {  // rows past the end are zeros, and 0 / x takes the long way through the division
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float2 gf = unpack_bf16x2(g[j]), uf = unpack_bf16x2(u[j]);
-            g[j] = pack_bf16x2(gf.x / (1.f + __expf(-gf.x)) * uf.x, gf.y / (1.f + __expf(-gf.y)) * uf.y);
+            for (int j = 0; j < 32; ++j) {
+              const float2 gf = unpack_bf16x2(g[j]), uf = unpack_bf16x2(u[j]);
+              g[j] = pack_bf16x2(gf.x / (1.f + __expf(-gf.x)) * uf.x, gf.y / (1.f + __expf(-gf.y)) * uf.y);
+            }
           }
           store64(&maps.a[1], x, g);
         }
@@ -1386,10 +1388,14 @@ extern "C" int yf_gemm_swiglu(const void* X, const void* Wg, const void* Wu, voi
   return launch_gemm<256, 2, MODE_SWIGLU>(ops, 2, args, fa, 0, reinterpret_cast<cudaStream_t>(stream));
 }
 // Whether that is estimated to be faster than the best plain GEMM and a separate activation kernel (6 bytes per element of act
-// at 4 TB/s, 3 us): the epilogue of a tile takes some 15 us (exponentials, divisions and three stores in four warps), which
-// the next tile's main loop hides, but not the last one's and not where K is short.  Measured, F 11008, K 4096 (GEMM +
-// activation / fused, us): 2048 tokens 239 + 33 / 251, 8192 tokens 922 + 166 / 973, 1337 tokens 198 + 21 / 196; 300 tokens 65 + 6 /
-// 127, 512 x 1408 x 512 7 + 3 / 26: those stay separate.
+// at 4 TB/s, 3 us).  The epilogue of a tile takes 11.3 us (exponentials, divisions and three stores in four warps), 2.7 us of it also a
+// plain tile's; the next tile's main loop hides it, but not the last one's, and where K is short it hides the main loop.  Measured in
+// a stream of launches at the power cap, GEMM + activation / fused, us:
+//   F 11008, K 4096: 45 tokens 47 / 62, 300 72 / 84, 777 145 / 157, 999 175 / 158, 1337 222 / 216, 2048 323 / 284, 8192 1201 / 1015
+//   F 14336, K 4096: 777 tokens 176 / 199, 1337 282 / 291, 2048 421 / 365;  F 13824, K 5120: 300 tokens 98 / 116, 512 137 / 133
+//   F 28672, K 8192: 128 tokens 177 / 215, 777 686 / 757, 1337 1084 / 1098, 2048 1696 / 1534, 4096 3249 / 2957
+// (While rows past the end went through the epilogue's divisions, which take several times as long for 0 / x, fused tiles with such
+// rows cost 12 us more each: 1337 tokens 240, 777 187, 300 126 us at F 11008.)
 extern "C" int yf_gemm_swiglu_pays(int M, int F, int K) {
   if (M <= 0 || F <= 0 || K <= 0) return -1;
   if ((F % 128) || single_ctas_only()) return 0;  // the fused kernel has CTA pairs only
@@ -1398,8 +1404,9 @@ extern "C" int yf_gemm_swiglu_pays(int M, int F, int K) {
   make_plan(M, 2 * F, K, 0, 0, 0, true, 0, 0, &best);
   const TileShape& t = TILE_SHAPES[TILE_PAIR256];
   const long long tiles = (long long)((M + 255) / 256) * (F / 128), units = sms / 2;
-  const float loop = (float)num_k * t.kb_us;
-  const float fused = t.fixed_us + 10.f + (float)((tiles + units - 1) / units) * (loop > 15.f ? loop : 15.f);
+  const float loop = (float)num_k * t.kb_us, epi = 11.3f, longer = loop > epi ? loop : epi, shorter = loop > epi ? epi : loop;
+  const float us = (float)((tiles + units - 1) / units) * longer, read_us = ((float)M + 2.f * (float)F) * (float)K * 2.f / 5.2e6f;
+  const float fused = t.fixed_us + shorter - 2.7f + (us > read_us ? us + 0.1f * read_us : read_us + 0.1f * us);  // as in plan_us
   return fused <= best + 3.f + (float)M * (float)F * 6.f / 4e6f ? 1 : 0;
 }
 

@@ -30,3 +30,13 @@ def test_parts_of_a_key_tile_where_they_were_measured():
     best = {(1, 777, 64, 8): 4, (1, 1024, 64, 8): 4, (1, 2048, 64, 8): 2, (1, 2048, 32, 8): 2, (2, 777, 32, 8): 2, (8, 300, 32, 8): 1,
             (4, 1024, 32, 8): 1, (1, 4096, 28, 4): 7, (1, 1337, 28, 4): 7, (1, 2048, 8, 1): 8, (6, 512, 16, 2): 4, (2, 64, 2, 2): 1}
     assert dict(zip(best, _ask("yf_attn_bwd_head_parts", list(best)))) == best
+
+
+def test_fused_activation_where_it_was_measured():
+    """The faster choice where the sides were at least 8 % apart (the figures stand at the rule): whole and ragged tiles, few tokens
+    at large weights."""
+    best = {(999, 11008, 4096): 1, (2048, 11008, 4096): 1, (2500, 11008, 4096): 1, (8192, 11008, 4096): 1, (2048, 14336, 4096): 1,
+            (999, 13824, 5120): 1, (4096, 28672, 8192): 1, (45, 11008, 4096): 0, (300, 11008, 4096): 0, (777, 11008, 4096): 0,
+            (300, 13824, 5120): 0, (777, 14336, 4096): 0, (45, 22016, 8192): 0, (128, 22016, 8192): 0, (777, 22016, 8192): 0,
+            (128, 28672, 8192): 0, (777, 28672, 8192): 0}
+    assert dict(zip(best, _ask("yf_gemm_swiglu_pays", list(best)))) == best
