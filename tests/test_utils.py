@@ -3,6 +3,7 @@
 import io
 import json
 
+import pytest
 import torch
 
 
@@ -31,6 +32,30 @@ def test_profile_steps_writes_a_trace(tmp_path):
             torch.randn(32, 32).sum()
             prof.step()
     assert path.exists() and "traceEvents" in json.loads(path.read_text())
+
+
+@pytest.mark.parametrize("observer", ["profiler", "execution trace"])
+def test_phase_labels_reach_every_observer(tmp_path, observer):
+    """Ranges of the schedule are recorded for whatever watches them, not only under the autograd profiler."""
+    from yafsdp_b200.common import _NO_LABEL, phase_label
+
+    path = tmp_path / "trace.json"
+    assert phase_label("YaFSDP::idle") is _NO_LABEL
+    if observer == "profiler":
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+            with phase_label("YaFSDP::pre_forward", "layers.0"):
+                torch.ones(2).sum()
+        prof.export_chrome_trace(str(path))
+    else:
+        trace = torch.profiler.ExecutionTraceObserver()
+        trace.register_callback(str(path))
+        trace.start()
+        with phase_label("YaFSDP::pre_forward", "layers.0"):
+            torch.ones(2).sum()
+        trace.stop()
+        trace.unregister_callback()
+    assert "YaFSDP::pre_forward (layers.0)" in path.read_text()
+    assert phase_label("YaFSDP::idle") is _NO_LABEL
 
 
 def test_checkpoint_module_recomputes():

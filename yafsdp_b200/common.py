@@ -6,11 +6,13 @@ Parity: ``ya_fsdp/_common.py:13-74``.
 from __future__ import annotations
 
 import contextlib
+import ctypes
 import enum
 import logging
+import os
 import traceback
 from dataclasses import dataclass
-from typing import Any
+from typing import Any, Callable
 
 import torch
 import torch.distributed as dist
@@ -21,10 +23,24 @@ logger = logging.getLogger("yafsdp_b200")
 _NO_LABEL = contextlib.nullcontext()
 
 
+def _observers() -> "Callable[[], bool]":
+    """``at::hasCallbacks``: whether anything observes ``record_function`` ranges on this thread (a profiler, an execution-trace
+    observer, an on-demand trace).  PyTorch exports it from its C++ library only; without it the answer is always yes."""
+    try:
+        has = ctypes.CDLL(os.path.join(os.path.dirname(torch.__file__), "lib", "libtorch_cpu.so"))._ZN2at12hasCallbacksEv
+    except (OSError, AttributeError):
+        return lambda: True
+    has.restype, has.argtypes = ctypes.c_bool, []
+    return has  # type: ignore[no-any-return]
+
+
+_observed = _observers()
+
+
 def phase_label(name: str, of: str = "") -> Any:
-    """``record_function`` range ``name (of)`` while a profiler is active, nothing otherwise: entering and leaving a range costs
-    4 to 8 us of host time, 35 times in a step of a two-layer model."""
-    if not torch.autograd._profiler_enabled():  # type: ignore[attr-defined]
+    """``record_function`` range ``name (of)`` where something would see it, nothing otherwise: entering and leaving a range
+    costs 4 to 12 us of host time, 35 times in a step of a two-layer model; the question 0.4 us."""
+    if not _observed():
         return _NO_LABEL
     return torch.profiler.record_function(f"{name} ({of})" if of else name)
 
