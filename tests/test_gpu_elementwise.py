@@ -248,6 +248,39 @@ def test_clip_grad_norm_with_a_tensor_as_limit(max_norm, form):
             dist.destroy_process_group()
 
 
+def test_in_place_writes_of_gradients_move_their_version():
+    """What the kernels change in place counts as changed for autograd: gradients that a backward pass adds to, and clipped ones."""
+    import torch.distributed as dist
+
+    from yafsdp_b200 import MixedPrecisionPolicy, fully_shard
+    from yafsdp_b200.optim import clip_grad_norm_
+
+    torch.cuda.set_device(0)
+    created = not dist.is_initialized()
+    if created:
+        dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1)
+    try:
+        model = torch.nn.Sequential(torch.nn.Linear(64, 64, device="cuda"), torch.nn.Linear(64, 8, device="cuda"))
+        fully_shard(model, mp_policy=MixedPrecisionPolicy(param_dtype=torch.bfloat16, reduce_dtype=torch.float32))
+        x = torch.randn(16, 64, device="cuda").bfloat16()
+        model(x).square().sum().backward()
+        grads = [p.grad._local_tensor for p in model.parameters()]
+        before = [g._version for g in grads]
+        values = [g.clone() for g in grads]
+        model(x).square().sum().backward()  # added to the gradients that are there
+        assert all(p.grad._local_tensor is g or p.grad._local_tensor.data_ptr() == g.data_ptr() for p, g in zip(model.parameters(), grads))
+        assert all(torch.allclose(g, 2 * v) for g, v in zip(grads, values))
+        added = [g._version for g in grads]
+        assert all(a > b for a, b in zip(added, before))
+        grads = [p.grad._local_tensor for p in model.parameters()]
+        added = [g._version for g in grads]
+        clip_grad_norm_(model, 1e-3)
+        assert all(g._version > a for g, a in zip(grads, added))
+    finally:
+        if created:
+            dist.destroy_process_group()
+
+
 @pytest.mark.parametrize("t,d", [(1, 8), (7, 1024), (700, 1032), (601, 2048), (1200, 4096), (297, 4104), (599, 8192)])
 def test_rmsnorm_bwd_weight_gradient_over_many_rows(t, d):
     """Every width class of the row walk, more rows than a wave holds: the weight gradient in a fixed order, cleared or added to,

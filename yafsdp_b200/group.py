@@ -1016,6 +1016,7 @@ class ParamGroup:
 
             with torch.cuda.device(self.device):
                 kernels.accum_bf16_to_f32_multi_(mine, accumulate)
+            torch.autograd.graph.increment_version([d for d, _ in mine])  # changed in place, behind autograd's back
         return rest
 
     def _finish_pushes(self) -> None:

@@ -338,7 +338,7 @@ def clip_grad_norm_(parameters: Iterable[torch.Tensor] | nn.Module, max_norm: fl
         with torch.cuda.device(dev):
             for _, r in runs:
                 kernels.scale_(r, coef)
-                torch.autograd.graph.increment_version(r)  # changed in place, behind autograd's back
+        torch.autograd.graph.increment_version([g._local_tensor for g in grads])  # type: ignore[attr-defined]  # changed in place, behind autograd's back
         return total
     for g in grads:
         (g._local_tensor if isinstance(g, RaggedShardDTensor) else g).mul_(coef)
