@@ -1154,11 +1154,10 @@ Plan make_plan(int M, int N, int K, int kind, int n_align, int sm_limit, bool ma
   return best;
 }
 
-unsigned long long next_nonce() {  // 56 bits, never 0, different in every launch of this process
+unsigned long long next_nonce() {  // 56 bits, never 0, another one in each of 2^56 launches of this process
   static std::atomic<unsigned long long> n{0};
-  unsigned long long z = n.fetch_add(1, std::memory_order_relaxed) + 1;
-  z *= 0x9E3779B97F4A7C15ull;  // odd: no two launches get the same word
-  return (z >> 8) | 1ull;
+  // modulo 2^56 multiplication by an odd number permutes: neighbours in time get words that differ in many places
+  return ((n.fetch_add(1, std::memory_order_relaxed) + 1) * 0x9E3779B97F4A7C15ull) & ((1ull << 56) - 1);
 }
 
 template <int MODE>
