@@ -1210,8 +1210,9 @@ int launch_plain(const Operands* ops, int n_ops, GemmArgs args, const FusedArgs&
   return launch_tile<MODE_PLAIN>(p.tile, ops, n_ops, args, fa, sm_limit, s);
 }
 
-// Tile shape of the fused modes: CTA pairs (256 x 256 tiles, half of B per CTA) whenever both extents fill such a tile;
-// single CTAs with 128 x 256 or 128 x 128 tiles for small or ragged problems.
+// The entries without a workspace.  Plain mode: make_plan, nothing split.  Tile shape of the fused modes: CTA pairs (256 x 256 tiles,
+// half of B per CTA) whenever both extents fill such a tile; single CTAs with 128 x 256 or 128 x 128 tiles for small or ragged
+// problems.
 int dispatch_gemm(const void* A, const void* B, const GemmArgs& args, const FusedArgs& fa, long long lda, long long ldb, int sm_limit,
                   cudaStream_t s) {
   const int M = args.M, N = args.N;
@@ -1269,7 +1270,6 @@ extern "C" int yf_gemm_bf16_sumsq(const void* A, const void* B, void* C, int M, 
   args.out_f32 = out_f32 ? 1 : 0;
   args.accumulate = accumulate ? 1 : 0;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  // 128x256 tiles unless N is small or the 256-wide tiling wastes more of the last column block
   FusedArgs fa;
   memset(&fa, 0, sizeof(fa));
   fa.sumsq = sumsq;
@@ -1300,8 +1300,8 @@ extern "C" int yf_gemm_bf16_residual(const void* A, const void* B, void* C, cons
 
 // The general form of the entries above.  `workspace` (256-byte aligned device memory that no other launch uses meanwhile, its
 // contents do not matter) lets the last wave's tiles be split along K; yf_gemm_workspace says how much a problem wants, with
-// less (or none) no tile is split.  kind: 0 bf16 output of a K-major A, 1 fp32 output, 2 any other.  tile, splits: 0 = chosen from the shape; else a Tile (TILE_SWAP with
-// kind 0 only) and 1 to MAX_SPLITS.
+// less (or none) no tile is split.  kind: 0 bf16 output of a K-major A, 1 fp32 output, 2 any other.  tile,
+// splits: 0 = chosen from the shape (make_plan); else a Tile (TILE_SWAP with kind 0 only) and 1 to MAX_SPLITS.
 extern "C" int yf_gemm_workspace(int M, int N, int K, int kind, int n_align, int sm_limit, int tile, int splits, long long* bytes) {
   if (M <= 0 || N <= 0 || K <= 0 || kind < 0 || kind > 2 || n_align < 0 || bytes == nullptr || tile < 0 || tile > 6 || splits < 0 || splits > MAX_SPLITS) return -1;
   *bytes = make_plan(M, N, K, kind, n_align, sm_limit, true, tile, splits).bytes;

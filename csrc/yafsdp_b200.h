@@ -54,7 +54,7 @@ int yf_gemm_bf16_scatter_grouped(int n, const void* const* A, const void* const*
 
 // ---- memory-bound kernels (elementwise.cu)
 int yf_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int T, int D, float eps, void* stream);
-/* dx (+ dres) and dw += column sums of dy * xhat; zero_dw: dw is cleared first, inside the dx kernel (no fill launch) */
+/* dx (+ dres) and dw += column sums of dy * xhat; zero_dw: what dw held before does not count (here: a memset, then atomic sums) */
 int yf_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float* rstd, const void* dres, void* dx,
                    float* dw, int zero_dw, int T, int D, void* stream);
 /* the same with the weight gradient summed in a fixed order and, optionally, *sumsq += its squares: partials [yf_rmsnorm_bwd_partials(T, D), D] fp32 scratch */

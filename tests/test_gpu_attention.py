@@ -191,3 +191,30 @@ def test_attention_fwd_adds_row_sums_in_the_order_of_the_keys():
     torch.cuda.synchronize()
     kernels.check_status()
     assert (lse.double() - math.log1p(2.0**-19)).abs().max().item() < 2.0**-24  # the next sum is 2^-20 away
+
+
+def test_attention_bwd_heads_in_several_groups():
+    """A dQ accumulator beyond 64 MB and heads for more than three groups: the CTAs go group by group, the last group is smaller.
+    Some heads against fp64 (P, dS and the results are rounded to bf16)."""
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(22)
+    b, s, h, d = 2, 2304, 32, 128
+    assert b * s * h * d * 4 > 64 << 20 and (2 * 148 + s // 128 - 1) // (s // 128) < b * h / 3  # the rule's two conditions on 148 SMs
+    qkv = torch.randn(b * s, 3 * h * d, device="cuda").bfloat16()
+    q, k, v = qkv[:, : h * d], qkv[:, h * d : 2 * h * d], qkv[:, 2 * h * d :]
+    scale = 1.0 / math.sqrt(d)
+    out, lse = kernels.attn_fwd(q, k, v, b, s, h, h, scale, True)
+    dout = torch.randn_like(out)
+    g = torch.full_like(qkv, float("nan"))
+    kernels.attn_bwd(q, k, v, out, dout, lse, g[:, : h * d], g[:, h * d : 2 * h * d], g[:, 2 * h * d :], b, s, h, h, scale, True)
+    torch.cuda.synchronize()
+    kernels.check_status()
+    assert not g.isnan().any()
+    for bi, hi in ((0, 0), (0, 16), (0, 17), (1, 1), (1, 2), (1, 19), (1, 31)):  # both sides of the groups' borders, first and last
+        rows = slice(bi * s, (bi + 1) * s)
+        qf, kf, vf = (x[rows, hi * d : (hi + 1) * d].double().view(1, s, 1, d).requires_grad_(True) for x in (q, k, v))
+        _ref(qf, kf, vf, True).backward(dout[rows, hi * d : (hi + 1) * d].double().view(1, s, 1, d))
+        for x, at in ((qf, hi), (kf, h + hi), (vf, 2 * h + hi)):
+            want = x.grad.reshape(s, d)
+            assert ((g[rows, at * d : (at + 1) * d].double() - want).norm() / want.norm()).item() < 2.0**-7

@@ -246,3 +246,98 @@ def test_gemm_without_a_usable_workspace(tile, splits, given):
     kernels.check_status()
     # the same plan as for a caller that asks for whole tiles
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("m,n,k,f32,split", [(45, 4096, 4096, False, False), (1337, 4096, 11008, False, False), (1337, 4096, 11008, True, True),
+                                             (999, 5120, 13824, True, True), (333, 5120, 13824, False, False), (2048, 2816, 512, False, False)])
+def test_gemm_plans_chosen_from_the_shape(m, n, k, f32, split):
+    """Nothing forced: few tokens (narrow tiles), ragged ones (swapped), a last wave in K ranges, whole pair tiles; against fp64.
+    fp32 sums of k products: a few sqrt(k) * 2^-24; a bf16 result: 2^-8."""
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(19)
+    a, b = torch.randn(m, k, device="cuda").bfloat16(), torch.randn(n, k, device="cuda").bfloat16()
+    assert (kernels._gemm_workspace(m, n, k, int(f32), 0, 0, 0, 0, 0) > 0) == split
+    got = kernels.gemm(a, b, out_dtype=torch.float32 if f32 else torch.bfloat16)
+    again = kernels.gemm(a, b, out_dtype=got.dtype)
+    ref = a.double() @ b.double().t()
+    torch.cuda.synchronize()
+    kernels.check_status()
+    assert ((got.double() - ref).norm() / ref.norm()).item() < (3.0 * k**0.5 * 2.0**-24 if f32 else 2.0**-8)
+    assert torch.equal(got, again)
+
+
+@pytest.mark.parametrize("rows", [[512, 256, 256], [256, 768, 24]])
+@pytest.mark.parametrize("tile,splits", [(1, 1), (5, 1), (2, 1), (1, 2)])
+def test_gemm_weight_in_pieces_wide_tiles(rows, tile, splits):
+    """Pieces of an [N, K] weight that start where pair tiles do: every CTA of a pair reads its half from the right piece."""
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(20)
+    cols, m = 1032, 600
+    parts = [torch.randn(r, cols, device="cuda").bfloat16() for r in rows]
+    a = torch.randn(m, cols, device="cuda").bfloat16()
+    got = kernels.gemm_parts(a, parts, tile=tile, splits=splits)
+    want = kernels.gemm(a, torch.cat(parts), tile=tile, splits=splits)
+    torch.cuda.synchronize()
+    kernels.check_status()
+    assert torch.equal(got, want)
+
+
+def test_entries_without_scratch():
+    """The C entries that Python does not call, against the general forms: plain GEMMs without a workspace, RMSNorm backward with atomic
+    weight sums, embedding backward without a norm, attention backward without parts."""
+    from yafsdp_b200 import _native
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(21)
+    lib, st = _native.lib(), torch.cuda.current_stream().cuda_stream
+    m, n, k = 333, 520, 1032
+    a, b = torch.randn(m, k, device="cuda").bfloat16(), torch.randn(n, k, device="cuda").bfloat16()
+    r = torch.randn(m, n, device="cuda").bfloat16()
+    low, f32, sq, res = torch.empty_like(r), torch.empty(m, n, device="cuda"), torch.zeros(1, device="cuda"), torch.empty_like(r)
+    p = [t.data_ptr() for t in (a, b)]
+    assert lib.yf_gemm_bf16(*p, low.data_ptr(), m, n, k, k, k, n, 0, 0, 0, 0, 0.5, 0, st) == 0
+    assert lib.yf_gemm_bf16_sumsq(*p, f32.data_ptr(), m, n, k, k, k, n, 0, 0, 1, 0, 1.0, 0, sq.data_ptr(), st) == 0
+    assert lib.yf_gemm_bf16_residual(*p, res.data_ptr(), r.data_ptr(), m, n, k, k, k, n, n, 0, 0, 1.0, 0, st) == 0
+    # whole tiles of every shape add the products in the same order
+    assert torch.equal(low, kernels.gemm(a, b, alpha=0.5, splits=1)) and torch.equal(f32, kernels.gemm(a, b, out_dtype=torch.float32, splits=1))
+    assert torch.equal(res, kernels.gemm(a, b, residual=r, splits=1))
+    assert abs(sq.item() / f32.double().pow(2).sum().item() - 1.0) < 2.0**-14  # fp32 sums over a thread's rows, then atomics
+
+    t, d = 700, 1032
+    x, dy = (torch.randn(t, d, device="cuda").bfloat16() for _ in range(2))
+    w = torch.ones(d, device="cuda").bfloat16()
+    _, rstd = kernels.rmsnorm_fwd(x, w, 1e-5)
+    for zero in (1, 0):
+        dw, want = torch.full((d,), 2.0, device="cuda"), torch.full((d,), 2.0, device="cuda")
+        dx = torch.empty_like(x)
+        assert lib.yf_rmsnorm_bwd(x.data_ptr(), w.data_ptr(), dy.data_ptr(), rstd.data_ptr(), None, dx.data_ptr(), dw.data_ptr(), zero, t, d, st) == 0
+        assert torch.equal(dx, kernels.rmsnorm_bwd(x, w, dy, rstd, want, zero_dw=bool(zero)))
+        assert torch.allclose(dw, want, rtol=1e-5, atol=t**0.5 * 1e-5)  # fp32 sums of t terms of about one in two orders
+
+    ids = torch.randint(0, 40, (t,), device="cuda")
+    table, want = torch.zeros(40, d, device="cuda"), torch.zeros(40, d, device="cuda")
+    assert lib.yf_embedding_bwd(dy.data_ptr(), ids.data_ptr(), table.data_ptr(), t, d, 40, st) == 0
+    kernels.embedding_bwd_(dy, ids, want)
+    assert torch.allclose(table, want, rtol=1e-5, atol=1e-4)  # some twenty fp32 additions in any order
+
+    bsz, s, hq, hkv = 1, 200, 4, 2
+    qkv = torch.randn(s, (hq + 2 * hkv) * 128, device="cuda").bfloat16()
+    q, kk, v = qkv[:, : hq * 128], qkv[:, hq * 128 : (hq + hkv) * 128], qkv[:, (hq + hkv) * 128 :]
+    out, lse = kernels.attn_fwd(q, kk, v, bsz, s, hq, hkv, 0.09, True)
+    dout = torch.randn_like(out)
+    got, want = torch.empty_like(qkv), torch.empty_like(qkv)
+    delta, acc = torch.empty(hq * s, device="cuda"), torch.empty(s * hq * 128, device="cuda")
+    ld = qkv.stride(0)
+
+    def views(g):
+        return g[:, : hq * 128], g[:, hq * 128 : (hq + hkv) * 128], g[:, (hq + hkv) * 128 :]
+
+    assert lib.yf_attn_bwd(*[x.data_ptr() for x in (q, kk, v, out, dout, lse, delta, acc, *views(got))], bsz, s, hq, hkv, ld, ld, out.stride(0),
+                           dout.stride(0), ld, ld, 0.09, 1, st) == 0
+    kernels.attn_bwd(q, kk, v, out, dout, lse, *views(want), bsz, s, hq, hkv, 0.09, True, head_parts=1)
+    torch.cuda.synchronize()
+    kernels.check_status()
+    assert torch.equal(got[:, hq * 128 :], want[:, hq * 128 :])
+    assert torch.allclose(got.float(), want.float(), rtol=2.0**-7, atol=1e-5)  # dq: fp32 sums in any order, one bf16 rounding

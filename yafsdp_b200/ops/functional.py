@@ -161,42 +161,21 @@ def flush_pushed(deferred: "list[tuple[Any, ...]]") -> None:
     deferred.clear()
 
 
-def _norm_weight_grad(w: torch.Tensor, fn: Any, self_zeroing: bool = False, self_norm: bool = False) -> torch.Tensor | None:
-    """Run ``fn(dw_fp32)`` (a kernel that accumulates into dw); returns the gradient unless sunk.
-    ``self_zeroing``: the kernel can clear its target itself and is called as ``fn(dw, zero)``.  ``self_norm``: the kernel can
-    sum the squares of a gradient that starts from zeros and is called as ``fn(dw, target or None)``; with both,
-    ``fn(dw, zero, target or None)``."""
+def _norm_weight_grad(w: torch.Tensor, fn: Any, self_zeroing: bool = True) -> torch.Tensor | None:
+    """Run ``fn(dw_fp32, zero, target)``, a kernel that accumulates into ``dw_fp32``; returns the gradient unless sunk.  ``zero``: the
+    kernel is to clear ``dw_fp32`` first (with ``self_zeroing`` only; else it starts from zeros already).  ``target``: where the
+    kernel adds the squares of the gradient, or ``None``; given only where the gradient starts from zeros and is final."""
     s = _sink(w)
+    if s is not None and not s.pushes() and s.local_ok:
+        zeroed_now = not s.would_accumulate()
+        view, _ = s.begin(zero=not self_zeroing)
+        fn(view, zeroed_now and self_zeroing, s.norm_target(not zeroed_now))
+        return None
+    dw = (torch.empty if self_zeroing else torch.zeros)(w.shape, device=w.device, dtype=torch.float32)
+    fn(dw, self_zeroing, None)
     if s is not None and s.pushes():
-        dw = torch.empty(w.shape, device=w.device, dtype=torch.float32) if self_zeroing else torch.zeros(w.shape, device=w.device, dtype=torch.float32)
-        fn(dw, True) if self_zeroing else fn(dw)
         s.push_from(dw)
         return None
-    if s is not None and s.local_ok:
-        zeroed_now = not s.would_accumulate()
-        if self_norm:
-            view, _ = s.begin(zero=not self_zeroing)
-            target = s.norm_target(not zeroed_now)
-            fn(view, zeroed_now, target) if self_zeroing else fn(view, target)
-            return None
-        if self_zeroing:
-            view, _ = s.begin(zero=False)
-            fn(view, zeroed_now)
-        else:
-            view, _ = s.begin(zero=True)
-            fn(view)
-        # the value is final (and its squares may be summed here) only if this call started from zeros: an earlier write
-        # of this backward pass or an earlier micro-batch's gradient makes it a partial sum
-        tgt = s.norm_target(not zeroed_now)
-        if tgt is not None:
-            kernels.sumsq_(view.reshape(-1), tgt)
-        return None
-    if self_zeroing:
-        dw = torch.empty(w.shape, device=w.device, dtype=torch.float32)
-        fn(dw, True)
-    else:
-        dw = torch.zeros(w.shape, device=w.device, dtype=torch.float32)
-        fn(dw)
     return dw.to(w.dtype)
 
 
@@ -217,7 +196,7 @@ class EmbeddingFn(torch.autograd.Function):
         (ids,) = ctx.saved_tensors
         table = ctx.table
         dout2 = _c(dout).view(-1, table.shape[1])
-        grad = _norm_weight_grad(table, lambda dw, sumsq=None: kernels.embedding_bwd_(dout2, ids.reshape(-1), dw, sumsq), self_norm=True)
+        grad = _norm_weight_grad(table, lambda dw, _, sq: kernels.embedding_bwd_(dout2, ids.reshape(-1), dw, sq), self_zeroing=False)
         return None, grad
 
 
@@ -288,7 +267,7 @@ class DecoderLayerFn(torch.autograd.Function):
         g_wg, g_wu = _WeightGrad([wg, wu]).run(dgu, n2, pushed)
         del dgu
         box: list[torch.Tensor] = []
-        g_n2 = _norm_weight_grad(w_n2, lambda dw, z, sq=None: box.append(kernels.rmsnorm_bwd(h, w_n2.detach(), dn2, rstd2, dw, dres=dout, zero_dw=z, sumsq=sq)), True, True)
+        g_n2 = _norm_weight_grad(w_n2, lambda dw, z, sq: box.append(kernels.rmsnorm_bwd(h, w_n2.detach(), dn2, rstd2, dw, dres=dout, zero_dw=z, sumsq=sq)))
         dh = box.pop()
         # ---- attention
         datt = kernels.gemm(dh, wo.detach(), b_mn_major=True)
@@ -304,7 +283,7 @@ class DecoderLayerFn(torch.autograd.Function):
             kernels.rope_(dqkv, cos_sin, dims.seq, 0, hq + hkv, hd, backward=True)
         dn1 = _gemm_fused(dqkv, w_qkv, b_mn_major=True)
         g_wq, g_wk, g_wv = _WeightGrad([wq, wk, wv]).run(dqkv, n1, pushed)
-        g_n1 = _norm_weight_grad(w_n1, lambda dw, z, sq=None: box.append(kernels.rmsnorm_bwd(x, w_n1.detach(), dn1, rstd1, dw, dres=dh, zero_dw=z, sumsq=sq)), True, True)
+        g_n1 = _norm_weight_grad(w_n1, lambda dw, z, sq: box.append(kernels.rmsnorm_bwd(x, w_n1.detach(), dn1, rstd1, dw, dres=dh, zero_dw=z, sumsq=sq)))
         dx = box.pop()
         flush_pushed(pushed)
         return dx, g_n1, g_wq, g_wk, g_wv, g_wo, g_n2, g_wg, g_wu, g_wd, None, None, None
@@ -337,7 +316,7 @@ class HeadLossFn(torch.autograd.Function):
         dn = kernels.gemm(dlogits, w_head.detach(), b_mn_major=True, alpha_tensor=scale)
         (g_head,) = _WeightGrad([w_head]).run(dlogits, n, scale=scale)
         box: list[torch.Tensor] = []
-        g_norm = _norm_weight_grad(w_norm, lambda dw, z, sq=None: box.append(kernels.rmsnorm_bwd(h, w_norm.detach(), dn, rstd, dw, zero_dw=z, sumsq=sq)), True, True)
+        g_norm = _norm_weight_grad(w_norm, lambda dw, z, sq: box.append(kernels.rmsnorm_bwd(h, w_norm.detach(), dn, rstd, dw, zero_dw=z, sumsq=sq)))
         return box.pop(), g_norm, g_head, None, None
 
 
@@ -360,7 +339,7 @@ class HeadLogitsFn(torch.autograd.Function):
         dn = kernels.gemm(dlogits, w_head.detach(), b_mn_major=True)
         (g_head,) = _WeightGrad([w_head]).run(dlogits, n)
         box: list[torch.Tensor] = []
-        g_norm = _norm_weight_grad(w_norm, lambda dw, z, sq=None: box.append(kernels.rmsnorm_bwd(h, w_norm.detach(), dn, rstd, dw, zero_dw=z, sumsq=sq)), True, True)
+        g_norm = _norm_weight_grad(w_norm, lambda dw, z, sq: box.append(kernels.rmsnorm_bwd(h, w_norm.detach(), dn, rstd, dw, zero_dw=z, sumsq=sq)))
         return box.pop(), g_norm, g_head, None
 
 

@@ -269,8 +269,8 @@ def rmsnorm_fwd(x: torch.Tensor, w: torch.Tensor, eps: float) -> tuple[torch.Ten
 
 def rmsnorm_bwd(x: torch.Tensor, w: torch.Tensor, dy: torch.Tensor, rstd: torch.Tensor, dw_f32: torch.Tensor,
                 dres: torch.Tensor | None = None, zero_dw: bool = False, sumsq: torch.Tensor | None = None) -> torch.Tensor:
-    """Returns dx (+ dres when given); accumulates the weight gradient into the fp32 tensor ``dw_f32`` (``zero_dw``: the
-    kernel clears it first, which saves the caller a fill launch; ``sumsq``: ``+= sum(dw_f32**2)`` of the result)."""
+    """Returns dx (+ dres when given); accumulates the weight gradient into the fp32 tensor ``dw_f32`` (``zero_dw``: what
+    it held before does not count, the caller need not clear it; ``sumsq``: ``+= sum(dw_f32**2)`` of the result)."""
     t, d = x.shape
     dx = torch.empty_like(x)
     assert dw_f32.dtype == torch.float32 and dw_f32.numel() == d
