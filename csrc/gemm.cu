@@ -1048,8 +1048,16 @@ struct TileShape {
 };
 constexpr TileShape TILE_SHAPES[6] = {{0, 0, 0.f, 0.f}, {2, 256, 7.f, 0.36f}, {1, 256, 6.f, 0.40f}, {1, 128, 4.8f, 0.225f}, {1, 64, 4.2f, 0.155f}, {2, 128, 6.f, 0.20f}};
 
-// Estimated time of a tile shape and split count.  A tile takes its K blocks or, where K is short, its epilogue (15 ns per
-// column of fp32 output, 10.5 ns of bf16); no shape gets more than 5.2 TB/s out of HBM on operands that are read once.
+// What a tile takes whose K blocks take `loop` and whose epilogue takes `epi` us: they overlap, but both move data between the SM and
+// the L2.
+float tile_time(float loop, float epi) { return loop > epi ? loop + 0.4f * epi : epi + 0.4f * loop; }
+
+// Estimated time of a tile shape and split count.  The epilogue has a fixed part (larger for a pair) and one per column, fp32 or
+// bf16; no shape gets more than 5.2 TB/s out of HBM on operands that are read once.  Where K is short (weight gradients of few
+// tokens) the fixed part decides, us with tiles of pairs of 256 / 256 / 128 / 64 / pairs of 128 columns (* the choice):
+//   fp32 output [57344 x 8192 x 100] 399 / 334* / 363 / 513 / 574, [28672 x 4096 x 333] 146 / 139* / 142 / 163 / 199;
+//   bf16 [57344 x 8192 x 100] 307 / 254* / 304 / 383 / 410, [28672 x 4096 x 777] 157* / 173 / 213 / 300 / 213.
+// (With an epilogue of 15 and 10.5 ns per column and no fixed part every shape was estimated the same there, and the narrowest won.)
 // Splitting: an exchange of partial sums takes 6 to 18 us (a release and an acquire at GPU scope in an SM full of
 // asynchronous copies).  Whole tiles behind it hide it, unless a unit gets several ranges one after another.  Long GEMMs
 // run against the power cap, where idle units are not all lost, hence the factor of 1.1.
@@ -1059,12 +1067,13 @@ float plan_us(const TileShape& t, int M, int N, int K, int units, int splits, bo
   const int tile_m = BLOCK_M * t.cg, num_k = (K + BLOCK_K - 1) / BLOCK_K;
   const long long tiles = (long long)((M + tile_m - 1) / tile_m) * ((N + t.bn - 1) / t.bn);
   const long long full = tiles / units, rest = tiles - full * units;
-  const float epi = (float)t.bn * (out_f32 ? 0.015f : 0.0105f), loop = (float)num_k * t.kb_us, tile_us = loop > epi ? loop : epi;
+  const float epi = (t.cg == 2 ? 0.95f : 0.39f) + (float)t.bn * (out_f32 ? 0.0118f : 0.0083f);
+  const float loop = (float)num_k * t.kb_us, tile_us = tile_time(loop, epi);
   float us = (float)full * tile_us;
   if (rest > 0 && splits == 1) us += tile_us;
   if (rest > 0 && splits > 1) {
     const float rounds = (float)((rest * splits + units - 1) / units), part = loop / (float)splits;
-    us += rounds * ((rounds > 1.f && part < 9.f ? 9.f : part) + 4.f);
+    us += rounds * ((rounds > 1.f && part < 9.f ? 9.f : part) + 4.f) + tile_us - (loop > epi ? loop : epi);
     us *= 1.1f;
   }
   const float exchange_us = rest == 0 || splits == 1 ? 0.f : (full > 0 ? 3.f : 2.f + 4.f * (float)splits);
@@ -1074,7 +1083,7 @@ float plan_us(const TileShape& t, int M, int N, int K, int units, int splits, bo
 
 // The swapped form: pairs of 256 weight rows x bn tokens, for every number of token tiles.  A K block takes its MMAs (1.55 ns per
 // token with all units busy, a little more than the unswapped form: the epilogue transposes) or its loads (128 + bn / 2 rows at
-// 122 GB/s per SM), an epilogue 12 ns per token.  Best unswapped / swapped, us:
+// 122 GB/s per SM), an epilogue 2 us and 12 ns per token.  Best unswapped / swapped, us:
 //   [333 x 27648 x 5120] 98 / 84, [777 x 8192 x 22016] 265 / 218, [777 x 8192 x 8192] 96 / 84, [1337 x 22016 x 4096] 179 / 166,
 //   [1337 x 4096 x 4096] 42 / 38; [2048 x 22016 x 4096] 243 / 270 and [999 x 27648 x 5120] 199 / 209 stay unswapped.
 float swap_us(int M, int N, int K, int units, int* bn) {
@@ -1086,7 +1095,7 @@ float swap_us(int M, int N, int K, int units, int* bn) {
     if (w > 256 || w < 16) continue;
     const long long tiles = (long long)rows * ((M + w - 1) / w), waves = (tiles + units - 1) / units;
     const float mma = 0.00155f * (float)w, load = (128.f + 0.5f * (float)w) * 0.00105f, loop = (float)num_k * (mma > load ? mma : load);
-    const float epi = 0.012f * (float)w, us = (float)waves * (loop > epi ? loop : epi);
+    const float epi = 2.f + 0.012f * (float)w, us = (float)waves * tile_time(loop, epi);
     const float t = 7.f + (us > read_us ? us + 0.1f * read_us : read_us + 0.1f * us);
     if (t < best) {
       best = t;
@@ -1306,6 +1315,12 @@ extern "C" int yf_gemm_workspace(int M, int N, int K, int kind, int n_align, int
   if (M <= 0 || N <= 0 || K <= 0 || kind < 0 || kind > 2 || n_align < 0 || bytes == nullptr || tile < 0 || tile > 6 || splits < 0 || splits > MAX_SPLITS) return -1;
   *bytes = make_plan(M, N, K, kind, n_align, sm_limit, true, tile, splits).bytes;
   return 0;
+}
+// the Tile that is chosen, plus 16 * (K ranges of the last wave's tiles); kind and n_align as above
+extern "C" int yf_gemm_plan(int M, int N, int K, int kind, int n_align, int sm_limit) {
+  if (M <= 0 || N <= 0 || K <= 0 || kind < 0 || kind > 2 || n_align < 0) return -1;
+  const Plan p = make_plan(M, N, K, kind, n_align, sm_limit, true, 0, 0);
+  return p.tile + 16 * p.splits;
 }
 extern "C" int yf_gemm_bf16_ws(const void* A, const void* B, void* C, const void* R, int M, int N, int K, long long lda, long long ldb,
                                long long ldc, long long ldr, int a_mn, int b_mn, int out_f32, int accumulate, float alpha, int sm_limit,

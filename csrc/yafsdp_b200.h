@@ -27,6 +27,7 @@ int yf_gemm_bf16_residual(const void* A, const void* B, void* C, const void* R, 
 /* The general form: optional residual R, optional sumsq, a workspace for splitting the last wave along K (see gemm.cu), a tile
    shape and a split count (0 = chosen).  yf_gemm_workspace: the workspace bytes that a problem wants. */
 int yf_gemm_workspace(int M, int N, int K, int kind, int n_align, int sm_limit, int tile, int splits, long long* bytes);
+int yf_gemm_plan(int M, int N, int K, int kind, int n_align, int sm_limit);  /* tile + 16 * splits that would be chosen */
 int yf_gemm_bf16_ws(const void* A, const void* B, void* C, const void* R, int M, int N, int K, long long lda, long long ldb,
                     long long ldc, long long ldr, int a_mn, int b_mn, int out_f32, int accumulate, float alpha, int sm_limit,
                     const float* alpha_ptr, float* sumsq, void* workspace, long long workspace_bytes, int tile, int splits, void* stream);

@@ -177,6 +177,7 @@ def _declare(l: ctypes.CDLL) -> None:
         "yf_gemm_bf16_sumsq": [_P, _P, _P, _I, _I, _I, _L, _L, _L, _I, _I, _I, _I, _F, _I, _P, _P],
         "yf_gemm_bf16_residual": [_P, _P, _P, _P, _I, _I, _I, _L, _L, _L, _L, _I, _I, _F, _I, _P],
         "yf_gemm_workspace": [_I, _I, _I, _I, _I, _I, _I, _I, _P],
+        "yf_gemm_plan": [_I, _I, _I, _I, _I, _I],
         "yf_gemm_bf16_ws": [_P, _P, _P, _P, _I, _I, _I, _L, _L, _L, _L, _I, _I, _I, _I, _F, _I, _P, _P, _P, _L, _I, _I, _P],
         "yf_gemm_swiglu": [_P, _P, _P, _P, _P, _I, _I, _I, _L, _L, _L, _L, _L, _P],
         "yf_gemm_swiglu_pays": [_I, _I, _I],
