@@ -73,8 +73,9 @@ __host__ __device__ inline long long part_tile(int part, int B, int b, int n_kt,
 
 // Order of the CTAs: heads are taken in groups, within a group key tile by key tile with the heads fastest, so that all heads'
 // long walks start first.  One group holds all heads unless the dQ accumulator outgrows the L2 and there are heads for three
-// groups; then a group has two CTAs per SM, whose sums stay in the L2 (2 x 4096 tokens x 32 heads: 1235 us in one group,
-// 1036 us in groups of ten heads; 1 x 8192 x 32/8 heads, 1661 us in one group and 1772 us in two, stays whole).
+// groups; then a group has two CTAs per SM, whose sums stay in the L2.  It pays for many sequences or long ones: 8 x 2048 tokens x 32
+// heads 1449 us in one group, 1247 in groups of 19; 2 x 8192 x 32 3516 / 3438 in groups of five; 2 x 2304 x 32 393 / 380; 2 x 4096 x
+// 32 971 / 995 in groups of ten; 1 x 4096 x 64 984 / 1013.  1 x 8192 x 32/8 stays whole: 1543 us, 1572 in two groups.
 YF_DEVINL void head_group_order(int cta, int n_pos, int n_heads, int group, int& pos, int& head) {
   const int per_group = n_pos * group;
   const int g = cta / per_group;
@@ -286,7 +287,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       // queries [0, hidden) of the tile do not see this key: those in front of it, all when the key is past the end
       const int hidden = key >= args.S ? BQ : (args.causal ? key - q0 : 0);
       const bool any_hidden = __any_sync(0xffffffffu, hidden > 0);
-      // 32 queries at a time: everything stays in registers (a spill goes to the L2: shared memory leaves no L1)
+      // 32 queries at a time: all but a few words (28 bytes, 52 with shared key tiles) stay in registers; a spill goes to the L2, as
+      // shared memory leaves no L1
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t s[32], dp[32], pk[16], dk[16];

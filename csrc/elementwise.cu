@@ -515,8 +515,10 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
   }
 }
 
-// The loss's two scalars, one block each: bound by the latency of a launch.  (As comparison, sum, clamp, cast and reciprocal, and as
-// sum and product, they were seven launches of 2 to 4 us.)
+// The loss's two scalars, one block each: bound by the latency of a launch up to some 10^5 values.  Device time, us, against PyTorch's
+// comparison, sum, clamp, cast and reciprocal / sum and product: 8192 tokens 2.2 against 12 / 2.2 against 4.4; 131072 tokens 6.5 against
+// 19 / 4.6 against 10; 524288 tokens 19 against 19 / 11 against 10; 1048576 tokens 36 against 20 / 20 against 11 (next to 0.2 s of head
+// GEMMs).
 constexpr int ONE_BLOCK = 1024;
 __global__ void __launch_bounds__(ONE_BLOCK) inv_valid_labels_kernel(const long long* __restrict__ labels, long long n, float* __restrict__ out) {
   __shared__ int count;

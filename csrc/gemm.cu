@@ -287,6 +287,8 @@ __device__ void gather_comm_role(const FusedArgs& fa, long long b_bytes, long lo
   for (long long i = done; i < stored; ++i) publish(i);
 }
 
+// 128 registers a thread, 28 672 of the SM's 65 536: blocks of the pull reduce-scatter (64 registers) and of AdamW find room next to a
+// persistent CTA.  The split instantiations spill 120 to 132 bytes for it, the SwiGLU one 12, around their epilogues.
 template <int BLOCK_N, int CG, int MODE>
 __global__ void __maxnreg__(128)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ CUtensorMap tma_c, GemmArgs args, FusedArgs fa) {
