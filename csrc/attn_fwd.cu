@@ -7,10 +7,10 @@
 //   warps 2-5   softmax of tile 0, warps 6-9 of tile 1: one thread per query row (TMEM lane == row)
 // While one tile's softmax runs, the tensor cores work for the other one.  TMEM (512 columns): S_0, S_1, O_0, O_1, 128
 // columns of fp32 each; P_i (bf16, 64 columns) takes the place of S_i, whose row its thread has read into registers, and is
-// the MMA's A operand from there, so the probabilities never go through shared memory.  A row belongs to one thread: no
-// exchange and no barrier among the softmax threads.
+// the MMA's A operand from there, so the probabilities never go through shared memory.  A row belongs to one thread: the
+// softmax threads exchange nothing but one bit per block, at a barrier of the tile's four warps (below).
 // The output accumulates in TMEM over all key blocks (O += P V).  The exponent's reference maximum is only moved when
-// some row of a warp has grown by more than 2^8 since it was set (then the warp rescales its rows of O in TMEM and its
+// some row of a tile has grown by more than 2^8 since it was set (then its warps rescale their rows of O in TMEM and their
 // sums); otherwise P is taken relative to the older maximum (values up to 2^8, harmless in bf16 / fp32), and the final
 // division by the row sum makes the result exact again.
 // Bound: per 128 x 128 block the two MMAs take 1024 cycles and the 16 384 exponentials at 16 per cycle as long, on
@@ -60,6 +60,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   uint64_t* p_ready = bars + 12;        // [2] per tile
   uint64_t* o_full = bars + 14;         // [2] per tile
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);  // [2] per tile: 1 + the block at which one of its warps has given up
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -88,6 +89,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       mbar_init(&s_full[s], 1);
       mbar_init(&p_ready[s], 4);  // one arrival per softmax warp of the tile
       mbar_init(&o_full[s], 1);
+      dead[s] = 0;
     }
     mbar_fence_init();
   }
@@ -196,14 +198,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     const int limit = args.causal ? min(qrow, args.S - 1) : (args.S - 1);
     bool alive = true;
     for (int j = 0; j < n; ++j) {
-      // a bounded wait that runs out ends the warp's work (the lanes decide together: TMEM accesses are warp-wide)
-      if (!__all_sync(0xffffffffu, mbar_wait(&s_full[i], j & 1, 120 + i))) { alive = false; break; }
-      tc_fence_after();
+      // a bounded wait that runs out ends the work of the tile's four warps: they meet at the barrier below, so the one that gives up
+      // says so there (the lanes of a warp decide together: TMEM accesses are warp-wide)
+      alive = alive && __all_sync(0xffffffffu, mbar_wait(&s_full[i], j & 1, 120 + i));
       const int kv0 = j * BKV;
       uint32_t sc[4][32];
+      if (alive) {
+        tc_fence_after();
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld32(tS + c * 32, sc[c]);
-      tmem_ld_wait();
+        for (int c = 0; c < 4; ++c) tmem_ld32(tS + c * 32, sc[c]);
+        tmem_ld_wait();
+      } else {
+        dead[i] = j + 1;
+      }
       if (kv0 + BKV - 1 > limit) {  // only the blocks on the diagonal and the last one have masked keys
 #pragma unroll
         for (int c = 0; c < 4; ++c)
@@ -219,12 +226,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         for (int t = 1; t < 32; ++t) mx4[c] = fmaxf(mx4[c], __uint_as_float(sc[c][t]));
       }
       const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      const bool grew = (j == 0) || (mx != -INFINITY && (m_run == -INFINITY || (mx - m_run) * sl2 > RESCALE_LOG2));
-      if (__any_sync(0xffffffffu, grew)) {
+      const bool grew = !alive || j == 0 || (mx != -INFINITY && (m_run == -INFINITY || (mx - m_run) * sl2 > RESCALE_LOG2));
+      // The four warps of a tile move their rows' maxima together: a row's bits then depend on its tile alone and repeat those of
+      // kernels that deal the rows to warps in another way.  The barrier costs 4 % at 2048 tokens x 32 heads (49 -> 51 us) and 8 % at
+      // 8192 x 32/8 (570 -> 615 us), less than 0.2 % of a layer's forward and backward.
+      if (i == 0 ? named_bar_or(1, 128, grew) : named_bar_or(2, 128, grew)) {
+        if (dead[i] == j + 1) { alive = false; break; }  // not a later block's: who gives up there waits for this warp there
         const float m_new = fmaxf(m_run, mx);
         if (j > 0) {
           // O holds sums relative to the old maximum: wait for the last P V to land, then scale this warp's rows
-          if (!__all_sync(0xffffffffu, mbar_wait(&o_full[i], (j - 1) & 1, 122 + i))) { alive = false; break; }
+          alive = __all_sync(0xffffffffu, mbar_wait(&o_full[i], (j - 1) & 1, 122 + i));
+          if (!alive) continue;  // to the next barrier, where the others learn of it
           tc_fence_after();
           const float alpha = (m_run == -INFINITY) ? 0.f : fast_exp2((m_run - m_new) * sl2);
 #pragma unroll 1

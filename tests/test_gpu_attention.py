@@ -218,3 +218,28 @@ def test_attention_bwd_heads_in_several_groups():
         for x, at in ((qf, hi), (kf, h + hi), (vf, 2 * h + hi)):
             want = x.grad.reshape(s, d)
             assert ((g[rows, at * d : (at + 1) * d].double() - want).norm() / want.norm()).item() < 2.0**-7
+
+
+def test_attention_fwd_moves_the_reference_of_a_whole_tile():
+    """A row whose scores grow by more than 2^8 behind the first key block moves the reference of the exponents for the 128 rows of
+    its tile, and for no others: a row's bits do not depend on how rows are dealt to warps.  The second weight is 2^0.5 relative to
+    the first block's maximum, which bf16 rounds to 181 / 128, and cancels the first value exactly; relative to its own maximum it is 1
+    and leaves 1 - 181 / 128 * 2^-0.5 of a row sum of 1 + 2^-0.5."""
+    from yafsdp_b200.ops import kernels
+
+    s, d, scale = 256, 128, 0.6931471824645996  # scale * log2(e) is 1 in fp32: weights are powers of two
+    qkv = torch.zeros(s, 3 * d, device="cuda").bfloat16()
+    q, k, v = qkv[:, :d], qkv[:, d : 2 * d], qkv[:, 2 * d :]
+    q[:, 0] = 1.0
+    q[70, 1] = 1.0  # the row that grows: third warp of the first tile
+    k[:, 0] = -100.0
+    k[0, 0], k[128, 0], k[128, 1] = 0.0, 0.5, 16.0
+    v[0], v[128] = -181.0 / 128.0, 1.0
+    out, _ = kernels.attn_fwd(q, k, v, 1, s, 1, 1, scale, False)
+    torch.cuda.synchronize()
+    kernels.check_status()
+    moved = (1.0 - 181.0 / 128.0 * 0.5**0.5) / (1.0 + 0.5**0.5)
+    rows = [r for r in range(128) if r != 70]
+    assert torch.allclose(out[rows].double(), torch.tensor(moved, dtype=torch.float64, device="cuda"), rtol=2.0**-6)  # bf16, and a difference near 1e-4
+    assert (out[128:] == 0).all()
+    assert (out[70].double() - 1.0).abs().max().item() < 2.0**-8
