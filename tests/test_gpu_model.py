@@ -99,6 +99,44 @@ def test_sharded_world1_matches_unsharded_model_on_gpu():
             dist.destroy_process_group()
 
 
+@pytest.mark.parametrize("place", ["adjacent", "apart", "off by one element"])
+def test_decoder_layer_with_fused_activation(monkeypatch, place):
+    """A layer at a size where gate, up and their activation are one kernel, wherever the two weights lie (an address that TMA
+    cannot read goes through a copy), with and without gradients, against the same layer on the separate kernels: the same
+    rounding points, fp32 sums of 4096 products in another order at most."""
+    from yafsdp_b200.ops import functional as Fn
+    from yafsdp_b200.ops import kernels
+
+    torch.manual_seed(1)
+    d, f, s = 4096, 11008, 1024
+    dims = Fn.LayerDims(1, s, 32, 32, 128, 1e-5)
+    assert kernels.swiglu_pays(s, f, d, 0)
+
+    def w(*shape):
+        return torch.randn(*shape, device="cuda").mul_(0.02).bfloat16().requires_grad_(True)
+
+    flat = torch.randn(2 * f * d + 64, device="cuda").mul_(0.02).bfloat16()
+    gap = {"adjacent": 0, "apart": 64, "off by one element": 1}[place]
+    wg, wu = (flat[at : at + f * d].view(f, d).requires_grad_(True) for at in (0, f * d + gap))
+    assert wg.is_contiguous() and wu.is_contiguous() and (wu.data_ptr() % 16 == 0) == (gap != 1)
+    n1, n2 = (torch.ones(d, device="cuda").bfloat16().requires_grad_(True) for _ in range(2))
+    ws = [n1, w(d, d), w(d, d), w(d, d), w(d, d), n2, wg, wu, w(d, f)]
+    x = torch.randn(s, d, device="cuda").bfloat16().requires_grad_(True)
+    dout = torch.randn(s, d, device="cuda").bfloat16()
+    cs = Fn.rope_table(s, 128, 10000.0, "cuda")
+    got = Fn.decoder_layer(x, *ws, cs, dims)
+    grads = torch.autograd.grad(got, [x, *ws], dout)
+    with torch.no_grad():
+        assert torch.equal(Fn.decoder_layer(x, *ws, cs, dims), got)
+    monkeypatch.setattr(kernels, "swiglu_pays", lambda *a: False)
+    want = Fn.decoder_layer(x, *ws, cs, dims)
+    wanted = torch.autograd.grad(want, [x, *ws], dout)
+    torch.cuda.synchronize()
+    kernels.check_status()
+    for a, b in zip((got, *grads), (want, *wanted)):
+        assert a.shape == b.shape and ((a.double() - b.double()).norm() / b.double().norm()).item() < 2.0**-8
+
+
 def test_optimizer_overlap_matches_plain_stepping():
     """AdamW on a side stream under the next forward gives the same parameters as stepping in line."""
     import os
@@ -217,41 +255,3 @@ def test_fused_gradient_norm_with_micro_batches_on_gpu():
     finally:
         if created:
             dist.destroy_process_group()
-
-
-@pytest.mark.parametrize("place", ["adjacent", "apart", "off by one element"])
-def test_decoder_layer_with_fused_activation(monkeypatch, place):
-    """A layer at a size where gate, up and their activation are one kernel, wherever the two weights lie (an address that TMA
-    cannot read goes through a copy), with and without gradients, against the same layer on the separate kernels: the same
-    rounding points, fp32 sums of 4096 products in another order at most."""
-    from yafsdp_b200.ops import functional as Fn
-    from yafsdp_b200.ops import kernels
-
-    torch.manual_seed(1)
-    d, f, s = 4096, 11008, 1024
-    dims = Fn.LayerDims(1, s, 32, 32, 128, 1e-5)
-    assert kernels.swiglu_pays(s, f, d, 0)
-
-    def w(*shape):
-        return torch.randn(*shape, device="cuda").mul_(0.02).bfloat16().requires_grad_(True)
-
-    flat = torch.randn(2 * f * d + 64, device="cuda").mul_(0.02).bfloat16()
-    gap = {"adjacent": 0, "apart": 64, "off by one element": 1}[place]
-    wg, wu = (flat[at : at + f * d].view(f, d).requires_grad_(True) for at in (0, f * d + gap))
-    assert wg.is_contiguous() and wu.is_contiguous() and (wu.data_ptr() % 16 == 0) == (gap != 1)
-    n1, n2 = (torch.ones(d, device="cuda").bfloat16().requires_grad_(True) for _ in range(2))
-    ws = [n1, w(d, d), w(d, d), w(d, d), w(d, d), n2, wg, wu, w(d, f)]
-    x = torch.randn(s, d, device="cuda").bfloat16().requires_grad_(True)
-    dout = torch.randn(s, d, device="cuda").bfloat16()
-    cs = Fn.rope_table(s, 128, 10000.0, "cuda")
-    got = Fn.decoder_layer(x, *ws, cs, dims)
-    grads = torch.autograd.grad(got, [x, *ws], dout)
-    with torch.no_grad():
-        assert torch.equal(Fn.decoder_layer(x, *ws, cs, dims), got)
-    monkeypatch.setattr(kernels, "swiglu_pays", lambda *a: False)
-    want = Fn.decoder_layer(x, *ws, cs, dims)
-    wanted = torch.autograd.grad(want, [x, *ws], dout)
-    torch.cuda.synchronize()
-    kernels.check_status()
-    for a, b in zip((got, *grads), (want, *wanted)):
-        assert a.shape == b.shape and ((a.double() - b.double()).norm() / b.double().norm()).item() < 2.0**-8
